@@ -1,0 +1,1065 @@
+// Coarse correction of the gradient-corrected multicolour SSOR.
+//
+// SSOR on the edges and on the gradients removes the error that varies from
+// edge to edge; what is left is smooth, and its reduction takes as many
+// iterations as the mesh is cells wide.  Following Hiptmair and Xu (SIAM J.
+// Numer. Anal. 45, 2007) the smooth part of an edge field is represented by
+// nodal functions: the gradient of a scalar potential and a vector field whose
+// three components are taken one by one,
+//
+//     z += sum_{c=0..3} Q_c B_c Q_c^T r,   Q_0 = G T,  Q_k = Pi_k T,
+//
+// with G the edge-node incidence, (Pi_k v)_e = (x_head - x_tail)_k (v_head +
+// v_tail) / 2 and T the trilinear interpolation from a tensor-product grid
+// about twice as coarse as the mesh (its planes are quantiles of the node
+// coordinates, so a graded mesh gets a graded grid and an unstructured one
+// planes where its nodes are).  B_c is one symmetric V-cycle on the Galerkin
+// matrices Q_c^T A Q_c, kept as pairs (K, M) like the edge matrix, over grids
+// halved per axis; its smoother is l1-Jacobi, D = sum_j |K_ij| + i omega
+// sum_j |M_ij|, which needs no estimate of the largest eigenvalue on stretched
+// cells.  Everything is complex symmetric, so COCG applies as before.
+// Measured to 1e-10 on a B200: 461 -> 59 iterations and 370 -> 70 ms on a 48x48x32-cell mesh (8
+// systems, FP64), about 850 -> 65 and 1,290 -> 151 ms on 88x88x56 (one system), 110 -> 43 and
+// 30 -> 16 ms on 12x12x9, where an iteration is all launches and grid barriers.
+//
+// The four components and the systems are independent below the restriction,
+// so the lower levels of the V-cycle run as one block per (component, system)
+// with its vectors in shared memory and no grid-wide step at all; only levels
+// of more than COARSE_TAIL nodes take launches of their own.
+#include <algorithm>
+#include <cmath>
+
+#include "afem_hybrid.h"
+
+namespace afem {
+
+namespace {
+
+constexpr int MAXS = 32;              // row length of the partial sums (systems)
+constexpr int COARSE_TAIL = 1600;     // nodes of the first level the one-block cycle takes
+constexpr int COARSE_STOP = 60;       // a grid of at most this many nodes is the coarsest
+constexpr int COARSE_SWEEPS = 4;      // smoothing sweeps on the coarsest grid
+constexpr int TAIL_THREADS = 1024;
+constexpr size_t TAIL_VALS = 14000;   // shared complex values of the one-block cycle (224 KB in FP64)
+constexpr int COARSE_MIN_NODES = 64;  // smaller meshes keep the SSOR corrections alone
+
+inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
+
+template <class T>
+struct CV;
+template <>
+struct CV<double> {
+  using V = double2;
+};
+template <>
+struct CV<float> {
+  using V = float2;
+};
+
+__device__ __forceinline__ int pk(int i, int j, int k) { return i | (j << 10) | (k << 20); }
+
+// ------------------------------------------------------------------ pattern (once per mesh)
+__global__ void k_edge_vec(const double* __restrict__ xyz, const int32_t* __restrict__ line, int n,
+                           double* __restrict__ te) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const double* a = xyz + 3L * (line[2L * e] - 1);
+  const double* b = xyz + 3L * (line[2L * e + 1] - 1);
+  for (int d = 0; d < 3; ++d) te[3L * e + d] = b[d] - a[d];
+}
+
+__device__ __forceinline__ int find_plane(const double* __restrict__ p, int n, double x) {
+  int lo = 0, hi = n - 1;  // p[lo] <= x < p[hi] as far as x lies inside
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (p[m] <= x) lo = m;
+    else hi = m;
+  }
+  return lo;
+}
+
+// Cell of each mesh node in its mesh's level-1 grid and its position there; counts the supports.
+// planes: the meshes' x, y and z planes one after another, from pofs[mesh].
+__global__ void k_node_cells(const double* __restrict__ xyz, int node, const uint8_t* __restrict__ seg,
+                             const CoarseGrid* __restrict__ grids, const double* __restrict__ planes,
+                             const int32_t* __restrict__ pofs, int32_t* __restrict__ corner,
+                             double* __restrict__ frac, int32_t* __restrict__ cnt) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= node) return;
+  const int sg = seg ? seg[a] : 0;
+  const CoarseGrid g = grids[(long)sg * COARSE_LEVELS];
+  const int np[3] = {g.nx, g.ny, g.nz};
+  const double* p = planes + pofs[sg];
+  int ijk[3];
+  double f[3];
+  for (int d = 0; d < 3; ++d) {
+    const double x = xyz[3L * a + d];
+    const int i = find_plane(p, np[d], x);
+    double t = (x - p[i]) / (p[i + 1] - p[i]);
+    t = t > 0.0 ? (t < 1.0 ? t : 1.0) : 0.0;
+    ijk[d] = i;
+    f[d] = t;
+    frac[3L * a + d] = t;
+    p += np[d];
+  }
+  corner[a] = pk(ijk[0], ijk[1], ijk[2]);
+  const int base = g.off + ijk[0] + g.nx * (ijk[1] + g.ny * ijk[2]);
+  for (int q = 0; q < 8; ++q) {
+    const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+    if ((dx ? f[0] : 1 - f[0]) * (dy ? f[1] : 1 - f[1]) * (dz ? f[2] : 1 - f[2]) != 0.0)
+      atomicAdd(cnt + base + dx + g.nx * (dy + g.ny * dz), 1);
+  }
+}
+
+__global__ void k_support_fill(int node, const uint8_t* __restrict__ seg, const CoarseGrid* __restrict__ grids,
+                               const int32_t* __restrict__ corner, const double* __restrict__ frac,
+                               const int32_t* __restrict__ lptr, int32_t* __restrict__ cur,
+                               int32_t* __restrict__ lidx) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= node) return;
+  const CoarseGrid g = grids[(long)(seg ? seg[a] : 0) * COARSE_LEVELS];
+  const int c = corner[a];
+  const double fx = frac[3L * a], fy = frac[3L * a + 1], fz = frac[3L * a + 2];
+  const int base = g.off + (c & 1023) + g.nx * (((c >> 10) & 1023) + g.ny * (c >> 20));
+  for (int q = 0; q < 8; ++q) {
+    const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+    if ((dx ? fx : 1 - fx) * (dy ? fy : 1 - fy) * (dz ? fz : 1 - fz) != 0.0) {
+      const int ci = base + dx + g.nx * (dy + g.ny * dz);
+      lidx[lptr[ci] + atomicAdd(cur + ci, 1)] = a;
+    }
+  }
+}
+
+// The atomics above fill a support in any order: sorted ascending, sums over it have one order
+// (insertion sort: ~27 nodes on a box mesh).
+__global__ void k_support_sort(int n1, const int32_t* __restrict__ lptr, int32_t* __restrict__ lidx) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n1) return;
+  const int b = lptr[c], e = lptr[c + 1];
+  for (int i = b + 1; i < e; ++i) {
+    const int v = lidx[i];
+    int j = i;
+    for (; j > b && lidx[j - 1] > v; --j) lidx[j] = lidx[j - 1];
+    lidx[j] = v;
+  }
+}
+
+__global__ void k_cseg(int nseg, const CoarseGrid* __restrict__ grids, int n1, uint8_t* __restrict__ cseg) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n1) return;
+  int s = 0;
+  while (s + 1 < nseg && c >= grids[(long)(s + 1) * COARSE_LEVELS].off) ++s;
+  cseg[c] = (uint8_t)s;
+}
+
+// ------------------------------------------------------------------ values (once per assembly)
+// A node with a Dirichlet edge takes no part in the correction: its interpolation is zero.
+__global__ void k_free_cells(int node, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist,
+                             const uint8_t* __restrict__ bc, const uint8_t* __restrict__ seg,
+                             const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ corner,
+                             int32_t* __restrict__ cell) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= node) return;
+  bool fixed = false;
+  for (int q = nptr[a]; q < nptr[a + 1]; ++q) fixed |= bc[nlist[q] >> 1] != 0;
+  const CoarseGrid g = grids[(long)(seg ? seg[a] : 0) * COARSE_LEVELS];
+  const int c = corner[a];
+  cell[a] = fixed ? -1 : g.off + (c & 1023) + g.nx * (((c >> 10) & 1023) + g.ny * (c >> 20));
+}
+
+// trilinear weight of grid node (i, j, k) at a position in the cell with lowest corner c
+__device__ __forceinline__ double corner_weight(int i, int j, int k, int c, double fx, double fy, double fz) {
+  const int dx = i - (c & 1023), dy = j - ((c >> 10) & 1023), dz = k - (c >> 20);
+  const double wx = dx == 0 ? 1.0 - fx : (dx == 1 ? fx : 0.0);
+  const double wy = dy == 0 ? 1.0 - fy : (dy == 1 ? fy : 0.0);
+  const double wz = dz == 0 ? 1.0 - fz : (dz == 1 ? fz : 0.0);
+  return wx * wy * wz;
+}
+
+__global__ void k_support_weights(int n1, const uint8_t* __restrict__ cseg, const CoarseGrid* __restrict__ grids,
+                                  const int32_t* __restrict__ lptr, const int32_t* __restrict__ lidx,
+                                  const int32_t* __restrict__ corner, const double* __restrict__ frac,
+                                  const int32_t* __restrict__ cell, double* __restrict__ lw) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n1) return;
+  const CoarseGrid g = grids[(long)cseg[c] * COARSE_LEVELS];
+  const int l = c - g.off, i = l % g.nx, j = (l / g.nx) % g.ny, k = l / (g.nx * g.ny);
+  for (int p = lptr[c]; p < lptr[c + 1]; ++p) {
+    const int a = lidx[p];
+    lw[p] = cell[a] < 0 ? 0.0
+                        : corner_weight(i, j, k, corner[a], frac[3L * a], frac[3L * a + 1], frac[3L * a + 2]);
+  }
+}
+
+// Nodal matrices of the vector components on the node graph, Pi_k^T P A P Pi_k: a warp per row,
+// a lane per entry (so an entry stays in registers over the row's edges); n3[3 * entry + k].
+__global__ void __launch_bounds__(256)
+    k_node_values3(const int32_t* __restrict__ line, const uint8_t* __restrict__ bc, int node,
+                   const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist,
+                   const int32_t* __restrict__ erow, const int32_t* __restrict__ ecol,
+                   const double2* __restrict__ ekm, const double* __restrict__ te,
+                   const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, double2* __restrict__ n3) {
+  const int a = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (a >= node) return;
+  const int r0 = rowptr[a], r1 = rowptr[a + 1];
+  for (int q0 = r0; q0 < r1; q0 += 32) {
+    const int q = q0 + lane, b = q < r1 ? col[q] + 1 : 0;  // node ids in line are 1-based
+    double2 acc[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (int i = nptr[a]; i < nptr[a + 1]; ++i) {
+      const int e = nlist[i] >> 1;
+      if (bc[e]) continue;
+      const double ex = 0.25 * te[3L * e], ey = 0.25 * te[3L * e + 1], ez = 0.25 * te[3L * e + 2];
+      for (int k = erow[e]; k < erow[e + 1]; ++k) {
+        const int f = ecol[k];
+        if (bc[f]) continue;
+        if (line[2L * f] == b || line[2L * f + 1] == b) {
+          const double2 v = ekm[k];
+          const double wx = ex * te[3L * f], wy = ey * te[3L * f + 1], wz = ez * te[3L * f + 2];
+          acc[0].x += wx * v.x; acc[0].y += wx * v.y;
+          acc[1].x += wy * v.x; acc[1].y += wy * v.y;
+          acc[2].x += wz * v.x; acc[2].y += wz * v.y;
+        }
+      }
+    }
+    if (q < r1)
+      for (int k = 0; k < 3; ++k) n3[3L * q + k] = acc[k];
+  }
+}
+
+// the row sums of |K| and |M| over the warp's slots; dead rows (zero diagonal) give zero
+__device__ __forceinline__ void store_row(const double2 (&acc)[4], int lane, const CoarseGrid& g, int l,
+                                          double2* __restrict__ km, double2* __restrict__ l1) {
+  for (int c = 0; c < 4; ++c) {
+    if (lane < 27) km[108L * g.off + (long)(c * 27 + lane) * g.n + l] = acc[c];
+    double sk = lane < 27 ? fabs(acc[c].x) : 0.0, sm = lane < 27 ? fabs(acc[c].y) : 0.0;
+    for (int m = 16; m > 0; m >>= 1) {
+      sk += __shfl_xor_sync(0xffffffffu, sk, m);
+      sm += __shfl_xor_sync(0xffffffffu, sm, m);
+    }
+    const double dk = __shfl_sync(0xffffffffu, acc[c].x, 13), dm = __shfl_sync(0xffffffffu, acc[c].y, 13);
+    if (lane == 0) l1[4L * (g.off + l) + c] = (dk == 0.0 && dm == 0.0) ? make_double2(0.0, 0.0) : make_double2(sk, sm);
+  }
+}
+
+// Level 1: T^T N_c T, a warp per grid node, a lane per slot
+__global__ void __launch_bounds__(256)
+    k_galerkin_mesh(int n1, const uint8_t* __restrict__ cseg, const CoarseGrid* __restrict__ grids,
+                    const int32_t* __restrict__ lptr, const int32_t* __restrict__ lidx,
+                    const double* __restrict__ lw, const int32_t* __restrict__ corner,
+                    const double* __restrict__ frac, const int32_t* __restrict__ cell,
+                    const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                    const double2* __restrict__ n0, const double2* __restrict__ n3, double2* __restrict__ km,
+                    double2* __restrict__ l1) {
+  const int c = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (c >= n1) return;
+  const CoarseGrid g = grids[(long)cseg[c] * COARSE_LEVELS];
+  const int l = c - g.off;
+  const int i = l % g.nx + lane % 3 - 1, j = (l / g.nx) % g.ny + (lane / 3) % 3 - 1,
+            k = l / (g.nx * g.ny) + lane / 9 - 1;
+  double2 acc[4] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+  for (int p = lptr[c]; p < lptr[c + 1]; ++p) {
+    const double wa = lw[p];
+    if (wa == 0.0) continue;
+    const int a = lidx[p];
+    for (int q = rowptr[a]; q < rowptr[a + 1]; ++q) {
+      const int b = col[q];
+      if (cell[b] < 0) continue;
+      const double w = wa * corner_weight(i, j, k, corner[b], frac[3L * b], frac[3L * b + 1], frac[3L * b + 2]);
+      if (w == 0.0) continue;
+      const double2 v = n0[q];
+      acc[0].x += w * v.x; acc[0].y += w * v.y;
+      for (int m = 0; m < 3; ++m) {
+        const double2 u = n3[3L * q + m];
+        acc[m + 1].x += w * u.x; acc[m + 1].y += w * u.y;
+      }
+    }
+  }
+  store_row(acc, lane, g, l, km, l1);
+}
+
+// weight of plane I of the next level at plane i of this one
+__device__ __forceinline__ double axis_weight(int i, int I, bool halved, int nc, double w) {
+  const int ci = min(halved ? i >> 1 : i, nc - 2);
+  return I == ci ? 1.0 - w : (I == ci + 1 ? w : 0.0);
+}
+
+// Level l + 1 from level l of each mesh that has both: P^T A P, a warp per node, a lane per slot
+__global__ void __launch_bounds__(256)
+    k_galerkin_grid(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int lev,
+                    const double* __restrict__ axw, double2* __restrict__ km, double2* __restrict__ l1) {
+  const int sg = blockIdx.y;
+  if (lev + 1 >= levels[sg]) return;
+  const CoarseGrid f = grids[(long)sg * COARSE_LEVELS + lev], g = grids[(long)sg * COARSE_LEVELS + lev + 1];
+  const int l = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (l >= g.n) return;
+  const bool hx = f.halved & 1, hy = f.halved & 2, hz = f.halved & 4;
+  const int I = l % g.nx, J = (l / g.nx) % g.ny, K = l / (g.nx * g.ny);
+  const int si = I + lane % 3 - 1, sj = J + (lane / 3) % 3 - 1, sk = K + lane / 9 - 1;
+  const int i0 = hx ? max(0, 2 * I - 1) : I, i1 = hx ? min(f.nx - 1, 2 * I + 1) : I;
+  const int j0 = hy ? max(0, 2 * J - 1) : J, j1 = hy ? min(f.ny - 1, 2 * J + 1) : J;
+  const int k0 = hz ? max(0, 2 * K - 1) : K, k1 = hz ? min(f.nz - 1, 2 * K + 1) : K;
+  double2 acc[4] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+  for (int k = k0; k <= k1; ++k)
+    for (int j = j0; j <= j1; ++j)
+      for (int i = i0; i <= i1; ++i) {
+        const double wa = axis_weight(i, I, hx, g.nx, axw[f.wx + i]) * axis_weight(j, J, hy, g.ny, axw[f.wy + j]) *
+                          axis_weight(k, K, hz, g.nz, axw[f.wz + k]);
+        if (wa == 0.0) continue;
+        const int a = i + f.nx * (j + f.ny * k);
+        for (int s = 0; s < 27; ++s) {
+          const int bi = i + s % 3 - 1, bj = j + (s / 3) % 3 - 1, bk = k + s / 9 - 1;
+          if (bi < 0 || bi >= f.nx || bj < 0 || bj >= f.ny || bk < 0 || bk >= f.nz) continue;
+          const double w = wa * axis_weight(bi, si, hx, g.nx, axw[f.wx + bi]) *
+                           axis_weight(bj, sj, hy, g.ny, axw[f.wy + bj]) *
+                           axis_weight(bk, sk, hz, g.nz, axw[f.wz + bk]);
+          if (w == 0.0) continue;
+          for (int c = 0; c < 4; ++c) {
+            const double2 v = km[108L * f.off + (long)(c * 27 + s) * f.n + a];
+            acc[c].x += w * v.x; acc[c].y += w * v.y;
+          }
+        }
+      }
+  store_row(acc, lane, g, l, km, l1);
+}
+
+__global__ void k_to_float(const double2* __restrict__ in, float2* __restrict__ out, long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    out[i] = make_float2((float)in[i].x, (float)in[i].y);
+}
+
+// ------------------------------------------------------------------ application
+// t_a = sum of g_ea r_e over the non-Dirichlet edges of node a, and the vector components'
+// t3_a = sum of te_e r_e / 2 (the sums run in the COCG type)
+template <class T, class PT, int NS>
+__global__ void __launch_bounds__(256)
+    k_node_restrict(int node, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist,
+                    const uint8_t* __restrict__ bc, const double* __restrict__ te,
+                    const typename CV<T>::V* __restrict__ r, typename CV<PT>::V* __restrict__ t,
+                    typename CV<PT>::V* __restrict__ t3, const int* __restrict__ done) {
+  if (*done) return;
+  const long total = (long)node * NS;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int a = (int)(i / NS), s = (int)(i % NS);
+    T gx = 0, gy = 0, vx[3] = {0, 0, 0}, vy[3] = {0, 0, 0};
+    const int q1 = __ldg(nptr + a + 1);
+    for (int q = __ldg(nptr + a); q < q1; ++q) {
+      const int v = __ldg(nlist + q), e = v >> 1;
+      if (__ldg(bc + e)) continue;
+      const typename CV<T>::V re = r[(long)e * NS + s];
+      if (v & 1) { gx -= re.x; gy -= re.y; }
+      else { gx += re.x; gy += re.y; }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const T h = (T)(0.5 * __ldg(te + 3L * e + d));
+        vx[d] += h * re.x;
+        vy[d] += h * re.y;
+      }
+    }
+    typename CV<PT>::V o;
+    o.x = (PT)gx; o.y = (PT)gy;
+    t[i] = o;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      o.x = (PT)vx[d]; o.y = (PT)vy[d];
+      t3[((long)a * 3 + d) * NS + s] = o;
+    }
+  }
+}
+
+// D^-1 v with D the l1 row sums (0 on a dead row)
+template <class T>
+__device__ __forceinline__ typename CV<T>::V l1_solve(double2 d, double om, typename CV<T>::V v) {
+  typename CV<T>::V o;
+  const double k = d.x, m = om * d.y, s = k * k + m * m;
+  const double inv = s > 0.0 ? 1.0 / s : 0.0;
+  const T ix = (T)(k * inv), iy = (T)(-m * inv);
+  o.x = ix * v.x - iy * v.y;
+  o.y = ix * v.y + iy * v.x;
+  return o;
+}
+
+// R = T^T t at level 1 and Z = D^-1 R
+template <class T, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_grid_restrict(int n1, const uint8_t* __restrict__ cseg, const int32_t* __restrict__ lptr,
+                    const int32_t* __restrict__ lidx, const double* __restrict__ lw,
+                    const typename CV<T>::V* __restrict__ t, const typename CV<T>::V* __restrict__ t3,
+                    const double2* __restrict__ l1, const double* __restrict__ omega,
+                    typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ Z,
+                    const int* __restrict__ done) {
+  if (*done) return;
+  const long total = (long)n1 * 4 * NS;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int s = (int)(i % NS), cc = (int)(i / NS) & 3, c = (int)(i / (4 * NS));
+    typename CV<T>::V acc;
+    acc.x = 0; acc.y = 0;
+    const int p1 = __ldg(lptr + c + 1);
+    for (int p = __ldg(lptr + c); p < p1; ++p) {
+      const int a = __ldg(lidx + p);
+      const T w = (T)__ldg(lw + p);
+      const typename CV<T>::V v = cc == 0 ? t[(long)a * NS + s] : t3[((long)a * 3 + cc - 1) * NS + s];
+      acc.x += w * v.x;
+      acc.y += w * v.y;
+    }
+    if (l1[4L * c + cc].x == 0.0 && l1[4L * c + cc].y == 0.0) { acc.x = 0; acc.y = 0; }
+    R[i] = acc;
+    Z[i] = l1_solve<T>(l1[4L * c + cc], omega[SEG ? (int)cseg[c] : s], acc);
+  }
+}
+
+// (A v)_(node, comp) for one system; v and km of one grid, vs the stride between nodes of v
+template <class T>
+__device__ __forceinline__ typename CV<T>::V grid_row(const CoarseGrid& g, int l, int comp, double om,
+                                                      const typename CV<T>::V* __restrict__ km,
+                                                      const typename CV<T>::V* v, long vs) {
+  const int i = l % g.nx, jk = l / g.nx, j = jk % g.ny, k = jk / g.ny;
+  const typename CV<T>::V* a = km + 108L * g.off + (long)comp * 27 * g.n + l;
+  T t1x = 0, t1y = 0, t2x = 0, t2y = 0;
+#pragma unroll
+  for (int dk = -1; dk <= 1; ++dk) {
+    if (k + dk < 0 || k + dk >= g.nz) continue;
+#pragma unroll
+    for (int dj = -1; dj <= 1; ++dj) {
+      if (j + dj < 0 || j + dj >= g.ny) continue;
+#pragma unroll
+      for (int di = -1; di <= 1; ++di) {
+        if (i + di < 0 || i + di >= g.nx) continue;
+        const typename CV<T>::V m = a[(long)((di + 1) + 3 * (dj + 1) + 9 * (dk + 1)) * g.n];
+        const typename CV<T>::V w = v[(long)(l + di + g.nx * (dj + g.ny * dk)) * vs];
+        t1x += m.x * w.x; t1y += m.x * w.y;
+        t2x += m.y * w.x; t2y += m.y * w.y;
+      }
+    }
+  }
+  typename CV<T>::V o;
+  o.x = t1x - (T)om * t2y;
+  o.y = t1y + (T)om * t2x;
+  return o;
+}
+
+// (P^T v) at node l of the next level g; v on level f
+template <class T>
+__device__ __forceinline__ typename CV<T>::V grid_down(const CoarseGrid& f, const CoarseGrid& g, int l,
+                                                       const double* __restrict__ axw, const typename CV<T>::V* v,
+                                                       long vs) {
+  const bool hx = f.halved & 1, hy = f.halved & 2, hz = f.halved & 4;
+  const int I = l % g.nx, J = (l / g.nx) % g.ny, K = l / (g.nx * g.ny);
+  const int i0 = hx ? max(0, 2 * I - 1) : I, i1 = hx ? min(f.nx - 1, 2 * I + 1) : I;
+  const int j0 = hy ? max(0, 2 * J - 1) : J, j1 = hy ? min(f.ny - 1, 2 * J + 1) : J;
+  const int k0 = hz ? max(0, 2 * K - 1) : K, k1 = hz ? min(f.nz - 1, 2 * K + 1) : K;
+  typename CV<T>::V o;
+  o.x = 0; o.y = 0;
+  for (int k = k0; k <= k1; ++k) {
+    const double wk = axis_weight(k, K, hz, g.nz, __ldg(axw + f.wz + k));
+    for (int j = j0; j <= j1; ++j) {
+      const double wj = wk * axis_weight(j, J, hy, g.ny, __ldg(axw + f.wy + j));
+      for (int i = i0; i <= i1; ++i) {
+        const T w = (T)(wj * axis_weight(i, I, hx, g.nx, __ldg(axw + f.wx + i)));
+        const typename CV<T>::V x = v[(long)(i + f.nx * (j + f.ny * k)) * vs];
+        o.x += w * x.x;
+        o.y += w * x.y;
+      }
+    }
+  }
+  return o;
+}
+
+// (P v) at node l of level f; v on the next level g
+template <class T>
+__device__ __forceinline__ typename CV<T>::V grid_up(const CoarseGrid& f, const CoarseGrid& g, int l,
+                                                     const double* __restrict__ axw, const typename CV<T>::V* v,
+                                                     long vs) {
+  const int i = l % f.nx, j = (l / f.nx) % f.ny, k = l / (f.nx * f.ny);
+  const int I = min((f.halved & 1) ? i >> 1 : i, g.nx - 2), J = min((f.halved & 2) ? j >> 1 : j, g.ny - 2),
+            K = min((f.halved & 4) ? k >> 1 : k, g.nz - 2);
+  const double fx = __ldg(axw + f.wx + i), fy = __ldg(axw + f.wy + j), fz = __ldg(axw + f.wz + k);
+  typename CV<T>::V o;
+  o.x = 0; o.y = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+    const double wd = (dx ? fx : 1.0 - fx) * (dy ? fy : 1.0 - fy) * (dz ? fz : 1.0 - fz);
+    if (wd == 0.0) continue;
+    const T w = (T)wd;
+    const typename CV<T>::V x = v[(long)(I + dx + g.nx * (J + dy + g.ny * (K + dz))) * vs];
+    o.x += w * x.x;
+    o.y += w * x.y;
+  }
+  return o;
+}
+
+// Levels too large for one block: the steps of the V-cycle as launches over (node, component,
+// system), systems fastest.  STEP 0: O = R - A Z (pre-smoothed residual); 1: R, Z of the next
+// level g from O; 2: Z += P O_g; 3: O = Z + D^-1 (R - A Z), with R^T O partial sums when part is set.
+template <class T, int NS, int STEP>
+__global__ void __launch_bounds__(256)
+    k_grid_step(const CoarseGrid f, const CoarseGrid g, const typename CV<T>::V* __restrict__ km,
+                const double2* __restrict__ l1, const double* __restrict__ axw, const double* __restrict__ omega,
+                typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ Z, typename CV<T>::V* __restrict__ O,
+                const int* __restrict__ done, double* __restrict__ part) {
+  if (*done) return;
+  constexpr long VS = 4L * NS;
+  const CoarseGrid& w = STEP == 1 ? g : f;
+  const long total = (long)w.n * VS, fo = f.off * VS, go = g.off * VS;
+  double px = 0.0, py = 0.0;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int s = (int)(i % NS), c = (int)(i / NS) & 3, l = (int)(i / VS);
+    const long in = i % VS;  // component and system
+    if constexpr (STEP == 0) {
+      const typename CV<T>::V a = grid_row<T>(f, l, c, omega[s], km, Z + fo + in, VS);
+      typename CV<T>::V v = R[fo + i];
+      v.x -= a.x; v.y -= a.y;
+      O[fo + i] = v;
+    } else if constexpr (STEP == 1) {
+      const double2 d = l1[4L * (g.off + l) + c];
+      typename CV<T>::V v = grid_down<T>(f, g, l, axw, O + fo + in, VS);
+      if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
+      R[go + i] = v;
+      Z[go + i] = l1_solve<T>(d, omega[s], v);
+    } else if constexpr (STEP == 2) {
+      const double2 d = l1[4L * (f.off + l) + c];
+      if (d.x == 0.0 && d.y == 0.0) continue;
+      const typename CV<T>::V u = grid_up<T>(f, g, l, axw, O + go + in, VS);
+      typename CV<T>::V z = Z[fo + i];
+      z.x += u.x; z.y += u.y;
+      Z[fo + i] = z;
+    } else {
+      const typename CV<T>::V a = grid_row<T>(f, l, c, omega[s], km, Z + fo + in, VS);
+      const typename CV<T>::V r = R[fo + i];
+      typename CV<T>::V z = Z[fo + i], e;
+      e.x = r.x - a.x; e.y = r.y - a.y;
+      e = l1_solve<T>(l1[4L * (f.off + l) + c], omega[s], e);
+      z.x += e.x; z.y += e.y;
+      O[fo + i] = z;
+      px += (double)r.x * (double)z.x - (double)r.y * (double)z.y;
+      py += (double)r.x * (double)z.y + (double)r.y * (double)z.x;
+    }
+  }
+  if constexpr (STEP == 3) {
+    if (!part) return;
+    // the grid's stride is a multiple of 32, so a lane keeps its system
+    __shared__ double red[8][32][2];
+#pragma unroll
+    for (int m = NS; m < 32; m <<= 1) {
+      px += __shfl_xor_sync(0xffffffffu, px, m);
+      py += __shfl_xor_sync(0xffffffffu, py, m);
+    }
+    red[threadIdx.x >> 5][threadIdx.x & 31][0] = px;
+    red[threadIdx.x >> 5][threadIdx.x & 31][1] = py;
+    __syncthreads();
+    if (threadIdx.x < NS) {
+      double x = 0.0, y = 0.0;
+      for (int b = 0; b < 8; ++b) { x += red[b][threadIdx.x][0]; y += red[b][threadIdx.x][1]; }
+      part[((long)blockIdx.x * MAXS + threadIdx.x) * 4] = x;
+      part[((long)blockIdx.x * MAXS + threadIdx.x) * 4 + 1] = y;
+    }
+  }
+}
+
+// The V-cycle from level `top` down, one block per (component, system) -- in a packed batch per
+// (component, mesh) -- with the levels' R and Z and one scratch vector in shared memory.  Reads R
+// of the top level, writes its O; part (top = 0, one matrix): the component's share of rho.
+template <class T, int NS, bool SEG>
+__global__ void __launch_bounds__(TAIL_THREADS)
+    k_grid_tail(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int top,
+                const typename CV<T>::V* __restrict__ km, const double2* __restrict__ l1,
+                const double* __restrict__ axw, const double* __restrict__ omega,
+                const typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ O,
+                const int* __restrict__ done, double* __restrict__ part) {
+  using V = typename CV<T>::V;
+  if (*done) return;
+  extern __shared__ double2 tail_smem[];
+  V* sh = reinterpret_cast<V*>(tail_smem);
+  __shared__ CoarseGrid gs[COARSE_LEVELS];
+  __shared__ int so[COARSE_LEVELS + 1];
+  const int comp = blockIdx.x, sg = SEG ? (int)blockIdx.y : 0, s = SEG ? 0 : (int)blockIdx.y;
+  const double om = omega[blockIdx.y];
+  const int nl = levels[sg];
+  if (threadIdx.x < nl) gs[threadIdx.x] = grids[(long)sg * COARSE_LEVELS + threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {  // R of level l at so[l], Z behind it; the scratch after all levels
+    int o = 0;
+    for (int l = top; l < nl; ++l) { so[l] = o; o += 2 * gs[l].n; }
+    so[nl] = o;
+  }
+  __syncthreads();
+  V* tmp = sh + so[nl];
+  constexpr long VS = 4L * NS;
+  {
+    const CoarseGrid& g = gs[top];
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) sh[so[top] + i] = R[((long)(g.off + i) * 4 + comp) * NS + s];
+  }
+  __syncthreads();
+  for (int l = top; l < nl; ++l) {  // down: z = D^-1 r, then the residual to the next level
+    const CoarseGrid& g = gs[l];
+    V* r = sh + so[l];
+    V* z = r + g.n;
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = l1_solve<T>(l1[4L * (g.off + i) + comp], om, r[i]);
+    __syncthreads();
+    if (l + 1 == nl) {
+      for (int k = 1; k < COARSE_SWEEPS; ++k) {
+        for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+          const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+          V e = r[i];
+          e.x -= a.x; e.y -= a.y;
+          e = l1_solve<T>(l1[4L * (g.off + i) + comp], om, e);
+          e.x += z[i].x; e.y += z[i].y;
+          tmp[i] = e;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = tmp[i];
+        __syncthreads();
+      }
+      break;
+    }
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+      const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+      V e = r[i];
+      e.x -= a.x; e.y -= a.y;
+      tmp[i] = e;
+    }
+    __syncthreads();
+    const CoarseGrid& n = gs[l + 1];
+    for (int i = threadIdx.x; i < n.n; i += TAIL_THREADS) {
+      V v = grid_down<T>(g, n, i, axw, tmp, 1);
+      const double2 d = l1[4L * (n.off + i) + comp];
+      if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
+      sh[so[l + 1] + i] = v;
+    }
+    __syncthreads();
+  }
+  for (int l = nl - 2; l >= top; --l) {  // up: z += P z_next, then one sweep
+    const CoarseGrid& g = gs[l];
+    V* r = sh + so[l];
+    V* z = r + g.n;
+    const V* zc = sh + so[l + 1] + gs[l + 1].n;
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+      const double2 d = l1[4L * (g.off + i) + comp];
+      if (d.x == 0.0 && d.y == 0.0) continue;
+      const V u = grid_up<T>(g, gs[l + 1], i, axw, zc, 1);
+      z[i].x += u.x; z[i].y += u.y;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+      const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+      V e = r[i];
+      e.x -= a.x; e.y -= a.y;
+      e = l1_solve<T>(l1[4L * (g.off + i) + comp], om, e);
+      e.x += z[i].x; e.y += z[i].y;
+      tmp[i] = e;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = tmp[i];
+    __syncthreads();
+  }
+  const CoarseGrid& g = gs[top];
+  const V* r = sh + so[top];
+  const V* z = r + g.n;
+  double px = 0.0, py = 0.0;
+  for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+    O[((long)(g.off + i) * 4 + comp) * NS + s] = z[i];
+    px += (double)r[i].x * (double)z[i].x - (double)r[i].y * (double)z[i].y;
+    py += (double)r[i].x * (double)z[i].y + (double)r[i].y * (double)z[i].x;
+  }
+  if (!part) return;
+  __shared__ double red[TAIL_THREADS / 32][2];
+  for (int m = 16; m > 0; m >>= 1) {
+    px += __shfl_xor_sync(0xffffffffu, px, m);
+    py += __shfl_xor_sync(0xffffffffu, py, m);
+  }
+  if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5][0] = px; red[threadIdx.x >> 5][1] = py; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    px = py = 0.0;
+    for (int b = 0; b < TAIL_THREADS / 32; ++b) { px += red[b][0]; py += red[b][1]; }
+    part[((long)comp * MAXS + s) * 4] = px;
+    part[((long)comp * MAXS + s) * 4 + 1] = py;
+  }
+}
+
+// w = (u + T O_0, T O_1, T O_2, T O_3) at every mesh node, [node][4][system]
+template <class T, int NS>
+__global__ void __launch_bounds__(256)
+    k_node_prolong(int node, const uint8_t* __restrict__ seg, const CoarseGrid* __restrict__ grids,
+                   const int32_t* __restrict__ cell, const double* __restrict__ frac,
+                   const typename CV<T>::V* __restrict__ O, const typename CV<T>::V* __restrict__ u,
+                   typename CV<T>::V* __restrict__ w, const int* __restrict__ done) {
+  using V = typename CV<T>::V;
+  if (*done) return;
+  const long total = (long)node * 4 * NS;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const int s = (int)(i % NS), c = (int)(i / NS) & 3, a = (int)(i / (4 * NS));
+    V o;
+    o.x = 0; o.y = 0;
+    const int b = __ldg(cell + a);
+    if (b >= 0) {
+      const CoarseGrid* g = grids + (long)(seg ? (int)__ldg(seg + a) : 0) * COARSE_LEVELS;
+      const int nx = g->nx, nxy = nx * g->ny;
+      const double fx = __ldg(frac + 3L * a), fy = __ldg(frac + 3L * a + 1), fz = __ldg(frac + 3L * a + 2);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+        const double wd = (dx ? fx : 1.0 - fx) * (dy ? fy : 1.0 - fy) * (dz ? fz : 1.0 - fz);
+        if (wd == 0.0) continue;
+        const T wt = (T)wd;
+        const V x = O[((long)(b + dx + nx * dy + nxy * dz) * 4 + c) * NS + s];
+        o.x += wt * x.x;
+        o.y += wt * x.y;
+      }
+    }
+    if (c == 0) {
+      const V v = u[(long)a * NS + s];
+      o.x += v.x;
+      o.y += v.y;
+    }
+    w[i] = o;
+  }
+}
+
+// ------------------------------------------------------------------ host: grids of one mesh
+// Planes of one axis: about m slabs holding equal shares of the nodes, ends at the extent.  The
+// coordinates are binned (a node layer of a box mesh falls into one bin, whose smallest coordinate
+// stands for it), so a plane passes through the nodes of a layered mesh.
+void axis_planes(const double* xyz, int a0, int a1, int d, int m, std::vector<double>& out) {
+  constexpr int BINS = 8192;
+  double lo = xyz[3L * a0 + d], hi = lo;
+  for (int a = a0; a < a1; ++a) {
+    lo = std::min(lo, xyz[3L * a + d]);
+    hi = std::max(hi, xyz[3L * a + d]);
+  }
+  out.clear();
+  out.push_back(lo);
+  if (m > 1 && hi > lo) {
+    std::vector<int> cnt(BINS, 0);
+    std::vector<double> low(BINS, hi);
+    const double sc = BINS / (hi - lo);
+    for (int a = a0; a < a1; ++a) {
+      const double x = xyz[3L * a + d];
+      const int b = std::min(BINS - 1, std::max(0, (int)((x - lo) * sc)));
+      cnt[b] += 1;
+      low[b] = std::min(low[b], x);
+    }
+    const double share = (double)(a1 - a0) / m;
+    // a slab's upper plane is the first layer at which the nodes below and on it exceed its share
+    long cum = 0;
+    int j = 1;
+    for (int b = 0; b < BINS && j < m; ++b) {
+      if (!cnt[b]) continue;
+      cum += cnt[b];
+      if ((double)cum > j * share + 0.5) {
+        if (low[b] > out.back() && low[b] < hi) out.push_back(low[b]);
+        while (j < m && (double)cum > j * share + 0.5) ++j;
+      }
+    }
+  }
+  out.push_back(hi);
+}
+
+}  // namespace
+
+size_t coarse_bytes(const HybridState* h, int ns, int pb) {
+  const CoarseState* co = h->co;
+  return (size_t)2 * pb * ns * (3 * 4 * (size_t)co->ntot + 7 * (size_t)h->node);
+}
+
+// The grids of every mesh and the mesh nodes' places in them.  Slabs per axis: half the node
+// layers, estimated from the mean edge extent along the axis (over the edges that have one), scaled
+// down together where the product would exceed an eighth of the nodes (unstructured meshes).
+void coarse_pattern(afem_ctx* c) {
+  HybridState* h = c->hyb;
+  if (!h->co) h->co = new CoarseState();
+  CoarseState* co = h->co;
+  cudaStream_t s = c->stream;
+  const int node = c->node, nline = c->nline, nseg = std::max(1, c->nseg);
+  co->on = false;
+  co->values_gen = -1;
+  co->nseg = nseg;
+  std::vector<double> xyz(3L * node);
+  std::vector<int32_t> ln(2L * nline);
+  c->xyz.download(xyz.data(), xyz.size(), s);
+  c->line.download(ln.data(), ln.size(), s);
+  AFEM_CUDA(cudaStreamSynchronize(s));
+  co->grids.assign((size_t)nseg * COARSE_LEVELS, CoarseGrid());
+  co->levels.assign(nseg, 0);
+  std::vector<std::vector<double>> pls[3];
+  std::vector<double> planes;
+  std::vector<int32_t> pofs(nseg);
+  for (int d = 0; d < 3; ++d) pls[d].resize(nseg);
+  int e0 = 0, off = 0;
+  for (int sg = 0; sg < nseg; ++sg) {
+    const int a0 = c->nseg > 0 ? c->seg_node_ptr[sg] : 0, a1 = c->nseg > 0 ? c->seg_node_ptr[sg + 1] : node;
+    const int e1 = c->nseg > 0 ? c->seg_row_ptr[sg + 1] : nline;
+    double ext[3], cells[3], prod = 1.0;
+    for (int d = 0; d < 3; ++d) {
+      double lo = 1e300, hi = -1e300, sum = 0.0;
+      long cnt = 0;
+      for (int a = a0; a < a1; ++a) {
+        lo = std::min(lo, xyz[3L * a + d]);
+        hi = std::max(hi, xyz[3L * a + d]);
+      }
+      ext[d] = hi - lo;
+      if (!(ext[d] > 0.0) || !std::isfinite(ext[d])) return;  // a flat or unreadable mesh: no correction
+      for (int e = e0; e < e1; ++e) {
+        const double t = std::fabs(xyz[3L * (ln[2L * e + 1] - 1) + d] - xyz[3L * (ln[2L * e] - 1) + d]);
+        if (t > 1e-9 * ext[d]) { sum += t; cnt += 1; }
+      }
+      if (!cnt || !std::isfinite(sum)) return;
+      cells[d] = std::max(1.0, 0.5 * ext[d] * cnt / sum);
+      prod *= cells[d];
+    }
+    e0 = e1;
+    if (a1 - a0 < COARSE_MIN_NODES && nseg == 1) return;
+    double scale = prod > (a1 - a0) / 8.0 ? std::cbrt((a1 - a0) / 8.0 / prod) : 1.0;
+    CoarseGrid* G = co->grids.data() + (size_t)sg * COARSE_LEVELS;
+    for (;;) {  // packed batches: the whole cycle of a mesh has to fit one block
+      long n1 = 1;
+      for (int d = 0; d < 3; ++d) {
+        const int m = std::min(256, std::max(1, (int)std::lround(cells[d] * scale)));
+        axis_planes(xyz.data(), a0, a1, d, m, pls[d][sg]);
+        n1 *= (long)pls[d][sg].size();
+      }
+      if (nseg == 1 || n1 * 3.4 < TAIL_VALS || scale < 1e-3) break;
+      scale *= 0.9;
+    }
+    pofs[sg] = (int)planes.size();
+    for (int d = 0; d < 3; ++d) planes.insert(planes.end(), pls[d][sg].begin(), pls[d][sg].end());
+    G[0].nx = (int)pls[0][sg].size();
+    G[0].ny = (int)pls[1][sg].size();
+    G[0].nz = (int)pls[2][sg].size();
+    G[0].n = G[0].nx * G[0].ny * G[0].nz;
+    G[0].off = off;
+    off += G[0].n;
+    co->levels[sg] = 1;
+  }
+  co->n1 = off;
+  co->nlev = 1;
+  std::vector<double> axw;
+  for (int sg = 0; sg < nseg; ++sg) {
+    CoarseGrid* G = co->grids.data() + (size_t)sg * COARSE_LEVELS;
+    int l = 0;
+    for (; l + 1 < COARSE_LEVELS && G[l].n > COARSE_STOP && std::max(G[l].nx, std::max(G[l].ny, G[l].nz)) > 3; ++l) {
+      int* np[3] = {&G[l].nx, &G[l].ny, &G[l].nz};
+      int* nc[3] = {&G[l + 1].nx, &G[l + 1].ny, &G[l + 1].nz};
+      int* wo[3] = {&G[l].wx, &G[l].wy, &G[l].wz};
+      for (int d = 0; d < 3; ++d) {
+        std::vector<double>& p = pls[d][sg];
+        const bool half = p.size() > 3;
+        std::vector<double> q;
+        if (half) {
+          G[l].halved |= 1 << d;
+          for (size_t i = 0; i + 1 < p.size(); i += 2) q.push_back(p[i]);
+          q.push_back(p.back());
+        } else {
+          q = p;
+        }
+        *wo[d] = (int)axw.size();
+        for (size_t i = 0; i < p.size(); ++i) {
+          const size_t ci = std::min(half ? i / 2 : i, q.size() - 2);
+          axw.push_back((p[i] - q[ci]) / (q[ci + 1] - q[ci]));
+        }
+        *nc[d] = (int)q.size();
+        (void)np;
+        p = q;
+      }
+      G[l + 1].n = G[l + 1].nx * G[l + 1].ny * G[l + 1].nz;
+      G[l + 1].off = off;
+      off += G[l + 1].n;
+    }
+    co->levels[sg] = l + 1;
+    co->nlev = std::max(co->nlev, l + 1);
+  }
+  co->ntot = off;
+  co->tail = 0;
+  if (nseg == 1)
+    while (co->grids[co->tail].n > COARSE_TAIL && co->tail + 1 < co->levels[0]) ++co->tail;
+  co->tail_vals = 0;
+  for (int sg = 0; sg < nseg; ++sg) {
+    size_t v = co->grids[(size_t)sg * COARSE_LEVELS + co->tail].n;
+    for (int l = co->tail; l < co->levels[sg]; ++l) v += 2 * (size_t)co->grids[(size_t)sg * COARSE_LEVELS + l].n;
+    co->tail_vals = std::max(co->tail_vals, v);
+  }
+  if (co->tail_vals > TAIL_VALS) return;
+  if (axw.empty()) axw.push_back(0.0);
+  co->d_grids.upload(co->grids.data(), co->grids.size(), s);
+  co->d_levels.upload(co->levels.data(), co->levels.size(), s);
+  co->planes.upload(planes.data(), planes.size(), s);
+  co->axw.upload(axw.data(), axw.size(), s);
+  DBuf<int32_t> dpofs, cnt;
+  dpofs.upload(pofs.data(), pofs.size(), s);
+  co->corner.alloc(node);
+  co->frac.alloc(3L * node);
+  co->cell.alloc(node);
+  co->te.alloc(3L * nline);
+  co->cseg.alloc(co->n1);
+  cnt.alloc(co->n1);
+  cnt.zero(s);
+  const uint8_t* seg = c->nseg > 0 ? h->seg.p : nullptr;
+  k_edge_vec<<<nblk(nline, 256), 256, 0, s>>>(c->xyz.p, c->line.p, nline, co->te.p);
+  count_launch();
+  k_node_cells<<<nblk(node, 256), 256, 0, s>>>(c->xyz.p, node, seg, co->d_grids.p, co->planes.p, dpofs.p,
+                                               co->corner.p, co->frac.p, cnt.p);
+  count_launch();
+  k_cseg<<<nblk(co->n1, 256), 256, 0, s>>>(nseg, co->d_grids.p, co->n1, co->cseg.p);
+  count_launch();
+  long total = 0;
+  co->lptr.alloc(co->n1 + 1);
+  exclusive_scan(cnt.p, co->lptr.p, co->n1, s, &total);
+  co->lidx.alloc(std::max(1L, total));
+  co->lw.alloc(std::max(1L, total));
+  cnt.zero(s);
+  k_support_fill<<<nblk(node, 256), 256, 0, s>>>(node, seg, co->d_grids.p, co->corner.p, co->frac.p, co->lptr.p,
+                                                 cnt.p, co->lidx.p);
+  count_launch();
+  k_support_sort<<<nblk(co->n1, 128), 128, 0, s>>>(co->n1, co->lptr.p, co->lidx.p);
+  count_launch();
+  co->n3.alloc(3 * h->nnz);
+  co->km.alloc(108L * co->ntot);
+  co->l1.alloc(4L * co->ntot);
+  AFEM_CUDA(cudaStreamSynchronize(s));  // the host vectors above go out of scope
+  co->on = true;
+}
+
+void coarse_values(afem_ctx* c) {
+  HybridState* h = c->hyb;
+  CoarseState* co = h->co;
+  if (!co || !co->on || co->values_gen == c->assemble_gen) return;
+  cudaStream_t s = c->stream;
+  const int node = c->node;
+  const uint8_t* seg = c->nseg > 0 ? h->seg.p : nullptr;
+  k_free_cells<<<nblk(node, 256), 256, 0, s>>>(node, h->nptr.p, h->nlist.p, c->bc.p, seg, co->d_grids.p, co->corner.p,
+                                               co->cell.p);
+  count_launch();
+  k_support_weights<<<nblk(co->n1, 128), 128, 0, s>>>(co->n1, co->cseg.p, co->d_grids.p, co->lptr.p, co->lidx.p,
+                                                      co->corner.p, co->frac.p, co->cell.p, co->lw.p);
+  count_launch();
+  k_node_values3<<<nblk(32L * node, 256), 256, 0, s>>>(c->line.p, c->bc.p, node, h->nptr.p, h->nlist.p, c->rowptr.p,
+                                                       c->col.p, c->km.p, co->te.p, h->rowptr.p, h->col.p, co->n3.p);
+  count_launch();
+  k_galerkin_mesh<<<nblk(32L * co->n1, 256), 256, 0, s>>>(co->n1, co->cseg.p, co->d_grids.p, co->lptr.p, co->lidx.p,
+                                                          co->lw.p, co->corner.p, co->frac.p, co->cell.p, h->rowptr.p,
+                                                          h->col.p, h->km.p, co->n3.p, co->km.p, co->l1.p);
+  count_launch();
+  for (int l = 0; l + 1 < co->nlev; ++l) {
+    int nmax = 1;
+    for (int sg = 0; sg < co->nseg; ++sg)
+      if (l + 1 < co->levels[sg]) nmax = std::max(nmax, co->grids[(size_t)sg * COARSE_LEVELS + l + 1].n);
+    k_galerkin_grid<<<dim3(nblk(32L * nmax, 256), co->nseg), 256, 0, s>>>(co->d_grids.p, co->d_levels.p, l, co->axw.p,
+                                                                          co->km.p, co->l1.p);
+    count_launch();
+  }
+  co->kmf_valid = false;
+  co->values_gen = c->assemble_gen;
+}
+
+// FP32 copy of the Galerkin matrices (outside any graph capture)
+void coarse_float(afem_ctx* c) {
+  CoarseState* co = c->hyb->co;
+  if (!co || !co->on || co->kmf_valid) return;
+  co->kmf.alloc(co->km.n);
+  k_to_float<<<c->num_sms * 8, 256, 0, c->stream>>>(co->km.p, co->kmf.p, (long)co->km.n);
+  count_launch();
+  co->kmf_valid = true;
+}
+
+void coarse_destroy(HybridState* h) {
+  delete h->co;
+  h->co = nullptr;
+}
+
+namespace {
+
+template <class PT>
+struct Carve {  // work vectors of a solve: R, Z, O of every grid, the nodal t3 and w
+  using V = typename CV<PT>::V;
+  V *R, *Z, *O, *t3, *w;
+  Carve(const HybridState* h, void* buf, int ns) {
+    const size_t g = (size_t)4 * ns * h->co->ntot, nn = (size_t)ns * h->node;
+    R = static_cast<V*>(buf);
+    Z = R + g;
+    O = Z + g;
+    w = O + g;
+    t3 = w + 4 * nn;
+  }
+};
+
+template <class PT>
+const typename CV<PT>::V* grid_km(const CoarseState* co) {
+  if constexpr (sizeof(PT) == 8) return co->km.p;
+  else return co->kmf.p;
+}
+
+}  // namespace
+
+template <class T, class PT, int NS, bool SEG>
+int coarse_down(afem_ctx* c, const CoarseArgs& a) {
+  using V = typename CV<PT>::V;
+  HybridState* h = c->hyb;
+  CoarseState* co = h->co;
+  cudaStream_t s = c->stream;
+  const Carve<PT> w(h, a.buf, NS);
+  const V* km = grid_km<PT>(co);
+  const int wide = c->num_sms * 8;
+  k_node_restrict<T, PT, NS><<<std::min((unsigned)wide, nblk((long)h->node * NS, 256)), 256, 0, s>>>(
+      h->node, h->nptr.p, h->nlist.p, c->bc.p, co->te.p, static_cast<const typename CV<T>::V*>(a.r),
+      static_cast<V*>(a.t), w.t3, a.done);
+  count_launch();
+  k_grid_restrict<PT, NS, SEG><<<std::min((unsigned)wide, nblk(4L * co->n1 * NS, 256)), 256, 0, s>>>(
+      co->n1, co->cseg.p, co->lptr.p, co->lidx.p, co->lw.p, static_cast<const V*>(a.t), w.t3, co->l1.p, a.omega, w.R,
+      w.Z, a.done);
+  count_launch();
+  auto step = [&](auto tag, int l, int nodes, double* part) {
+    constexpr int ST = decltype(tag)::value;
+    const unsigned g = std::min(nblk(4L * nodes * NS, 256), (unsigned)std::min(wide, a.max_blocks));
+    k_grid_step<PT, NS, ST><<<g, 256, 0, s>>>(co->grids[l], co->grids[l + 1], km, co->l1.p, co->axw.p, a.omega, w.R,
+                                              w.Z, w.O, a.done, part);
+    count_launch();
+    return (int)g;
+  };
+  if constexpr (!SEG)
+    for (int l = 0; l < co->tail; ++l) {
+      step(std::integral_constant<int, 0>(), l, co->grids[l].n, nullptr);
+      step(std::integral_constant<int, 1>(), l, co->grids[l + 1].n, nullptr);
+    }
+  const size_t smem = sizeof(V) * co->tail_vals;
+  auto tail = k_grid_tail<PT, NS, SEG>;
+  AFEM_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int blocks = 4;
+  tail<<<dim3(4, SEG ? co->nseg : NS), TAIL_THREADS, smem, s>>>(co->d_grids.p, co->d_levels.p, co->tail, km, co->l1.p,
+                                                                co->axw.p, a.omega, w.R, w.O, a.done,
+                                                                co->tail == 0 && !SEG ? a.part : nullptr);
+  count_launch();
+  if constexpr (!SEG)
+    for (int l = co->tail - 1; l >= 0; --l) {
+      step(std::integral_constant<int, 2>(), l, co->grids[l].n, nullptr);
+      blocks = step(std::integral_constant<int, 3>(), l, co->grids[l].n, l == 0 ? a.part : nullptr);
+    }
+  return blocks;
+}
+
+template <class PT, int NS, bool SEG>
+const void* coarse_up(afem_ctx* c, const CoarseArgs& a) {
+  using V = typename CV<PT>::V;
+  HybridState* h = c->hyb;
+  const Carve<PT> w(h, a.buf, NS);
+  k_node_prolong<PT, NS><<<std::min((unsigned)(c->num_sms * 8), nblk(4L * h->node * NS, 256)), 256, 0, c->stream>>>(
+      h->node, SEG ? h->seg.p : nullptr, h->co->d_grids.p, h->co->cell.p, h->co->frac.p, w.O,
+      static_cast<const V*>(a.u), w.w, a.done);
+  count_launch();
+  return w.w;
+}
+
+#define AFEM_COARSE(NS, SEG)                                                    \
+  template int coarse_down<double, double, NS, SEG>(afem_ctx*, const CoarseArgs&); \
+  template int coarse_down<double, float, NS, SEG>(afem_ctx*, const CoarseArgs&);  \
+  template int coarse_down<float, float, NS, SEG>(afem_ctx*, const CoarseArgs&);   \
+  template const void* coarse_up<double, NS, SEG>(afem_ctx*, const CoarseArgs&);   \
+  template const void* coarse_up<float, NS, SEG>(afem_ctx*, const CoarseArgs&);
+AFEM_COARSE(1, false)
+AFEM_COARSE(2, false)
+AFEM_COARSE(4, false)
+AFEM_COARSE(8, false)
+AFEM_COARSE(16, false)
+AFEM_COARSE(1, true)
+#undef AFEM_COARSE
+
+}  // namespace afem

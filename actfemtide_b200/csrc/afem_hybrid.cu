@@ -73,7 +73,7 @@ inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
-void hybrid_prepare(afem_ctx* c) {
+void hybrid_prepare(afem_ctx* c, bool coarse) {
   AFEM_REQUIRE(c->node > 0 && c->nline > 0 && c->line.p, AFEM_ESTATE,
                "hybrid preconditioner: needs the mesh (not available for a system loaded in split layout)");
   AFEM_REQUIRE(c->assembled, AFEM_ESTATE, "hybrid preconditioner: assemble first");
@@ -152,6 +152,7 @@ void hybrid_prepare(afem_ctx* c) {
     h->live.alloc(node);
     h->pattern_ready = true;
     h->values_gen = -1;
+    h->coarse_ready = false;
   }
   if (h->values_gen != c->assemble_gen) {
     k_node_values<<<nblk(node, 128), 128, 0, s>>>(c->line.p, c->bc.p, node, h->nptr.p, h->nlist.p, c->rowptr.p,
@@ -176,6 +177,12 @@ void hybrid_prepare(afem_ctx* c) {
     count_launch();
     AFEM_CUDA(cudaStreamSynchronize(s));
     h->seg_nseg = c->nseg;
+    h->coarse_ready = false;
+  }
+  if (coarse) {
+    if (!h->coarse_ready) coarse_pattern(c);
+    h->coarse_ready = true;
+    coarse_values(c);
   }
   AFEM_CUDA(cudaStreamSynchronize(s));
 }
@@ -188,13 +195,14 @@ void hybrid_invalidate(afem_ctx* c) {
 }
 
 void hybrid_destroy(afem_ctx* c) {
+  if (c->hyb) coarse_destroy(c->hyb);
   delete c->hyb;
   c->hyb = nullptr;
 }
 
 // Host only: the nodal matrix of the last preparation, for tests.
 void hybrid_export(afem_ctx* c, int* node, long* nnz, int32_t* rowptr, int32_t* col, double* km) {
-  hybrid_prepare(c);
+  hybrid_prepare(c, false);
   HybridState* h = c->hyb;
   if (node) *node = h->node;
   if (nnz) *nnz = h->nnz;

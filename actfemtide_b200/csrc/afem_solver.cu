@@ -89,6 +89,7 @@ struct SolverWork {
   DBuf<double> rms;                 // per-system rms(r) for the learned preconditioner
   DBuf<double2> ht, hy, hdd;        // gradient-space correction: nodal rhs, solution, 1/diag (FP64 inner)
   DBuf<float2> htf, hyf, hddf;      // the same for the FP32 inner solve
+  DBuf<unsigned char> cbuf;         // coarse correction: work vectors (coarse_bytes)
   int nmc_blocks = 0;               // co-resident grid of the nodal multicolour sweeps
   int rpw64 = 0, rpw32 = 0;         // SpMV rows per warp chosen by tune_spmv (0 = not tuned; 8: 4 systems per lane)
   int spmv_grid[2][5] = {};         // one-wave grid of each SpMV variant (FP64 / FP32), 0 = not known yet
@@ -101,6 +102,7 @@ struct SolverWork {
   DBuf<unsigned> flag_f, flag_b;
   DBuf<double> part;                // partial sums [block][sys][4]
   DBuf<double> part2;               // nodal share of rho (hybrid), same layout
+  DBuf<double> part3;               // coarse correction's share of rho, same layout
   DBuf<SysScal> sc;
   DBuf<Ctrl> ctrl;
   Ctrl* h_ctrl = nullptr;           // pinned mirror
@@ -1090,14 +1092,39 @@ __device__ __forceinline__ void seg_warp_add(double (*red)[MAX_SYS][NVAL], int s
   }
 }
 
-// z_e += u_head(e) - u_tail(e) on the non-Dirichlet edges, then rho = r^T z partial sums (slots 0, 1)
+// The nodal correction of edge e for system s of NS: u_head - u_tail, or with edge vectors te (coarse
+// correction on, u then [node][4][system]) also te . (v_head + v_tail) / 2 of the vector part v.
+template <class T, class PT, int NS>
+__device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restrict__ line,
+                                                        const typename Cx<PT>::V* __restrict__ u,
+                                                        const double* __restrict__ te, long e, int s) {
+  using PV = typename Cx<PT>::V;
+  const long ih = __ldg(line + 2 * e + 1) - 1, it = __ldg(line + 2 * e) - 1;
+  if (!te) {
+    const PV uh = u[ih * NS + s], ut = u[it * NS + s];
+    return Cx<T>::make((T)(uh.x - ut.x), (T)(uh.y - ut.y));
+  }
+  const PV* ph = u + ih * 4 * NS + s;
+  const PV* pt = u + it * 4 * NS + s;
+  T x = (T)(ph[0].x - pt[0].x), y = (T)(ph[0].y - pt[0].y);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const T h = (T)(0.5 * __ldg(te + 3 * e + d));
+    const PV a = ph[(d + 1) * NS], b = pt[(d + 1) * NS];
+    x += h * ((T)a.x + (T)b.x);
+    y += h * ((T)a.y + (T)b.y);
+  }
+  return Cx<T>::make(x, y);
+}
+
+// z_e += the nodal correction on the non-Dirichlet edges, then rho = r^T z partial sums (slots 0, 1)
 // (u, z in the preconditioner type PT, r in the COCG type T)
 template <class T, class PT, int NS, bool SEG>
 __global__ void __launch_bounds__(256)
     k_grad_add(int n, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
                const typename Cx<PT>::V* __restrict__ u, typename Cx<PT>::V* __restrict__ z,
                const typename Cx<T>::V* __restrict__ r, const Ctrl* __restrict__ ctrl, double* __restrict__ part,
-               const uint8_t* __restrict__ seg) {
+               const uint8_t* __restrict__ seg, const double* __restrict__ te) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   static_assert(!SEG || NS == 1, "packed batches hold one system per row");
@@ -1115,9 +1142,8 @@ __global__ void __launch_bounds__(256)
       const int e = (int)(i / NS), s = (int)(i % NS);
       PV zi = z[i];
       if (!__ldg(bc + e)) {
-        const PV uh = u[(long)(__ldg(line + 2 * e + 1) - 1) * NS + s];
-        const PV ut = u[(long)(__ldg(line + 2 * e) - 1) * NS + s];
-        zi = Cx<PT>::make(zi.x + (uh.x - ut.x), zi.y + (uh.y - ut.y));
+        const PV d = nodal_term<PT, PT, NS>(line, u, te, e, s);
+        zi = Cx<PT>::make(zi.x + d.x, zi.y + d.y);
         z[i] = zi;
       }
       const V ri = r[i];
@@ -1195,7 +1221,8 @@ template <class T, class PT, int NS, bool SEG = false>
 __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
                        const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg,
                        double2* __restrict__ x, int nsys, const int32_t* __restrict__ line,
-                       const uint8_t* __restrict__ bc, const typename Cx<PT>::V* __restrict__ u) {
+                       const uint8_t* __restrict__ bc, const typename Cx<PT>::V* __restrict__ u,
+                       const double* __restrict__ te) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   const bool done = ctrl->done;
@@ -1226,10 +1253,8 @@ __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename
     if (u) {
       const int e = (int)(i / NS);
       if (!__ldg(bc + e)) {
-        const int sn = SEG ? 0 : s;
-        const PV uh = u[(long)(__ldg(line + 2 * e + 1) - 1) * NS + sn];
-        const PV ut = u[(long)(__ldg(line + 2 * e) - 1) * NS + sn];
-        zi = Cx<T>::make(zi.x + (T)(uh.x - ut.x), zi.y + (T)(uh.y - ut.y));
+        const V d = nodal_term<T, PT, NS>(line, u, te, e, SEG ? 0 : s);
+        zi = Cx<T>::make(zi.x + d.x, zi.y + d.y);
       }
     }
     if (first) {
@@ -1252,7 +1277,7 @@ template <class T, class PT, int NS>
 __global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
                            const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, double2* __restrict__ x,
                            int nsys, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
-                           const typename Cx<PT>::V* __restrict__ u) {
+                           const typename Cx<PT>::V* __restrict__ u, const double* __restrict__ te) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   constexpr int SP = 2, GPR = NS / SP;  // systems per thread, threads per row
@@ -1302,12 +1327,26 @@ __global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, type
 #pragma unroll
     for (int j = 0; j < SP; ++j) zi[j] = Cx<T>::make((T)zp[j].x, (T)zp[j].y);
     if (u && !__ldg(bc + e)) {
+      const int nc = te ? 4 : 1;  // components of a nodal row (see nodal_term)
+      const PV* ph = u + (long)(__ldg(line + 2 * e + 1) - 1) * nc * NS + s0;
+      const PV* pt = u + (long)(__ldg(line + 2 * e) - 1) * nc * NS + s0;
       PV uh[SP], ut[SP];
-      load_spl<PV, NS, SP, false>(u + (long)(__ldg(line + 2 * e + 1) - 1) * NS + s0, uh);
-      load_spl<PV, NS, SP, false>(u + (long)(__ldg(line + 2 * e) - 1) * NS + s0, ut);
+      load_spl<PV, NS, SP, false>(ph, uh);
+      load_spl<PV, NS, SP, false>(pt, ut);
 #pragma unroll
       for (int j = 0; j < SP; ++j)
         zi[j] = Cx<T>::make(zi[j].x + (T)(uh[j].x - ut[j].x), zi[j].y + (T)(uh[j].y - ut[j].y));
+      if (te) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const T h = (T)(0.5 * __ldg(te + 3L * e + d));
+          load_spl<PV, NS, SP, false>(ph + (d + 1) * NS, uh);
+          load_spl<PV, NS, SP, false>(pt + (d + 1) * NS, ut);
+#pragma unroll
+          for (int j = 0; j < SP; ++j)
+            zi[j] = Cx<T>::make(zi[j].x + h * ((T)uh[j].x + (T)ut[j].x), zi[j].y + h * ((T)uh[j].y + (T)ut[j].y));
+        }
+      }
     }
     if (first) {
       store_spl<V, SP>(p + base, zi);
@@ -1645,9 +1684,10 @@ __global__ void k_scal_r(SysScal* sc, Ctrl* ctrl, const double* part, int nblock
 __device__ __forceinline__ double2 d_cdiv(double2 a, double2 b) { return cdiv(a, b); }
 
 // part2 (nullable): the nodal correction's share r^T G u = t^T u of rho, summed by
-// the backward nodal sweep when the gradient add is folded into the p update
+// the backward nodal sweep when the gradient add is folded into the p update; part3
+// (nullable): the coarse correction's share
 __global__ void k_scal_rho(SysScal* sc, Ctrl* ctrl, const double* part, int nblocks, int ns, int flexible,
-                           const double* part2, int nblocks2) {
+                           const double* part2, int nblocks2, const double* part3, int nblocks3) {
   if (ctrl->done) return;
   const int s = threadIdx.x >> 5;
   if (s >= ns) return;
@@ -1659,6 +1699,13 @@ __global__ void k_scal_rho(SysScal* sc, Ctrl* ctrl, const double* part, int nblo
     sum_partials(part2, nblocks2, s, 0, v2, 2);
     v[0] += v2[0];
     v[1] += v2[1];
+  }
+  if (part3) {
+    double v3[2];
+    __syncwarp();
+    sum_partials(part3, nblocks3, s, 0, v3, 2);
+    v[0] += v3[0];
+    v[1] += v3[1];
   }
   if ((threadIdx.x & 31) == 0) {
     SysScal& S = sc[s];
@@ -2061,7 +2108,8 @@ int tune_spmv(afem_ctx* c, SolverWork* w) {
 // T: COCG vectors and the SpMV; PT: the multicolour preconditioner (its matrix
 // copies and vectors); PT differs from T only on the multicolour path.
 template <class T, class PT, int NS, bool SEG>
-void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, cudaEvent_t* ev) {
+void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, const double* d_omega,
+                       cudaEvent_t* ev) {
   using I = Inner<T, NS>;
   using P = Inner<PT, NS>;
   using V = typename I::V;
@@ -2114,24 +2162,45 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[3], s));
   int rho_blocks = mc ? w->mcb_blocks : sweep_blocks;
+  const bool coarse = mode == AFEM_PRECOND_HYBRID && c->hyb->co && c->hyb->co->on;
+  int coarse_blocks = 0;
+  const void* nodal = nullptr;
+  CoarseArgs ca{};
   if (hyb) {
     // z += G SSOR_node(G^T r): folded into the p update, or (packed batches, learned
     // base) a pass of its own that takes the rho partials again from the corrected z
     HybridState* h = c->hyb;
     const int node = h->node;
     const uint8_t* hs = SEG ? h->seg.p : nullptr;
-    k_grad_t<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(node, h->nptr.p, h->nlist.p, c->bc.p, (const V*)I::R(w),
-                                                        P::HT(w), w->ctrl.p);
-    count_launch();
+    nodal = P::HY(w);
+    if (coarse) {
+      ca.r = I::R(w);
+      ca.t = P::HT(w);
+      ca.u = P::HY(w);
+      ca.buf = w->cbuf.p;
+      ca.omega = d_omega;
+      ca.done = &w->ctrl.p->done;
+      ca.part = fold_grad ? w->part3.p : nullptr;
+      ca.max_blocks = w->nblocks;
+      coarse_blocks = coarse_down<T, PT, NS, SEG>(c, ca);
+    } else {
+      k_grad_t<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(node, h->nptr.p, h->nlist.p, c->bc.p, (const V*)I::R(w),
+                                                          P::HT(w), w->ctrl.p);
+      count_launch();
+    }
+    if (ev) AFEM_CUDA(cudaEventRecord(ev[8], s));
     for (int bwd = 0; bwd < 2; ++bwd)
       launch_coop(k_nsweep_mc<PT, NS, SEG>, w->nmc_blocks, s, (const int32_t*)(bwd ? h->uptr.p : h->lptr.p),
                   (const int32_t*)(bwd ? h->ucol.p : h->lcol.p), bwd ? P::HUKM(c) : P::HLKM(c),
                   (const PV*)P::HT(w), P::HY(w), (const PV*)P::HDD(w), (const int32_t*)h->perm.p,
                   (const int32_t*)h->cptr.p, h->ncolors, (const SysScal*)w->sc.p, (const Ctrl*)w->ctrl.p, hs, bwd,
                   (fold_grad && bwd) ? w->part2.p : (double*)nullptr);
+    if (ev) AFEM_CUDA(cudaEventRecord(ev[9], s));
+    if (coarse) nodal = coarse_up<PT, NS, SEG>(c, ca);
     if (!fold_grad) {
-      k_grad_add<T, PT, NS, SEG><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const PV*)P::HY(w), P::Z(w),
-                                                              (const V*)I::R(w), w->ctrl.p, w->part.p, sg);
+      k_grad_add<T, PT, NS, SEG><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const PV*)nodal, P::Z(w),
+                                                              (const V*)I::R(w), w->ctrl.p, w->part.p, sg,
+                                                              coarse ? c->hyb->co->te.p : (const double*)nullptr);
       count_launch();
       rho_blocks = w->nblocks;
     }
@@ -2147,19 +2216,21 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
     }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[4], s));
   k_scal_rho<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, rho_blocks, nsys, learned ? 1 : 0,
-                                        fold_grad ? w->part2.p : (const double*)nullptr, w->nmc_blocks);
+                                        fold_grad ? w->part2.p : (const double*)nullptr, w->nmc_blocks,
+                                        coarse && fold_grad ? w->part3.p : (const double*)nullptr, coarse_blocks);
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
+  const double* te = coarse && fold_grad ? c->hyb->co->te.p : nullptr;
   if constexpr (NS == 16 && !SEG)
     k_pupd_spl<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr,
-        fold_grad ? c->bc.p : (const uint8_t*)nullptr, fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr);
+        fold_grad ? c->bc.p : (const uint8_t*)nullptr, fold_grad ? (const PV*)nodal : (const PV*)nullptr, te);
   else
     k_pupd<T, PT, NS, SEG><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr, fold_grad ? c->bc.p : (const uint8_t*)nullptr,
-        fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr);
+        fold_grad ? (const PV*)nodal : (const PV*)nullptr, te);
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
   const int spmv_grid = launch_spmv<T, NS, SEG>(c, w, sizeof(T) == 8 ? w->rpw64 : w->rpw32, I::KM(c, w),
@@ -2272,6 +2343,12 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
         h->kmf_valid = true;
       }
     }
+    if (precond == AFEM_PRECOND_HYBRID && h->co && h->co->on) {
+      if (sizeof(PT) == 4) coarse_float(c);
+      const size_t need = coarse_bytes(h, NS, sizeof(PT));
+      if (w->cbuf.n < need) w->cbuf.alloc(need);
+      w->part3.alloc((size_t)w->nblocks * MAX_SYS * 4);
+    }
   }
   w->sd = o->sigma_diag > 0 ? o->sigma_diag : 1.0;
   setup_dd<T, PT, NS, SEG>(c, w, use_hyb ? AFEM_PRECOND_HYBRID : precond, w->sd);
@@ -2304,14 +2381,15 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   AFEM_CUDA(cudaMemcpyAsync(&w->ctrl.p->epoch, &w->epoch_host, sizeof(unsigned), cudaMemcpyHostToDevice, s));
   int iters_done = 0;
   const int chunk = check_every > 0 ? check_every : 32;
-  // profiling: 8 events per iteration of a chunk (fwd | scal | bwd | nodal correction | scal | pupd | spmv)
+  // profiling: 10 events per iteration of a chunk (fwd | scal | bwd | coarse down | nodal sweeps | coarse up |
+  // scal | pupd | spmv)
   const bool prof = c->prof.on;
   std::vector<cudaEvent_t> evs;
   if (prof) {
-    evs.resize(8L * chunk);
+    evs.resize(10L * chunk);
     for (auto& e : evs) AFEM_CUDA(cudaEventCreate(&e));
   }
-  auto ev_of = [&](int k) -> cudaEvent_t* { return prof ? &evs[8L * k] : nullptr; };
+  auto ev_of = [&](int k) -> cudaEvent_t* { return prof ? &evs[10L * k] : nullptr; };
   cudaGraphExec_t gexec = nullptr;
   long graph_kernels = 0;  // kernel nodes of the captured chunk (launch count per graph launch)
   bool use_graph = o->use_graph != 0 && !prof;
@@ -2322,7 +2400,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       bool ok = true;
       g_capturing = 1;
       try {
-        for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, ev_of(k));
+        for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, d_omega, ev_of(k));
       } catch (const Error&) {
         ok = false;
       }
@@ -2374,7 +2452,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       AFEM_CUDA(cudaGraphLaunch(gexec, s));
       count_launch(graph_kernels);
     } else {
-      for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, ev_of(k));
+      for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, d_omega, ev_of(k));
     }
     AFEM_CUDA(cudaMemcpyAsync(w->h_ctrl, w->ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
     AFEM_CUDA(cudaStreamSynchronize(s));
@@ -2383,18 +2461,20 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       // count only iterations that ran to their last kernel
       const int executed = std::min(chunk, w->h_ctrl->iter - iter_before);
       const char* tag = sizeof(T) == 8 ? (sizeof(PT) == 8 ? "fp64" : "fp64pc32") : "fp32";
-      char nf[64], nb[64], nh[64], np_[64], ns_[64];
+      char nf[64], nb[64], nh[64], nc_[64], np_[64], ns_[64];
       const char* kind = SEG ? "seg" : "ns";
       const int cnt = SEG ? nsys : NS;
       const bool mcs = mode == AFEM_PRECOND_SSOR_MC || use_hyb;
       snprintf(nf, sizeof nf, "cocg_fwd_sweep%s_%s_%s%d", mcs ? "_mc" : "", tag, kind, cnt);
       snprintf(nb, sizeof nb, "cocg_bwd_sweep%s_%s_%s%d", mcs ? "_mc" : "", tag, kind, cnt);
       snprintf(nh, sizeof nh, "cocg_nodal_correction_%s_%s%d", tag, kind, cnt);
+      snprintf(nc_, sizeof nc_, "cocg_coarse_correction_%s_%s%d", tag, kind, cnt);
+      const bool crs = mode == AFEM_PRECOND_HYBRID && c->hyb->co && c->hyb->co->on;
       snprintf(np_, sizeof np_, "cocg_p_update_%s_%s%d", tag, kind, cnt);
       snprintf(ns_, sizeof ns_, "cocg_spmv_%s_%s%d_rpw%d", tag, kind, cnt, sizeof(T) == 8 ? w->rpw64 : w->rpw32);
       for (int k = 0; k < executed; ++k) {
         float a = 0, b = 0, h = 0, d = 0, e = 0;
-        cudaEvent_t* E = &evs[8L * k];
+        cudaEvent_t* E = &evs[10L * k];
         if (cudaEventElapsedTime(&a, E[0], E[1]) != cudaSuccess || cudaEventElapsedTime(&b, E[2], E[3]) != cudaSuccess ||
             cudaEventElapsedTime(&h, E[3], E[4]) != cudaSuccess || cudaEventElapsedTime(&d, E[5], E[6]) != cudaSuccess ||
             cudaEventElapsedTime(&e, E[6], E[7]) != cudaSuccess) {
@@ -2403,6 +2483,12 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
         }
         c->prof.add(nf, a);
         c->prof.add(nb, b);
+        float cd = 0, nd = 0, cu = 0;
+        if (crs && cudaEventElapsedTime(&cd, E[3], E[8]) == cudaSuccess &&
+            cudaEventElapsedTime(&nd, E[8], E[9]) == cudaSuccess && cudaEventElapsedTime(&cu, E[9], E[4]) == cudaSuccess) {
+          c->prof.add(nc_, cd + cu);
+          h = nd;
+        }
         if (use_hyb) c->prof.add(nh, h);
         c->prof.add(np_, d);
         c->prof.add(ns_, e);
@@ -2753,7 +2839,7 @@ int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, cons
   }
   if (o->precond == AFEM_PRECOND_HYBRID || (o->precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1)) {
     HostTimer ht(c, "host_setup_hybrid");
-    hybrid_prepare(c);
+    hybrid_prepare(c, true);
   }
   if (c->nseg > 0) {
     AFEM_REQUIRE(nsys == c->nseg, AFEM_EINVAL, "solve: a packed batch solves one system per mesh (nsys = nseg)");
@@ -2777,7 +2863,7 @@ void precond_apply_device(afem_ctx* c, double omega, const double2* r, double2* 
   AFEM_REQUIRE(c->nseg == 0, AFEM_EINVAL, "preconditioner: packed batches are not supported here");
   build_schedule(c, false);
   ensure_mc_values(c);
-  hybrid_prepare(c);
+  hybrid_prepare(c, false);
   SolverWork* w = ensure_work<1, false>(c, 1, false);
   cudaStream_t s = c->stream;
   const int n = c->nline;
@@ -2820,7 +2906,8 @@ void precond_apply_device(afem_ctx* c, double omega, const double2* r, double2* 
                 (const uint8_t*)nullptr, bwd, (double*)nullptr);
   k_grad_add<double, double, 1, false><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const double2*)w->hy.p,
                                                                   w->z.p, (const double2*)w->r.p, w->ctrl.p,
-                                                                  w->part.p, (const uint8_t*)nullptr);
+                                                                  w->part.p, (const uint8_t*)nullptr,
+                                                                  (const double*)nullptr);
   count_launch();
   AFEM_CUDA(cudaMemcpyAsync(z, w->z.p, sizeof(double2) * n, cudaMemcpyDeviceToDevice, s));
   AFEM_CUDA(cudaStreamSynchronize(s));

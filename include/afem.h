@@ -57,7 +57,8 @@ typedef enum afem_precond {
   AFEM_PRECOND_LEARNED = 4,  /* flexible COCG with the learned network; SSOR-COCG restart when it stalls */
   AFEM_PRECOND_SSOR_MC = 5,  /* SSOR of the colour-permuted matrix: every sweep is ~10 parallel passes */
   AFEM_PRECOND_HYBRID = 6    /* multicolour SSOR plus a gradient-space correction G SSOR_node(G^T r)
-                                (Hiptmair's hybrid smoother, additive); needs the mesh */
+                                (Hiptmair's hybrid smoother, additive) and, in afem_solve, a coarse-grid
+                                correction in the nodal scalar and vector spaces; needs the mesh */
 } afem_precond;
 
 typedef enum afem_precision {

@@ -1,0 +1,118 @@
+"""Coarse correction of the gradient-corrected COCG on the GPU (AFEM_PRECOND_HYBRID).
+
+The solution must be the system's own: the oracle's FP64 true residual of the device solution at the
+asked tolerance, and (small meshes) site fields within 1e-6 of a direct solve of the oracle's assembly.
+The meshes are where the grids and the cycle can go wrong: two planes on an axis, odd and even plane
+counts, one flat axis, graded cells, jittered nodes (every node inside a cell), a mesh below the
+correction's minimum, level-1 grids on both sides of the one-block cycle's limit, packed batches.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+import scipy.sparse.linalg as sla
+
+from actfemtide_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fw(gpulib):
+    from actfemtide_b200.forward import Forward
+    f = Forward(0)
+    yield f
+    f.close()
+
+
+def _jitter(m, amp):
+    """The mesh with its interior nodes moved by up to amp of the smallest cell (tags and orientation kept)."""
+    rng = np.random.default_rng(5)
+    lo, hi = m.xyz.min(axis=0), m.xyz.max(axis=0)
+    h = (hi - lo) / m.dims
+    inner = np.all((m.xyz > lo + 0.5 * h) & (m.xyz < hi - 0.5 * h), axis=1)
+    xyz = m.xyz + inner[:, None] * rng.uniform(-amp, amp, m.xyz.shape) * h
+    sites = m.sites + np.array([0.3, 0.2, -0.4])
+    return dataclasses.replace(m, xyz=xyz, sites=sites)
+
+
+CASES = {
+    "2x2x4_below_minimum": lambda: synth.tiny_model(),
+    "3x5x4": lambda: synth.tidal_box(3, 5, 4, seed=1, block=False, site_grid=(-5.0, 5.0), half_km=10.0),
+    "12x2x6_flat": lambda: synth.tidal_box(12, 2, 6, seed=2, grf=True, block=False),
+    "9x10x7": lambda: synth.tidal_box(9, 10, 7, seed=3, grf=True, block=False),
+    "8x8x8_jittered": lambda: _jitter(synth.tidal_box(8, 8, 8, seed=4, grf=True, block=False), 0.2),
+}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "pc32"])
+@pytest.mark.parametrize("name", CASES)
+def test_small_meshes_match_a_direct_solve(fw, oracle, name, precision):
+    m = CASES[name]()
+    of = oracle.OracleForward(m)
+    A = of.assemble(m.freqs[0])
+    x = sla.spsolve(A.to_scipy().tocsc(), A.b)
+    ref = np.asarray(of.sites(x, m.freqs[0])[0]).reshape(5, -1)
+    fw.load_model(m)
+    fw.assemble()
+    for ns in (1, 2, 16):
+        r = fw.solve(np.full(ns, m.freqs[0]), precond="HYBRID", precision=precision, tol=1e-9, maxit=2000)
+        assert r.ok and r.resid_true <= 1e-9, (ns, r)
+        assert oracle.true_residual(A, fw.solution(ns - 1)) <= 1.01e-9
+        out = fw.sites(m.sites)
+        assert np.abs(out - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dims", [(22, 22, 22), (24, 24, 20), (40, 26, 17)])
+def test_grids_around_the_one_block_limit(fw, oracle, dims):
+    """Level-1 grids of 12^3 = 1,728, 13 x 13 x 11 = 1,859 and about 21 x 14 x 9 nodes: launches for the first
+    level, one block below; the iteration count stays that of a mesh a quarter as wide."""
+    m = synth.tidal_box(*dims, seed=6, grf=True, block=False)
+    of = oracle.OracleForward(m)
+    A = of.assemble(m.freqs[0])
+    fw.load_model(m)
+    fw.assemble()
+    for ns, precision in ((1, "fp64"), (4, "pc32"), (8, "fp64")):
+        r = fw.solve(np.full(ns, m.freqs[0]), precond="HYBRID", precision=precision, tol=1e-9, maxit=2000)
+        assert r.ok and r.iterations < 90, (ns, r)
+        assert oracle.true_residual(A, fw.solution(ns - 1)) <= 1.01e-9
+
+
+def test_mixed_precision_uses_the_correction(fw):
+    """FP32 inner solve (conductive everywhere, where FP32 holds): converges with the correction in FP32."""
+    m = synth.tidal_box(10, 9, 8, seed=7, block=False)
+    fw.load_model(m)
+    fw.set_sigma(np.ones(m.ntet))
+    fw.assemble()
+    r = fw.solve([m.freqs[0]] * 2, precond="HYBRID", precision="mixed", tol=1e-8, maxit=5000)
+    assert r.ok and r.resid_true <= 1e-8, r
+
+
+@pytest.mark.parametrize("precision", ["fp64", "pc32"])
+def test_packed_meshes_of_different_depth(fw, oracle, precision):
+    """Packed meshes whose hierarchies have different numbers of levels, one of them a handful of cells."""
+    parts = [synth.tidal_box(nx, ny, nz, seed=20 + k, field_seed=30 + k, grf=True, block=False, name=f"p{k}")
+             for k, (nx, ny, nz) in enumerate([(2, 3, 2), (9, 8, 7), (20, 6, 11), (26, 25, 20)])]
+    pk = synth.pack(parts)
+    fw.load_packed(pk)
+    fw.assemble()
+    r = fw.solve([m.freqs[0] for m in parts], precond="HYBRID", precision=precision, tol=1e-9, maxit=3000)
+    assert r.ok, r
+    for k, m in enumerate(parts):
+        A = oracle.OracleForward(m).assemble(m.freqs[0])
+        assert oracle.true_residual(A, fw.solution(k)) <= 1.01e-9
+
+
+def test_new_conductivities_and_bounds_rebuild_the_matrices(fw, oracle):
+    """The Galerkin matrices follow the assembly: other conductivities, then other Dirichlet bounds."""
+    m = synth.tidal_box(8, 9, 8, seed=9, grf=True, block=False)
+    fw.load_model(m)
+    for sig, dz in ((m.sigma_land, 0.0), (m.sigma_land[::-1].copy(), 0.0), (m.sigma_land, 13.0)):
+        m2 = dataclasses.replace(m, sigma_land=sig, bounds=dict(m.bounds, zmax=m.bounds["zmax"] - dz))
+        fw.set_cond(m2.sigma_air, m2.sigma_ocean, 1, sigma_file=m2.sigma_land)
+        b = m2.bounds
+        fw.set_bounds(b["zmin"], b["zmax"], b["xout"], b["yout"])
+        fw.assemble()
+        A = oracle.OracleForward(m2).assemble(m2.freqs[0])
+        r = fw.solve(m2.freqs[0], precond="HYBRID", tol=1e-9, maxit=2000)
+        assert r.ok and oracle.true_residual(A, fw.solution(0)) <= 1.01e-9, r
