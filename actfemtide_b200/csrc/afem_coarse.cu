@@ -35,7 +35,6 @@ namespace afem {
 
 namespace {
 
-constexpr int MAXS = 32;              // row length of the partial sums (systems)
 constexpr int COARSE_TAIL = 1600;     // nodes of the first level the one-block cycle takes
 constexpr int COARSE_STOP = 60;       // a grid of at most this many nodes is the coarsest
 constexpr int COARSE_SWEEPS = 4;      // smoothing sweeps on the coarsest grid
@@ -328,44 +327,6 @@ __global__ void k_to_float(const double2* __restrict__ in, float2* __restrict__ 
 }
 
 // ------------------------------------------------------------------ application
-// t_a = sum of g_ea r_e over the non-Dirichlet edges of node a, and the vector components'
-// t3_a = sum of te_e r_e / 2 (the sums run in the COCG type)
-template <class T, class PT, int NS>
-__global__ void __launch_bounds__(256)
-    k_node_restrict(int node, const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist,
-                    const uint8_t* __restrict__ bc, const double* __restrict__ te,
-                    const typename CV<T>::V* __restrict__ r, typename CV<PT>::V* __restrict__ t,
-                    typename CV<PT>::V* __restrict__ t3, const int* __restrict__ done) {
-  if (*done) return;
-  const long total = (long)node * NS;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int a = (int)(i / NS), s = (int)(i % NS);
-    T gx = 0, gy = 0, vx[3] = {0, 0, 0}, vy[3] = {0, 0, 0};
-    const int q1 = __ldg(nptr + a + 1);
-    for (int q = __ldg(nptr + a); q < q1; ++q) {
-      const int v = __ldg(nlist + q), e = v >> 1;
-      if (__ldg(bc + e)) continue;
-      const typename CV<T>::V re = r[(long)e * NS + s];
-      if (v & 1) { gx -= re.x; gy -= re.y; }
-      else { gx += re.x; gy += re.y; }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const T h = (T)(0.5 * __ldg(te + 3L * e + d));
-        vx[d] += h * re.x;
-        vy[d] += h * re.y;
-      }
-    }
-    typename CV<PT>::V o;
-    o.x = (PT)gx; o.y = (PT)gy;
-    t[i] = o;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      o.x = (PT)vx[d]; o.y = (PT)vy[d];
-      t3[((long)a * 3 + d) * NS + s] = o;
-    }
-  }
-}
-
 // D^-1 v with D the l1 row sums (0 on a dead row)
 template <class T>
 __device__ __forceinline__ typename CV<T>::V l1_solve(double2 d, double om, typename CV<T>::V v) {
@@ -378,12 +339,30 @@ __device__ __forceinline__ typename CV<T>::V l1_solve(double2 d, double om, type
   return o;
 }
 
+// (T^T t) of level-1 node c, component cc, system s; t [mesh node][4][system]
+template <class T, int NS>
+__device__ __forceinline__ typename CV<T>::V mesh_down(int c, int cc, int s, const int32_t* __restrict__ lptr,
+                                                       const int32_t* __restrict__ lidx,
+                                                       const double* __restrict__ lw,
+                                                       const typename CV<T>::V* __restrict__ t) {
+  typename CV<T>::V acc;
+  acc.x = 0; acc.y = 0;
+  const int p1 = __ldg(lptr + c + 1);
+#pragma unroll 4
+  for (int p = __ldg(lptr + c); p < p1; ++p) {
+    const T w = (T)__ldg(lw + p);
+    const typename CV<T>::V v = t[((long)__ldg(lidx + p) * 4 + cc) * NS + s];
+    acc.x += w * v.x;
+    acc.y += w * v.y;
+  }
+  return acc;
+}
+
 // R = T^T t at level 1 and Z = D^-1 R
-template <class T, int NS, bool SEG>
+template <class T, int NS>
 __global__ void __launch_bounds__(256)
-    k_grid_restrict(int n1, const uint8_t* __restrict__ cseg, const int32_t* __restrict__ lptr,
-                    const int32_t* __restrict__ lidx, const double* __restrict__ lw,
-                    const typename CV<T>::V* __restrict__ t, const typename CV<T>::V* __restrict__ t3,
+    k_grid_restrict(int n1, const int32_t* __restrict__ lptr, const int32_t* __restrict__ lidx,
+                    const double* __restrict__ lw, const typename CV<T>::V* __restrict__ t,
                     const double2* __restrict__ l1, const double* __restrict__ omega,
                     typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ Z,
                     const int* __restrict__ done) {
@@ -391,19 +370,11 @@ __global__ void __launch_bounds__(256)
   const long total = (long)n1 * 4 * NS;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
     const int s = (int)(i % NS), cc = (int)(i / NS) & 3, c = (int)(i / (4 * NS));
-    typename CV<T>::V acc;
-    acc.x = 0; acc.y = 0;
-    const int p1 = __ldg(lptr + c + 1);
-    for (int p = __ldg(lptr + c); p < p1; ++p) {
-      const int a = __ldg(lidx + p);
-      const T w = (T)__ldg(lw + p);
-      const typename CV<T>::V v = cc == 0 ? t[(long)a * NS + s] : t3[((long)a * 3 + cc - 1) * NS + s];
-      acc.x += w * v.x;
-      acc.y += w * v.y;
-    }
-    if (l1[4L * c + cc].x == 0.0 && l1[4L * c + cc].y == 0.0) { acc.x = 0; acc.y = 0; }
-    R[i] = acc;
-    Z[i] = l1_solve<T>(l1[4L * c + cc], omega[SEG ? (int)cseg[c] : s], acc);
+    const double2 d = l1[4L * c + cc];
+    typename CV<T>::V v = mesh_down<T, NS>(c, cc, s, lptr, lidx, lw, t);
+    if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
+    R[i] = v;
+    Z[i] = l1_solve<T>(d, omega[s], v);
   }
 }
 
@@ -490,13 +461,13 @@ __device__ __forceinline__ typename CV<T>::V grid_up(const CoarseGrid& f, const 
 
 // Levels too large for one block: the steps of the V-cycle as launches over (node, component,
 // system), systems fastest.  STEP 0: O = R - A Z (pre-smoothed residual); 1: R, Z of the next
-// level g from O; 2: Z += P O_g; 3: O = Z + D^-1 (R - A Z), with R^T O partial sums when part is set.
+// level g from O; 2: Z += P O_g; 3: O = Z + D^-1 (R - A Z), and with rho set the share R^T O of rho.
 template <class T, int NS, int STEP>
 __global__ void __launch_bounds__(256)
     k_grid_step(const CoarseGrid f, const CoarseGrid g, const typename CV<T>::V* __restrict__ km,
                 const double2* __restrict__ l1, const double* __restrict__ axw, const double* __restrict__ omega,
                 typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ Z, typename CV<T>::V* __restrict__ O,
-                const int* __restrict__ done, double* __restrict__ part) {
+                const int* __restrict__ done, double2* __restrict__ rho, RedSet red) {
   if (*done) return;
   constexpr long VS = 4L * NS;
   const CoarseGrid& w = STEP == 1 ? g : f;
@@ -536,36 +507,30 @@ __global__ void __launch_bounds__(256)
     }
   }
   if constexpr (STEP == 3) {
-    if (!part) return;
+    if (!rho) return;
     // the grid's stride is a multiple of 32, so a lane keeps its system
-    __shared__ double red[8][32][2];
-#pragma unroll
-    for (int m = NS; m < 32; m <<= 1) {
-      px += __shfl_xor_sync(0xffffffffu, px, m);
-      py += __shfl_xor_sync(0xffffffffu, py, m);
-    }
-    red[threadIdx.x >> 5][threadIdx.x & 31][0] = px;
-    red[threadIdx.x >> 5][threadIdx.x & 31][1] = py;
-    __syncthreads();
-    if (threadIdx.x < NS) {
-      double x = 0.0, y = 0.0;
-      for (int b = 0; b < 8; ++b) { x += red[b][threadIdx.x][0]; y += red[b][threadIdx.x][1]; }
-      part[((long)blockIdx.x * MAXS + threadIdx.x) * 4] = x;
-      part[((long)blockIdx.x * MAXS + threadIdx.x) * 4 + 1] = y;
+    __shared__ double2 sums[RED_SYS];
+    double v[1][2] = {{px, py}};
+    block_pair<NS, 1, NS>(v, threadIdx.x % NS, true, red, blockIdx.x);
+    if (reduce_blocks(red, blockIdx.x, gridDim.x, NS, sums) && threadIdx.x < NS) {
+      rho[threadIdx.x] = sums[threadIdx.x];
+      for (int c = 1; c < 4; ++c) rho[c * RED_SYS + threadIdx.x] = make_double2(0.0, 0.0);
     }
   }
 }
 
 // The V-cycle from level `top` down, one block per (component, system) -- in a packed batch per
-// (component, mesh) -- with the levels' R and Z and one scratch vector in shared memory.  Reads R
-// of the top level, writes its O; part (top = 0, one matrix): the component's share of rho.
+// (component, mesh) -- with the levels' R and Z and one scratch vector in shared memory.  Starts from
+// R of the top level, or (top = 0) from the mesh nodes' t, and writes the top level's O; rho
+// (top = 0): the component's share of rho of its system.
 template <class T, int NS, bool SEG>
 __global__ void __launch_bounds__(TAIL_THREADS)
     k_grid_tail(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int top,
                 const typename CV<T>::V* __restrict__ km, const double2* __restrict__ l1,
                 const double* __restrict__ axw, const double* __restrict__ omega,
                 const typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ O,
-                const int* __restrict__ done, double* __restrict__ part) {
+                const int32_t* __restrict__ lptr, const int32_t* __restrict__ lidx, const double* __restrict__ lw,
+                const typename CV<T>::V* __restrict__ t, const int* __restrict__ done, double2* __restrict__ rho) {
   using V = typename CV<T>::V;
   if (*done) return;
   extern __shared__ double2 tail_smem[];
@@ -587,7 +552,17 @@ __global__ void __launch_bounds__(TAIL_THREADS)
   constexpr long VS = 4L * NS;
   {
     const CoarseGrid& g = gs[top];
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) sh[so[top] + i] = R[((long)(g.off + i) * 4 + comp) * NS + s];
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+      V v;
+      if (top) {
+        v = R[((long)(g.off + i) * 4 + comp) * NS + s];
+      } else {
+        const double2 d = l1[4L * (g.off + i) + comp];
+        v = mesh_down<T, NS>(g.off + i, comp, s, lptr, lidx, lw, t);
+        if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
+      }
+      sh[so[top] + i] = v;
+    }
   }
   __syncthreads();
   for (int l = top; l < nl; ++l) {  // down: z = D^-1 r, then the residual to the next level
@@ -661,7 +636,7 @@ __global__ void __launch_bounds__(TAIL_THREADS)
     px += (double)r[i].x * (double)z[i].x - (double)r[i].y * (double)z[i].y;
     py += (double)r[i].x * (double)z[i].y + (double)r[i].y * (double)z[i].x;
   }
-  if (!part) return;
+  if (!rho) return;
   __shared__ double red[TAIL_THREADS / 32][2];
   for (int m = 16; m > 0; m >>= 1) {
     px += __shfl_xor_sync(0xffffffffu, px, m);
@@ -672,47 +647,7 @@ __global__ void __launch_bounds__(TAIL_THREADS)
   if (threadIdx.x == 0) {
     px = py = 0.0;
     for (int b = 0; b < TAIL_THREADS / 32; ++b) { px += red[b][0]; py += red[b][1]; }
-    part[((long)comp * MAXS + s) * 4] = px;
-    part[((long)comp * MAXS + s) * 4 + 1] = py;
-  }
-}
-
-// w = (u + T O_0, T O_1, T O_2, T O_3) at every mesh node, [node][4][system]
-template <class T, int NS>
-__global__ void __launch_bounds__(256)
-    k_node_prolong(int node, const uint8_t* __restrict__ seg, const CoarseGrid* __restrict__ grids,
-                   const int32_t* __restrict__ cell, const double* __restrict__ frac,
-                   const typename CV<T>::V* __restrict__ O, const typename CV<T>::V* __restrict__ u,
-                   typename CV<T>::V* __restrict__ w, const int* __restrict__ done) {
-  using V = typename CV<T>::V;
-  if (*done) return;
-  const long total = (long)node * 4 * NS;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int s = (int)(i % NS), c = (int)(i / NS) & 3, a = (int)(i / (4 * NS));
-    V o;
-    o.x = 0; o.y = 0;
-    const int b = __ldg(cell + a);
-    if (b >= 0) {
-      const CoarseGrid* g = grids + (long)(seg ? (int)__ldg(seg + a) : 0) * COARSE_LEVELS;
-      const int nx = g->nx, nxy = nx * g->ny;
-      const double fx = __ldg(frac + 3L * a), fy = __ldg(frac + 3L * a + 1), fz = __ldg(frac + 3L * a + 2);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
-        const double wd = (dx ? fx : 1.0 - fx) * (dy ? fy : 1.0 - fy) * (dz ? fz : 1.0 - fz);
-        if (wd == 0.0) continue;
-        const T wt = (T)wd;
-        const V x = O[((long)(b + dx + nx * dy + nxy * dz) * 4 + c) * NS + s];
-        o.x += wt * x.x;
-        o.y += wt * x.y;
-      }
-    }
-    if (c == 0) {
-      const V v = u[(long)a * NS + s];
-      o.x += v.x;
-      o.y += v.y;
-    }
-    w[i] = o;
+    rho[comp * RED_SYS + blockIdx.y] = make_double2(px, py);
   }
 }
 
@@ -759,7 +694,7 @@ void axis_planes(const double* xyz, int a0, int a1, int d, int m, std::vector<do
 
 size_t coarse_bytes(const HybridState* h, int ns, int pb) {
   const CoarseState* co = h->co;
-  return (size_t)2 * pb * ns * (3 * 4 * (size_t)co->ntot + 7 * (size_t)h->node);
+  return (size_t)2 * pb * ns * 3 * 4 * (size_t)co->ntot;
 }
 
 // The grids of every mesh and the mesh nodes' places in them.  Slabs per axis: half the node
@@ -966,54 +901,31 @@ void coarse_destroy(HybridState* h) {
   h->co = nullptr;
 }
 
-namespace {
-
-template <class PT>
-struct Carve {  // work vectors of a solve: R, Z, O of every grid, the nodal t3 and w
+template <class PT, int NS, bool SEG>
+const void* coarse_cycle(afem_ctx* c, const CoarseArgs& a) {
   using V = typename CV<PT>::V;
-  V *R, *Z, *O, *t3, *w;
-  Carve(const HybridState* h, void* buf, int ns) {
-    const size_t g = (size_t)4 * ns * h->co->ntot, nn = (size_t)ns * h->node;
-    R = static_cast<V*>(buf);
-    Z = R + g;
-    O = Z + g;
-    w = O + g;
-    t3 = w + 4 * nn;
-  }
-};
-
-template <class PT>
-const typename CV<PT>::V* grid_km(const CoarseState* co) {
-  if constexpr (sizeof(PT) == 8) return co->km.p;
-  else return co->kmf.p;
-}
-
-}  // namespace
-
-template <class T, class PT, int NS, bool SEG>
-int coarse_down(afem_ctx* c, const CoarseArgs& a) {
-  using V = typename CV<PT>::V;
-  HybridState* h = c->hyb;
-  CoarseState* co = h->co;
+  CoarseState* co = c->hyb->co;
   cudaStream_t s = c->stream;
-  const Carve<PT> w(h, a.buf, NS);
-  const V* km = grid_km<PT>(co);
-  const int wide = c->num_sms * 8;
-  k_node_restrict<T, PT, NS><<<std::min((unsigned)wide, nblk((long)h->node * NS, 256)), 256, 0, s>>>(
-      h->node, h->nptr.p, h->nlist.p, c->bc.p, co->te.p, static_cast<const typename CV<T>::V*>(a.r),
-      static_cast<V*>(a.t), w.t3, a.done);
-  count_launch();
-  k_grid_restrict<PT, NS, SEG><<<std::min((unsigned)wide, nblk(4L * co->n1 * NS, 256)), 256, 0, s>>>(
-      co->n1, co->cseg.p, co->lptr.p, co->lidx.p, co->lw.p, static_cast<const V*>(a.t), w.t3, co->l1.p, a.omega, w.R,
-      w.Z, a.done);
-  count_launch();
-  auto step = [&](auto tag, int l, int nodes, double* part) {
-    constexpr int ST = decltype(tag)::value;
-    const unsigned g = std::min(nblk(4L * nodes * NS, 256), (unsigned)std::min(wide, a.max_blocks));
-    k_grid_step<PT, NS, ST><<<g, 256, 0, s>>>(co->grids[l], co->grids[l + 1], km, co->l1.p, co->axw.p, a.omega, w.R,
-                                              w.Z, w.O, a.done, part);
+  const size_t vec = (size_t)4 * NS * co->ntot;
+  V* R = static_cast<V*>(a.buf);
+  V* Z = R + vec;
+  V* O = Z + vec;
+  const V* t = static_cast<const V*>(a.t);
+  const V* km;
+  if constexpr (sizeof(PT) == 8) km = co->km.p;
+  else km = co->kmf.p;
+  const unsigned wide = c->num_sms * 8;
+  if (co->tail > 0) {
+    k_grid_restrict<PT, NS><<<std::min(wide, nblk(4L * co->n1 * NS, 256)), 256, 0, s>>>(
+        co->n1, co->lptr.p, co->lidx.p, co->lw.p, t, co->l1.p, a.omega, R, Z, a.done);
     count_launch();
-    return (int)g;
+  }
+  auto step = [&](auto tag, int l, int nodes, double2* rho) {
+    constexpr int ST = decltype(tag)::value;
+    const unsigned g = std::min(nblk(4L * nodes * NS, 256), std::min(wide, (unsigned)a.red.rows));
+    k_grid_step<PT, NS, ST><<<g, 256, 0, s>>>(co->grids[l], co->grids[l + 1], km, co->l1.p, co->axw.p, a.omega, R, Z,
+                                              O, a.done, rho, a.red);
+    count_launch();
   };
   if constexpr (!SEG)
     for (int l = 0; l < co->tail; ++l) {
@@ -1023,37 +935,21 @@ int coarse_down(afem_ctx* c, const CoarseArgs& a) {
   const size_t smem = sizeof(V) * co->tail_vals;
   auto tail = k_grid_tail<PT, NS, SEG>;
   AFEM_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int blocks = 4;
-  tail<<<dim3(4, SEG ? co->nseg : NS), TAIL_THREADS, smem, s>>>(co->d_grids.p, co->d_levels.p, co->tail, km, co->l1.p,
-                                                                co->axw.p, a.omega, w.R, w.O, a.done,
-                                                                co->tail == 0 && !SEG ? a.part : nullptr);
+  tail<<<dim3(4, SEG ? co->nseg : NS), TAIL_THREADS, smem, s>>>(
+      co->d_grids.p, co->d_levels.p, co->tail, km, co->l1.p, co->axw.p, a.omega, R, O, co->lptr.p, co->lidx.p,
+      co->lw.p, t, a.done, co->tail == 0 ? a.rho : nullptr);
   count_launch();
   if constexpr (!SEG)
     for (int l = co->tail - 1; l >= 0; --l) {
       step(std::integral_constant<int, 2>(), l, co->grids[l].n, nullptr);
-      blocks = step(std::integral_constant<int, 3>(), l, co->grids[l].n, l == 0 ? a.part : nullptr);
+      step(std::integral_constant<int, 3>(), l, co->grids[l].n, l == 0 ? a.rho : nullptr);
     }
-  return blocks;
+  return O;
 }
 
-template <class PT, int NS, bool SEG>
-const void* coarse_up(afem_ctx* c, const CoarseArgs& a) {
-  using V = typename CV<PT>::V;
-  HybridState* h = c->hyb;
-  const Carve<PT> w(h, a.buf, NS);
-  k_node_prolong<PT, NS><<<std::min((unsigned)(c->num_sms * 8), nblk(4L * h->node * NS, 256)), 256, 0, c->stream>>>(
-      h->node, SEG ? h->seg.p : nullptr, h->co->d_grids.p, h->co->cell.p, h->co->frac.p, w.O,
-      static_cast<const V*>(a.u), w.w, a.done);
-  count_launch();
-  return w.w;
-}
-
-#define AFEM_COARSE(NS, SEG)                                                    \
-  template int coarse_down<double, double, NS, SEG>(afem_ctx*, const CoarseArgs&); \
-  template int coarse_down<double, float, NS, SEG>(afem_ctx*, const CoarseArgs&);  \
-  template int coarse_down<float, float, NS, SEG>(afem_ctx*, const CoarseArgs&);   \
-  template const void* coarse_up<double, NS, SEG>(afem_ctx*, const CoarseArgs&);   \
-  template const void* coarse_up<float, NS, SEG>(afem_ctx*, const CoarseArgs&);
+#define AFEM_COARSE(NS, SEG)                                                                 \
+  template const void* coarse_cycle<double, NS, SEG>(afem_ctx*, const CoarseArgs&);          \
+  template const void* coarse_cycle<float, NS, SEG>(afem_ctx*, const CoarseArgs&);
 AFEM_COARSE(1, false)
 AFEM_COARSE(2, false)
 AFEM_COARSE(4, false)

@@ -73,7 +73,7 @@ inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
 
-void hybrid_prepare(afem_ctx* c, bool coarse) {
+void hybrid_prepare(afem_ctx* c, bool coarse, bool colours) {
   AFEM_REQUIRE(c->node > 0 && c->nline > 0 && c->line.p, AFEM_ESTATE,
                "hybrid preconditioner: needs the mesh (not available for a system loaded in split layout)");
   AFEM_REQUIRE(c->assembled, AFEM_ESTATE, "hybrid preconditioner: assemble first");
@@ -134,6 +134,25 @@ void hybrid_prepare(afem_ctx* c, bool coarse) {
     h->rowptr.upload(rp.data(), rp.size(), s);
     h->col.upload(cl.data(), cl.size(), s);
     h->diagpos.upload(dp.data(), dp.size(), s);
+    h->km.alloc(nnz);
+    h->live.alloc(node);
+    h->pattern_ready = true;
+    h->values_gen = -1;
+    h->coarse_ready = h->colours_ready = false;
+    AFEM_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
+  }
+  if (h->values_gen != c->assemble_gen) {
+    k_node_values<<<nblk(node, 128), 128, 0, s>>>(c->line.p, c->bc.p, node, h->nptr.p, h->nlist.p, c->rowptr.p,
+                                                   c->col.p, c->km.p, h->rowptr.p, h->col.p, h->km.p, h->live.p);
+    count_launch();
+    h->values_gen = c->assemble_gen;
+    h->kmf_valid = false;
+  }
+  if (colours && !h->colours_ready) {
+    std::vector<int32_t> rp(node + 1), cl(h->nnz);
+    h->rowptr.download(rp.data(), rp.size(), s);
+    h->col.download(cl.data(), cl.size(), s);
+    AFEM_CUDA(cudaStreamSynchronize(s));
     std::vector<int32_t> pm(node), cptr(256);
     std::vector<uint8_t> color(node);
     // multicolour order of the node graph (host greedy colouring, as for the edges)
@@ -148,16 +167,11 @@ void hybrid_prepare(afem_ctx* c, bool coarse) {
                       h->uptr, h->ucol, h->usrc, nullptr);
     h->lkm.alloc(h->lcol.n);
     h->ukm.alloc(h->ucol.n);
-    h->km.alloc(nnz);
-    h->live.alloc(node);
-    h->pattern_ready = true;
-    h->values_gen = -1;
-    h->coarse_ready = false;
+    AFEM_CUDA(cudaStreamSynchronize(s));
+    h->colours_ready = true;
+    h->split_gen = -1;
   }
-  if (h->values_gen != c->assemble_gen) {
-    k_node_values<<<nblk(node, 128), 128, 0, s>>>(c->line.p, c->bc.p, node, h->nptr.p, h->nlist.p, c->rowptr.p,
-                                                   c->col.p, c->km.p, h->rowptr.p, h->col.p, h->km.p, h->live.p);
-    count_launch();
+  if (colours && h->split_gen != c->assemble_gen) {
     if (h->lcol.n) {
       k_gather_km<<<nblk((long)h->lcol.n, 256), 256, 0, s>>>(h->km.p, h->lsrc.p, (long)h->lcol.n, h->lkm.p);
       count_launch();
@@ -166,7 +180,7 @@ void hybrid_prepare(afem_ctx* c, bool coarse) {
       k_gather_km<<<nblk((long)h->ucol.n, 256), 256, 0, s>>>(h->km.p, h->usrc.p, (long)h->ucol.n, h->ukm.p);
       count_launch();
     }
-    h->values_gen = c->assemble_gen;
+    h->split_gen = c->assemble_gen;
     h->kmf_valid = false;
   }
   if (c->nseg > 0 && (int)h->seg_nseg != c->nseg) {
@@ -202,7 +216,7 @@ void hybrid_destroy(afem_ctx* c) {
 
 // Host only: the nodal matrix of the last preparation, for tests.
 void hybrid_export(afem_ctx* c, int* node, long* nnz, int32_t* rowptr, int32_t* col, double* km) {
-  hybrid_prepare(c, false);
+  hybrid_prepare(c, false, false);
   HybridState* h = c->hyb;
   if (node) *node = h->node;
   if (nnz) *nnz = h->nnz;

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "afem_internal.h"
+#include "afem_reduce.cuh"
 
 namespace afem {
 
@@ -11,6 +12,8 @@ struct HybridState {
   int node = 0, nline = 0;
   long nnz = 0;
   bool pattern_ready = false;
+  bool colours_ready = false;   // the multicolour order and its split rows
+  long split_gen = -1;          // assembly generation of lkm / ukm
   bool coarse_ready = false;    // co was set up for this mesh (it may have found no hierarchy)
   long values_gen = -1;         // assembly generation the values belong to
   DBuf<int32_t> nptr, nlist;    // node -> incident edges (edge << 1 | tail flag), ascending
@@ -73,8 +76,9 @@ struct CoarseState {
   DBuf<double2> l1;             // (sum |K|, sum |M|) of each row, [(off + node) * 4 + comp]; 0: dead row
 };
 
-// pattern + colouring (once per mesh), values (once per assembly); coarse: also the coarse correction
-void hybrid_prepare(afem_ctx* c, bool coarse);
+// node graph (once per mesh) and A_G (once per assembly); coarse: also the coarse correction;
+// colours: also the colouring and the colour-ordered rows of the nodal sweeps
+void hybrid_prepare(afem_ctx* c, bool coarse, bool colours);
 void hybrid_invalidate(afem_ctx* c);  // the mesh changed
 void hybrid_destroy(afem_ctx* c);
 void hybrid_export(afem_ctx* c, int* node, long* nnz, int32_t* rowptr, int32_t* col, double* km);
@@ -88,20 +92,15 @@ void coarse_destroy(HybridState* h);
 // Bytes of the work vectors of one solve (pb: bytes of a preconditioner real, ns systems per row)
 size_t coarse_bytes(const HybridState* h, int ns, int pb);
 struct CoarseArgs {
-  const void* r;        // COCG residual [row][system]
-  void* t;              // G^T r [node][system] (written)
-  const void* u;        // nodal SSOR solution [node][system]
+  const void* t;        // mesh nodes' right-hand sides (G^T r, Pi_k^T r) [node][4][system]
   void* buf;            // coarse_bytes
   const double* omega;  // per system
   const int* done;      // the batch has finished: every kernel returns
-  double* part;         // partial sums of the correction's share of rho, [block][MAX_SYS][4]
-  int max_blocks;       // rows of part
+  double2* rho;         // the correction's share of rho, 4 rows of RED_SYS values (to be added up)
+  RedSet red;           // block sums
 };
-// t = G^T r, the vector components' restriction and the V-cycle; returns the blocks that wrote part
-template <class T, class PT, int NS, bool SEG>
-int coarse_down(afem_ctx* c, const CoarseArgs& a);
-// w = the nodal correction [node][4][system]: u plus the coarse potential, and the three vector components
+// The V-cycle of every component and system; returns the level-1 values [grid node][4][system].
 template <class PT, int NS, bool SEG>
-const void* coarse_up(afem_ctx* c, const CoarseArgs& a);
+const void* coarse_cycle(afem_ctx* c, const CoarseArgs& a);
 
 }  // namespace afem

@@ -260,7 +260,8 @@ namespace afem {
 // afem_mesh.cu
 void build_lines_device(afem_ctx* c);     // MKLINE_V2 + MKN6 on the device
 void build_pattern_device(afem_ctx* c);   // adjacency + full CSR pattern
-void build_schedule(afem_ctx* c, bool levels);  // colouring + split rows; the level schedules when asked
+// levels: the natural-order level schedules; colours: the colouring and the split rows
+void build_schedule(afem_ctx* c, bool levels, bool colours);
 void exclusive_scan(const int32_t* in, int32_t* out, int n, cudaStream_t s, long* total_host);
 int compute_coloring(int n, const int32_t* rp, const int32_t* cl, uint8_t* color, int32_t* perm, int32_t* cptr,
                      int max_colors);  // greedy distance-1 colouring, rows sorted by colour

@@ -478,8 +478,8 @@ void split_rows_device(afem_ctx* c, const int32_t* rp, const int32_t* cl, const 
   count_launch();
 }
 
-void build_schedule(afem_ctx* c, bool levels) {
-  if (c->schedule_ready && (!levels || c->levels_ready)) return;
+void build_schedule(afem_ctx* c, bool levels, bool colours) {
+  if ((!colours || c->schedule_ready) && (!levels || c->levels_ready)) return;
   const int n = c->nline;
   cudaStream_t s = c->stream;
   // host copies of the pattern for the colouring (left uninitialised: filled by the copies)
@@ -498,7 +498,7 @@ void build_schedule(afem_ctx* c, bool levels) {
     AFEM_CUDA(cudaStreamSynchronize(s));
     c->levels_ready = true;
   }
-  if (c->schedule_ready) return;
+  if (!colours || c->schedule_ready) return;
   std::vector<uint8_t> color(n);
   std::vector<int32_t> pm(n), cptr(256);
   const int nc = compute_coloring(n, rp.get(), cl.get(), color.data(), pm.data(), cptr.data(), 255);

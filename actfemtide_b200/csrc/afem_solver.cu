@@ -34,6 +34,7 @@
 
 #include "afem_hybrid.h"
 #include "afem_internal.h"
+#include "afem_reduce.cuh"
 
 namespace afem {
 
@@ -77,6 +78,7 @@ struct SolverWork {
   int nsys = 0;     // systems of the current solve: ns, or the meshes of a packed batch
   bool seg = false; // packed batch: vectors hold one system per row
   int nblocks = 0;  // persistent grid size (blocks of 256 threads)
+  int prows = 0;    // rows of the partial-sum arrays
   DBuf<double2> x, b;               // FP64 solution and right-hand side [row][sys]
   DBuf<double2> xacc;               // FP64 solution accumulated over the refinement steps (kept between solves)
   DBuf<double2> r64;                // FP64 true residual
@@ -89,7 +91,15 @@ struct SolverWork {
   DBuf<double> rms;                 // per-system rms(r) for the learned preconditioner
   DBuf<double2> ht, hy, hdd;        // gradient-space correction: nodal rhs, solution, 1/diag (FP64 inner)
   DBuf<float2> htf, hyf, hddf;      // the same for the FP32 inner solve
-  DBuf<unsigned char> cbuf;         // coarse correction: work vectors (coarse_bytes)
+  DBuf<unsigned char> cbuf, nbuf;   // smoothed iteration: the grids' vectors; the mesh nodes' right-hand
+                                    // sides and corrections, [node][4][system] each
+  DBuf<double2> dkm;                // (K, M) diagonal in row order
+  DBuf<double> cheb;                // polynomial coefficients of the smoother: edges, nodes
+  DBuf<double2> pw;                 // power iteration: two vectors (K and M parts as x, y)
+  long cheb_gen = -1;               // assembly generation of dkm and cheb
+  DBuf<double2> red;                // block sums finished inside a launch: RED_SETS sets (red_set)
+  DBuf<unsigned> cnt;               // their counters
+  DBuf<double2> rho;                // shares of rho: the edges', then 4 rows of the grids'
   int nmc_blocks = 0;               // co-resident grid of the nodal multicolour sweeps
   int rpw64 = 0, rpw32 = 0;         // SpMV rows per warp chosen by tune_spmv (0 = not tuned; 8: 4 systems per lane)
   int spmv_grid[2][5] = {};         // one-wave grid of each SpMV variant (FP64 / FP32), 0 = not known yet
@@ -97,12 +107,10 @@ struct SolverWork {
   int mcb_blocks = 0;               // and of the backward one (fewer registers: more blocks)
   double sd = 1.0;                  // SSOR diagonal scale of the current solve (DD = 1 / (sd D))
   bool no_window = false;           // COCG13_single semantics: no stagnation window, run to the cap
-  bool kmf_valid = false;            // kmf matches the assembly
-  bool mcf_valid = false;            // mc_lkmf / mc_ukmf match the assembly
+  long kmf_gen = -1, mcf_gen = -1;   // assembly generations of kmf and of mc_lkmf / mc_ukmf
   DBuf<unsigned> flag_f, flag_b;
   DBuf<double> part;                // partial sums [block][sys][4]
   DBuf<double> part2;               // nodal share of rho (hybrid), same layout
-  DBuf<double> part3;               // coarse correction's share of rho, same layout
   DBuf<SysScal> sc;
   DBuf<Ctrl> ctrl;
   Ctrl* h_ctrl = nullptr;           // pinned mirror
@@ -215,7 +223,7 @@ __device__ __forceinline__ void row_gather(const int32_t* __restrict__ cols, con
 #ifndef AFEM_SPMV_CHUNK
 #define AFEM_SPMV_CHUNK 4  // rounds per chunk in the SpMV
 #endif
-// The first row of this warp's first round in for_rows<RPW, CH>(p0, ..).
+// The first row of this warp's first round in for_rows<RPW>(p0, .., CH, ..).
 template <int RPW, int CH>
 __device__ __forceinline__ int first_round(int p0) {
   return p0 + (int)blockIdx.x * CH * (int)(blockDim.x >> 5) * RPW + (int)(threadIdx.x >> 5) * RPW;
@@ -225,11 +233,12 @@ __device__ __forceinline__ int first_round(int p0) {
 // are pos0 + sub (sub < RPW), live below `end`; `next` is the first row of the
 // warp's following round (-1 after the last), so that a body can load the next
 // rows' indices while it gathers for the current ones.
-template <int RPW, int CH, class F>
-__device__ __forceinline__ void for_rows(int p0, int p1, F body) {
+template <int RPW, class F>
+__device__ __forceinline__ void for_rows(int p0, int p1, int ch, F body, int bid = (int)blockIdx.x,
+                                         int nb = (int)gridDim.x) {
   const int wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
-  const int chunk = CH * nwb * RPW, cstride = (int)gridDim.x * chunk;
-  int cb = p0 + (int)blockIdx.x * chunk, pos0 = cb + wib * RPW;
+  const int chunk = ch * nwb * RPW, cstride = nb * chunk;
+  int cb = p0 + bid * chunk, pos0 = cb + wib * RPW;
   if (cb < p1 && pos0 >= min(cb + chunk, p1)) cb = p1;  // no round of this warp in the (last, partial) chunk
   while (cb < p1) {
     const int ce = min(cb + chunk, p1);
@@ -286,6 +295,20 @@ __device__ __forceinline__ void seg_partials(double (*red)[MAX_SYS][NVAL], doubl
     double acc = 0.0;
     for (int sl = 0; sl < SLOTS; ++sl) acc += red[sl][sid][k];
     part[((long)blockIdx.x * MAX_SYS + sid) * 4 + k] = acc;
+  }
+}
+
+// The same into a set of block sums (first two values of a slot).
+template <int SLOTS, int NVAL>
+__device__ __forceinline__ void seg_pair(double (*red)[MAX_SYS][NVAL], const RedSet& R, int bid) {
+  __syncthreads();
+  for (int t = threadIdx.x; t < MAX_SYS; t += blockDim.x) {
+    double2 a = make_double2(0.0, 0.0);
+    for (int sl = 0; sl < SLOTS; ++sl) {
+      a.x += red[sl][t][0];
+      if constexpr (NVAL > 1) a.y += red[sl][t][1];
+    }
+    R.part[(long)t * R.rows + bid] = a;
   }
 }
 
@@ -772,7 +795,7 @@ __global__ void __launch_bounds__(256, (mc_min_blocks<NS, SEG>()))
       }
     };
     fetch(first_round<S::RPW, AFEM_SWEEP_CHUNK>(p0) + sub);
-    for_rows<S::RPW, AFEM_SWEEP_CHUNK>(p0, p1, [&](int pos0, int cend, int next) {
+    for_rows<S::RPW>(p0, p1, AFEM_SWEEP_CHUNK, [&](int pos0, int cend, int next) {
       const int pos = pos0 + sub;
       const bool live = pos < cend;
       const int row = live ? nrow : 0;
@@ -882,7 +905,7 @@ __global__ void __launch_bounds__(256, (mc_min_blocks<NS, SEG>()))
       }
     };
     fetch(first_round<S::RPW, AFEM_SWEEP_CHUNK>(p0) + sub);
-    for_rows<S::RPW, AFEM_SWEEP_CHUNK>(p0, p1, [&](int pos0, int cend, int next) {
+    for_rows<S::RPW>(p0, p1, AFEM_SWEEP_CHUNK, [&](int pos0, int cend, int next) {
       const int pos = pos0 + sub;
       const bool live = pos < cend;
       const int row = live ? nrow : 0;
@@ -1017,7 +1040,7 @@ __global__ void __launch_bounds__(256, (mc_min_blocks<NS, SEG>()))
       }
     };
     fetch(first_round<S::RPW, AFEM_SWEEP_CHUNK>(p0) + sub);
-    for_rows<S::RPW, AFEM_SWEEP_CHUNK>(p0, p1, [&](int pos0, int cend, int next) {
+    for_rows<S::RPW>(p0, p1, AFEM_SWEEP_CHUNK, [&](int pos0, int cend, int next) {
       const int pos = pos0 + sub;
       const bool live = pos < cend;
       const int row = live ? nrow : 0;
@@ -1092,39 +1115,32 @@ __device__ __forceinline__ void seg_warp_add(double (*red)[MAX_SYS][NVAL], int s
   }
 }
 
-// The nodal correction of edge e for system s of NS: u_head - u_tail, or with edge vectors te (coarse
-// correction on, u then [node][4][system]) also te . (v_head + v_tail) / 2 of the vector part v.
-template <class T, class PT, int NS>
-__device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restrict__ line,
-                                                        const typename Cx<PT>::V* __restrict__ u,
-                                                        const double* __restrict__ te, long e, int s) {
-  using PV = typename Cx<PT>::V;
-  const long ih = __ldg(line + 2 * e + 1) - 1, it = __ldg(line + 2 * e) - 1;
-  if (!te) {
-    const PV uh = u[ih * NS + s], ut = u[it * NS + s];
-    return Cx<T>::make((T)(uh.x - ut.x), (T)(uh.y - ut.y));
-  }
-  const PV* ph = u + ih * 4 * NS + s;
-  const PV* pt = u + it * 4 * NS + s;
-  T x = (T)(ph[0].x - pt[0].x), y = (T)(ph[0].y - pt[0].y);
+// The same for a warp that mostly lies in one mesh: one shuffle sum then, lane by lane otherwise.
+template <int NVAL>
+__device__ __forceinline__ void seg_warp_sum(double (*red)[MAX_SYS][NVAL], int slot, int sid, const double (&v)[NVAL]) {
+  const int s0 = __shfl_sync(0xffffffffu, sid, 0);
+  if (__all_sync(0xffffffffu, sid == s0)) {
+    if (s0 < 0) return;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const T h = (T)(0.5 * __ldg(te + 3 * e + d));
-    const PV a = ph[(d + 1) * NS], b = pt[(d + 1) * NS];
-    x += h * ((T)a.x + (T)b.x);
-    y += h * ((T)a.y + (T)b.y);
+    for (int k = 0; k < NVAL; ++k) {
+      double a = v[k];
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) a += __shfl_xor_sync(0xffffffffu, a, m);
+      if ((threadIdx.x & 31) == 0) red[slot][s0][k] += a;
+    }
+    return;
   }
-  return Cx<T>::make(x, y);
+  seg_warp_add<NVAL>(red, slot, sid, v);
 }
 
-// z_e += the nodal correction on the non-Dirichlet edges, then rho = r^T z partial sums (slots 0, 1)
+// z_e += u_head(e) - u_tail(e) on the non-Dirichlet edges, then rho = r^T z partial sums (slots 0, 1)
 // (u, z in the preconditioner type PT, r in the COCG type T)
 template <class T, class PT, int NS, bool SEG>
 __global__ void __launch_bounds__(256)
     k_grad_add(int n, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
                const typename Cx<PT>::V* __restrict__ u, typename Cx<PT>::V* __restrict__ z,
                const typename Cx<T>::V* __restrict__ r, const Ctrl* __restrict__ ctrl, double* __restrict__ part,
-               const uint8_t* __restrict__ seg, const double* __restrict__ te) {
+               const uint8_t* __restrict__ seg) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   static_assert(!SEG || NS == 1, "packed batches hold one system per row");
@@ -1142,8 +1158,9 @@ __global__ void __launch_bounds__(256)
       const int e = (int)(i / NS), s = (int)(i % NS);
       PV zi = z[i];
       if (!__ldg(bc + e)) {
-        const PV d = nodal_term<PT, PT, NS>(line, u, te, e, s);
-        zi = Cx<PT>::make(zi.x + d.x, zi.y + d.y);
+        const PV uh = u[(long)(__ldg(line + 2 * e + 1) - 1) * NS + s];
+        const PV ut = u[(long)(__ldg(line + 2 * e) - 1) * NS + s];
+        zi = Cx<PT>::make(zi.x + (uh.x - ut.x), zi.y + (uh.y - ut.y));
         z[i] = zi;
       }
       const V ri = r[i];
@@ -1211,11 +1228,111 @@ __global__ void k_dd_node(const double2* __restrict__ km, const int32_t* __restr
   }
 }
 
+// ------------------------------------------------------------------ scalar steps
+__device__ __forceinline__ void sum_partials(const double* part, int nblocks, int s, int k, double* out,
+                                             int nvals) {
+  // one warp per system; deterministic order
+  __shared__ double sh[32][4];
+  const int lane = threadIdx.x & 31;
+  for (int v = 0; v < nvals; ++v) {
+    double acc = 0.0;
+    for (int b = lane; b < nblocks; b += 32) acc += __ldcg(part + ((long)b * MAX_SYS + s) * 4 + k + v);
+    for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    sh[threadIdx.x >> 5][v] = acc;
+  }
+  __syncwarp();
+  for (int v = 0; v < nvals; ++v) out[v] = sh[threadIdx.x >> 5][v];
+  __syncwarp();
+}
+
+__device__ __forceinline__ double2 d_cdiv(double2 a, double2 b) { return cdiv(a, b); }
+
+// The three scalar steps of an iteration, run by one block on the sums v[system]:
+// ||r||^2 -> RESID, convergence, iteration cap, pending x update;
+__device__ __forceinline__ void finish_r(SysScal* sc, Ctrl* ctrl, const double2* v, int nsys) {
+  __shared__ int any_active;
+  if (threadIdx.x == 0) any_active = 0;
+  __syncthreads();
+  if (threadIdx.x < nsys) {
+    SysScal& S = sc[threadIdx.x];
+    S.xpend = S.active && ctrl->iter > 0;
+    if (S.active) {
+      S.rr = v[threadIdx.x].x;
+      S.resid = sqrt(S.rr / S.bnrm2);
+      if (ctrl->iter > 0) S.iter += 1;
+      if (!isfinite(S.resid)) { S.active = 0; S.status = AFEM_ENONFINITE; }
+      else if (S.resid <= ctrl->tol && ctrl->iter > 0) { S.active = 0; S.status = AFEM_OK; }
+      else if (ctrl->iter >= ctrl->maxit) { S.active = 0; S.status = AFEM_EMAXITER; }
+      else any_active = 1;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && !any_active) ctrl->done = 1;
+}
+
+// rho = r^T z from the edges', the nodes' and the grids' shares -> beta;
+__device__ __forceinline__ void finish_rho(SysScal* sc, const Ctrl* ctrl, const double2* v, const double2* edge,
+                                           const double2* grid, int nsys) {
+  if (threadIdx.x >= nsys) return;
+  SysScal& S = sc[threadIdx.x];
+  double2 a = cadd(v[threadIdx.x], __ldcg(edge + threadIdx.x));
+  for (int c = 0; c < 4; ++c) a = cadd(a, __ldcg(grid + c * MAX_SYS + threadIdx.x));
+  S.rho = a;
+  if (S.active) {
+    if (a.x == 0.0 && a.y == 0.0) { S.active = 0; S.status = AFEM_EBREAKDOWN; }
+    else if (ctrl->iter > 0) S.beta = d_cdiv(S.rho, S.rho1);
+  }
+}
+
+// p^T q -> alpha, and the iteration count.
+__device__ __forceinline__ void finish_pq(SysScal* sc, Ctrl* ctrl, const double2* v, int nsys) {
+  if (threadIdx.x < nsys) {
+    SysScal& S = sc[threadIdx.x];
+    S.pq = v[threadIdx.x];
+    if (S.active) {
+      if (S.pq.x == 0.0 && S.pq.y == 0.0) { S.active = 0; S.status = AFEM_EBREAKDOWN; S.alpha = make_double2(0, 0); }
+      else S.alpha = d_cdiv(S.rho, S.pq);
+      S.rho1 = S.rho;
+    } else {
+      S.alpha = make_double2(0.0, 0.0);
+    }
+  }
+  if (threadIdx.x == 0) {
+    ctrl->iter += 1;
+    ctrl->epoch += 1;
+  }
+}
+
 // ------------------------------------------------------------------ p update, SpMV
+// The nodal correction of edge e for system s of NS: u_head - u_tail, or with edge vectors te (coarse
+// correction on, u then [node][4][system]) also te . (v_head + v_tail) / 2 of the vector part v.
+template <class T, class PT, int NS>
+__device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restrict__ line,
+                                                        const typename Cx<PT>::V* __restrict__ u,
+                                                        const double* __restrict__ te, long e, int s) {
+  using PV = typename Cx<PT>::V;
+  const long ih = __ldg(line + 2 * e + 1) - 1, it = __ldg(line + 2 * e) - 1;
+  if (!te) {
+    const PV uh = u[ih * NS + s], ut = u[it * NS + s];
+    return Cx<T>::make((T)(uh.x - ut.x), (T)(uh.y - ut.y));
+  }
+  const PV* ph = u + ih * 4 * NS + s;
+  const PV* pt = u + it * 4 * NS + s;
+  T x = (T)(ph[0].x - pt[0].x), y = (T)(ph[0].y - pt[0].y);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const T h = (T)(0.5 * __ldg(te + 3 * e + d));
+    const PV a = ph[(d + 1) * NS], b = pt[(d + 1) * NS];
+    x += h * ((T)a.x + (T)b.x);
+    y += h * ((T)a.y + (T)b.y);
+  }
+  return Cx<T>::make(x, y);
+}
+
 // Multicolour path (x != nullptr): first x += alpha p with the old p for the
 // systems whose update is pending (also after the residual check ended the
-// solve).  Hybrid preconditioner with the gradient add folded in (u != nullptr):
-// z_e + u_head(e) - u_tail(e) on the non-Dirichlet edges stands for z.
+// solve).  Hybrid preconditioner with the nodal part folded in (u != nullptr):
+// z_e + the nodal correction (nodal_term) on the non-Dirichlet edges stands for z.
 // (p in the COCG type T; z and u in the preconditioner type PT)
 template <class T, class PT, int NS, bool SEG = false>
 __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
@@ -1372,7 +1489,8 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
     k_spmv(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
            const typename Cx<T>::V* __restrict__ km, int n, const typename Cx<T>::V* __restrict__ p,
            typename Cx<T>::V* __restrict__ q, const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl,
-           double* __restrict__ part, const typename Cx<T>::V* __restrict__ bvec, const uint8_t* __restrict__ seg) {
+           double* __restrict__ part, const typename Cx<T>::V* __restrict__ bvec, const uint8_t* __restrict__ seg,
+           RedSet R = RedSet{}, int nsys = 0, int ch = AFEM_SPMV_CHUNK) {
   using V = typename Cx<T>::V;
   constexpr int NG = NS / SPL;   // lanes of a row that hold different systems
   static_assert(NG * RPW <= 32, "rows per warp times lanes per row must fit a warp");
@@ -1398,10 +1516,10 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
   int nk0 = 0, nk1 = 0;
   {
     const int wib = threadIdx.x >> 5;
-    const int first = (int)blockIdx.x * AFEM_SPMV_CHUNK * (int)(blockDim.x >> 5) * RPW + wib * RPW + sub;
+    const int first = (int)blockIdx.x * ch * (int)(blockDim.x >> 5) * RPW + wib * RPW + sub;
     if (first < n) { nk0 = __ldg(rowptr + first); nk1 = __ldg(rowptr + first + 1); }
   }
-  for_rows<RPW, AFEM_SPMV_CHUNK>(0, n, [&](int row0, int cend, int next) {
+  for_rows<RPW>(0, n, ch, [&](int row0, int cend, int next) {
     const int row = row0 + sub;
     const bool live = row < cend;
     int sid = s0;
@@ -1448,11 +1566,511 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
       store_spl<V, SPL>(q + base, qi);
     }
   });
-  if constexpr (SEG) {
-    seg_partials<8 * RPW, 3>(red, part);
+  if (!R.part) {
+    if constexpr (SEG) seg_partials<8 * RPW, 3>(red, part);
+    else block_partials_spl<NS, SPL, LPR, NACC>(acc, s0, g == 0, part);
     return;
   }
-  block_partials_spl<NS, SPL, LPR, NACC>(acc, s0, g == 0, part);
+  // smoothed iteration: alpha is formed here
+  __shared__ double2 sums[MAX_SYS];
+  if constexpr (SEG) {
+    seg_pair<8 * RPW, 3>(red, R, blockIdx.x);
+  } else {
+    double pq[SPL][2];
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) {
+      pq[i][0] = acc[i][0];
+      pq[i][1] = acc[i][1];
+    }
+    block_pair<NS, SPL, LPR>(pq, s0, g == 0, R, blockIdx.x);
+  }
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
+    finish_pq(const_cast<SysScal*>(sc), const_cast<Ctrl*>(ctrl), sums, nsys);
+}
+
+// ------------------------------------------------------------------ smoothed iteration
+// The iteration of the gradient-corrected preconditioner with its coarse correction (afem_coarse.cu).
+// What the correction leaves to the smoother is local, so the smoother need not be a triangular
+// sweep: on the edges it is the Chebyshev polynomial of degree 2 in D^-1 A,
+//
+//     z = c1 s - c2 D^-1 A s,   s = D^-1 r,   D = diag(A),
+//
+// and the same on the nodes with A_G.  Both are one pass with no dependence between rows: the colour
+// sweeps spent 40 grid barriers an iteration (0.24 of 0.35 ms on 12x12x9 cells) and read the matrix
+// by halves through a colour permutation.  Iterations to 1e-10 on 32x32x24 cells: 52 with the sweeps,
+// 55 here (67 with D_G^-1 alone on the nodes).
+// An iteration is
+//   k_r_update:    r -= alpha q, s = D^-1 r, ||r||^2 -> convergence;
+//   k_smooth:      the edges' z, and the mesh nodes' right-hand sides G^T r, Pi_k^T r;
+//   coarse_cycle:  the V-cycles;
+//   k_node_prolong: the nodal correction w at the mesh nodes, with the nodes' smoother; rho -> beta;
+//   k_pupd:        x += alpha p, p = z + (correction of w) + beta p;
+//   k_spmv:        q = A p, p^T q -> alpha.
+// The scalar steps run in the last block of the kernel that produced their sums.
+constexpr double CHEB_SAFETY = 1.15;  // on the power iteration's estimate of the largest eigenvalue
+constexpr double CHEB_RATIO = 8.0;    // the smoothed interval is [b / 8, b]
+constexpr int CHEB_POWER = 8;         // steps of the power iteration
+// The smoothed iteration's recursive residual goes to this fraction of the tolerance before the true
+// residual is judged.  At the same residual its error is spread differently from the sweeps': the
+// phases of an MT model's small impedances were 2 to 12e-10 off where the sweeps left 3 to 4e-10
+// (residual 3e-12).  The three to six iterations this costs keep the fields as exact as they were.
+constexpr double SMOOTH_MARGIN = 0.3;
+
+// Lane geometry of k_smooth's edge part: SPL systems per lane, RPW rows per warp, G lanes share a
+// row's entries.  Four rows (or more, where a row's lanes are fewer) keep enough gathers in flight.
+template <int NS, bool SEG>
+struct SmShape {
+  static constexpr int SPL = NS >= 8 ? 2 : 1;
+  static constexpr int NG = NS / SPL;
+  static constexpr int RPW = NG >= 8 || NS < 8 ? 4 : 8;
+  static constexpr int LPR = 32 / RPW;
+  static constexpr int G = LPR / NG;
+};
+// ... and of its node part: SPL systems per lane, 8 lanes per node (4 nodes per warp)
+template <int NS>
+struct NdShape {
+  static constexpr int SPL = NS >= 2 ? 2 : 1;
+  static constexpr int NG = NS / SPL;
+  static constexpr int G = 8 / NG;
+};
+
+// r -= alpha q (the previous iteration's), s = D^-1 r and ||r||^2.  A thread takes SP consecutive
+// systems of a row (one 32-byte access in FP64); the grid's stride is a multiple of the threads per
+// row, so a thread keeps its systems.
+template <class T, class PT, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_r_update(int n, typename Cx<T>::V* __restrict__ r, const typename Cx<T>::V* __restrict__ q,
+               typename Cx<PT>::V* __restrict__ s, const double2* __restrict__ dkm, SysScal* sc, Ctrl* ctrl,
+               const uint8_t* __restrict__ seg, RedSet R, int nsys) {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  constexpr int SP = NS >= 2 ? 2 : 1, GPR = NS / SP;
+  if (ctrl->done) {
+    // the x update pending when the solve ended was applied by that iteration's p update
+    if (blockIdx.x == 0 && threadIdx.x < nsys) sc[threadIdx.x].xpend = 0;
+    return;
+  }
+  const bool update = ctrl->iter > 0;
+  const long total = (long)n * GPR, stride = (long)gridDim.x * blockDim.x;
+  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int s0 = SEG ? 0 : (int)(i0 % GPR) * SP;
+  double2 al[SP];
+  double om[SP], rr[SP][2];
+  bool act[SP];
+#pragma unroll
+  for (int j = 0; j < SP; ++j) {
+    al[j] = sc[s0 + j].alpha;
+    om[j] = sc[s0 + j].omega;
+    act[j] = update && sc[s0 + j].active;
+    rr[j][0] = rr[j][1] = 0.0;
+  }
+  double (*red)[MAX_SYS][1] = nullptr;
+  if constexpr (SEG) red = seg_sums<8, 1>();
+  const long span = SEG ? (total + stride - 1) / stride * stride : total;  // SEG: whole warps (shuffles)
+  for (long i = i0; i < span; i += stride) {
+    int sid = -1;
+    double e = 0.0;
+    if (i < total) {
+      const long row = i / GPR, base = row * NS + s0;
+      if constexpr (SEG) {
+        sid = __ldg(seg + row);
+        al[0] = sc[sid].alpha;
+        om[0] = sc[sid].omega;
+        act[0] = update && sc[sid].active;
+      }
+      V ri[SP];
+      load_spl<V, NS, SP, false>(r + base, ri);
+      bool any = false;
+#pragma unroll
+      for (int j = 0; j < SP; ++j) any |= act[j];
+      if (any) {
+        V qi[SP];
+        load_spl<V, NS, SP, false>(q + base, qi);
+#pragma unroll
+        for (int j = 0; j < SP; ++j)
+          if (act[j])
+            ri[j] = Cx<T>::make((T)((double)ri[j].x - (al[j].x * (double)qi[j].x - al[j].y * (double)qi[j].y)),
+                                (T)((double)ri[j].y - (al[j].x * (double)qi[j].y + al[j].y * (double)qi[j].x)));
+        store_spl<V, SP>(r + base, ri);
+      }
+      const double2 dg = __ldg(dkm + row);
+      PV so[SP];
+#pragma unroll
+      for (int j = 0; j < SP; ++j) {
+        const double v = (double)ri[j].x * (double)ri[j].x + (double)ri[j].y * (double)ri[j].y;
+        if constexpr (SEG) e = v;
+        else rr[j][0] += v;
+        const double2 dd = ssor_dd(dg, om[j], 1.0);
+        const PT dx = (PT)dd.x, dy = (PT)dd.y, wx = (PT)ri[j].x, wy = (PT)ri[j].y;
+        so[j] = Cx<PT>::make(wx * dx - wy * dy, wx * dy + wy * dx);
+      }
+      store_spl<PV, SP>(s + base, so);
+    }
+    if constexpr (SEG) {
+      const double v[1] = {e};
+      seg_warp_sum<1>(red, threadIdx.x >> 5, sid, v);
+    }
+  }
+  __shared__ double2 sums[MAX_SYS];
+  if constexpr (SEG) seg_pair<8, 1>(red, R, blockIdx.x);
+  else block_pair<NS, SP, GPR>(rr, s0, true, R, blockIdx.x);
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_r(sc, ctrl, sums, nsys);
+}
+
+// Blocks below nbe: z = c1 s - c2 D^-1 A s by rows, and the edges' share r^T z of rho.  The others:
+// the mesh nodes' right-hand sides t = (G^T r, Pi_x^T r, Pi_y^T r, Pi_z^T r) over the non-Dirichlet
+// edges of a node, and hs = D_G^-1 t_0.  Neither reads what the other writes.
+template <class T, class PT, int NS, bool SEG>
+__global__ void __launch_bounds__(256, (NS >= 8 ? MC_MIN_BLOCKS : 0))
+    k_smooth(int nbe, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+             const typename Cx<PT>::V* __restrict__ km, int n, const typename Cx<PT>::V* __restrict__ sv,
+             const typename Cx<T>::V* __restrict__ r, typename Cx<PT>::V* __restrict__ z,
+             const double2* __restrict__ dkm, const double* __restrict__ coef, int node,
+             const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist, const uint8_t* __restrict__ bc,
+             const double* __restrict__ te, const typename Cx<PT>::V* __restrict__ hdd,
+             typename Cx<PT>::V* __restrict__ t, typename Cx<PT>::V* __restrict__ hs,
+             const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg, int ch,
+             RedSet R, int nsys, double2* __restrict__ edge_rho) {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  if (ctrl->done) return;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if ((int)blockIdx.x < nbe) {
+    double (*red)[MAX_SYS][2] = nullptr;
+    if constexpr (SEG) red = seg_sums<32, 2>();
+    using S = SmShape<NS, SEG>;
+    constexpr int SPL = S::SPL;
+    const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+    const PT c1 = (PT)coef[0], c2 = (PT)coef[1];
+    double om[SPL], acc[SPL][2];
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) {
+      om[i] = sc[s0 + i].omega;
+      acc[i][0] = acc[i][1] = 0.0;
+    }
+    int nk0 = 0, nk1 = 0;
+    {
+      const int first = (int)blockIdx.x * ch * 8 * S::RPW + w * S::RPW + sub;
+      if (first < n) { nk0 = __ldg(rowptr + first); nk1 = __ldg(rowptr + first + 1); }
+    }
+    for_rows<S::RPW>(0, n, ch, [&](int row0, int cend, int next) {
+      const int row = row0 + sub;
+      const bool live = row < cend;
+      int sid = 0;
+      if constexpr (SEG) {
+        sid = live ? (int)__ldg(seg + row) : 0;
+        om[0] = sc[sid].omega;
+      }
+      const int k0 = live ? nk0 : 0, k1 = live ? nk1 : 0;
+      if (next >= 0 && next + sub < n) { nk0 = __ldg(rowptr + next + sub); nk1 = __ldg(rowptr + next + sub + 1); }
+      PT t1x[SPL], t1y[SPL], t2x[SPL], t2y[SPL];
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) t1x[i] = t1y[i] = t2x[i] = t2y[i] = 0;
+      row_gather_spl<PT, NS, S::G, SPL, true>(col, km, sv, k0 + g, k1, s0, t1x, t1y, t2x, t2y);
+      group_sum<PT, SPL, S::NG, S::LPR>(t1x, t1y, t2x, t2y);
+      if (g == 0 && live) {
+        const long base = (long)row * NS + s0;
+        const double2 dg = __ldg(dkm + row);
+        PV si[SPL], zo[SPL];
+        V ri[SPL];
+        load_spl<PV, NS, SPL, false, true>(sv + base, si);
+        load_spl<V, NS, SPL, false, true>(r + base, ri);
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) {
+          const PT o = (PT)om[i];
+          const PT ax = t1x[i] - o * t2y[i], ay = t1y[i] + o * t2x[i];
+          const double2 dd = ssor_dd(dg, om[i], 1.0);
+          const PT dx = (PT)dd.x, dy = (PT)dd.y;
+          zo[i] = Cx<PT>::make(c1 * si[i].x - c2 * (ax * dx - ay * dy), c1 * si[i].y - c2 * (ax * dy + ay * dx));
+          const double e0 = (double)ri[i].x * (double)zo[i].x - (double)ri[i].y * (double)zo[i].y;
+          const double e1 = (double)ri[i].x * (double)zo[i].y + (double)ri[i].y * (double)zo[i].x;
+          if constexpr (SEG) {
+            red[w * 4 + sub][sid][0] += e0;
+            red[w * 4 + sub][sid][1] += e1;
+          } else {
+            acc[i][0] += e0;
+            acc[i][1] += e1;
+          }
+        }
+        store_spl<PV, SPL>(z + base, zo);
+      }
+    }, (int)blockIdx.x, nbe);
+    __shared__ double2 sums[MAX_SYS];
+    if constexpr (SEG) seg_pair<32, 2>(red, R, blockIdx.x);
+    else block_pair<NS, SPL, S::LPR>(acc, s0, g == 0, R, blockIdx.x);
+    if (reduce_blocks(R, blockIdx.x, nbe, nsys, sums) && threadIdx.x < nsys) edge_rho[threadIdx.x] = sums[threadIdx.x];
+  } else {
+    using S = NdShape<NS>;
+    constexpr int SPL = S::SPL;
+    const int sub = lane >> 3, ql = lane & 7, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+    const int nb = (int)gridDim.x - nbe, b0 = (int)blockIdx.x - nbe;
+    for (int a0 = (b0 * 8 + w) * 4; a0 < node; a0 += nb * 32) {
+      const int a = a0 + sub;
+      const bool live = a < node;
+      T v[4][SPL][2];
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) v[d][i][0] = v[d][i][1] = 0;
+      const int q1 = live ? __ldg(nptr + a + 1) : 0;
+      for (int k = (live ? __ldg(nptr + a) : 0) + g; k < q1; k += S::G) {
+        const int ent = __ldg(nlist + k), e = ent >> 1;
+        if (__ldg(bc + e)) continue;
+        V re[SPL];
+        load_spl<V, NS, SPL, false, true>(r + (long)e * NS + s0, re);
+        const T sg = (ent & 1) ? (T)-1 : (T)1;
+        const T hx = (T)(0.5 * __ldg(te + 3L * e)), hy = (T)(0.5 * __ldg(te + 3L * e + 1)),
+                hz = (T)(0.5 * __ldg(te + 3L * e + 2));
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) {
+          v[0][i][0] += sg * re[i].x; v[0][i][1] += sg * re[i].y;
+          v[1][i][0] += hx * re[i].x; v[1][i][1] += hx * re[i].y;
+          v[2][i][0] += hy * re[i].x; v[2][i][1] += hy * re[i].y;
+          v[3][i][0] += hz * re[i].x; v[3][i][1] += hz * re[i].y;
+        }
+      }
+#pragma unroll
+      for (int m = S::NG; m < 8; m <<= 1)
+#pragma unroll
+        for (int d = 0; d < 4; ++d)
+#pragma unroll
+          for (int i = 0; i < SPL; ++i) {
+            v[d][i][0] += shfl_xor(v[d][i][0], m);
+            v[d][i][1] += shfl_xor(v[d][i][1], m);
+          }
+      if (live && g == 0) {
+#pragma unroll
+        for (int d = 0; d < 4; ++d) {
+          PV o[SPL];
+#pragma unroll
+          for (int i = 0; i < SPL; ++i) o[i] = Cx<PT>::make((PT)v[d][i][0], (PT)v[d][i][1]);
+          store_spl<PV, SPL>(t + ((long)a * 4 + d) * NS + s0, o);
+        }
+        PV dd[SPL], o[SPL];
+        load_spl<PV, NS, SPL, false, true>(hdd + (long)a * NS + s0, dd);
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) {
+          const PT tx = (PT)v[0][i][0], ty = (PT)v[0][i][1];
+          o[i] = Cx<PT>::make(tx * dd[i].x - ty * dd[i].y, tx * dd[i].y + ty * dd[i].x);
+        }
+        store_spl<PV, SPL>(hs + (long)a * NS + s0, o);
+      }
+    }
+  }
+}
+
+// w = (u + T O_0, T O_1, T O_2, T O_3) at every mesh node, in [node][4][system], with the nodes'
+// smoother u = c1 hs - c2 D_G^-1 A_G hs (the polynomial of the edges, on A_G = G^T A G) and their
+// share t_0^T u of rho; the last block forms rho and beta.  coef: the edges' and the nodes' pairs.
+template <class T, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_node_prolong(int node, const uint8_t* __restrict__ nseg, const CoarseGrid* __restrict__ grids,
+                   const int32_t* __restrict__ cell, const double* __restrict__ frac,
+                   const typename Cx<T>::V* __restrict__ O, const typename Cx<T>::V* __restrict__ t,
+                   const typename Cx<T>::V* __restrict__ hs, const typename Cx<T>::V* __restrict__ hdd,
+                   const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                   const double2* __restrict__ km, const double* __restrict__ coef, typename Cx<T>::V* __restrict__ w,
+                   SysScal* sc, const Ctrl* ctrl, RedSet R, int nsys, const double2* edge_rho, const double2* grid_rho) {
+  using V = typename Cx<T>::V;
+  if (ctrl->done) return;
+  constexpr int SP = NS >= 2 ? 2 : 1, GPC = NS / SP, GPR = 4 * GPC;
+  const long total = (long)node * GPR, stride = (long)gridDim.x * blockDim.x;
+  const T c1 = (T)coef[2], c2 = (T)coef[3];
+  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const int c = (int)(i0 % GPR) / GPC, s0 = (int)(i0 % GPC) * SP;  // the stride is a multiple of GPR
+  double om[SP], acc[SP][2];
+#pragma unroll
+  for (int j = 0; j < SP; ++j) {
+    om[j] = SEG ? 0.0 : sc[s0 + j].omega;
+    acc[j][0] = acc[j][1] = 0.0;
+  }
+  double (*red)[MAX_SYS][2] = nullptr;
+  if constexpr (SEG) red = seg_sums<8, 2>();
+  const long span = SEG ? (total + stride - 1) / stride * stride : total;  // SEG: whole warps (shuffles)
+  for (long i = i0; i < span; i += stride) {
+    const int a = (int)(i / GPR);
+    int sid = -1;
+    double e[2] = {0.0, 0.0};
+    if (i < total) {
+      if constexpr (SEG) sid = __ldg(nseg + a);
+      V o[SP];
+#pragma unroll
+      for (int j = 0; j < SP; ++j) o[j] = Cx<T>::make(0, 0);
+      if (c == 0) {
+        if constexpr (SEG) om[0] = sc[sid].omega;
+        T t1x[SP], t1y[SP], t2x[SP], t2y[SP];
+#pragma unroll
+        for (int j = 0; j < SP; ++j) t1x[j] = t1y[j] = t2x[j] = t2y[j] = 0;
+        const int k1 = __ldg(rowptr + a + 1);
+#pragma unroll 4
+        for (int k = __ldg(rowptr + a); k < k1; ++k) {
+          const double2 m = __ldg(km + k);
+          V x[SP];
+          load_spl<V, NS, SP, false, true>(hs + (long)__ldg(col + k) * NS + s0, x);
+#pragma unroll
+          for (int j = 0; j < SP; ++j) {
+            t1x[j] += (T)m.x * x[j].x; t1y[j] += (T)m.x * x[j].y;
+            t2x[j] += (T)m.y * x[j].x; t2y[j] += (T)m.y * x[j].y;
+          }
+        }
+        V ti[SP], si[SP], dd[SP];
+        load_spl<V, NS, SP, false, true>(t + (long)a * 4 * NS + s0, ti);
+        load_spl<V, NS, SP, false, true>(hs + (long)a * NS + s0, si);
+        load_spl<V, NS, SP, false, true>(hdd + (long)a * NS + s0, dd);
+#pragma unroll
+        for (int j = 0; j < SP; ++j) {
+          const T ax = t1x[j] - (T)om[j] * t2y[j], ay = t1y[j] + (T)om[j] * t2x[j];
+          o[j].x = c1 * si[j].x - c2 * (ax * dd[j].x - ay * dd[j].y);
+          o[j].y = c1 * si[j].y - c2 * (ax * dd[j].y + ay * dd[j].x);
+          const double ex = (double)ti[j].x * (double)o[j].x - (double)ti[j].y * (double)o[j].y;
+          const double ey = (double)ti[j].x * (double)o[j].y + (double)ti[j].y * (double)o[j].x;
+          if constexpr (SEG) {
+            e[0] = ex;
+            e[1] = ey;
+          } else {
+            acc[j][0] += ex;
+            acc[j][1] += ey;
+          }
+        }
+      }
+      const int b = __ldg(cell + a);
+      if (b >= 0) {
+        const CoarseGrid* g = grids + (SEG ? (long)sid * COARSE_LEVELS : 0);
+        const int nx = g->nx, nxy = nx * g->ny;
+        const double fx = __ldg(frac + 3L * a), fy = __ldg(frac + 3L * a + 1), fz = __ldg(frac + 3L * a + 2);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int dx = q & 1, dy = (q >> 1) & 1, dz = q >> 2;
+          const double wd = (dx ? fx : 1.0 - fx) * (dy ? fy : 1.0 - fy) * (dz ? fz : 1.0 - fz);
+          if (wd == 0.0) continue;
+          const T wt = (T)wd;
+          V x[SP];
+          load_spl<V, NS, SP, false, true>(O + ((long)(b + dx + nx * dy + nxy * dz) * 4 + c) * NS + s0, x);
+#pragma unroll
+          for (int j = 0; j < SP; ++j) {
+            o[j].x += wt * x[j].x;
+            o[j].y += wt * x[j].y;
+          }
+        }
+      }
+      store_spl<V, SP>(w + ((long)a * 4 + c) * NS + s0, o);
+    }
+    if constexpr (SEG) seg_warp_sum<2>(red, threadIdx.x >> 5, sid, e);
+  }
+  __shared__ double2 sums[MAX_SYS];
+  if constexpr (SEG) {
+    seg_pair<8, 2>(red, R, blockIdx.x);
+  } else {
+    // the lanes of component 0 hold the values
+    block_pair<NS, SP, GPR>(acc, s0, (int)(threadIdx.x % GPR) < GPC, R, blockIdx.x);
+  }
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_rho(sc, ctrl, sums, edge_rho, grid_rho, nsys);
+}
+
+// One step of the power iteration on D_K^-1 K and D_M^-1 M at once (x and y of the vectors): 8 lanes
+// per row; first: the start vector is a hash of the row in [-1, 1].  The last block of the last step
+// turns the two Rayleigh quotients into the smoother's coefficients: [b / CHEB_RATIO, b] with b
+// CHEB_SAFETY times the larger quotient (|x^H A x| <= b |x^H D x| at every frequency, as K and M are
+// semi-definite).
+__device__ __forceinline__ void cheb_coefficients(double lam, double fallback, double* coef) {
+  if (!(lam > 0.5 && lam < 64.0)) lam = fallback;  // an unusable estimate (non-finite values end the solve by themselves)
+  const double b = CHEB_SAFETY * lam, a = b / CHEB_RATIO;
+  const double th = 0.5 * (b + a), de = 0.5 * (b - a), sg = th / de, rho0 = 1.0 / sg, rn = 1.0 / (2.0 * sg - rho0);
+  coef[0] = (1.0 + rn * rho0) / th + 2.0 * rn / de;
+  coef[1] = 2.0 * rn / (de * th);
+}
+__device__ __forceinline__ double power_start(int row) {
+  unsigned h = (unsigned)row * 2654435761u;
+  h ^= h >> 15;
+  h *= 2246822519u;
+  h ^= h >> 13;
+  return (double)(h & 0xffff) / 32768.0 - 1.0;
+}
+__global__ void __launch_bounds__(256)
+    k_power(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const double2* __restrict__ km, int n,
+            const double2* __restrict__ dkm, const double2* __restrict__ in, double2* __restrict__ out, int first,
+            RedSet R, double* __restrict__ coef) {
+  const int lane = threadIdx.x & 31, sub = lane >> 3, g = lane & 7;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (long r0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; r0 < n; r0 += (long)gridDim.x * 32) {
+    const int row = (int)r0 + sub;
+    double kx = 0.0, my = 0.0;
+    if (row < n)
+      for (int k = __ldg(rowptr + row) + g; k < __ldg(rowptr + row + 1); k += 8) {
+        const int j = __ldg(col + k);
+        const double2 a = km[k];
+        const double2 v = first ? make_double2(power_start(j), power_start(j)) : in[j];
+        kx += a.x * v.x;
+        my += a.y * v.y;
+      }
+    for (int m = 1; m < 8; m <<= 1) {
+      kx += shfl_xor(kx, m);
+      my += shfl_xor(my, m);
+    }
+    if (row < n && g == 0) {
+      const double2 d = dkm[row];
+      const double2 v = first ? make_double2(power_start(row), power_start(row)) : in[row];
+      s[0] += v.x * kx; s[1] += v.x * v.x * d.x;
+      s[2] += v.y * my; s[3] += v.y * v.y * d.y;
+      out[row] = make_double2(d.x != 0.0 ? kx / d.x : 0.0, d.y != 0.0 ? my / d.y : 0.0);
+    }
+  }
+  if (!coef) return;
+  // two sums as two "systems": K's quotient and M's
+  __shared__ double2 sums[MAX_SYS];
+  double v[2][2] = {{s[0], s[1]}, {s[2], s[3]}};
+  block_pair<2, 2, 1>(v, 0, true, R, blockIdx.x);
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, 2, sums) && threadIdx.x == 0) {
+    double lam = sums[0].y > 0.0 ? sums[0].x / sums[0].y : 0.0;
+    if (sums[1].y > 0.0) lam = fmax(lam, sums[1].x / sums[1].y);
+    cheb_coefficients(lam, 3.5, coef);
+  }
+}
+
+// Steps of a power iteration on D_G^-1 A_G at each mesh's first frequency (8 lanes per node); the
+// last one leaves the quotient of the last two vectors' norms in coefficients like k_power's.
+__global__ void __launch_bounds__(256)
+    k_node_power(int node, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                 const double2* __restrict__ km, const int32_t* __restrict__ diagpos, const uint8_t* __restrict__ live,
+                 const uint8_t* __restrict__ nseg, const double* __restrict__ omega, const double2* __restrict__ in,
+                 double2* __restrict__ out, int first, RedSet R, double* __restrict__ coef) {
+  const int lane = threadIdx.x & 31, sub = lane >> 3, g = lane & 7;
+  double s[1][2] = {{0.0, 0.0}};
+  for (long r0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; r0 < node; r0 += (long)gridDim.x * 32) {
+    const int a = (int)r0 + sub;
+    double kx = 0.0, ky = 0.0;
+    if (a < node) {
+      const double om = omega[nseg ? (int)nseg[a] : 0];
+      for (int k = rowptr[a] + g; k < rowptr[a + 1]; k += 8) {
+        const int j = col[k];
+        const double2 m = km[k];
+        const double2 v = first ? make_double2(power_start(j), 0.0) : in[j];
+        kx += m.x * v.x - om * m.y * v.y;
+        ky += m.x * v.y + om * m.y * v.x;
+      }
+      for (int m = 1; m < 8; m <<= 1) {
+        kx += __shfl_xor_sync(0xffu << (8 * sub), kx, m);
+        ky += __shfl_xor_sync(0xffu << (8 * sub), ky, m);
+      }
+      if (g == 0) {
+        const double2 d = km[diagpos[a]];
+        const double2 D = make_double2(d.x, om * d.y);
+        const double2 v = first ? make_double2(power_start(a), 0.0) : in[a];
+        double2 o = make_double2(0.0, 0.0);
+        if (live[a] && (D.x != 0.0 || D.y != 0.0)) {
+          o = cdiv(make_double2(kx, ky), D);
+          s[0][0] += o.x * o.x + o.y * o.y;
+          s[0][1] += v.x * v.x + v.y * v.y;
+        }
+        out[a] = o;
+      }
+    }
+  }
+  if (!coef) return;
+  __shared__ double2 sums[MAX_SYS];
+  block_pair<1, 1, 1>(s, 0, true, R, blockIdx.x);
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, 1, sums) && threadIdx.x == 0)
+    cheb_coefficients(sums[0].y > 0.0 ? sqrt(sums[0].x / sums[0].y) : 0.0, 2.0, coef + 2);
 }
 
 // ------------------------------------------------------------------ tiled SpMV (16 systems, FP64)
@@ -1627,21 +2245,6 @@ __global__ void __launch_bounds__(256, 3)
 }
 
 // ------------------------------------------------------------------ scalar kernels
-__device__ __forceinline__ void sum_partials(const double* part, int nblocks, int s, int k, double* out,
-                                             int nvals) {
-  // one warp per system; deterministic order
-  __shared__ double sh[32][4];
-  const int lane = threadIdx.x & 31;
-  for (int v = 0; v < nvals; ++v) {
-    double acc = 0.0;
-    for (int b = lane; b < nblocks; b += 32) acc += part[((long)b * MAX_SYS + s) * 4 + k + v];
-    for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    sh[threadIdx.x >> 5][v] = acc;
-  }
-  __syncwarp();
-  for (int v = 0; v < nvals; ++v) out[v] = sh[threadIdx.x >> 5][v];
-}
-
 // defer_x (multicolour path): the sweep updated r only; x += alpha p of an active
 // system is marked pending and applied by the p update of the same iteration,
 // which also runs when this kernel ends the solve.
@@ -1681,13 +2284,10 @@ __global__ void k_scal_r(SysScal* sc, Ctrl* ctrl, const double* part, int nblock
   if (threadIdx.x == 0 && finished) ctrl->done = 1;
 }
 
-__device__ __forceinline__ double2 d_cdiv(double2 a, double2 b) { return cdiv(a, b); }
-
 // part2 (nullable): the nodal correction's share r^T G u = t^T u of rho, summed by
-// the backward nodal sweep when the gradient add is folded into the p update; part3
-// (nullable): the coarse correction's share
+// the backward nodal sweep when the gradient add is folded into the p update
 __global__ void k_scal_rho(SysScal* sc, Ctrl* ctrl, const double* part, int nblocks, int ns, int flexible,
-                           const double* part2, int nblocks2, const double* part3, int nblocks3) {
+                           const double* part2, int nblocks2) {
   if (ctrl->done) return;
   const int s = threadIdx.x >> 5;
   if (s >= ns) return;
@@ -1699,13 +2299,6 @@ __global__ void k_scal_rho(SysScal* sc, Ctrl* ctrl, const double* part, int nblo
     sum_partials(part2, nblocks2, s, 0, v2, 2);
     v[0] += v2[0];
     v[1] += v2[1];
-  }
-  if (part3) {
-    double v3[2];
-    __syncwarp();
-    sum_partials(part3, nblocks3, s, 0, v3, 2);
-    v[0] += v3[0];
-    v[1] += v3[1];
   }
   if ((threadIdx.x & 31) == 0) {
     SysScal& S = sc[s];
@@ -1976,7 +2569,7 @@ int one_wave_grid(afem_ctx* c, K kernel, int cap, size_t smem = 0) {
 
 // The SpMV variants: rpw rows per warp with a lane per system (1, 2, 4), or, at 16
 // systems, 8 rows per warp with 4 systems per lane (rpw = 8).  Returns the grid it
-// used (the number of partial sums its consumer adds).
+// used (the number of partial sums its consumer adds).  R: the last block forms alpha (not the tiles).
 // Build the tiled SpMV's column lists once per pattern (two passes of k_spt_build:
 // count, scan, fill).  Synchronises the stream; called before any graph capture.
 void ensure_spmv_tiles(afem_ctx* c) {
@@ -2004,9 +2597,15 @@ void ensure_spmv_tiles(afem_ctx* c) {
   c->spt_ready = true;
 }
 
+// Rounds per chunk of for_rows in a grid of nb blocks: the SpMV's, unless the rows are too few to
+// give every block a chunk (a mesh of 10,000 rows would leave three blocks of four idle).
+int row_chunk(int n, int nb, int rows_per_warp) {
+  return (long)nb * 8 * rows_per_warp * AFEM_SPMV_CHUNK <= n ? AFEM_SPMV_CHUNK : 1;
+}
+
 template <class T, int NS, bool SEG>
 int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km, const typename Cx<T>::V* p,
-                typename Cx<T>::V* q, const Ctrl* ctrl, const typename Cx<T>::V* bvec) {
+                typename Cx<T>::V* q, const Ctrl* ctrl, const typename Cx<T>::V* bvec, RedSet R = RedSet{}, int ch = AFEM_SPMV_CHUNK) {
   cudaStream_t s = c->stream;
   const int n = w->n;
   const int32_t* rp = c->rowptr.p;
@@ -2014,6 +2613,13 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
   const uint8_t* sg = SEG ? c->seg_of_row.p : nullptr;
   const int vi = rpw == 16 ? 4 : rpw == 8 ? 3 : rpw == 4 ? 2 : rpw == 2 ? 1 : 0;
   int& grid = w->spmv_grid[sizeof(T) == 8 ? 0 : 1][vi];
+  const bool fit = ch == 0;  // chunk and grid by the number of rows
+  auto shape = [&](int rows_per_warp) {
+    if (!fit) return grid;
+    const int g = std::max(1, std::min(grid, (n + 8 * rows_per_warp - 1) / (8 * rows_per_warp)));
+    ch = row_chunk(n, g, rows_per_warp);
+    return g;
+  };
   if constexpr (NS == 16 && !SEG && sizeof(T) == 8) {
     if (rpw == 16 && !bvec) {  // tiles staged in shared memory (built by ensure_spmv_tiles)
       AFEM_REQUIRE(c->spt_ready, AFEM_ESTATE, "SpMV: tiles not built");
@@ -2029,30 +2635,18 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
       return grid;
     }
   }
-  if constexpr (NS == 16 && !SEG) {
-    if (rpw == 8 && !bvec) {  // AFEM_MC_SPL systems per lane, 2 * AFEM_MC_SPL rows per warp (q = A p only)
-      auto k = k_spmv<T, NS, 2 * AFEM_MC_SPL, SEG, AFEM_MC_SPL>;
-      if (!grid) grid = one_wave_grid(c, k, w->nblocks);
-      k<<<grid, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg);
-      count_launch();
-      return grid;
-    }
-  }
-  if (rpw == 4 && NS * 4 <= 32) {
-    auto k = k_spmv<T, NS, (NS * 4 <= 32 ? 4 : 1), SEG>;
+  auto run = [&](auto k, int rows_per_warp) {
     if (!grid) grid = one_wave_grid(c, k, w->nblocks);
-    k<<<grid, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg);
-  } else if (rpw == 2 && NS * 2 <= 32) {
-    auto k = k_spmv<T, NS, (NS * 2 <= 32 ? 2 : 1), SEG>;
-    if (!grid) grid = one_wave_grid(c, k, w->nblocks);
-    k<<<grid, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg);
-  } else {
-    auto k = k_spmv<T, NS, 1, SEG>;
-    if (!grid) grid = one_wave_grid(c, k, w->nblocks);
-    k<<<grid, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg);
-  }
-  count_launch();
-  return grid;
+    const int g = shape(rows_per_warp);
+    k<<<g, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg, R, w->nsys, ch);
+    count_launch();
+    return g;
+  };
+  if constexpr (NS == 16 && !SEG)  // AFEM_MC_SPL systems per lane, 2 * AFEM_MC_SPL rows per warp (q = A p only)
+    if (rpw == 8 && !bvec) return run(k_spmv<T, NS, 2 * AFEM_MC_SPL, SEG, AFEM_MC_SPL>, 2 * AFEM_MC_SPL);
+  if (rpw == 4 && NS * 4 <= 32) return run(k_spmv<T, NS, (NS * 4 <= 32 ? 4 : 1), SEG>, 4);
+  if (rpw == 2 && NS * 2 <= 32) return run(k_spmv<T, NS, (NS * 2 <= 32 ? 2 : 1), SEG>, 2);
+  return run(k_spmv<T, NS, 1, SEG>, 1);
 }
 
 // Rows-per-warp autotuner: times each variant on this matrix (q = A p with the
@@ -2108,8 +2702,7 @@ int tune_spmv(afem_ctx* c, SolverWork* w) {
 // T: COCG vectors and the SpMV; PT: the multicolour preconditioner (its matrix
 // copies and vectors); PT differs from T only on the multicolour path.
 template <class T, class PT, int NS, bool SEG>
-void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, const double* d_omega,
-                       cudaEvent_t* ev) {
+void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, cudaEvent_t* ev) {
   using I = Inner<T, NS>;
   using P = Inner<PT, NS>;
   using V = typename I::V;
@@ -2162,45 +2755,24 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[3], s));
   int rho_blocks = mc ? w->mcb_blocks : sweep_blocks;
-  const bool coarse = mode == AFEM_PRECOND_HYBRID && c->hyb->co && c->hyb->co->on;
-  int coarse_blocks = 0;
-  const void* nodal = nullptr;
-  CoarseArgs ca{};
   if (hyb) {
     // z += G SSOR_node(G^T r): folded into the p update, or (packed batches, learned
     // base) a pass of its own that takes the rho partials again from the corrected z
     HybridState* h = c->hyb;
     const int node = h->node;
     const uint8_t* hs = SEG ? h->seg.p : nullptr;
-    nodal = P::HY(w);
-    if (coarse) {
-      ca.r = I::R(w);
-      ca.t = P::HT(w);
-      ca.u = P::HY(w);
-      ca.buf = w->cbuf.p;
-      ca.omega = d_omega;
-      ca.done = &w->ctrl.p->done;
-      ca.part = fold_grad ? w->part3.p : nullptr;
-      ca.max_blocks = w->nblocks;
-      coarse_blocks = coarse_down<T, PT, NS, SEG>(c, ca);
-    } else {
-      k_grad_t<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(node, h->nptr.p, h->nlist.p, c->bc.p, (const V*)I::R(w),
-                                                          P::HT(w), w->ctrl.p);
-      count_launch();
-    }
-    if (ev) AFEM_CUDA(cudaEventRecord(ev[8], s));
+    k_grad_t<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(node, h->nptr.p, h->nlist.p, c->bc.p, (const V*)I::R(w),
+                                                        P::HT(w), w->ctrl.p);
+    count_launch();
     for (int bwd = 0; bwd < 2; ++bwd)
       launch_coop(k_nsweep_mc<PT, NS, SEG>, w->nmc_blocks, s, (const int32_t*)(bwd ? h->uptr.p : h->lptr.p),
                   (const int32_t*)(bwd ? h->ucol.p : h->lcol.p), bwd ? P::HUKM(c) : P::HLKM(c),
                   (const PV*)P::HT(w), P::HY(w), (const PV*)P::HDD(w), (const int32_t*)h->perm.p,
                   (const int32_t*)h->cptr.p, h->ncolors, (const SysScal*)w->sc.p, (const Ctrl*)w->ctrl.p, hs, bwd,
                   (fold_grad && bwd) ? w->part2.p : (double*)nullptr);
-    if (ev) AFEM_CUDA(cudaEventRecord(ev[9], s));
-    if (coarse) nodal = coarse_up<PT, NS, SEG>(c, ca);
     if (!fold_grad) {
-      k_grad_add<T, PT, NS, SEG><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const PV*)nodal, P::Z(w),
-                                                              (const V*)I::R(w), w->ctrl.p, w->part.p, sg,
-                                                              coarse ? c->hyb->co->te.p : (const double*)nullptr);
+      k_grad_add<T, PT, NS, SEG><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const PV*)P::HY(w), P::Z(w),
+                                                              (const V*)I::R(w), w->ctrl.p, w->part.p, sg);
       count_launch();
       rho_blocks = w->nblocks;
     }
@@ -2216,21 +2788,19 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
     }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[4], s));
   k_scal_rho<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, rho_blocks, nsys, learned ? 1 : 0,
-                                        fold_grad ? w->part2.p : (const double*)nullptr, w->nmc_blocks,
-                                        coarse && fold_grad ? w->part3.p : (const double*)nullptr, coarse_blocks);
+                                        fold_grad ? w->part2.p : (const double*)nullptr, w->nmc_blocks);
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
-  const double* te = coarse && fold_grad ? c->hyb->co->te.p : nullptr;
   if constexpr (NS == 16 && !SEG)
     k_pupd_spl<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr,
-        fold_grad ? c->bc.p : (const uint8_t*)nullptr, fold_grad ? (const PV*)nodal : (const PV*)nullptr, te);
+        fold_grad ? c->bc.p : (const uint8_t*)nullptr, fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr, (const double*)nullptr);
   else
     k_pupd<T, PT, NS, SEG><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr, fold_grad ? c->bc.p : (const uint8_t*)nullptr,
-        fold_grad ? (const PV*)nodal : (const PV*)nullptr, te);
+        fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr, (const double*)nullptr);
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
   const int spmv_grid = launch_spmv<T, NS, SEG>(c, w, sizeof(T) == 8 ? w->rpw64 : w->rpw32, I::KM(c, w),
@@ -2240,6 +2810,113 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   count_launch();
 }
 
+// Whether a solve takes the smoothed iteration: the gradient-corrected preconditioner with a coarse
+// hierarchy, at SIGMA_DIAG = 1 (other values scale the SSOR sweeps' diagonal and keep those sweeps).
+bool smoothed(const afem_ctx* c, const SolverWork* w, int precond) {
+  return precond == AFEM_PRECOND_HYBRID && w->sd == 1.0 && c->hyb && c->hyb->co && c->hyb->co->on;
+}
+
+// The sets of block sums (each kernel its own: a kernel may start while the one before it ends).
+enum { RED_R, RED_EDGE, RED_NODE, RED_PQ, RED_GRID, RED_SETS };
+RedSet red_set(SolverWork* w, int k) {
+  const long vals = (long)RED_SYS * (w->prows + RED_GROUPS);
+  double2* p = w->red.p + k * vals;
+  return RedSet{p, p + (long)RED_SYS * w->prows, w->cnt.p + k * (RED_GROUPS + 1), w->prows};
+}
+
+// One smoothed iteration (see k_r_update).
+template <class T, class PT, int NS, bool SEG>
+void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, cudaEvent_t* ev) {
+  using I = Inner<T, NS>;
+  using P = Inner<PT, NS>;
+  using V = typename I::V;
+  using PV = typename P::V;
+  cudaStream_t s = c->stream;
+  HybridState* h = c->hyb;
+  CoarseState* co = h->co;
+  const int n = w->n, node = h->node, nsys = w->nsys, wide = c->num_sms * 8;
+  const uint8_t* sg = SEG ? c->seg_of_row.p : nullptr;
+  const uint8_t* ns = SEG ? h->seg.p : nullptr;
+  PV* sv = reinterpret_cast<PV*>(w->dd.p);  // s; DD of the natural-order sweeps is not used here
+  PV* t = reinterpret_cast<PV*>(w->nbuf.p);
+  PV* nw = t + 4L * node * NS;
+  PV* hs = P::HY(w);
+  const PV* hdd = P::HDD(w);
+  auto grid = [&](long items) { return (int)std::max(1L, std::min((long)wide, (items + 255) / 256)); };
+  constexpr int SP = NS >= 2 ? 2 : 1;
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[0], s));
+  k_r_update<T, PT, NS, SEG><<<grid((long)n * NS / SP), 256, 0, s>>>(n, I::R(w), (const V*)I::Q(w), sv, w->dkm.p,
+                                                                   w->sc.p, w->ctrl.p, sg, red_set(w, RED_R), nsys);
+  count_launch();
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[1], s));
+  const int nbe = grid((long)n * SmShape<NS, SEG>::LPR), nbn = grid(8L * node);
+  const PV* km = sizeof(PT) == 8 ? (const PV*)c->km.p : (const PV*)w->kmf.p;
+  k_smooth<T, PT, NS, SEG><<<nbe + nbn, 256, 0, s>>>(
+      nbe, c->rowptr.p, c->col.p, km, n, sv, (const V*)I::R(w), P::Z(w), w->dkm.p, w->cheb.p, node, h->nptr.p,
+      h->nlist.p, c->bc.p, co->te.p, hdd, t, hs, w->sc.p, w->ctrl.p, sg,
+      row_chunk(n, nbe, SmShape<NS, SEG>::RPW), red_set(w, RED_EDGE), nsys, w->rho.p);
+  count_launch();
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[2], s));
+  const CoarseArgs ca{t, w->cbuf.p, d_omega, &w->ctrl.p->done, w->rho.p + MAX_SYS, red_set(w, RED_GRID)};
+  const void* sol = coarse_cycle<PT, NS, SEG>(c, ca);
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[3], s));
+  k_node_prolong<PT, NS, SEG><<<grid(4L * node * NS / SP), 256, 0, s>>>(
+      node, ns, co->d_grids.p, co->cell.p, co->frac.p, static_cast<const PV*>(sol), t, hs, hdd, h->rowptr.p, h->col.p,
+      h->km.p, w->cheb.p, nw, w->sc.p, w->ctrl.p, red_set(w, RED_NODE), nsys, w->rho.p, w->rho.p + MAX_SYS);
+  count_launch();
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[4], s));
+  if constexpr (NS >= 2)
+    k_pupd_spl<T, PT, NS><<<grid((long)n * NS / 2), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p,
+                                                             w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw,
+                                                             co->te.p);
+  else
+    k_pupd<T, PT, NS, SEG><<<grid((long)n * NS), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg,
+                                                          w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw, co->te.p);
+  count_launch();
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
+  const int rpw = sizeof(T) == 8 ? w->rpw64 : w->rpw32;
+  const bool tiles = rpw == 16;
+  const int sgrid = launch_spmv<T, NS, SEG>(c, w, rpw, I::KM(c, w), (const V*)I::P(w), I::Q(w), w->ctrl.p,
+                                            (const V*)nullptr, tiles ? RedSet{} : red_set(w, RED_PQ), 0);
+  if (tiles) {
+    k_scal_pq<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, sgrid, nsys);
+    count_launch();
+  }
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
+}
+
+// Row-order diagonal and smoother coefficients: the edges' once per assembly (k_power covers every
+// frequency), the nodes' once per solve (k_node_power).
+void smoother_values(afem_ctx* c, SolverWork* w, const double* d_omega) {
+  cudaStream_t s = c->stream;
+  HybridState* h = c->hyb;
+  const int n = w->n, node = h->node;
+  auto grid = [&](long rows) { return (int)std::max(1L, std::min((long)c->num_sms * 8, (rows + 31) / 32)); };
+  const RedSet R = red_set(w, RED_EDGE);
+  const long m = std::max(n, node);  // (a mesh may have nodes without edges)
+  w->cheb.alloc(4);
+  w->pw.alloc(2 * m);
+  if (w->cheb_gen != c->assemble_gen) {
+    w->dkm.alloc(n);
+    k_gather_entries<double2><<<c->num_sms * 8, 256, 0, s>>>(c->km.p, c->diagpos.p, (long)n, w->dkm.p);
+    count_launch();
+    for (int k = 0; k < CHEB_POWER; ++k) {
+      k_power<<<grid(n), 256, 0, s>>>(c->rowptr.p, c->col.p, c->km.p, n, w->dkm.p, w->pw.p + (k & 1 ? m : 0),
+                                      w->pw.p + (k & 1 ? 0 : m), k == 0, R,
+                                      k + 1 == CHEB_POWER ? w->cheb.p : (double*)nullptr);
+      count_launch();
+    }
+    w->cheb_gen = c->assemble_gen;
+  }
+  for (int k = 0; k < CHEB_POWER; ++k) {
+    k_node_power<<<grid(node), 256, 0, s>>>(node, h->rowptr.p, h->col.p, h->km.p, h->diagpos.p, h->live.p,
+                                            c->nseg > 0 ? h->seg.p : nullptr, d_omega, w->pw.p + (k & 1 ? m : 0),
+                                            w->pw.p + (k & 1 ? 0 : m), k == 0, R,
+                                            k + 1 == CHEB_POWER ? w->cheb.p : (double*)nullptr);
+    count_launch();
+  }
+}
+
 // FP64 true residual r64 = b - A x; returns per-system ||r||^2 and ||b||^2 on the host.
 template <int NS, bool SEG>
 void true_residual(afem_ctx* c, SolverWork* w, std::vector<double>& rr, std::vector<double>& bb) {
@@ -2247,7 +2924,8 @@ void true_residual(afem_ctx* c, SolverWork* w, std::vector<double>& rr, std::vec
   const int nsys = w->nsys;
   k_spmv<double, NS, 1, SEG><<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p, c->km.p,
                                                         w->n, w->x.p, w->r64.p, w->sc.p, (const Ctrl*)nullptr,
-                                                        w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr);
+                                                        w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr,
+                                                        RedSet{}, 0, AFEM_SPMV_CHUNK);
   count_launch();
   DBuf<double> out;
   out.alloc(2 * nsys);
@@ -2312,7 +2990,8 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
     AFEM_CUDA(cudaMemsetAsync(w->x.p, 0, sizeof(double2) * total, s));
     k_spmv<double, NS, 1, SEG><<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p,
                                                           c->km.p, n, w->x.p, w->q.p, w->sc.p, (const Ctrl*)nullptr,
-                                                          w->part.p, w->r64.p, SEG ? c->seg_of_row.p : nullptr);
+                                                          w->part.p, w->r64.p, SEG ? c->seg_of_row.p : nullptr,
+                                                          RedSet{}, 0, AFEM_SPMV_CHUNK);
     count_launch();
   }
   k_init_sys<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, w->nblocks, nsys, tol, maxit, d_omega,
@@ -2326,7 +3005,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       w->ht.alloc(nt); w->hy.alloc(nt); w->hdd.alloc(nt);
     } else {
       w->htf.alloc(nt); w->hyf.alloc(nt); w->hddf.alloc(nt);
-      if (!h->kmf_valid || h->kmf.n != (size_t)h->nnz) {
+      if (!smoothed(c, w, precond) && (!h->kmf_valid || h->kmf.n != (size_t)h->nnz)) {
         h->kmf.alloc(h->nnz);
         k_convert<float2, double2><<<c->num_sms * 8, 256, 0, s>>>(h->km.p, h->kmf.p, h->nnz);
         count_launch();
@@ -2343,14 +3022,15 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
         h->kmf_valid = true;
       }
     }
-    if (precond == AFEM_PRECOND_HYBRID && h->co && h->co->on) {
+    if (smoothed(c, w, precond)) {
       if (sizeof(PT) == 4) coarse_float(c);
       const size_t need = coarse_bytes(h, NS, sizeof(PT));
       if (w->cbuf.n < need) w->cbuf.alloc(need);
-      w->part3.alloc((size_t)w->nblocks * MAX_SYS * 4);
+      const size_t nodal = 8 * (size_t)h->node * NS * 2 * sizeof(PT);
+      if (w->nbuf.n < nodal) w->nbuf.alloc(nodal);
+      smoother_values(c, w, d_omega);
     }
   }
-  w->sd = o->sigma_diag > 0 ? o->sigma_diag : 1.0;
   setup_dd<T, PT, NS, SEG>(c, w, use_hyb ? AFEM_PRECOND_HYBRID : precond, w->sd);
   const int mode = precond;
   {
@@ -2381,15 +3061,20 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   AFEM_CUDA(cudaMemcpyAsync(&w->ctrl.p->epoch, &w->epoch_host, sizeof(unsigned), cudaMemcpyHostToDevice, s));
   int iters_done = 0;
   const int chunk = check_every > 0 ? check_every : 32;
-  // profiling: 10 events per iteration of a chunk (fwd | scal | bwd | coarse down | nodal sweeps | coarse up |
-  // scal | pupd | spmv)
+  // profiling: 8 events per iteration of a chunk (fwd | scal | bwd | nodal correction | scal | pupd | spmv,
+  // or r update | smoother | coarse cycle | prolongation | pupd | spmv)
   const bool prof = c->prof.on;
   std::vector<cudaEvent_t> evs;
   if (prof) {
-    evs.resize(10L * chunk);
+    evs.resize(8L * chunk);
     for (auto& e : evs) AFEM_CUDA(cudaEventCreate(&e));
   }
-  auto ev_of = [&](int k) -> cudaEvent_t* { return prof ? &evs[10L * k] : nullptr; };
+  auto ev_of = [&](int k) -> cudaEvent_t* { return prof ? &evs[8L * k] : nullptr; };
+  const bool smooth = smoothed(c, w, mode);
+  auto enqueue = [&](int k) {
+    if (smooth) enqueue_smoothed<T, PT, NS, SEG>(c, w, d_omega, ev_of(k));
+    else enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, ev_of(k));
+  };
   cudaGraphExec_t gexec = nullptr;
   long graph_kernels = 0;  // kernel nodes of the captured chunk (launch count per graph launch)
   bool use_graph = o->use_graph != 0 && !prof;
@@ -2400,7 +3085,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       bool ok = true;
       g_capturing = 1;
       try {
-        for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, d_omega, ev_of(k));
+        for (int k = 0; k < chunk; ++k) enqueue(k);
       } catch (const Error&) {
         ok = false;
       }
@@ -2452,7 +3137,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       AFEM_CUDA(cudaGraphLaunch(gexec, s));
       count_launch(graph_kernels);
     } else {
-      for (int k = 0; k < chunk; ++k) enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, d_omega, ev_of(k));
+      for (int k = 0; k < chunk; ++k) enqueue(k);
     }
     AFEM_CUDA(cudaMemcpyAsync(w->h_ctrl, w->ctrl.p, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
     AFEM_CUDA(cudaStreamSynchronize(s));
@@ -2461,20 +3146,32 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       // count only iterations that ran to their last kernel
       const int executed = std::min(chunk, w->h_ctrl->iter - iter_before);
       const char* tag = sizeof(T) == 8 ? (sizeof(PT) == 8 ? "fp64" : "fp64pc32") : "fp32";
-      char nf[64], nb[64], nh[64], nc_[64], np_[64], ns_[64];
+      char nf[64], nb[64], nh[64], np_[64], ns_[64];
       const char* kind = SEG ? "seg" : "ns";
       const int cnt = SEG ? nsys : NS;
       const bool mcs = mode == AFEM_PRECOND_SSOR_MC || use_hyb;
       snprintf(nf, sizeof nf, "cocg_fwd_sweep%s_%s_%s%d", mcs ? "_mc" : "", tag, kind, cnt);
       snprintf(nb, sizeof nb, "cocg_bwd_sweep%s_%s_%s%d", mcs ? "_mc" : "", tag, kind, cnt);
       snprintf(nh, sizeof nh, "cocg_nodal_correction_%s_%s%d", tag, kind, cnt);
-      snprintf(nc_, sizeof nc_, "cocg_coarse_correction_%s_%s%d", tag, kind, cnt);
-      const bool crs = mode == AFEM_PRECOND_HYBRID && c->hyb->co && c->hyb->co->on;
       snprintf(np_, sizeof np_, "cocg_p_update_%s_%s%d", tag, kind, cnt);
       snprintf(ns_, sizeof ns_, "cocg_spmv_%s_%s%d_rpw%d", tag, kind, cnt, sizeof(T) == 8 ? w->rpw64 : w->rpw32);
       for (int k = 0; k < executed; ++k) {
         float a = 0, b = 0, h = 0, d = 0, e = 0;
-        cudaEvent_t* E = &evs[10L * k];
+        cudaEvent_t* E = &evs[8L * k];
+        if (smooth) {
+          static const char* const step[6] = {"cocg_r_update", "cocg_smoother", "cocg_coarse_cycle", "cocg_prolongation",
+                                              "cocg_p_update", "cocg_spmv"};
+          for (int j = 0; j < 6; ++j) {
+            float ms = 0;
+            if (cudaEventElapsedTime(&ms, E[j], E[j + 1]) != cudaSuccess) {
+              cudaGetLastError();
+              break;
+            }
+            if (j < 5) snprintf(nh, sizeof nh, "%s_%s_%s%d", step[j], tag, kind, cnt);
+            c->prof.add(j < 5 ? nh : ns_, ms);
+          }
+          continue;
+        }
         if (cudaEventElapsedTime(&a, E[0], E[1]) != cudaSuccess || cudaEventElapsedTime(&b, E[2], E[3]) != cudaSuccess ||
             cudaEventElapsedTime(&h, E[3], E[4]) != cudaSuccess || cudaEventElapsedTime(&d, E[5], E[6]) != cudaSuccess ||
             cudaEventElapsedTime(&e, E[6], E[7]) != cudaSuccess) {
@@ -2483,12 +3180,6 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
         }
         c->prof.add(nf, a);
         c->prof.add(nb, b);
-        float cd = 0, nd = 0, cu = 0;
-        if (crs && cudaEventElapsedTime(&cd, E[3], E[8]) == cudaSuccess &&
-            cudaEventElapsedTime(&nd, E[8], E[9]) == cudaSuccess && cudaEventElapsedTime(&cu, E[9], E[4]) == cudaSuccess) {
-          c->prof.add(nc_, cd + cu);
-          h = nd;
-        }
         if (use_hyb) c->prof.add(nh, h);
         c->prof.add(np_, d);
         c->prof.add(ns_, e);
@@ -2570,14 +3261,16 @@ SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false) {
     w->rf.alloc(total); w->pf.alloc(total); w->qf.alloc(total); w->ddf.alloc(total);
   }
   if ((mixed || pc32) && w->zf.n != (size_t)total) w->zf.alloc(total);
-  if (mixed && (!w->kmf_valid || w->kmf.n != (size_t)c->nnz)) {
+  if ((mixed || pc32) && (w->kmf_gen != c->assemble_gen || w->kmf.n != (size_t)c->nnz)) {
     w->kmf.alloc(c->nnz);
     k_convert<float2, double2><<<c->num_sms * 8, 256, 0, s>>>(c->km.p, w->kmf.p, c->nnz);
     count_launch();
-    w->kmf_valid = true;
+    w->kmf_gen = c->assemble_gen;
   }
   // FP32 copies of the colour-ordered split rows (mixed inner solve, FP32 preconditioner)
-  if ((mixed || pc32) && (!w->mcf_valid || w->mc_lkmf.n != c->mc_lcol.n)) {
+  // (where the colour-ordered rows are in use: the smoothed iteration has none)
+  if ((mixed || pc32) && c->mc_vals_gen == c->assemble_gen &&
+      (w->mcf_gen != c->assemble_gen || w->mc_lkmf.n != c->mc_lcol.n)) {
     const long nl = (long)c->mc_lcol.n, nu = (long)c->mc_ucol.n;
     w->mc_lkmf.alloc(nl);
     w->mc_ukmf.alloc(nu);
@@ -2589,7 +3282,7 @@ SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false) {
       k_gather_entries<float2><<<c->num_sms * 8, 256, 0, s>>>(c->km.p, c->mc_usrc.p, nu, w->mc_ukmf.p);
       count_launch();
     }
-    w->mcf_valid = true;
+    w->mcf_gen = c->assemble_gen;
   }
   {
     int b1 = 0;
@@ -2608,8 +3301,15 @@ SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false) {
       w->nblocks = std::max(w->nblocks, coresident_blocks(k_fwd<float, NS, SEG>, c->num_sms));
       w->nblocks = std::max(w->nblocks, coresident_blocks(k_bwd<float, NS, SEG>, c->num_sms));
     }
-    w->part.alloc((size_t)w->nblocks * MAX_SYS * 4);
-    w->part2.alloc((size_t)w->nblocks * MAX_SYS * 4);
+    w->prows = std::max(w->nblocks, c->num_sms * 8);
+    w->part.alloc((size_t)w->prows * MAX_SYS * 4);
+    w->part2.alloc((size_t)w->prows * MAX_SYS * 4);
+    w->red.alloc((size_t)RED_SETS * RED_SYS * (w->prows + RED_GROUPS));
+    w->rho.alloc(5 * MAX_SYS);
+    if (!w->cnt.p) {
+      w->cnt.alloc(RED_SETS * (RED_GROUPS + 1));
+      w->cnt.zero(s);
+    }
   }
   return w;
 }
@@ -2682,6 +3382,7 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
   }
   const bool recursive_only = ex && ex->recursive_only;
   w->no_window = recursive_only;
+  w->sd = o->sigma_diag > 0 ? o->sigma_diag : 1.0;
   const double tol = o->tol > 0 ? o->tol : 1e-8;
   const int maxit = o->maxit > 0 ? o->maxit : 100000;
   int it_total = 0, refinements = 0;
@@ -2699,7 +3400,7 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
     // residual relative to ||r64||; ask for the reduction still missing,
     // never below what FP32 can deliver in the mixed mode.
     double inner_tol = std::min(0.5, 0.5 * tol / prev);
-    if (outer == 0) inner_tol = tol * tol_scale;
+    if (outer == 0) inner_tol = tol * tol_scale * (smoothed(c, w, precond_now) ? SMOOTH_MARGIN : 1.0);
     if (mixed) inner_tol = std::max(inner_tol, o->inner_tol > 0 ? o->inner_tol : 1e-5);
     const int left = maxit - it_total;
     if (left <= 0) break;
@@ -2826,20 +3527,23 @@ void ensure_mc_values(afem_ctx* c) {
 int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, const afem_solve_opts* o,
                  afem_solve_stats* st, const SolveExtra* ex) {
   AFEM_REQUIRE(c->assembled, AFEM_ESTATE, "solve: system not assembled");
-  // the multicolour paths never read the natural-order level schedules
-  const bool mc_only = o->precond == AFEM_PRECOND_HYBRID || o->precond == AFEM_PRECOND_SSOR_MC ||
-                       (o->precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1);
-  {
-    HostTimer ht(c, "host_setup_schedule");
-    build_schedule(c, !mc_only);
+  const bool hyb = o->precond == AFEM_PRECOND_HYBRID || (o->precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1);
+  if (hyb) {
+    HostTimer ht(c, "host_setup_hybrid");
+    hybrid_prepare(c, true, false);
   }
-  {
+  // the smoothed iteration needs no colouring, the multicolour sweeps no natural-order levels
+  const bool smooth = o->precond == AFEM_PRECOND_HYBRID && (o->sigma_diag <= 0 || o->sigma_diag == 1.0) &&
+                      c->hyb->co->on;
+  const bool mc = o->precond == AFEM_PRECOND_SSOR_MC || (hyb && !smooth);
+  if (!smooth) {
+    HostTimer ht(c, "host_setup_schedule");
+    build_schedule(c, !mc, mc);
+  }
+  if (mc) {
     HostTimer ht(c, "host_setup_mc_values");
     ensure_mc_values(c);
-  }
-  if (o->precond == AFEM_PRECOND_HYBRID || (o->precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1)) {
-    HostTimer ht(c, "host_setup_hybrid");
-    hybrid_prepare(c, true);
+    if (hyb) hybrid_prepare(c, true, true);
   }
   if (c->nseg > 0) {
     AFEM_REQUIRE(nsys == c->nseg, AFEM_EINVAL, "solve: a packed batch solves one system per mesh (nsys = nseg)");
@@ -2861,9 +3565,9 @@ int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, cons
 void precond_apply_device(afem_ctx* c, double omega, const double2* r, double2* z) {
   AFEM_REQUIRE(c->assembled, AFEM_ESTATE, "preconditioner: system not assembled");
   AFEM_REQUIRE(c->nseg == 0, AFEM_EINVAL, "preconditioner: packed batches are not supported here");
-  build_schedule(c, false);
+  build_schedule(c, false, true);
   ensure_mc_values(c);
-  hybrid_prepare(c, false);
+  hybrid_prepare(c, false, true);
   SolverWork* w = ensure_work<1, false>(c, 1, false);
   cudaStream_t s = c->stream;
   const int n = c->nline;
@@ -2906,8 +3610,7 @@ void precond_apply_device(afem_ctx* c, double omega, const double2* r, double2* 
                 (const uint8_t*)nullptr, bwd, (double*)nullptr);
   k_grad_add<double, double, 1, false><<<w->nblocks, 256, 0, s>>>(n, c->line.p, c->bc.p, (const double2*)w->hy.p,
                                                                   w->z.p, (const double2*)w->r.p, w->ctrl.p,
-                                                                  w->part.p, (const uint8_t*)nullptr,
-                                                                  (const double*)nullptr);
+                                                                  w->part.p, (const uint8_t*)nullptr);
   count_launch();
   AFEM_CUDA(cudaMemcpyAsync(z, w->z.p, sizeof(double2) * n, cudaMemcpyDeviceToDevice, s));
   AFEM_CUDA(cudaStreamSynchronize(s));
@@ -2935,7 +3638,7 @@ void get_residual(afem_ctx* c, int k, double* r) {
 // depends on the pattern only), so repeated solves take the same reduction
 // order and give the same bits.
 void invalidate_work(afem_ctx* c) {
-  if (c->work) c->work->kmf_valid = c->work->mcf_valid = false;
+  if (c->work) c->work->kmf_gen = c->work->mcf_gen = -1;
 }
 
 // A new pattern: also tune the SpMV again (ensure_work re-allocates when the
@@ -2943,7 +3646,7 @@ void invalidate_work(afem_ctx* c) {
 void invalidate_pattern_work(afem_ctx* c) {
   c->spt_ready = false;
   if (c->work) {
-    c->work->kmf_valid = c->work->mcf_valid = false;
+    c->work->kmf_gen = c->work->mcf_gen = -1;
     c->work->rpw64 = c->work->rpw32 = 0;
   }
   c->nsys = 0;  // the old solutions belong to the old pattern
