@@ -35,11 +35,13 @@ namespace afem {
 
 namespace {
 
-constexpr int COARSE_TAIL = 1600;     // nodes of the first level the one-block cycle takes
-constexpr int COARSE_STOP = 60;       // a grid of at most this many nodes is the coarsest
+constexpr int COARSE_TAIL = 500;      // nodes of the first level the one-block cycle takes
+constexpr int COARSE_STOP = 300;      // a grid of at most this many nodes is the coarsest
 constexpr int COARSE_SWEEPS = 4;      // smoothing sweeps on the coarsest grid
-constexpr int TAIL_THREADS = 1024;
-constexpr size_t TAIL_VALS = 14000;   // shared complex values of the one-block cycle (224 KB in FP64)
+constexpr int TAIL_THREADS = 512;
+constexpr size_t TAIL_BYTES = 212 << 10;  // its shared memory (vectors, and the matrices that fit)
+constexpr size_t TAIL_VALS = TAIL_BYTES / 16;
+constexpr int TAIL_AXIS = 1024;       // axis weights of its levels
 constexpr int COARSE_MIN_NODES = 64;  // smaller meshes keep the SSOR corrections alone
 
 inline unsigned nblk(long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -190,90 +192,89 @@ __global__ void k_support_weights(int n1, const uint8_t* __restrict__ cseg, cons
   }
 }
 
-// Nodal matrices of the vector components on the node graph, Pi_k^T P A P Pi_k: a warp per row,
-// a lane per entry (so an entry stays in registers over the row's edges); n3[3 * entry + k].
-__global__ void __launch_bounds__(256)
-    k_node_values3(const int32_t* __restrict__ line, const uint8_t* __restrict__ bc, int node,
-                   const int32_t* __restrict__ nptr, const int32_t* __restrict__ nlist,
-                   const int32_t* __restrict__ erow, const int32_t* __restrict__ ecol,
-                   const double2* __restrict__ ekm, const double* __restrict__ te,
-                   const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, double2* __restrict__ n3) {
-  const int a = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (a >= node) return;
-  const int r0 = rowptr[a], r1 = rowptr[a + 1];
-  for (int q0 = r0; q0 < r1; q0 += 32) {
-    const int q = q0 + lane, b = q < r1 ? col[q] + 1 : 0;  // node ids in line are 1-based
-    double2 acc[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    for (int i = nptr[a]; i < nptr[a + 1]; ++i) {
-      const int e = nlist[i] >> 1;
-      if (bc[e]) continue;
-      const double ex = 0.25 * te[3L * e], ey = 0.25 * te[3L * e + 1], ez = 0.25 * te[3L * e + 2];
-      for (int k = erow[e]; k < erow[e + 1]; ++k) {
-        const int f = ecol[k];
-        if (bc[f]) continue;
-        if (line[2L * f] == b || line[2L * f + 1] == b) {
-          const double2 v = ekm[k];
-          const double wx = ex * te[3L * f], wy = ey * te[3L * f + 1], wz = ez * te[3L * f + 2];
-          acc[0].x += wx * v.x; acc[0].y += wx * v.y;
-          acc[1].x += wy * v.x; acc[1].y += wy * v.y;
-          acc[2].x += wz * v.x; acc[2].y += wz * v.y;
-        }
-      }
-    }
-    if (q < r1)
-      for (int k = 0; k < 3; ++k) n3[3L * q + k] = acc[k];
-  }
-}
-
-// the row sums of |K| and |M| over the warp's slots; dead rows (zero diagonal) give zero
-__device__ __forceinline__ void store_row(const double2 (&acc)[4], int lane, const CoarseGrid& g, int l,
+// One component's row from the warp's slots (lane < 27), with the row sums of |K| and |M|; a dead
+// row (zero diagonal) gets zero sums.
+__device__ __forceinline__ void store_row(double2 v, int lane, int c, const CoarseGrid& g, int l,
                                           double2* __restrict__ km, double2* __restrict__ l1) {
-  for (int c = 0; c < 4; ++c) {
-    if (lane < 27) km[108L * g.off + (long)(c * 27 + lane) * g.n + l] = acc[c];
-    double sk = lane < 27 ? fabs(acc[c].x) : 0.0, sm = lane < 27 ? fabs(acc[c].y) : 0.0;
-    for (int m = 16; m > 0; m >>= 1) {
-      sk += __shfl_xor_sync(0xffffffffu, sk, m);
-      sm += __shfl_xor_sync(0xffffffffu, sm, m);
-    }
-    const double dk = __shfl_sync(0xffffffffu, acc[c].x, 13), dm = __shfl_sync(0xffffffffu, acc[c].y, 13);
-    if (lane == 0) l1[4L * (g.off + l) + c] = (dk == 0.0 && dm == 0.0) ? make_double2(0.0, 0.0) : make_double2(sk, sm);
+  if (lane < 27) km[108L * g.off + (long)(c * 27 + lane) * g.n + l] = v;
+  double sk = lane < 27 ? fabs(v.x) : 0.0, sm = lane < 27 ? fabs(v.y) : 0.0;
+  for (int m = 16; m > 0; m >>= 1) {
+    sk += __shfl_xor_sync(0xffffffffu, sk, m);
+    sm += __shfl_xor_sync(0xffffffffu, sm, m);
   }
+  const double dk = __shfl_sync(0xffffffffu, v.x, 13), dm = __shfl_sync(0xffffffffu, v.y, 13);
+  if (lane == 0) l1[4L * (g.off + l) + c] = (dk == 0.0 && dm == 0.0) ? make_double2(0.0, 0.0) : make_double2(sk, sm);
 }
 
-// Level 1: T^T N_c T, a warp per grid node, a lane per slot
-__global__ void __launch_bounds__(256)
-    k_galerkin_mesh(int n1, const uint8_t* __restrict__ cseg, const CoarseGrid* __restrict__ grids,
+// Level 1: T^T N_c T.  A block of four warps per grid node, a lane per slot; the warps take the
+// support's mesh nodes in turn.  The entries of a mesh node's row are fetched by 32 lanes at once and
+// handed round through shared memory, so a row costs one load latency and not one per entry (a lane
+// per slot reading entry by entry took 2.8 ms on 88x88x56 cells and 0.22 ms on 12x12x9).
+constexpr int GM_WARPS = 4;
+struct MeshEntry {  // a nodal row's entry: its column's place in the grid and the four components
+  double fx, fy, fz;
+  int corner, pad;
+  double2 v[4];
+};
+__global__ void __launch_bounds__(32 * GM_WARPS)
+    k_galerkin_mesh(const uint8_t* __restrict__ cseg, const CoarseGrid* __restrict__ grids,
                     const int32_t* __restrict__ lptr, const int32_t* __restrict__ lidx,
                     const double* __restrict__ lw, const int32_t* __restrict__ corner,
                     const double* __restrict__ frac, const int32_t* __restrict__ cell,
                     const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                     const double2* __restrict__ n0, const double2* __restrict__ n3, double2* __restrict__ km,
                     double2* __restrict__ l1) {
-  const int c = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (c >= n1) return;
+  __shared__ MeshEntry ent[GM_WARPS][32];
+  __shared__ double2 sum[GM_WARPS][4][32];
+  const int c = blockIdx.x, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const CoarseGrid g = grids[(long)cseg[c] * COARSE_LEVELS];
   const int l = c - g.off;
   const int i = l % g.nx + lane % 3 - 1, j = (l / g.nx) % g.ny + (lane / 3) % 3 - 1,
             k = l / (g.nx * g.ny) + lane / 9 - 1;
   double2 acc[4] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-  for (int p = lptr[c]; p < lptr[c + 1]; ++p) {
+  for (int p = lptr[c] + w; p < lptr[c + 1]; p += GM_WARPS) {
     const double wa = lw[p];
     if (wa == 0.0) continue;
-    const int a = lidx[p];
-    for (int q = rowptr[a]; q < rowptr[a + 1]; ++q) {
-      const int b = col[q];
-      if (cell[b] < 0) continue;
-      const double w = wa * corner_weight(i, j, k, corner[b], frac[3L * b], frac[3L * b + 1], frac[3L * b + 2]);
-      if (w == 0.0) continue;
-      const double2 v = n0[q];
-      acc[0].x += w * v.x; acc[0].y += w * v.y;
-      for (int m = 0; m < 3; ++m) {
-        const double2 u = n3[3L * q + m];
-        acc[m + 1].x += w * u.x; acc[m + 1].y += w * u.y;
+    const int a = lidx[p], r1 = rowptr[a + 1];
+    for (int q0 = rowptr[a]; q0 < r1; q0 += 32) {
+      const int q = q0 + lane;
+      bool take = false;
+      MeshEntry x;
+      if (q < r1) {
+        const int b = col[q];
+        take = cell[b] >= 0;
+        x.corner = corner[b];
+        x.fx = frac[3L * b]; x.fy = frac[3L * b + 1]; x.fz = frac[3L * b + 2];
+        x.v[0] = n0[q];
+        for (int m = 0; m < 3; ++m) x.v[m + 1] = n3[3L * q + m];
       }
+      const unsigned have = __ballot_sync(0xffffffffu, take);
+      if (take) ent[w][__popc(have & ((1u << lane) - 1))] = x;
+      __syncwarp();
+      const int cnt = __popc(have);
+      for (int e = 0; e < cnt; ++e) {
+        const MeshEntry& y = ent[w][e];
+        const double wt = wa * corner_weight(i, j, k, y.corner, y.fx, y.fy, y.fz);
+        if (wt != 0.0)
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            acc[m].x += wt * y.v[m].x;
+            acc[m].y += wt * y.v[m].y;
+          }
+      }
+      __syncwarp();
     }
   }
-  store_row(acc, lane, g, l, km, l1);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) sum[w][m][lane] = acc[m];
+  __syncthreads();
+  // warp m adds component m
+  double2 v = sum[0][w][lane];
+  for (int u = 1; u < GM_WARPS; ++u) {
+    v.x += sum[u][w][lane].x;
+    v.y += sum[u][w][lane].y;
+  }
+  store_row(v, lane, w, g, l, km, l1);
 }
 
 // weight of plane I of the next level at plane i of this one
@@ -282,43 +283,98 @@ __device__ __forceinline__ double axis_weight(int i, int I, bool halved, int nc,
   return I == ci ? 1.0 - w : (I == ci + 1 ? w : 0.0);
 }
 
-// Level l + 1 from level l of each mesh that has both: P^T A P, a warp per node, a lane per slot
-__global__ void __launch_bounds__(256)
+// Level l + 1 from level l of each mesh that has both: P^T A P with P the product of three axis
+// interpolations, applied axis by axis.  A block per node of the next level, a warp per component: the
+// up to 27 x 27 entries around the node go to shared memory (one latency), then the axes are
+// contracted one after another, 9 terms a value (a lane per slot reading the 729 entries in turn
+// took 0.3 to 0.5 ms a level whatever its size).
+__global__ void __launch_bounds__(128)
     k_galerkin_grid(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int lev,
                     const double* __restrict__ axw, double2* __restrict__ km, double2* __restrict__ l1) {
+  __shared__ double W[3][27];          // [axis][fine plane ii][fine slot s][coarse slot S]
+  __shared__ double2 E[4][27 * 9];     // fine entries of three x planes at a time, then the y stage
+  __shared__ double2 X[4][27 * 9];     // after the x axis: [kk][jj][sz][sy][SX]
   const int sg = blockIdx.y;
   if (lev + 1 >= levels[sg]) return;
   const CoarseGrid f = grids[(long)sg * COARSE_LEVELS + lev], g = grids[(long)sg * COARSE_LEVELS + lev + 1];
-  const int l = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int l = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (l >= g.n) return;
-  const bool hx = f.halved & 1, hy = f.halved & 2, hz = f.halved & 4;
-  const int I = l % g.nx, J = (l / g.nx) % g.ny, K = l / (g.nx * g.ny);
-  const int si = I + lane % 3 - 1, sj = J + (lane / 3) % 3 - 1, sk = K + lane / 9 - 1;
-  const int i0 = hx ? max(0, 2 * I - 1) : I, i1 = hx ? min(f.nx - 1, 2 * I + 1) : I;
-  const int j0 = hy ? max(0, 2 * J - 1) : J, j1 = hy ? min(f.ny - 1, 2 * J + 1) : J;
-  const int k0 = hz ? max(0, 2 * K - 1) : K, k1 = hz ? min(f.nz - 1, 2 * K + 1) : K;
-  double2 acc[4] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-  for (int k = k0; k <= k1; ++k)
-    for (int j = j0; j <= j1; ++j)
-      for (int i = i0; i <= i1; ++i) {
-        const double wa = axis_weight(i, I, hx, g.nx, axw[f.wx + i]) * axis_weight(j, J, hy, g.ny, axw[f.wy + j]) *
-                          axis_weight(k, K, hz, g.nz, axw[f.wz + k]);
-        if (wa == 0.0) continue;
-        const int a = i + f.nx * (j + f.ny * k);
-        for (int s = 0; s < 27; ++s) {
-          const int bi = i + s % 3 - 1, bj = j + (s / 3) % 3 - 1, bk = k + s / 9 - 1;
-          if (bi < 0 || bi >= f.nx || bj < 0 || bj >= f.ny || bk < 0 || bk >= f.nz) continue;
-          const double w = wa * axis_weight(bi, si, hx, g.nx, axw[f.wx + bi]) *
-                           axis_weight(bj, sj, hy, g.ny, axw[f.wy + bj]) *
-                           axis_weight(bk, sk, hz, g.nz, axw[f.wz + bk]);
-          if (w == 0.0) continue;
-          for (int c = 0; c < 4; ++c) {
-            const double2 v = km[108L * f.off + (long)(c * 27 + s) * f.n + a];
-            acc[c].x += w * v.x; acc[c].y += w * v.y;
-          }
+  const int N[3] = {g.nx, g.ny, g.nz}, n[3] = {f.nx, f.ny, f.nz}, wo[3] = {f.wx, f.wy, f.wz};
+  const int I[3] = {l % g.nx, (l / g.nx) % g.ny, l / (g.nx * g.ny)};
+  int lo[3], cnt[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const bool h = (f.halved >> d) & 1;
+    lo[d] = h ? max(0, 2 * I[d] - 1) : I[d];
+    cnt[d] = (h ? min(n[d] - 1, 2 * I[d] + 1) : I[d]) - lo[d] + 1;
+  }
+  if (threadIdx.x < 81) {
+    const int d = threadIdx.x / 27, ii = threadIdx.x % 27 / 9, s = threadIdx.x % 9 / 3 - 1, S = threadIdx.x % 3 - 1;
+    const bool h = (f.halved >> d) & 1;
+    const int i = lo[d] + ii, b = i + s;
+    double w = 0.0;
+    if (ii < cnt[d] && b >= 0 && b < n[d])
+      w = axis_weight(i, I[d], h, N[d], axw[wo[d] + i]) * axis_weight(b, I[d] + S, h, N[d], axw[wo[d] + b]);
+    W[d][threadIdx.x % 27] = w;
+  }
+  __syncthreads();
+  const double2* A = km + 108L * f.off + (long)c * 27 * f.n;
+  // x axis, three fine planes kk in turn: E[ii][jj][slot] (9 x 27 entries), X[kk][jj][sz][sy][SX]
+  for (int kk = 0; kk < 3; ++kk) {
+    for (int q = lane; q < 243; q += 32) {
+      const int ii = q % 3, jj = q / 3 % 3, s = q / 9;
+      double2 v = make_double2(0.0, 0.0);
+      if (ii < cnt[0] && jj < cnt[1] && kk < cnt[2])
+        v = A[(long)s * f.n + (lo[0] + ii) + f.nx * ((lo[1] + jj) + f.ny * (lo[2] + kk))];
+      E[c][q] = v;
+    }
+    __syncwarp();
+    for (int q = lane; q < 81; q += 32) {  // q = SX + 3 (sy + 3 (sz + 3 jj))
+      const int SX = q % 3, sy = q / 3 % 3, sz = q / 9 % 3, jj = q / 27;
+      double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+      for (int ii = 0; ii < 3; ++ii)
+#pragma unroll
+        for (int sx = 0; sx < 3; ++sx) {
+          const double w = W[0][ii * 9 + sx * 3 + SX];
+          const double2 e = E[c][ii + 3 * jj + 9 * (sx + 3 * sy + 9 * sz)];
+          v.x += w * e.x;
+          v.y += w * e.y;
         }
+      X[c][q + 81 * kk] = v;
+    }
+    __syncwarp();
+  }
+  // y axis: Y[kk][sz][SY][SX] in E
+  for (int q = lane; q < 81; q += 32) {  // q = SX + 3 (SY + 3 (sz + 3 kk))
+    const int SX = q % 3, SY = q / 3 % 3, sz = q / 9 % 3, kk = q / 27;
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int jj = 0; jj < 3; ++jj)
+#pragma unroll
+      for (int sy = 0; sy < 3; ++sy) {
+        const double w = W[1][jj * 9 + sy * 3 + SY];
+        const double2 e = X[c][SX + 3 * (sy + 3 * (sz + 3 * jj)) + 81 * kk];
+        v.x += w * e.x;
+        v.y += w * e.y;
       }
-  store_row(acc, lane, g, l, km, l1);
+    E[c][q] = v;
+  }
+  __syncwarp();
+  double2 v = make_double2(0.0, 0.0);
+  if (lane < 27) {
+    const int SZ = lane / 9;
+#pragma unroll
+    for (int kk = 0; kk < 3; ++kk)
+#pragma unroll
+      for (int sz = 0; sz < 3; ++sz) {
+        const double w = W[2][kk * 9 + sz * 3 + SZ];
+        const double2 e = E[c][lane % 9 + 9 * (sz + 3 * kk)];
+        v.x += w * e.x;
+        v.y += w * e.y;
+      }
+  }
+  store_row(v, lane, c, g, l, km, l1);
 }
 
 __global__ void k_to_float(const double2* __restrict__ in, float2* __restrict__ out, long n) {
@@ -339,9 +395,10 @@ __device__ __forceinline__ typename CV<T>::V l1_solve(double2 d, double om, type
   return o;
 }
 
-// (T^T t) of level-1 node c, component cc, system s; t [mesh node][4][system]
-template <class T, int NS>
-__device__ __forceinline__ typename CV<T>::V mesh_down(int c, int cc, int s, const int32_t* __restrict__ lptr,
+// (T^T t) of level-1 node c, component cc, system s; t [mesh node][4][system].  Over the support's
+// nodes p0 + q, p0 + q + G, ...: G lanes may share a support.
+template <class T, int NS, int G>
+__device__ __forceinline__ typename CV<T>::V mesh_down(int c, int cc, int s, int q, const int32_t* __restrict__ lptr,
                                                        const int32_t* __restrict__ lidx,
                                                        const double* __restrict__ lw,
                                                        const typename CV<T>::V* __restrict__ t) {
@@ -349,13 +406,21 @@ __device__ __forceinline__ typename CV<T>::V mesh_down(int c, int cc, int s, con
   acc.x = 0; acc.y = 0;
   const int p1 = __ldg(lptr + c + 1);
 #pragma unroll 4
-  for (int p = __ldg(lptr + c); p < p1; ++p) {
+  for (int p = __ldg(lptr + c) + q; p < p1; p += G) {
     const T w = (T)__ldg(lw + p);
     const typename CV<T>::V v = t[((long)__ldg(lidx + p) * 4 + cc) * NS + s];
     acc.x += w * v.x;
     acc.y += w * v.y;
   }
   return acc;
+}
+
+template <class T>
+__device__ __forceinline__ typename CV<T>::V cm(typename CV<T>::V a, typename CV<T>::V b) {
+  typename CV<T>::V o;
+  o.x = a.x * b.x - a.y * b.y;
+  o.y = a.x * b.y + a.y * b.x;
+  return o;
 }
 
 // R = T^T t at level 1 and Z = D^-1 R
@@ -371,35 +436,39 @@ __global__ void __launch_bounds__(256)
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
     const int s = (int)(i % NS), cc = (int)(i / NS) & 3, c = (int)(i / (4 * NS));
     const double2 d = l1[4L * c + cc];
-    typename CV<T>::V v = mesh_down<T, NS>(c, cc, s, lptr, lidx, lw, t);
+    typename CV<T>::V v = mesh_down<T, NS, 1>(c, cc, s, 0, lptr, lidx, lw, t);
     if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
     R[i] = v;
     Z[i] = l1_solve<T>(d, omega[s], v);
   }
 }
 
-// (A v)_(node, comp) for one system; v and km of one grid, vs the stride between nodes of v
+// (A v) at a node for one component and system: a = the component's first slot at the node, as =
+// the stride between slots; v the vector at the node's own entry, vs its stride between nodes.  Slots
+// outside the grid hold zeros, so they may be multiplied with any value (the node's own): no
+// branches, and three entries are in flight together (nine cost registers and so resident warps).
 template <class T>
-__device__ __forceinline__ typename CV<T>::V grid_row(const CoarseGrid& g, int l, int comp, double om,
-                                                      const typename CV<T>::V* __restrict__ km,
+__device__ __forceinline__ typename CV<T>::V grid_row(const CoarseGrid& g, int l, double om,
+                                                      const typename CV<T>::V* __restrict__ a, long as,
                                                       const typename CV<T>::V* v, long vs) {
   const int i = l % g.nx, jk = l / g.nx, j = jk % g.ny, k = jk / g.ny;
-  const typename CV<T>::V* a = km + 108L * g.off + (long)comp * 27 * g.n + l;
+  const bool x0 = i > 0, x1 = i + 1 < g.nx, y0 = j > 0, y1 = j + 1 < g.ny, z0 = k > 0, z1 = k + 1 < g.nz;
   T t1x = 0, t1y = 0, t2x = 0, t2y = 0;
 #pragma unroll
-  for (int dk = -1; dk <= 1; ++dk) {
-    if (k + dk < 0 || k + dk >= g.nz) continue;
+  for (int b = 0; b < 27; b += 3) {
+    typename CV<T>::V m[3], w[3];
 #pragma unroll
-    for (int dj = -1; dj <= 1; ++dj) {
-      if (j + dj < 0 || j + dj >= g.ny) continue;
+    for (int q = 0; q < 3; ++q) {
+      const int s = b + q, di = s % 3 - 1, dj = s / 3 % 3 - 1, dk = s / 9 - 1;
+      const bool ok = (dk < 0 ? z0 : (dk > 0 ? z1 : true)) && (dj < 0 ? y0 : (dj > 0 ? y1 : true)) &&
+                      (di < 0 ? x0 : (di > 0 ? x1 : true));
+      m[q] = a[(long)s * as];
+      w[q] = v[ok ? (long)(di + g.nx * (dj + g.ny * dk)) * vs : 0L];
+    }
 #pragma unroll
-      for (int di = -1; di <= 1; ++di) {
-        if (i + di < 0 || i + di >= g.nx) continue;
-        const typename CV<T>::V m = a[(long)((di + 1) + 3 * (dj + 1) + 9 * (dk + 1)) * g.n];
-        const typename CV<T>::V w = v[(long)(l + di + g.nx * (dj + g.ny * dk)) * vs];
-        t1x += m.x * w.x; t1y += m.x * w.y;
-        t2x += m.y * w.x; t2y += m.y * w.y;
-      }
+    for (int q = 0; q < 3; ++q) {
+      t1x += m[q].x * w[q].x; t1y += m[q].x * w[q].y;
+      t2x += m[q].y * w[q].x; t2y += m[q].y * w[q].y;
     }
   }
   typename CV<T>::V o;
@@ -411,7 +480,7 @@ __device__ __forceinline__ typename CV<T>::V grid_row(const CoarseGrid& g, int l
 // (P^T v) at node l of the next level g; v on level f
 template <class T>
 __device__ __forceinline__ typename CV<T>::V grid_down(const CoarseGrid& f, const CoarseGrid& g, int l,
-                                                       const double* __restrict__ axw, const typename CV<T>::V* v,
+                                                       const double* axw, const typename CV<T>::V* v,
                                                        long vs) {
   const bool hx = f.halved & 1, hy = f.halved & 2, hz = f.halved & 4;
   const int I = l % g.nx, J = (l / g.nx) % g.ny, K = l / (g.nx * g.ny);
@@ -421,11 +490,11 @@ __device__ __forceinline__ typename CV<T>::V grid_down(const CoarseGrid& f, cons
   typename CV<T>::V o;
   o.x = 0; o.y = 0;
   for (int k = k0; k <= k1; ++k) {
-    const double wk = axis_weight(k, K, hz, g.nz, __ldg(axw + f.wz + k));
+    const double wk = axis_weight(k, K, hz, g.nz, axw[f.wz + k]);
     for (int j = j0; j <= j1; ++j) {
-      const double wj = wk * axis_weight(j, J, hy, g.ny, __ldg(axw + f.wy + j));
+      const double wj = wk * axis_weight(j, J, hy, g.ny, axw[f.wy + j]);
       for (int i = i0; i <= i1; ++i) {
-        const T w = (T)(wj * axis_weight(i, I, hx, g.nx, __ldg(axw + f.wx + i)));
+        const T w = (T)(wj * axis_weight(i, I, hx, g.nx, axw[f.wx + i]));
         const typename CV<T>::V x = v[(long)(i + f.nx * (j + f.ny * k)) * vs];
         o.x += w * x.x;
         o.y += w * x.y;
@@ -438,12 +507,12 @@ __device__ __forceinline__ typename CV<T>::V grid_down(const CoarseGrid& f, cons
 // (P v) at node l of level f; v on the next level g
 template <class T>
 __device__ __forceinline__ typename CV<T>::V grid_up(const CoarseGrid& f, const CoarseGrid& g, int l,
-                                                     const double* __restrict__ axw, const typename CV<T>::V* v,
+                                                     const double* axw, const typename CV<T>::V* v,
                                                      long vs) {
   const int i = l % f.nx, j = (l / f.nx) % f.ny, k = l / (f.nx * f.ny);
   const int I = min((f.halved & 1) ? i >> 1 : i, g.nx - 2), J = min((f.halved & 2) ? j >> 1 : j, g.ny - 2),
             K = min((f.halved & 4) ? k >> 1 : k, g.nz - 2);
-  const double fx = __ldg(axw + f.wx + i), fy = __ldg(axw + f.wy + j), fz = __ldg(axw + f.wz + k);
+  const double fx = axw[f.wx + i], fy = axw[f.wy + j], fz = axw[f.wz + k];
   typename CV<T>::V o;
   o.x = 0; o.y = 0;
 #pragma unroll
@@ -477,7 +546,8 @@ __global__ void __launch_bounds__(256)
     const int s = (int)(i % NS), c = (int)(i / NS) & 3, l = (int)(i / VS);
     const long in = i % VS;  // component and system
     if constexpr (STEP == 0) {
-      const typename CV<T>::V a = grid_row<T>(f, l, c, omega[s], km, Z + fo + in, VS);
+      const typename CV<T>::V a = grid_row<T>(f, l, omega[s], km + 108L * f.off + (long)c * 27 * f.n + l, f.n,
+                                              Z + fo + i, VS);
       typename CV<T>::V v = R[fo + i];
       v.x -= a.x; v.y -= a.y;
       O[fo + i] = v;
@@ -495,7 +565,8 @@ __global__ void __launch_bounds__(256)
       z.x += u.x; z.y += u.y;
       Z[fo + i] = z;
     } else {
-      const typename CV<T>::V a = grid_row<T>(f, l, c, omega[s], km, Z + fo + in, VS);
+      const typename CV<T>::V a = grid_row<T>(f, l, omega[s], km + 108L * f.off + (long)c * 27 * f.n + l, f.n,
+                                              Z + fo + i, VS);
       const typename CV<T>::V r = R[fo + i];
       typename CV<T>::V z = Z[fo + i], e;
       e.x = r.x - a.x; e.y = r.y - a.y;
@@ -519,13 +590,62 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Half of grid_row's sum for the one-block cycle, where two lanes share a node: slots q, q + 2, ...
+// with the slots' node offsets `off` and the node's valid slots `ok` (bit per slot).
+template <class T>
+__device__ __forceinline__ void grid_half(int q, unsigned ok, const int* off, const typename CV<T>::V* __restrict__ a,
+                                          int as, const typename CV<T>::V* v, T (&t)[4]) {
+#pragma unroll
+  for (int b = 0; b < 14; b += 7) {
+    typename CV<T>::V m[7], w[7];
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+      const int s = min(q + 2 * (b + j), 26);
+      const bool in = q + 2 * (b + j) < 27 && ((ok >> s) & 1);
+      m[j] = a[(long)s * as];
+      w[j] = v[in ? off[s] : 0];
+      if (!in) m[j].x = m[j].y = 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+      t[0] += m[j].x * w[j].x; t[1] += m[j].x * w[j].y;
+      t[2] += m[j].y * w[j].x; t[3] += m[j].y * w[j].y;
+    }
+  }
+}
+
+// Valid slots of node (i, j, k): bit (di+1) + 3 (dj+1) + 9 (dk+1)
+__device__ __forceinline__ unsigned grid_mask(const CoarseGrid& g, int l) {
+  const int i = l % g.nx, jk = l / g.nx, j = jk % g.ny, k = jk / g.ny;
+  unsigned m = 0x7ffffffu;
+  if (i == 0) m &= ~0x1249249u;                 // di = -1: bits 0, 3, 6, ...
+  if (i + 1 == g.nx) m &= ~(0x1249249u << 2);   // di = +1
+  if (j == 0) m &= ~0x01c0e07u;                 // dj = -1: bits 0..2, 9..11, 18..20
+  if (j + 1 == g.ny) m &= ~(0x01c0e07u << 6);   // dj = +1
+  if (k == 0) m &= ~0x1ffu;                     // dk = -1
+  if (k + 1 == g.nz) m &= ~(0x1ffu << 18);      // dk = +1
+  return m;
+}
+
 // The V-cycle from level `top` down, one block per (component, system) -- in a packed batch per
-// (component, mesh) -- with the levels' R and Z and one scratch vector in shared memory.  Starts from
-// R of the top level, or (top = 0) from the mesh nodes' t, and writes the top level's O; rho
-// (top = 0): the component's share of rho of its system.
+// (component, mesh) -- with the levels' R, Z and D^-1 and one scratch vector in shared memory.
+// Starts from R of the top level, or (top = 0) from the mesh nodes' t, and writes the top level's O;
+// rho (top = 0): the component's share of rho of its system.
+// A step is one load latency long, so what bounds it is how many dependent loads it makes: the
+// matrices of the lower levels that fit are copied to shared memory while the restriction runs, the
+// inverse diagonals are formed once, the axis weights sit in shared memory, and the larger levels' rows
+// come seven entries at a time on two lanes a node.  49.6 -> 21 us a cycle on 12x12x9 cells (one 245-node grid,
+// whose four sweeps replaced two more levels).
+template <class T>
+__device__ __forceinline__ void copy_async(typename CV<T>::V* dst, const typename CV<T>::V* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (sizeof(T) == 8) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 template <class T, int NS, bool SEG>
 __global__ void __launch_bounds__(TAIL_THREADS)
-    k_grid_tail(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int top,
+    k_grid_tail(const CoarseGrid* __restrict__ grids, const int32_t* __restrict__ levels, int top, int vals,
                 const typename CV<T>::V* __restrict__ km, const double2* __restrict__ l1,
                 const double* __restrict__ axw, const double* __restrict__ omega,
                 const typename CV<T>::V* __restrict__ R, typename CV<T>::V* __restrict__ O,
@@ -534,72 +654,145 @@ __global__ void __launch_bounds__(TAIL_THREADS)
   using V = typename CV<T>::V;
   if (*done) return;
   extern __shared__ double2 tail_smem[];
-  V* sh = reinterpret_cast<V*>(tail_smem);
+  V* sh = reinterpret_cast<V*>(tail_smem);  // `vals` values
   __shared__ CoarseGrid gs[COARSE_LEVELS];
-  __shared__ int so[COARSE_LEVELS + 1];
+  __shared__ int so[COARSE_LEVELS], mo[COARSE_LEVELS];  // a level's vectors; its matrix (-1: in global memory)
+  __shared__ int scratch, off[COARSE_LEVELS][27];
+  __shared__ double aw[TAIL_AXIS];
   const int comp = blockIdx.x, sg = SEG ? (int)blockIdx.y : 0, s = SEG ? 0 : (int)blockIdx.y;
   const double om = omega[blockIdx.y];
   const int nl = levels[sg];
   if (threadIdx.x < nl) gs[threadIdx.x] = grids[(long)sg * COARSE_LEVELS + threadIdx.x];
   __syncthreads();
-  if (threadIdx.x == 0) {  // R of level l at so[l], Z behind it; the scratch after all levels
-    int o = 0;
-    for (int l = top; l < nl; ++l) { so[l] = o; o += 2 * gs[l].n; }
-    so[nl] = o;
+  for (int u = threadIdx.x; u < nl * 27; u += TAIL_THREADS) {
+    const int q = u % 27;
+    off[u / 27][q] = q % 3 - 1 + gs[u / 27].nx * (q / 3 % 3 - 1 + gs[u / 27].ny * (q / 9 - 1));
   }
-  __syncthreads();
-  V* tmp = sh + so[nl];
-  constexpr long VS = 4L * NS;
-  {
-    const CoarseGrid& g = gs[top];
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-      V v;
-      if (top) {
-        v = R[((long)(g.off + i) * 4 + comp) * NS + s];
-      } else {
-        const double2 d = l1[4L * (g.off + i) + comp];
-        v = mesh_down<T, NS>(g.off + i, comp, s, lptr, lidx, lw, t);
-        if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
-      }
-      sh[so[top] + i] = v;
+  const int aw0 = gs[top].wx;  // the axis weights of a mesh's levels are consecutive
+  if (threadIdx.x == 0) {      // a level: R, Z, D^-1; then the scratch; then matrices from the coarsest up
+    int o = 0;
+    for (int l = top; l < nl; ++l) { so[l] = o; o += 3 * gs[l].n; }
+    scratch = o;
+    o += gs[top].n;
+    for (int l = nl - 1; l >= top; --l) {
+      mo[l] = -1;
+      if (o + 27 * gs[l].n <= vals && (l == nl - 1 || mo[l + 1] >= 0)) { mo[l] = o; o += 27 * gs[l].n; }
     }
   }
   __syncthreads();
-  for (int l = top; l < nl; ++l) {  // down: z = D^-1 r, then the residual to the next level
+  for (int l = top; l < nl; ++l) {
+    if (mo[l] < 0) continue;
+    const V* src = km + 108L * gs[l].off + (long)comp * 27 * gs[l].n;
+    for (int i = threadIdx.x; i < 27 * gs[l].n; i += TAIL_THREADS) copy_async<T>(sh + mo[l] + i, src + i);
+  }
+  if (nl - 1 > top) {
+    const CoarseGrid& g = gs[nl - 2];
+    for (int i = threadIdx.x; i < g.wz + g.nz - aw0; i += TAIL_THREADS) aw[i] = axw[aw0 + i];
+  }
+  V* tmp = sh + scratch;
+  const double* ax = aw - aw0;
+  constexpr long VS = 4L * NS;
+  V one;
+  one.x = 1; one.y = 0;
+  for (int l = top; l < nl; ++l) {
+    const CoarseGrid& g = gs[l];
+    V* r = sh + so[l];
+    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+      const V d = l1_solve<T>(l1[4L * (g.off + i) + comp], om, one);
+      r[2 * g.n + i] = d;
+    }
+  }
+  __syncthreads();
+  {
+    const CoarseGrid& g = gs[top];
+    V* r = sh + so[top];
+    V* z = r + g.n;
+    const V* d = z + g.n;
+    if (top) {
+      for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
+        r[i] = R[((long)(g.off + i) * 4 + comp) * NS + s];
+        z[i] = cm<T>(d[i], r[i]);
+      }
+    } else {  // four lanes share a support
+      const int n4 = (4 * g.n + TAIL_THREADS - 1) / TAIL_THREADS * TAIL_THREADS;
+      for (int u = threadIdx.x; u < n4; u += TAIL_THREADS) {
+        const int i = u >> 2;
+        V v;
+        v.x = 0; v.y = 0;
+        if (i < g.n) v = mesh_down<T, NS, 4>(g.off + i, comp, s, u & 3, lptr, lidx, lw, t);
+#pragma unroll
+        for (int m = 1; m < 4; m <<= 1) {
+          v.x += __shfl_xor_sync(0xffffffffu, v.x, m);
+          v.y += __shfl_xor_sync(0xffffffffu, v.y, m);
+        }
+        if (i < g.n && (u & 3) == 0) {
+          if (d[i].x == 0 && d[i].y == 0) { v.x = 0; v.y = 0; }
+          r[i] = v;
+          z[i] = cm<T>(d[i], v);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  // f(i, (A z)_i) for every node of level l, two lanes a node
+  auto product = [&](int l, const V* z, auto f) {
+    const CoarseGrid& g = gs[l];
+    const V* a = mo[l] >= 0 ? sh + mo[l] : km + 108L * g.off + (long)comp * 27 * g.n;
+    const int n2 = (2 * g.n + TAIL_THREADS - 1) / TAIL_THREADS * TAIL_THREADS;
+    for (int u = threadIdx.x; u < n2; u += TAIL_THREADS) {
+      const int i = min(u >> 1, g.n - 1);
+      T t[4] = {0, 0, 0, 0};
+      grid_half<T>(u & 1, grid_mask(g, i), off[l], a + i, g.n, z + i, t);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) t[m] += __shfl_xor_sync(0xffffffffu, t[m], 1);
+      if ((u & 1) == 0 && (u >> 1) < g.n) {
+        V o;
+        o.x = t[0] - (T)om * t[3];
+        o.y = t[1] + (T)om * t[2];
+        f(i, o);
+      }
+    }
+  };
+  const V* zc = nullptr;  // the solution of the level below
+  for (int l = top; l < nl; ++l) {  // down: the residual of z = D^-1 r to the next level
     const CoarseGrid& g = gs[l];
     V* r = sh + so[l];
     V* z = r + g.n;
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = l1_solve<T>(l1[4L * (g.off + i) + comp], om, r[i]);
-    __syncthreads();
+    const V* d = z + g.n;
     if (l + 1 == nl) {
+      V* from = z;
+      V* to = tmp;
       for (int k = 1; k < COARSE_SWEEPS; ++k) {
-        for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-          const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+        product(l, from, [&](int i, V a) {
           V e = r[i];
           e.x -= a.x; e.y -= a.y;
-          e = l1_solve<T>(l1[4L * (g.off + i) + comp], om, e);
-          e.x += z[i].x; e.y += z[i].y;
-          tmp[i] = e;
-        }
+          e = cm<T>(d[i], e);
+          e.x += from[i].x; e.y += from[i].y;
+          to[i] = e;
+        });
         __syncthreads();
-        for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = tmp[i];
-        __syncthreads();
+        V* u = from;
+        from = to;
+        to = u;
       }
+      zc = from;
       break;
     }
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-      const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+    product(l, z, [&](int i, V a) {
       V e = r[i];
       e.x -= a.x; e.y -= a.y;
       tmp[i] = e;
-    }
+    });
     __syncthreads();
     const CoarseGrid& n = gs[l + 1];
+    V* rn = sh + so[l + 1];
     for (int i = threadIdx.x; i < n.n; i += TAIL_THREADS) {
-      V v = grid_down<T>(g, n, i, axw, tmp, 1);
-      const double2 d = l1[4L * (n.off + i) + comp];
-      if (d.x == 0.0 && d.y == 0.0) { v.x = 0; v.y = 0; }
-      sh[so[l + 1] + i] = v;
+      V v = grid_down<T>(g, n, i, ax, tmp, 1);
+      const V dn = rn[2 * n.n + i];
+      if (dn.x == 0 && dn.y == 0) { v.x = 0; v.y = 0; }
+      rn[i] = v;
+      rn[n.n + i] = cm<T>(dn, v);
     }
     __syncthreads();
   }
@@ -607,34 +800,31 @@ __global__ void __launch_bounds__(TAIL_THREADS)
     const CoarseGrid& g = gs[l];
     V* r = sh + so[l];
     V* z = r + g.n;
-    const V* zc = sh + so[l + 1] + gs[l + 1].n;
+    const V* d = z + g.n;
     for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-      const double2 d = l1[4L * (g.off + i) + comp];
-      if (d.x == 0.0 && d.y == 0.0) continue;
-      const V u = grid_up<T>(g, gs[l + 1], i, axw, zc, 1);
+      if (d[i].x == 0 && d[i].y == 0) continue;
+      const V u = grid_up<T>(g, gs[l + 1], i, ax, zc, 1);
       z[i].x += u.x; z[i].y += u.y;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-      const V a = grid_row<T>(g, i, comp, om, km, z, 1);
+    product(l, z, [&](int i, V a) {
       V e = r[i];
       e.x -= a.x; e.y -= a.y;
-      e = l1_solve<T>(l1[4L * (g.off + i) + comp], om, e);
+      e = cm<T>(d[i], e);
       e.x += z[i].x; e.y += z[i].y;
       tmp[i] = e;
-    }
+    });
     __syncthreads();
-    for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) z[i] = tmp[i];
-    __syncthreads();
+    zc = tmp;
   }
   const CoarseGrid& g = gs[top];
   const V* r = sh + so[top];
-  const V* z = r + g.n;
   double px = 0.0, py = 0.0;
   for (int i = threadIdx.x; i < g.n; i += TAIL_THREADS) {
-    O[((long)(g.off + i) * 4 + comp) * NS + s] = z[i];
-    px += (double)r[i].x * (double)z[i].x - (double)r[i].y * (double)z[i].y;
-    py += (double)r[i].x * (double)z[i].y + (double)r[i].y * (double)z[i].x;
+    const V z = zc[i];
+    O[((long)(g.off + i) * 4 + comp) * NS + s] = z;
+    px += (double)r[i].x * (double)z.x - (double)r[i].y * (double)z.y;
+    py += (double)r[i].x * (double)z.y + (double)r[i].y * (double)z.x;
   }
   if (!rho) return;
   __shared__ double red[TAIL_THREADS / 32][2];
@@ -753,7 +943,7 @@ void coarse_pattern(afem_ctx* c) {
         axis_planes(xyz.data(), a0, a1, d, m, pls[d][sg]);
         n1 *= (long)pls[d][sg].size();
       }
-      if (nseg == 1 || n1 * 3.4 < TAIL_VALS || scale < 1e-3) break;
+      if (nseg == 1 || n1 * 4.6 < TAIL_VALS || scale < 1e-3) break;
       scale *= 0.9;
     }
     pofs[sg] = (int)planes.size();
@@ -809,11 +999,17 @@ void coarse_pattern(afem_ctx* c) {
     while (co->grids[co->tail].n > COARSE_TAIL && co->tail + 1 < co->levels[0]) ++co->tail;
   co->tail_vals = 0;
   for (int sg = 0; sg < nseg; ++sg) {
-    size_t v = co->grids[(size_t)sg * COARSE_LEVELS + co->tail].n;
-    for (int l = co->tail; l < co->levels[sg]; ++l) v += 2 * (size_t)co->grids[(size_t)sg * COARSE_LEVELS + l].n;
-    co->tail_vals = std::max(co->tail_vals, v);
+    const CoarseGrid* G = co->grids.data() + (size_t)sg * COARSE_LEVELS;
+    size_t v = G[co->tail].n, ax = 0, all;
+    for (int l = co->tail; l < co->levels[sg]; ++l) {
+      v += 3 * (size_t)G[l].n;
+      ax += G[l].nx + G[l].ny + G[l].nz;
+    }
+    if (v > TAIL_VALS || ax > TAIL_AXIS) return;  // (a grid of hundreds of planes on one axis)
+    all = v;
+    for (int l = co->tail; l < co->levels[sg]; ++l) all += 27 * (size_t)G[l].n;
+    co->tail_vals = std::max(co->tail_vals, all);
   }
-  if (co->tail_vals > TAIL_VALS) return;
   if (axw.empty()) axw.push_back(0.0);
   co->d_grids.upload(co->grids.data(), co->grids.size(), s);
   co->d_levels.upload(co->levels.data(), co->levels.size(), s);
@@ -867,10 +1063,7 @@ void coarse_values(afem_ctx* c) {
   k_support_weights<<<nblk(co->n1, 128), 128, 0, s>>>(co->n1, co->cseg.p, co->d_grids.p, co->lptr.p, co->lidx.p,
                                                       co->corner.p, co->frac.p, co->cell.p, co->lw.p);
   count_launch();
-  k_node_values3<<<nblk(32L * node, 256), 256, 0, s>>>(c->line.p, c->bc.p, node, h->nptr.p, h->nlist.p, c->rowptr.p,
-                                                       c->col.p, c->km.p, co->te.p, h->rowptr.p, h->col.p, co->n3.p);
-  count_launch();
-  k_galerkin_mesh<<<nblk(32L * co->n1, 256), 256, 0, s>>>(co->n1, co->cseg.p, co->d_grids.p, co->lptr.p, co->lidx.p,
+  k_galerkin_mesh<<<co->n1, 32 * GM_WARPS, 0, s>>>(co->cseg.p, co->d_grids.p, co->lptr.p, co->lidx.p,
                                                           co->lw.p, co->corner.p, co->frac.p, co->cell.p, h->rowptr.p,
                                                           h->col.p, h->km.p, co->n3.p, co->km.p, co->l1.p);
   count_launch();
@@ -878,7 +1071,7 @@ void coarse_values(afem_ctx* c) {
     int nmax = 1;
     for (int sg = 0; sg < co->nseg; ++sg)
       if (l + 1 < co->levels[sg]) nmax = std::max(nmax, co->grids[(size_t)sg * COARSE_LEVELS + l + 1].n);
-    k_galerkin_grid<<<dim3(nblk(32L * nmax, 256), co->nseg), 256, 0, s>>>(co->d_grids.p, co->d_levels.p, l, co->axw.p,
+    k_galerkin_grid<<<dim3(nmax, co->nseg), 128, 0, s>>>(co->d_grids.p, co->d_levels.p, l, co->axw.p,
                                                                           co->km.p, co->l1.p);
     count_launch();
   }
@@ -932,11 +1125,11 @@ const void* coarse_cycle(afem_ctx* c, const CoarseArgs& a) {
       step(std::integral_constant<int, 0>(), l, co->grids[l].n, nullptr);
       step(std::integral_constant<int, 1>(), l, co->grids[l + 1].n, nullptr);
     }
-  const size_t smem = sizeof(V) * co->tail_vals;
+  const size_t smem = std::min(TAIL_BYTES, sizeof(V) * co->tail_vals);
   auto tail = k_grid_tail<PT, NS, SEG>;
   AFEM_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   tail<<<dim3(4, SEG ? co->nseg : NS), TAIL_THREADS, smem, s>>>(
-      co->d_grids.p, co->d_levels.p, co->tail, km, co->l1.p, co->axw.p, a.omega, R, O, co->lptr.p, co->lidx.p,
+      co->d_grids.p, co->d_levels.p, co->tail, (int)(smem / sizeof(V)), km, co->l1.p, co->axw.p, a.omega, R, O, co->lptr.p, co->lidx.p,
       co->lw.p, t, a.done, co->tail == 0 ? a.rho : nullptr);
   count_launch();
   if constexpr (!SEG)

@@ -310,6 +310,7 @@ struct SolveExtra {
   const double* x0 = nullptr;   // initial guess, [row][system] interleaved complex (host)
   bool recursive_only = false;  // stop on the recursive residual, no refinement (COCG13_single)
   const double* rhs = nullptr;  // caller right-hand sides, [row][system] interleaved complex (host)
+  double margin = 1.0;          // the recursive residual goes to this fraction of its target
 };
 int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, const afem_solve_opts* o,
                  afem_solve_stats* st, const SolveExtra* ex = nullptr);

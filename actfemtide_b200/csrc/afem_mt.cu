@@ -885,7 +885,11 @@ int mt_forward_device(afem_ctx* c, const afem_mt_cond* cond, int nfreq, const do
     std::vector<int> src(ns);
     for (int k = 0; k < ns; ++k) src[k] = k0 + k;
     afem_solve_stats sk{};
-    const int rc = solve_device(c, ns, fs.data() + k0, src.data(), o, &sk, nullptr);
+    // the phases of the small impedances (a hundredth of the others) magnify what the residual leaves: the
+    // recursion goes ten times further, about five of 115 iterations (phases 1e-9 off at 3e-12 before)
+    SolveExtra ex;
+    ex.margin = 0.1;
+    const int rc = solve_device(c, ns, fs.data() + k0, src.data(), o, &sk, &ex);
     if (rc != AFEM_OK && status == AFEM_OK) status = rc;
     its += sk.iterations;
     refs += sk.refinements;

@@ -1607,9 +1607,10 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
 //   k_pupd:        x += alpha p, p = z + (correction of w) + beta p;
 //   k_spmv:        q = A p, p^T q -> alpha.
 // The scalar steps run in the last block of the kernel that produced their sums.
-constexpr double CHEB_SAFETY = 1.15;  // on the power iteration's estimate of the largest eigenvalue
+constexpr double CHEB_SAFETY = 1.25;  // on the power iteration's estimate of the largest eigenvalue (0.79 of it
+                                      // after four steps on Kuhn meshes, from below)
 constexpr double CHEB_RATIO = 8.0;    // the smoothed interval is [b / 8, b]
-constexpr int CHEB_POWER = 8;         // steps of the power iteration
+constexpr int CHEB_POWER = 4;         // steps of the power iteration
 // The smoothed iteration's recursive residual goes to this fraction of the tolerance before the true
 // residual is judged.  At the same residual its error is spread differently from the sweeps': the
 // phases of an MT model's small impedances were 2 to 12e-10 off where the sweeps left 3 to 4e-10
@@ -3400,7 +3401,7 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
     // residual relative to ||r64||; ask for the reduction still missing,
     // never below what FP32 can deliver in the mixed mode.
     double inner_tol = std::min(0.5, 0.5 * tol / prev);
-    if (outer == 0) inner_tol = tol * tol_scale * (smoothed(c, w, precond_now) ? SMOOTH_MARGIN : 1.0);
+    if (outer == 0) inner_tol = tol * tol_scale * (smoothed(c, w, precond_now) ? SMOOTH_MARGIN * (ex ? ex->margin : 1.0) : 1.0);
     if (mixed) inner_tol = std::max(inner_tol, o->inner_tol > 0 ? o->inner_tol : 1e-5);
     const int left = maxit - it_total;
     if (left <= 0) break;
