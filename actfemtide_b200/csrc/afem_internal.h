@@ -89,6 +89,7 @@ struct DevStatus {
 
 // ---------------------------------------------------------------- limits
 constexpr int ROW_MAX = 64;      // maximum nonzeros of one matrix row (diagonal included)
+constexpr int SWEEP_ROWS = 20480; // rows up to which the natural-order sweeps may run in one block
 constexpr int EDGE_DEG_MAX = 64; // maximum tetrahedra sharing one edge
 constexpr int NODE_DEG_MAX = 100;// maximum tetrahedra sharing one node (MKLINE_V2 maxnele)
 constexpr int NODE_NBR_MAX = 128;// maximum edges leaving one node towards larger ids
@@ -198,6 +199,8 @@ struct afem_ctx {
   afem::DBuf<int32_t> perm_f;   // forward sweep: lower-triangle levels ascending, ties by row
   afem::DBuf<int32_t> perm_b;   // backward sweep: upper-triangle levels ascending, ties by row descending
   int levels_f = 0, levels_b = 0;
+  afem::DBuf<int32_t> lev_f, lev_b;  // positions at which the levels begin, levels + 1 values
+  afem::DBuf<int4> rows_f, rows_b;   // per position: row, range of its lower / upper entries (small systems)
   // multicolour sweeps: greedy colouring, rows sorted by colour
   afem::DBuf<uint8_t> color;    // nline
   afem::DBuf<int32_t> perm_mc;  // nline

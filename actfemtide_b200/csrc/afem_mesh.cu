@@ -348,9 +348,10 @@ void build_pattern_device(afem_ctx* c) {
 // unchanged, only the order in which rows are visited; a row's dependencies
 // always have a smaller level, so the order is topological.
 void compute_schedule(int n, const int32_t* rp, const int32_t* dp, const int32_t* cl, int32_t* perm_f,
-                      int32_t* perm_b, int* levels_f, int* levels_b) {
+                      int32_t* perm_b, int* levels_f, int* levels_b, std::vector<int32_t>* off_f = nullptr,
+                      std::vector<int32_t>* off_b = nullptr) {
   std::vector<int32_t> lev(n);
-  auto order = [&](bool forward, int32_t* perm, int* nlev) {
+  auto order = [&](bool forward, int32_t* perm, int* nlev, std::vector<int32_t>* off) {
     int mx = 0;
     if (forward) {
       for (int i = 0; i < n; ++i) {
@@ -371,14 +372,15 @@ void compute_schedule(int n, const int32_t* rp, const int32_t* dp, const int32_t
     std::vector<int32_t> cnt(mx + 2, 0);
     for (int i = 0; i < n; ++i) cnt[lev[i] + 1]++;
     for (int l = 0; l <= mx; ++l) cnt[l + 1] += cnt[l];
+    if (off) off->assign(cnt.begin(), cnt.begin() + *nlev + 1);  // level l: positions off[l] .. off[l+1]
     if (forward) {
       for (int i = 0; i < n; ++i) perm[cnt[lev[i]]++] = i;
     } else {
       for (int i = n - 1; i >= 0; --i) perm[cnt[lev[i]]++] = i;
     }
   };
-  order(true, perm_f, levels_f);
-  order(false, perm_b, levels_b);
+  order(true, perm_f, levels_f, off_f);
+  order(false, perm_b, levels_b, off_b);
 }
 
 // Greedy distance-1 colouring of the matrix graph in row order (each row takes
@@ -492,7 +494,19 @@ void build_schedule(afem_ctx* c, bool levels, bool colours) {
     std::vector<int32_t> pf(n), pb(n), dp(n);
     c->diagpos.download(dp.data(), n, s);
     AFEM_CUDA(cudaStreamSynchronize(s));
-    compute_schedule(n, rp.get(), dp.data(), cl.get(), pf.data(), pb.data(), &c->levels_f, &c->levels_b);
+    std::vector<int32_t> of, ob;
+    compute_schedule(n, rp.get(), dp.data(), cl.get(), pf.data(), pb.data(), &c->levels_f, &c->levels_b, &of, &ob);
+    c->lev_f.upload(of.data(), of.size(), s);
+    c->lev_b.upload(ob.data(), ob.size(), s);
+    std::vector<int4> rf, rb;
+    if (n <= SWEEP_ROWS) {
+      for (int i = 0; i < n; ++i) {
+        rf.push_back(make_int4(pf[i], rp[pf[i]], dp[pf[i]], 0));
+        rb.push_back(make_int4(pb[i], dp[pb[i]] + 1, rp[pb[i] + 1], 0));
+      }
+      c->rows_f.upload(rf.data(), n, s);
+      c->rows_b.upload(rb.data(), n, s);
+    }
     c->perm_f.upload(pf.data(), n, s);
     c->perm_b.upload(pb.data(), n, s);
     AFEM_CUDA(cudaStreamSynchronize(s));

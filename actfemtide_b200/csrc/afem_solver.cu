@@ -485,6 +485,120 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// ------------------------------------------------------------------ natural-order sweeps of small systems
+// The triangular sweep of k_fwd / k_bwd alone, for a system whose vector fits the shared memory of one
+// block: the rows of a dependency level are swept side by side (a warp per row, the lanes and sums of
+// k_fwd) and a block barrier parts the levels.  The sync-free sweeps pass every level through L2 flags
+// and polls, 6 us a level on 878 rows (380 us a sweep of 61 levels); here a level costs a barrier, the
+// arithmetic's latency and part of a load's, 1 us (60 us a sweep): a warp's rows come through a
+// pipeline, the range of the row after next and the entries of the next row on their way while a row is
+// swept.  (Entries by asynchronous copies into shared memory were no faster: 70 us.)  k_fwd and k_bwd still
+// run without their sweep (mode 3) for the updates and the partial sums, so a solve gives the same
+// bits by either path.
+constexpr int SWEEP_THREADS = 1024;
+constexpr int SWEEP_LEVELS = 12000;
+constexpr int SWEEP_BYTES = SWEEP_ROWS * 8;  // 160 KB: the vector (the levels' offsets come on top)
+
+template <class T, int NS, bool BWD>
+__global__ void __launch_bounds__(SWEEP_THREADS)
+    k_sweep_block(const int4* __restrict__ rows, const int32_t* __restrict__ col,
+                  const typename Cx<T>::V* __restrict__ km, int n, const typename Cx<T>::V* __restrict__ r,
+                  typename Cx<T>::V* __restrict__ y, const typename Cx<T>::V* __restrict__ dd,
+                  const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const int32_t* __restrict__ lev,
+                  int nlev) {
+  using V = typename Cx<T>::V;
+  if (ctrl->done) return;
+  constexpr int G = 32 / NS, NW = SWEEP_THREADS / 32;
+  extern __shared__ double2 sweep_smem[];
+  V* sv = reinterpret_cast<V*>(sweep_smem);           // y (forward) or z (backward), [row][system]
+  int* off = reinterpret_cast<int*>(sv + (long)n * NS);  // level l: positions off[l] .. off[l + 1]
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, s = lane % NS, g = lane / NS;
+  const T om = (T)sc[s].omega;
+  for (int i = threadIdx.x; i <= nlev; i += SWEEP_THREADS) off[i] = lev[i];
+  if constexpr (BWD)
+    for (int i = threadIdx.x; i < n * NS; i += SWEEP_THREADS) sv[i] = y[i];
+  __syncthreads();
+  // the warp's rows: position and level of the row whose range is fetched next
+  int pos = w, pl = 0;
+  auto settle = [&]() {
+    while (pl < nlev && pos >= off[pl + 1])
+      if (++pl < nlev) pos = off[pl] + w;
+  };
+  struct Row {
+    int row, k0, k1, level;
+  };
+  auto range = [&]() {
+    Row m{0, 0, 0, nlev};
+    if (pl < nlev) {
+      const int4 v = __ldg(rows + pos);
+      m = Row{v.x, v.y, v.z, pl};
+      pos += NW;
+      settle();
+    }
+    return m;
+  };
+  int j0 = 0;
+  V rv = Cx<T>::make(0, 0), dv = rv, a0 = rv;
+  auto entries = [&](const Row& m) {
+    if (m.level >= nlev) return;
+    if (g == 0) {
+      if constexpr (!BWD) rv = r[(long)m.row * NS + s];
+      dv = dd[(long)m.row * NS + s];
+    }
+    if (m.k0 + g < m.k1) {
+      j0 = __ldg(col + m.k0 + g);
+      a0 = km[m.k0 + g];
+    }
+  };
+  settle();
+  Row cur = range(), nxt = range();
+  entries(cur);
+  for (int l = 0; l < nlev; ++l) {
+    while (cur.level == l) {
+      const Row m = cur;
+      const int j = j0, len = m.k1 - m.k0;
+      const V a = a0, ri = rv, di = dv;
+      cur = nxt;
+      entries(cur);
+      nxt = range();
+      T t1x = 0, t1y = 0, t2x = 0, t2y = 0;
+      if (g < len) {
+        const V v = sv[(long)j * NS + s];
+        t1x += a.x * v.x; t1y += a.x * v.y;
+        t2x += a.y * v.x; t2y += a.y * v.y;
+      }
+      for (int k = m.k0 + g + G; k < m.k1; k += G) {
+        const V b = km[k], v = sv[(long)__ldg(col + k) * NS + s];
+        t1x += b.x * v.x; t1y += b.x * v.y;
+        t2x += b.y * v.x; t2y += b.y * v.y;
+      }
+      // group_reduce; the lanes past the row's entries hold zeros
+#pragma unroll
+      for (int q = NS; q < 32; q <<= 1)
+        if (q / NS < len) {
+          t1x += shfl_xor(t1x, q);
+          t1y += shfl_xor(t1y, q);
+          t2x += shfl_xor(t2x, q);
+          t2y += shfl_xor(t2y, q);
+        }
+      if (g == 0) {
+        const T ax = t1x - om * t2y, ay = t1y + om * t2x;
+        V o;
+        if constexpr (!BWD) {
+          const T wx = ri.x - ax, wy = ri.y - ay;
+          o = Cx<T>::make(wx * di.x - wy * di.y, wx * di.y + wy * di.x);
+        } else {
+          const V zi = sv[(long)m.row * NS + s];
+          o = Cx<T>::make(zi.x - (di.x * ax - di.y * ay), zi.y - (di.x * ay + di.y * ax));
+        }
+        sv[(long)m.row * NS + s] = o;
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < n * NS; i += SWEEP_THREADS) y[i] = sv[i];
+}
+
 // ------------------------------------------------------------------ multicolour sweeps
 // SSOR of the colour-permuted matrix: rows of one colour share no nonzero, so
 // the forward sweep updates colour 0, 1, ... in turn (each a parallel pass over
@@ -2699,6 +2813,27 @@ int tune_spmv(afem_ctx* c, SolverWork* w) {
   return pick;
 }
 
+// Whether the natural-order sweeps run in one block (k_sweep_block): the vector fits its shared memory.
+template <class T, int NS, bool SEG>
+bool block_sweeps(const afem_ctx* c, const SolverWork* w, int mode) {
+  return !SEG && mode <= AFEM_PRECOND_SSOR && (long)w->n * NS * (long)sizeof(typename Cx<T>::V) <= SWEEP_BYTES &&
+         std::max(c->levels_f, c->levels_b) < SWEEP_LEVELS;
+}
+
+template <class T, int NS, bool BWD>
+void launch_sweep_block(afem_ctx* c, SolverWork* w) {
+  using I = Inner<T, NS>;
+  using V = typename I::V;
+  auto k = k_sweep_block<T, NS, BWD>;
+  const int nlev = BWD ? c->levels_b : c->levels_f;
+  const int smem = (int)(sizeof(V) * w->n * NS + sizeof(int) * (nlev + 1));
+  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k<<<1, SWEEP_THREADS, smem, c->stream>>>(BWD ? c->rows_b.p : c->rows_f.p, c->col.p, I::KM(c, w), w->n,
+                                           (const V*)I::R(w), I::Z(w), (const V*)I::DD(w), w->sc.p, w->ctrl.p,
+                                           BWD ? c->lev_b.p : c->lev_f.p, nlev);
+  count_launch();
+}
+
 // One COCG iteration (7 launches; the learned preconditioner adds the network's 8).
 // T: COCG vectors and the SpMV; PT: the multicolour preconditioner (its matrix
 // copies and vectors); PT differs from T only on the multicolour path.
@@ -2723,6 +2858,7 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   // hybrid alone (one matrix): z + G u is formed inside the p update, and the
   // backward nodal sweep sums t^T u, the nodal share of rho
   const bool fold_grad = hyb && !lbase && !SEG;
+  const bool small = same && block_sweeps<T, NS, SEG>(c, w, mode);  // the sweeps proper in one block
   if (ev) AFEM_CUDA(cudaEventRecord(ev[0], s));
   if (mc) {  // the multicolour sweep updates r only: x += alpha p moves to the p update
     launch_coop(k_fwd_mc<T, PT, NS, SEG>, w->mc_blocks, s, (const int32_t*)c->mc_lptr.p,
@@ -2732,8 +2868,10 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   } else if constexpr (same) {
     launch_coop(k_fwd<T, NS, SEG>, sweep_blocks, s, (const int32_t*)c->rowptr.p, (const int32_t*)c->col.p,
                 (const int32_t*)c->diagpos.p, I::KM(c, w), n, I::R(w), I::Z(w), (const V*)I::P(w), (const V*)I::Q(w),
-                w->x.p, (const V*)I::DD(w), w->flag_f.p, mode, w->sc.p, w->ctrl.p, w->part.p, c->status.p, rp,
-                (const int32_t*)c->perm_f.p, sg);
+                w->x.p, (const V*)I::DD(w), w->flag_f.p, small ? (int)AFEM_PRECOND_NONE : mode, w->sc.p, w->ctrl.p,
+                w->part.p, c->status.p, rp, (const int32_t*)c->perm_f.p, sg);
+    if constexpr (!SEG)
+      if (small) launch_sweep_block<T, NS, false>(c, w);
   }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[1], s));
   const int swb = mc ? w->mc_blocks : sweep_blocks;
@@ -2749,9 +2887,11 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
                 (const int32_t*)c->perm_mc.p, (const int32_t*)c->color_ptr.p, c->ncolors, w->sc.p, w->ctrl.p,
                 w->part.p, sg, (const double2*)c->mc_dkm.p, w->sd);
   } else if constexpr (same) {
+    if constexpr (!SEG)
+      if (small) launch_sweep_block<T, NS, true>(c, w);
     launch_coop(k_bwd<T, NS, SEG>, sweep_blocks, s, (const int32_t*)c->rowptr.p, (const int32_t*)c->col.p,
                 (const int32_t*)c->diagpos.p, I::KM(c, w), n, (const V*)I::R(w), I::Z(w), (const V*)I::DD(w),
-                w->flag_b.p, mode, w->sc.p, w->ctrl.p, w->part.p, c->status.p, (const V*)rp,
+                w->flag_b.p, small ? (int)AFEM_PRECOND_NONE : mode, w->sc.p, w->ctrl.p, w->part.p, c->status.p, (const V*)rp,
                 (const int32_t*)c->perm_b.p, sg);
   }
   if (ev) AFEM_CUDA(cudaEventRecord(ev[3], s));
