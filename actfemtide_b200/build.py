@@ -21,7 +21,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 NOFMA = {"afem_assemble.cu", "afem_sites.cu", "afem_adjoint.cu", "afem_mt.cu"}
 SOURCES = ["afem_capi.cu", "afem_mesh.cu", "afem_assemble.cu", "afem_solver.cu", "afem_sites.cu", "afem_mpnn.cu",
            "afem_adjoint.cu", "afem_hybrid.cu", "afem_coarse.cu", "afem_mt.cu", "afem_io.cpp"]
-HEADERS = ["afem_internal.h", "afem_hybrid.h", "afem_reduce.cuh", os.path.join("..", "..", "include", "afem.h")]
+HEADERS = ["afem_internal.h", "afem_hybrid.h", "afem_reduce.cuh", "afem_coarse.cuh", os.path.join("..", "..", "include", "afem.h")]
 
 
 def _stale(target, deps):

@@ -74,11 +74,34 @@ __device__ __forceinline__ bool reduce_blocks(const RedSet& R, int bid, int nblk
   return true;
 }
 
+// The same sums by every block for itself, after a grid barrier: out[s] for s < nsys in shared memory.
+// (For grids of a few hundred blocks at most: each block reads all parts.)
+__device__ __forceinline__ void sum_blocks(const RedSet& R, int nblk, int nsys, double2* out) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int s = threadIdx.x >> 5; s < nsys; s += nw) {
+    double2 v = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int b = lane; b < nblk; b += 32) {
+      const double2 u = __ldcg(R.part + (long)s * R.rows + b);
+      v.x += u.x;
+      v.y += u.y;
+    }
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, m);
+      v.y += __shfl_xor_sync(0xffffffffu, v.y, m);
+    }
+    if (lane == 0) out[s] = v;
+  }
+  __syncthreads();
+}
+
 // The block's part from lanes that carry systems s0 .. s0 + SPL - 1 of a row of LPR lanes (values
 // zero on lanes that do not count): rows of a warp are folded by shuffles, warps in order.
+// buf: shared memory, NS values per warp of the block.
 template <int NS, int SPL, int LPR>
-__device__ __forceinline__ void block_pair(double (&v)[SPL][2], int s0, bool lead, const RedSet& R, int bid) {
-  __shared__ double2 red[32][NS];
+__device__ __forceinline__ void block_pair(double (&v)[SPL][2], int s0, bool lead, const RedSet& R, int bid,
+                                           double2* buf) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 #pragma unroll
   for (int m = LPR; m < 32; m <<= 1)
@@ -89,13 +112,13 @@ __device__ __forceinline__ void block_pair(double (&v)[SPL][2], int s0, bool lea
     }
   if (lane < LPR && lead)
 #pragma unroll
-    for (int i = 0; i < SPL; ++i) red[w][s0 + i] = make_double2(v[i][0], v[i][1]);
+    for (int i = 0; i < SPL; ++i) buf[w * NS + s0 + i] = make_double2(v[i][0], v[i][1]);
   __syncthreads();
   if (threadIdx.x < NS) {
     double2 a = make_double2(0.0, 0.0);
     for (int k = 0; k < nw; ++k) {
-      a.x += red[k][threadIdx.x].x;
-      a.y += red[k][threadIdx.x].y;
+      a.x += buf[k * NS + threadIdx.x].x;
+      a.y += buf[k * NS + threadIdx.x].y;
     }
     R.part[(long)threadIdx.x * R.rows + bid] = a;
   }

@@ -32,6 +32,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "afem_coarse.cuh"
 #include "afem_hybrid.h"
 #include "afem_internal.h"
 #include "afem_reduce.cuh"
@@ -1386,11 +1387,11 @@ __device__ __forceinline__ void finish_r(SysScal* sc, Ctrl* ctrl, const double2*
 
 // rho = r^T z from the edges', the nodes' and the grids' shares -> beta;
 __device__ __forceinline__ void finish_rho(SysScal* sc, const Ctrl* ctrl, const double2* v, const double2* edge,
-                                           const double2* grid, int nsys) {
+                                           const double2* grid, int ld, int nsys) {
   if (threadIdx.x >= nsys) return;
   SysScal& S = sc[threadIdx.x];
-  double2 a = cadd(v[threadIdx.x], __ldcg(edge + threadIdx.x));
-  for (int c = 0; c < 4; ++c) a = cadd(a, __ldcg(grid + c * MAX_SYS + threadIdx.x));
+  double2 a = cadd(v[threadIdx.x], edge[threadIdx.x]);
+  for (int c = 0; c < 4; ++c) a = cadd(a, grid[c * ld + threadIdx.x]);
   S.rho = a;
   if (S.active) {
     if (a.x == 0.0 && a.y == 0.0) { S.active = 0; S.status = AFEM_EBREAKDOWN; }
@@ -1448,24 +1449,15 @@ __device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restric
 // solve).  Hybrid preconditioner with the nodal part folded in (u != nullptr):
 // z_e + the nodal correction (nodal_term) on the non-Dirichlet edges stands for z.
 // (p in the COCG type T; z and u in the preconditioner type PT)
-template <class T, class PT, int NS, bool SEG = false>
-__global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
-                       const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg,
-                       double2* __restrict__ x, int nsys, const int32_t* __restrict__ line,
-                       const uint8_t* __restrict__ bc, const typename Cx<PT>::V* __restrict__ u,
-                       const double* __restrict__ te) {
+template <class T, class PT, int NS, bool SEG>
+__device__ __forceinline__ void pupd(int n, const typename Cx<PT>::V* z, typename Cx<T>::V* p, const SysScal* sc,
+                                     bool done, bool first, const uint8_t* seg, double2* x,
+                                     const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
+                                     const typename Cx<PT>::V* u, const double* __restrict__ te, int bid, int nb) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
-  const bool done = ctrl->done;
-  if (done) {
-    if (!x) return;
-    bool any = false;
-    for (int k = 0; k < nsys; ++k) any |= sc[k].xpend != 0;
-    if (!any) return;
-  }
-  const bool first = ctrl->iter == 0;
   const long total = (long)n * NS;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+  for (long i = bid * (long)blockDim.x + threadIdx.x; i < total; i += (long)nb * blockDim.x) {
     const int s = SEG ? (int)__ldg(seg + i) : (int)(i % NS);
     V pi = Cx<T>::make(0, 0);
     bool have_p = false;
@@ -1499,19 +1491,12 @@ __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename
   }
 }
 
-// k_pupd for 16 systems sharing a matrix: a thread takes 2 consecutive systems of
-// one row, so the 8 threads of a row read and write its FP64 values (p, x) as one
-// 256-byte run of 32-byte accesses and its FP32 values (z, u) as one 128-byte run
-// of 16-byte accesses; the systems' scalars stay in registers.  The grid-stride is
-// a multiple of 8, so a thread keeps the same 2 systems throughout.
-template <class T, class PT, int NS>
-__global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
-                           const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, double2* __restrict__ x,
-                           int nsys, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
-                           const typename Cx<PT>::V* __restrict__ u, const double* __restrict__ te) {
-  using V = typename Cx<T>::V;
-  using PV = typename Cx<PT>::V;
-  constexpr int SP = 2, GPR = NS / SP;  // systems per thread, threads per row
+template <class T, class PT, int NS, bool SEG = false>
+__global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
+                       const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg,
+                       double2* __restrict__ x, int nsys, const int32_t* __restrict__ line,
+                       const uint8_t* __restrict__ bc, const typename Cx<PT>::V* __restrict__ u,
+                       const double* __restrict__ te) {
   const bool done = ctrl->done;
   if (done) {
     if (!x) return;
@@ -1519,10 +1504,25 @@ __global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, type
     for (int k = 0; k < nsys; ++k) any |= sc[k].xpend != 0;
     if (!any) return;
   }
-  const bool first = ctrl->iter == 0;
+  pupd<T, PT, NS, SEG>(n, z, p, sc, done, ctrl->iter == 0, seg, x, line, bc, u, te, blockIdx.x, gridDim.x);
+}
+
+// k_pupd for 16 systems sharing a matrix: a thread takes 2 consecutive systems of
+// one row, so the 8 threads of a row read and write its FP64 values (p, x) as one
+// 256-byte run of 32-byte accesses and its FP32 values (z, u) as one 128-byte run
+// of 16-byte accesses; the systems' scalars stay in registers.  The grid-stride is
+// a multiple of 8, so a thread keeps the same 2 systems throughout.
+template <class T, class PT, int NS>
+__device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typename Cx<T>::V* p, const SysScal* sc,
+                                         bool done, bool first, double2* x, const int32_t* __restrict__ line,
+                                         const uint8_t* __restrict__ bc, const typename Cx<PT>::V* u,
+                                         const double* __restrict__ te, int bid, int nb) {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  constexpr int SP = 2, GPR = NS / SP;  // systems per thread, threads per row
   const long total = (long)n * GPR;
-  const long stride = (long)gridDim.x * blockDim.x;
-  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long stride = (long)nb * blockDim.x;
+  const long i0 = bid * (long)blockDim.x + threadIdx.x;
   const int s0 = (int)(i0 % GPR) * SP;
   double2 al[SP], be[SP];
   bool xp[SP], anyx = false;
@@ -1591,6 +1591,21 @@ __global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, type
       store_spl<V, SP>(p + base, po);
     }
   }
+}
+
+template <class T, class PT, int NS>
+__global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
+                           const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, double2* __restrict__ x,
+                           int nsys, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
+                           const typename Cx<PT>::V* __restrict__ u, const double* __restrict__ te) {
+  const bool done = ctrl->done;
+  if (done) {
+    if (!x) return;
+    bool any = false;
+    for (int k = 0; k < nsys; ++k) any |= sc[k].xpend != 0;
+    if (!any) return;
+  }
+  pupd_spl<T, PT, NS>(n, z, p, sc, done, ctrl->iter == 0, x, line, bc, u, te, blockIdx.x, gridDim.x);
 }
 
 // q = A p (COCG13_single.f90:273-288) and p^T q partial sums.  With
@@ -1696,7 +1711,8 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
       pq[i][0] = acc[i][0];
       pq[i][1] = acc[i][1];
     }
-    block_pair<NS, SPL, LPR>(pq, s0, g == 0, R, blockIdx.x);
+    __shared__ double2 buf[8 * NS];
+    block_pair<NS, SPL, LPR>(pq, s0, g == 0, R, blockIdx.x, buf);
   }
   if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
     finish_pq(const_cast<SysScal*>(sc), const_cast<Ctrl*>(ctrl), sums, nsys);
@@ -1753,21 +1769,14 @@ struct NdShape {
 // systems of a row (one 32-byte access in FP64); the grid's stride is a multiple of the threads per
 // row, so a thread keeps its systems.
 template <class T, class PT, int NS, bool SEG>
-__global__ void __launch_bounds__(256)
-    k_r_update(int n, typename Cx<T>::V* __restrict__ r, const typename Cx<T>::V* __restrict__ q,
-               typename Cx<PT>::V* __restrict__ s, const double2* __restrict__ dkm, SysScal* sc, Ctrl* ctrl,
-               const uint8_t* __restrict__ seg, RedSet R, int nsys) {
+__device__ __forceinline__ void r_update(int n, typename Cx<T>::V* r, const typename Cx<T>::V* q,
+                                         typename Cx<PT>::V* s, const double2* dkm, const SysScal* sc, bool update,
+                                         const uint8_t* seg, const RedSet& R, int bid, int nb, double2* buf) {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   constexpr int SP = NS >= 2 ? 2 : 1, GPR = NS / SP;
-  if (ctrl->done) {
-    // the x update pending when the solve ended was applied by that iteration's p update
-    if (blockIdx.x == 0 && threadIdx.x < nsys) sc[threadIdx.x].xpend = 0;
-    return;
-  }
-  const bool update = ctrl->iter > 0;
-  const long total = (long)n * GPR, stride = (long)gridDim.x * blockDim.x;
-  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long total = (long)n * GPR, stride = (long)nb * blockDim.x;
+  const long i0 = bid * (long)blockDim.x + threadIdx.x;
   const int s0 = SEG ? 0 : (int)(i0 % GPR) * SP;
   double2 al[SP];
   double om[SP], rr[SP][2];
@@ -1826,15 +1835,170 @@ __global__ void __launch_bounds__(256)
       seg_warp_sum<1>(red, threadIdx.x >> 5, sid, v);
     }
   }
-  __shared__ double2 sums[MAX_SYS];
-  if constexpr (SEG) seg_pair<8, 1>(red, R, blockIdx.x);
-  else block_pair<NS, SP, GPR>(rr, s0, true, R, blockIdx.x);
+  if constexpr (SEG) seg_pair<8, 1>(red, R, bid);
+  else block_pair<NS, SP, GPR>(rr, s0, true, R, bid, buf);
+}
+
+template <class T, class PT, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_r_update(int n, typename Cx<T>::V* __restrict__ r, const typename Cx<T>::V* __restrict__ q,
+               typename Cx<PT>::V* __restrict__ s, const double2* __restrict__ dkm, SysScal* sc, Ctrl* ctrl,
+               const uint8_t* __restrict__ seg, RedSet R, int nsys) {
+  if (ctrl->done) {
+    // the x update pending when the solve ended was applied by that iteration's p update
+    if (blockIdx.x == 0 && threadIdx.x < nsys) sc[threadIdx.x].xpend = 0;
+    return;
+  }
+  __shared__ double2 sums[MAX_SYS], buf[8 * NS];
+  r_update<T, PT, NS, SEG>(n, r, q, s, dkm, sc, ctrl->iter > 0, seg, R, blockIdx.x, gridDim.x, buf);
   if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_r(sc, ctrl, sums, nsys);
 }
 
-// Blocks below nbe: z = c1 s - c2 D^-1 A s by rows, and the edges' share r^T z of rho.  The others:
-// the mesh nodes' right-hand sides t = (G^T r, Pi_x^T r, Pi_y^T r, Pi_z^T r) over the non-Dirichlet
-// edges of a node, and hs = D_G^-1 t_0.  Neither reads what the other writes.
+// z = c1 s - c2 D^-1 A s by rows, and the edges' share r^T z of rho.  (RO: nothing of what is read is
+// written during the launch, see ld_v4d; bid of nb blocks take part.)
+template <class T, class PT, int NS, bool SEG, bool RO>
+__device__ __forceinline__ void smooth_edges(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                                             const typename Cx<PT>::V* __restrict__ km, int n,
+                                             const typename Cx<PT>::V* sv, const typename Cx<T>::V* r,
+                                             typename Cx<PT>::V* z, const double2* dkm, const double* coef,
+                                             const SysScal* sc, const uint8_t* seg, int ch, const RedSet& R, int bid,
+                                             int nb, double2* buf) {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double (*red)[MAX_SYS][2] = nullptr;
+  if constexpr (SEG) red = seg_sums<32, 2>();
+  using S = SmShape<NS, SEG>;
+  constexpr int SPL = S::SPL;
+  const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+  const PT c1 = (PT)coef[0], c2 = (PT)coef[1];
+  double om[SPL], acc[SPL][2];
+#pragma unroll
+  for (int i = 0; i < SPL; ++i) {
+    om[i] = sc[s0 + i].omega;
+    acc[i][0] = acc[i][1] = 0.0;
+  }
+  int nk0 = 0, nk1 = 0;
+  {
+    const int first = bid * ch * (int)(blockDim.x >> 5) * S::RPW + w * S::RPW + sub;
+    if (first < n) { nk0 = __ldg(rowptr + first); nk1 = __ldg(rowptr + first + 1); }
+  }
+  for_rows<S::RPW>(0, n, ch, [&](int row0, int cend, int next) {
+    const int row = row0 + sub;
+    const bool live = row < cend;
+    int sid = 0;
+    if constexpr (SEG) {
+      sid = live ? (int)__ldg(seg + row) : 0;
+      om[0] = sc[sid].omega;
+    }
+    const int k0 = live ? nk0 : 0, k1 = live ? nk1 : 0;
+    if (next >= 0 && next + sub < n) { nk0 = __ldg(rowptr + next + sub); nk1 = __ldg(rowptr + next + sub + 1); }
+    PT t1x[SPL], t1y[SPL], t2x[SPL], t2y[SPL];
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) t1x[i] = t1y[i] = t2x[i] = t2y[i] = 0;
+    row_gather_spl<PT, NS, S::G, SPL, RO>(col, km, sv, k0 + g, k1, s0, t1x, t1y, t2x, t2y);
+    group_sum<PT, SPL, S::NG, S::LPR>(t1x, t1y, t2x, t2y);
+    if (g == 0 && live) {
+      const long base = (long)row * NS + s0;
+      const double2 dg = __ldg(dkm + row);
+      PV si[SPL], zo[SPL];
+      V ri[SPL];
+      load_spl<PV, NS, SPL, false, RO>(sv + base, si);
+      load_spl<V, NS, SPL, false, RO>(r + base, ri);
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        const PT o = (PT)om[i];
+        const PT ax = t1x[i] - o * t2y[i], ay = t1y[i] + o * t2x[i];
+        const double2 dd = ssor_dd(dg, om[i], 1.0);
+        const PT dx = (PT)dd.x, dy = (PT)dd.y;
+        zo[i] = Cx<PT>::make(c1 * si[i].x - c2 * (ax * dx - ay * dy), c1 * si[i].y - c2 * (ax * dy + ay * dx));
+        const double e0 = (double)ri[i].x * (double)zo[i].x - (double)ri[i].y * (double)zo[i].y;
+        const double e1 = (double)ri[i].x * (double)zo[i].y + (double)ri[i].y * (double)zo[i].x;
+        if constexpr (SEG) {
+          red[w * 4 + sub][sid][0] += e0;
+          red[w * 4 + sub][sid][1] += e1;
+        } else {
+          acc[i][0] += e0;
+          acc[i][1] += e1;
+        }
+      }
+      store_spl<PV, SPL>(z + base, zo);
+    }
+  }, bid, nb);
+  if constexpr (SEG) seg_pair<32, 2>(red, R, bid);
+  else block_pair<NS, SPL, S::LPR>(acc, s0, g == 0, R, bid, buf);
+}
+
+// The mesh nodes' right-hand sides t = (G^T r, Pi_x^T r, Pi_y^T r, Pi_z^T r) over the non-Dirichlet
+// edges of a node, and hs = D_G^-1 t_0.
+template <class T, class PT, int NS, bool RO>
+__device__ __forceinline__ void restrict_nodes(int node, const int32_t* __restrict__ nptr,
+                                               const int32_t* __restrict__ nlist, const uint8_t* __restrict__ bc,
+                                               const double* __restrict__ te, const typename Cx<PT>::V* hdd,
+                                               const typename Cx<T>::V* r, typename Cx<PT>::V* t,
+                                               typename Cx<PT>::V* hs, int bid, int nb) {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  using S = NdShape<NS>;
+  constexpr int SPL = S::SPL;
+  const int sub = lane >> 3, ql = lane & 7, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+  const int nw = blockDim.x >> 5;
+  for (int a0 = (bid * nw + w) * 4; a0 < node; a0 += nb * nw * 4) {
+    const int a = a0 + sub;
+    const bool live = a < node;
+    T v[4][SPL][2];
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) v[d][i][0] = v[d][i][1] = 0;
+    const int q1 = live ? __ldg(nptr + a + 1) : 0;
+    for (int k = (live ? __ldg(nptr + a) : 0) + g; k < q1; k += S::G) {
+      const int ent = __ldg(nlist + k), e = ent >> 1;
+      if (__ldg(bc + e)) continue;
+      V re[SPL];
+      load_spl<V, NS, SPL, false, RO>(r + (long)e * NS + s0, re);
+      const T sg = (ent & 1) ? (T)-1 : (T)1;
+      const T hx = (T)(0.5 * __ldg(te + 3L * e)), hy = (T)(0.5 * __ldg(te + 3L * e + 1)),
+              hz = (T)(0.5 * __ldg(te + 3L * e + 2));
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        v[0][i][0] += sg * re[i].x; v[0][i][1] += sg * re[i].y;
+        v[1][i][0] += hx * re[i].x; v[1][i][1] += hx * re[i].y;
+        v[2][i][0] += hy * re[i].x; v[2][i][1] += hy * re[i].y;
+        v[3][i][0] += hz * re[i].x; v[3][i][1] += hz * re[i].y;
+      }
+    }
+#pragma unroll
+    for (int m = S::NG; m < 8; m <<= 1)
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) {
+          v[d][i][0] += shfl_xor(v[d][i][0], m);
+          v[d][i][1] += shfl_xor(v[d][i][1], m);
+        }
+    if (live && g == 0) {
+#pragma unroll
+      for (int d = 0; d < 4; ++d) {
+        PV o[SPL];
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) o[i] = Cx<PT>::make((PT)v[d][i][0], (PT)v[d][i][1]);
+        store_spl<PV, SPL>(t + ((long)a * 4 + d) * NS + s0, o);
+      }
+      PV dd[SPL], o[SPL];
+      load_spl<PV, NS, SPL, false, RO>(hdd + (long)a * NS + s0, dd);
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        const PT tx = (PT)v[0][i][0], ty = (PT)v[0][i][1];
+        o[i] = Cx<PT>::make(tx * dd[i].x - ty * dd[i].y, tx * dd[i].y + ty * dd[i].x);
+      }
+      store_spl<PV, SPL>(hs + (long)a * NS + s0, o);
+    }
+  }
+}
+
+// Blocks below nbe smooth the edges, the others restrict to the nodes: neither reads what the other writes.
 template <class T, class PT, int NS, bool SEG>
 __global__ void __launch_bounds__(256, (NS >= 8 ? MC_MIN_BLOCKS : 0))
     k_smooth(int nbe, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
@@ -1846,152 +2010,32 @@ __global__ void __launch_bounds__(256, (NS >= 8 ? MC_MIN_BLOCKS : 0))
              typename Cx<PT>::V* __restrict__ t, typename Cx<PT>::V* __restrict__ hs,
              const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg, int ch,
              RedSet R, int nsys, double2* __restrict__ edge_rho) {
-  using V = typename Cx<T>::V;
-  using PV = typename Cx<PT>::V;
   if (ctrl->done) return;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if ((int)blockIdx.x < nbe) {
-    double (*red)[MAX_SYS][2] = nullptr;
-    if constexpr (SEG) red = seg_sums<32, 2>();
-    using S = SmShape<NS, SEG>;
-    constexpr int SPL = S::SPL;
-    const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
-    const PT c1 = (PT)coef[0], c2 = (PT)coef[1];
-    double om[SPL], acc[SPL][2];
-#pragma unroll
-    for (int i = 0; i < SPL; ++i) {
-      om[i] = sc[s0 + i].omega;
-      acc[i][0] = acc[i][1] = 0.0;
-    }
-    int nk0 = 0, nk1 = 0;
-    {
-      const int first = (int)blockIdx.x * ch * 8 * S::RPW + w * S::RPW + sub;
-      if (first < n) { nk0 = __ldg(rowptr + first); nk1 = __ldg(rowptr + first + 1); }
-    }
-    for_rows<S::RPW>(0, n, ch, [&](int row0, int cend, int next) {
-      const int row = row0 + sub;
-      const bool live = row < cend;
-      int sid = 0;
-      if constexpr (SEG) {
-        sid = live ? (int)__ldg(seg + row) : 0;
-        om[0] = sc[sid].omega;
-      }
-      const int k0 = live ? nk0 : 0, k1 = live ? nk1 : 0;
-      if (next >= 0 && next + sub < n) { nk0 = __ldg(rowptr + next + sub); nk1 = __ldg(rowptr + next + sub + 1); }
-      PT t1x[SPL], t1y[SPL], t2x[SPL], t2y[SPL];
-#pragma unroll
-      for (int i = 0; i < SPL; ++i) t1x[i] = t1y[i] = t2x[i] = t2y[i] = 0;
-      row_gather_spl<PT, NS, S::G, SPL, true>(col, km, sv, k0 + g, k1, s0, t1x, t1y, t2x, t2y);
-      group_sum<PT, SPL, S::NG, S::LPR>(t1x, t1y, t2x, t2y);
-      if (g == 0 && live) {
-        const long base = (long)row * NS + s0;
-        const double2 dg = __ldg(dkm + row);
-        PV si[SPL], zo[SPL];
-        V ri[SPL];
-        load_spl<PV, NS, SPL, false, true>(sv + base, si);
-        load_spl<V, NS, SPL, false, true>(r + base, ri);
-#pragma unroll
-        for (int i = 0; i < SPL; ++i) {
-          const PT o = (PT)om[i];
-          const PT ax = t1x[i] - o * t2y[i], ay = t1y[i] + o * t2x[i];
-          const double2 dd = ssor_dd(dg, om[i], 1.0);
-          const PT dx = (PT)dd.x, dy = (PT)dd.y;
-          zo[i] = Cx<PT>::make(c1 * si[i].x - c2 * (ax * dx - ay * dy), c1 * si[i].y - c2 * (ax * dy + ay * dx));
-          const double e0 = (double)ri[i].x * (double)zo[i].x - (double)ri[i].y * (double)zo[i].y;
-          const double e1 = (double)ri[i].x * (double)zo[i].y + (double)ri[i].y * (double)zo[i].x;
-          if constexpr (SEG) {
-            red[w * 4 + sub][sid][0] += e0;
-            red[w * 4 + sub][sid][1] += e1;
-          } else {
-            acc[i][0] += e0;
-            acc[i][1] += e1;
-          }
-        }
-        store_spl<PV, SPL>(z + base, zo);
-      }
-    }, (int)blockIdx.x, nbe);
-    __shared__ double2 sums[MAX_SYS];
-    if constexpr (SEG) seg_pair<32, 2>(red, R, blockIdx.x);
-    else block_pair<NS, SPL, S::LPR>(acc, s0, g == 0, R, blockIdx.x);
+    __shared__ double2 sums[MAX_SYS], buf[8 * NS];
+    smooth_edges<T, PT, NS, SEG, true>(rowptr, col, km, n, sv, r, z, dkm, coef, sc, seg, ch, R, blockIdx.x, nbe, buf);
     if (reduce_blocks(R, blockIdx.x, nbe, nsys, sums) && threadIdx.x < nsys) edge_rho[threadIdx.x] = sums[threadIdx.x];
   } else {
-    using S = NdShape<NS>;
-    constexpr int SPL = S::SPL;
-    const int sub = lane >> 3, ql = lane & 7, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
-    const int nb = (int)gridDim.x - nbe, b0 = (int)blockIdx.x - nbe;
-    for (int a0 = (b0 * 8 + w) * 4; a0 < node; a0 += nb * 32) {
-      const int a = a0 + sub;
-      const bool live = a < node;
-      T v[4][SPL][2];
-#pragma unroll
-      for (int d = 0; d < 4; ++d)
-#pragma unroll
-        for (int i = 0; i < SPL; ++i) v[d][i][0] = v[d][i][1] = 0;
-      const int q1 = live ? __ldg(nptr + a + 1) : 0;
-      for (int k = (live ? __ldg(nptr + a) : 0) + g; k < q1; k += S::G) {
-        const int ent = __ldg(nlist + k), e = ent >> 1;
-        if (__ldg(bc + e)) continue;
-        V re[SPL];
-        load_spl<V, NS, SPL, false, true>(r + (long)e * NS + s0, re);
-        const T sg = (ent & 1) ? (T)-1 : (T)1;
-        const T hx = (T)(0.5 * __ldg(te + 3L * e)), hy = (T)(0.5 * __ldg(te + 3L * e + 1)),
-                hz = (T)(0.5 * __ldg(te + 3L * e + 2));
-#pragma unroll
-        for (int i = 0; i < SPL; ++i) {
-          v[0][i][0] += sg * re[i].x; v[0][i][1] += sg * re[i].y;
-          v[1][i][0] += hx * re[i].x; v[1][i][1] += hx * re[i].y;
-          v[2][i][0] += hy * re[i].x; v[2][i][1] += hy * re[i].y;
-          v[3][i][0] += hz * re[i].x; v[3][i][1] += hz * re[i].y;
-        }
-      }
-#pragma unroll
-      for (int m = S::NG; m < 8; m <<= 1)
-#pragma unroll
-        for (int d = 0; d < 4; ++d)
-#pragma unroll
-          for (int i = 0; i < SPL; ++i) {
-            v[d][i][0] += shfl_xor(v[d][i][0], m);
-            v[d][i][1] += shfl_xor(v[d][i][1], m);
-          }
-      if (live && g == 0) {
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-          PV o[SPL];
-#pragma unroll
-          for (int i = 0; i < SPL; ++i) o[i] = Cx<PT>::make((PT)v[d][i][0], (PT)v[d][i][1]);
-          store_spl<PV, SPL>(t + ((long)a * 4 + d) * NS + s0, o);
-        }
-        PV dd[SPL], o[SPL];
-        load_spl<PV, NS, SPL, false, true>(hdd + (long)a * NS + s0, dd);
-#pragma unroll
-        for (int i = 0; i < SPL; ++i) {
-          const PT tx = (PT)v[0][i][0], ty = (PT)v[0][i][1];
-          o[i] = Cx<PT>::make(tx * dd[i].x - ty * dd[i].y, tx * dd[i].y + ty * dd[i].x);
-        }
-        store_spl<PV, SPL>(hs + (long)a * NS + s0, o);
-      }
-    }
+    restrict_nodes<T, PT, NS, true>(node, nptr, nlist, bc, te, hdd, r, t, hs, (int)blockIdx.x - nbe,
+                                    (int)gridDim.x - nbe);
   }
 }
 
 // w = (u + T O_0, T O_1, T O_2, T O_3) at every mesh node, in [node][4][system], with the nodes'
 // smoother u = c1 hs - c2 D_G^-1 A_G hs (the polynomial of the edges, on A_G = G^T A G) and their
 // share t_0^T u of rho; the last block forms rho and beta.  coef: the edges' and the nodes' pairs.
-template <class T, int NS, bool SEG>
-__global__ void __launch_bounds__(256)
-    k_node_prolong(int node, const uint8_t* __restrict__ nseg, const CoarseGrid* __restrict__ grids,
-                   const int32_t* __restrict__ cell, const double* __restrict__ frac,
-                   const typename Cx<T>::V* __restrict__ O, const typename Cx<T>::V* __restrict__ t,
-                   const typename Cx<T>::V* __restrict__ hs, const typename Cx<T>::V* __restrict__ hdd,
-                   const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
-                   const double2* __restrict__ km, const double* __restrict__ coef, typename Cx<T>::V* __restrict__ w,
-                   SysScal* sc, const Ctrl* ctrl, RedSet R, int nsys, const double2* edge_rho, const double2* grid_rho) {
+template <class T, int NS, bool SEG, bool RO>
+__device__ __forceinline__ void prolong(int node, const uint8_t* nseg, const CoarseGrid* grids, const int32_t* cell,
+                                        const double* frac, const typename Cx<T>::V* O, const typename Cx<T>::V* t,
+                                        const typename Cx<T>::V* hs, const typename Cx<T>::V* hdd,
+                                        const int32_t* rowptr, const int32_t* col, const double2* km,
+                                        const double* coef, typename Cx<T>::V* w, const SysScal* sc, const RedSet& R,
+                                        int bid, int nb, double2* buf) {
   using V = typename Cx<T>::V;
-  if (ctrl->done) return;
   constexpr int SP = NS >= 2 ? 2 : 1, GPC = NS / SP, GPR = 4 * GPC;
-  const long total = (long)node * GPR, stride = (long)gridDim.x * blockDim.x;
+  const long total = (long)node * GPR, stride = (long)nb * blockDim.x;
   const T c1 = (T)coef[2], c2 = (T)coef[3];
-  const long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long i0 = bid * (long)blockDim.x + threadIdx.x;
   const int c = (int)(i0 % GPR) / GPC, s0 = (int)(i0 % GPC) * SP;  // the stride is a multiple of GPR
   double om[SP], acc[SP][2];
 #pragma unroll
@@ -2021,7 +2065,7 @@ __global__ void __launch_bounds__(256)
         for (int k = __ldg(rowptr + a); k < k1; ++k) {
           const double2 m = __ldg(km + k);
           V x[SP];
-          load_spl<V, NS, SP, false, true>(hs + (long)__ldg(col + k) * NS + s0, x);
+          load_spl<V, NS, SP, false, RO>(hs + (long)__ldg(col + k) * NS + s0, x);
 #pragma unroll
           for (int j = 0; j < SP; ++j) {
             t1x[j] += (T)m.x * x[j].x; t1y[j] += (T)m.x * x[j].y;
@@ -2029,9 +2073,9 @@ __global__ void __launch_bounds__(256)
           }
         }
         V ti[SP], si[SP], dd[SP];
-        load_spl<V, NS, SP, false, true>(t + (long)a * 4 * NS + s0, ti);
-        load_spl<V, NS, SP, false, true>(hs + (long)a * NS + s0, si);
-        load_spl<V, NS, SP, false, true>(hdd + (long)a * NS + s0, dd);
+        load_spl<V, NS, SP, false, RO>(t + (long)a * 4 * NS + s0, ti);
+        load_spl<V, NS, SP, false, RO>(hs + (long)a * NS + s0, si);
+        load_spl<V, NS, SP, false, RO>(hdd + (long)a * NS + s0, dd);
 #pragma unroll
         for (int j = 0; j < SP; ++j) {
           const T ax = t1x[j] - (T)om[j] * t2y[j], ay = t1y[j] + (T)om[j] * t2x[j];
@@ -2060,7 +2104,7 @@ __global__ void __launch_bounds__(256)
           if (wd == 0.0) continue;
           const T wt = (T)wd;
           V x[SP];
-          load_spl<V, NS, SP, false, true>(O + ((long)(b + dx + nx * dy + nxy * dz) * 4 + c) * NS + s0, x);
+          load_spl<V, NS, SP, false, RO>(O + ((long)(b + dx + nx * dy + nxy * dz) * 4 + c) * NS + s0, x);
 #pragma unroll
           for (int j = 0; j < SP; ++j) {
             o[j].x += wt * x[j].x;
@@ -2072,14 +2116,25 @@ __global__ void __launch_bounds__(256)
     }
     if constexpr (SEG) seg_warp_sum<2>(red, threadIdx.x >> 5, sid, e);
   }
-  __shared__ double2 sums[MAX_SYS];
-  if constexpr (SEG) {
-    seg_pair<8, 2>(red, R, blockIdx.x);
-  } else {
-    // the lanes of component 0 hold the values
-    block_pair<NS, SP, GPR>(acc, s0, (int)(threadIdx.x % GPR) < GPC, R, blockIdx.x);
-  }
-  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_rho(sc, ctrl, sums, edge_rho, grid_rho, nsys);
+  if constexpr (SEG) seg_pair<8, 2>(red, R, bid);
+  else block_pair<NS, SP, GPR>(acc, s0, (int)(threadIdx.x % GPR) < GPC, R, bid, buf);  // component 0's lanes
+}
+
+template <class T, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_node_prolong(int node, const uint8_t* __restrict__ nseg, const CoarseGrid* __restrict__ grids,
+                   const int32_t* __restrict__ cell, const double* __restrict__ frac,
+                   const typename Cx<T>::V* __restrict__ O, const typename Cx<T>::V* __restrict__ t,
+                   const typename Cx<T>::V* __restrict__ hs, const typename Cx<T>::V* __restrict__ hdd,
+                   const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                   const double2* __restrict__ km, const double* __restrict__ coef, typename Cx<T>::V* __restrict__ w,
+                   SysScal* sc, const Ctrl* ctrl, RedSet R, int nsys, const double2* edge_rho, const double2* grid_rho) {
+  if (ctrl->done) return;
+  __shared__ double2 sums[MAX_SYS], buf[8 * NS];
+  prolong<T, NS, SEG, true>(node, nseg, grids, cell, frac, O, t, hs, hdd, rowptr, col, km, coef, w, sc, R, blockIdx.x,
+                            gridDim.x, buf);
+  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
+    finish_rho(sc, ctrl, sums, edge_rho, grid_rho, MAX_SYS, nsys);
 }
 
 // One step of the power iteration on D_K^-1 K and D_M^-1 M at once (x and y of the vectors): 8 lanes
@@ -2134,7 +2189,8 @@ __global__ void __launch_bounds__(256)
   // two sums as two "systems": K's quotient and M's
   __shared__ double2 sums[MAX_SYS];
   double v[2][2] = {{s[0], s[1]}, {s[2], s[3]}};
-  block_pair<2, 2, 1>(v, 0, true, R, blockIdx.x);
+  __shared__ double2 buf[16];
+  block_pair<2, 2, 1>(v, 0, true, R, blockIdx.x, buf);
   if (reduce_blocks(R, blockIdx.x, gridDim.x, 2, sums) && threadIdx.x == 0) {
     double lam = sums[0].y > 0.0 ? sums[0].x / sums[0].y : 0.0;
     if (sums[1].y > 0.0) lam = fmax(lam, sums[1].x / sums[1].y);
@@ -2183,9 +2239,174 @@ __global__ void __launch_bounds__(256)
   }
   if (!coef) return;
   __shared__ double2 sums[MAX_SYS];
-  block_pair<1, 1, 1>(s, 0, true, R, blockIdx.x);
+  __shared__ double2 buf[8];
+  block_pair<1, 1, 1>(s, 0, true, R, blockIdx.x, buf);
   if (reduce_blocks(R, blockIdx.x, gridDim.x, 1, sums) && threadIdx.x == 0)
     cheb_coefficients(sums[0].y > 0.0 ? sqrt(sums[0].x / sums[0].y) : 0.0, 2.0, coef + 2);
+}
+
+// ------------------------------------------------------------------ one-launch iteration of small systems
+// The smoothed iteration of a system too small to fill the device: a launch boundary and a sum across
+// blocks cost 5 to 7 us each there, six or more times an iteration, against 1 to 4 us of work.  One
+// cooperative kernel of a block per SM runs many iterations, with a grid barrier between the steps;
+// every block adds the parts of a sum for itself after the barrier and keeps its own copy of the
+// scalars, so no block waits for another's scalar step.  The blocks that have no V-cycle smooth the
+// edges meanwhile.  Steps and formulas are those of k_r_update ... k_spmv.
+constexpr int SMALL_THREADS = TAIL_THREADS;
+constexpr size_t SMALL_BYTES = 196 << 10;  // the cycle's shared memory
+// Rows x (systems + 2) -- the vectors' and the matrix's share of the work -- up to which it is the
+// faster form.  Us an iteration, one launch / launches per step: 1 system 54 / 78 at 10,000 rows, 113 / 138
+// at 100,000, 199 / 191 at 180,000; 4 systems 65 / 85 at 10,000, 189 / 201 at 100,000, 328 / 282 at 180,000;
+// 16 systems 80 / 95 at 10,000, 147 / 155 at 23,000, 256 / 211 at 48,000.
+constexpr long SMALL_ITEMS = 480000;
+
+template <class T, class PT>
+struct SmallArgs {
+  using V = typename Cx<T>::V;
+  using PV = typename Cx<PT>::V;
+  // static data
+  int n, node, nsys, steps, vals, top;
+  const int32_t *rowptr, *col, *line, *nptr, *nlist, *hrow, *hcol, *cell, *lptr, *lidx, *levels;
+  const uint8_t* bc;
+  const V* km;     // the COCG's matrix
+  const PV* kmp;   // the smoother's copy
+  const double2 *dkm, *hkm, *l1;
+  const double *te, *frac, *axw, *lw, *cheb, *omega;
+  const CoarseGrid* grids;
+  const PV *gkm, *hdd;
+  // written during the launch
+  V *r, *p, *q;
+  PV *z, *sv, *t, *w, *hs, *R, *Z, *O;
+  double2 *x, *rho;
+  SysScal* sc;
+  Ctrl* ctrl;
+  RedSet red_r, red_edge, red_node, red_pq, red_grid;
+};
+
+// q = A p and p^T q, lane geometry of the smoother's edges
+template <class T, int NS>
+__device__ __forceinline__ void spmv_rows(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                                          const typename Cx<T>::V* __restrict__ km, int n, const typename Cx<T>::V* p,
+                                          typename Cx<T>::V* q, const SysScal* sc, const RedSet& R, int bid, int nb,
+                                          double2* buf) {
+  using V = typename Cx<T>::V;
+  using S = SmShape<NS, false>;
+  constexpr int SPL = S::SPL;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+  double acc[SPL][2];
+#pragma unroll
+  for (int i = 0; i < SPL; ++i) acc[i][0] = acc[i][1] = 0.0;
+  for (int row0 = (bid * nw + w) * S::RPW; row0 < n; row0 += nb * nw * S::RPW) {
+    const int row = row0 + sub;
+    const bool live = row < n;
+    const int k0 = live ? __ldg(rowptr + row) : 0, k1 = live ? __ldg(rowptr + row + 1) : 0;
+    T t1x[SPL], t1y[SPL], t2x[SPL], t2y[SPL];
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) t1x[i] = t1y[i] = t2x[i] = t2y[i] = 0;
+    row_gather_spl<T, NS, S::G, SPL, false>(col, km, p, k0 + g, k1, s0, t1x, t1y, t2x, t2y);
+    group_sum<T, SPL, S::NG, S::LPR>(t1x, t1y, t2x, t2y);
+    if (g == 0 && live) {
+      const long base = (long)row * NS + s0;
+      V own[SPL], qi[SPL];
+      load_spl<V, NS, SPL, false>(p + base, own);
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        const T o = (T)sc[s0 + i].omega;
+        qi[i] = Cx<T>::make(t1x[i] - o * t2y[i], t1y[i] + o * t2x[i]);
+        acc[i][0] += (double)own[i].x * (double)qi[i].x - (double)own[i].y * (double)qi[i].y;
+        acc[i][1] += (double)own[i].x * (double)qi[i].y + (double)own[i].y * (double)qi[i].x;
+      }
+      store_spl<V, SPL>(q + base, qi);
+    }
+  }
+  block_pair<NS, SPL, S::LPR>(acc, s0, g == 0, R, bid, buf);
+}
+
+template <class T, class PT, int NS>
+__global__ void __launch_bounds__(SMALL_THREADS) k_small(const __grid_constant__ SmallArgs<T, PT> a) {
+  using PV = typename Cx<PT>::V;
+  if (a.ctrl->done) return;  // uniform over the grid
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  extern __shared__ double2 small_smem[];
+  __shared__ SysScal sc[NS];
+  __shared__ Ctrl ctrl;
+  __shared__ double2 sums[MAX_SYS], edge[MAX_SYS], grho[4 * NS], buf[SMALL_THREADS / 32 * NS];
+  const int bid = blockIdx.x, nb = gridDim.x;
+  if (threadIdx.x < NS) sc[threadIdx.x] = a.sc[threadIdx.x];
+  if (threadIdx.x == 0) ctrl = *a.ctrl;
+  __syncthreads();
+  grid.sync();  // every block holds the state before block 0 may write it back
+  const int nt = 4 * NS;       // blocks of the cycle, the others smooth the edges (nb > nt)
+  for (int it = 0; it < a.steps; ++it) {
+    r_update<T, PT, NS, false>(a.n, a.r, a.q, a.sv, a.dkm, sc, ctrl.iter > 0, nullptr, a.red_r, bid, nb, buf);
+    grid.sync();
+    sum_blocks(a.red_r, nb, NS, sums);
+    finish_r(sc, &ctrl, sums, NS);
+    __syncthreads();
+    if (!ctrl.done) {
+      restrict_nodes<T, PT, NS, false>(a.node, a.nptr, a.nlist, a.bc, a.te, a.hdd, a.r, a.t, a.hs, bid, nb);
+      grid.sync();
+      double v[1][2];
+      if (a.top > 0) {
+        grid_restrict<PT, NS>(a.grids[0].n, a.lptr, a.lidx, a.lw, a.t, a.l1, a.omega, a.R, a.Z, bid, nb);
+        grid.sync();
+        for (int l = 0; l < a.top; ++l) {
+          grid_step<PT, NS, 0>(a.grids[l], a.grids[l + 1], a.gkm, a.l1, a.axw, a.omega, a.R, a.Z, a.O, v, bid, nb);
+          grid.sync();
+          grid_step<PT, NS, 1>(a.grids[l], a.grids[l + 1], a.gkm, a.l1, a.axw, a.omega, a.R, a.Z, a.O, v, bid, nb);
+          grid.sync();
+        }
+      }
+      if (bid < nt)
+        grid_tail<PT, NS, false>(bid & 3, bid >> 2, reinterpret_cast<PV*>(small_smem), a.grids, a.levels, a.top,
+                                 a.vals, a.gkm, a.l1, a.axw, a.omega, a.R, a.O, a.lptr, a.lidx, a.lw, a.t,
+                                 a.top == 0 ? a.rho : nullptr);
+      else
+        smooth_edges<T, PT, NS, false, false>(a.rowptr, a.col, a.kmp, a.n, a.sv, a.r, a.z, a.dkm, a.cheb, sc, nullptr,
+                                              1, a.red_edge, bid - nt, nb - nt, buf);
+      grid.sync();
+      for (int l = a.top - 1; l >= 0; --l) {
+        grid_step<PT, NS, 2>(a.grids[l], a.grids[l + 1], a.gkm, a.l1, a.axw, a.omega, a.R, a.Z, a.O, v, bid, nb);
+        grid.sync();
+        grid_step<PT, NS, 3>(a.grids[l], a.grids[l + 1], a.gkm, a.l1, a.axw, a.omega, a.R, a.Z, a.O, v, bid, nb);
+        if (l == 0) block_pair<NS, 1, NS>(v, threadIdx.x % NS, true, a.red_grid, bid, buf);
+        grid.sync();
+      }
+      prolong<PT, NS, false, false>(a.node, nullptr, a.grids, a.cell, a.frac, a.O, a.t, a.hs, a.hdd, a.hrow, a.hcol,
+                                    a.hkm, a.cheb, a.w, sc, a.red_node, bid, nb, buf);
+      grid.sync();
+      sum_blocks(a.red_edge, nb - nt, NS, edge);
+      if (a.top > 0) sum_blocks(a.red_grid, nb, NS, grho);
+      for (int i = threadIdx.x; i < 4 * NS; i += SMALL_THREADS) {
+        if (a.top == 0) grho[i] = __ldcg(a.rho + (i / NS) * MAX_SYS + i % NS);
+        else if (i >= NS) grho[i] = make_double2(0.0, 0.0);
+      }
+      sum_blocks(a.red_node, nb, NS, sums);
+      finish_rho(sc, &ctrl, sums, edge, grho, NS, NS);
+      __syncthreads();
+    }
+    // also when this iteration's residual ended the solve: x += alpha p may be pending
+    if constexpr (NS >= 2)
+      pupd_spl<T, PT, NS>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, a.x, a.line, a.bc, a.w, a.te, bid, nb);
+    else
+      pupd<T, PT, NS, false>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, nullptr, a.x, a.line, a.bc, a.w, a.te, bid,
+                             nb);
+    if (ctrl.done) break;
+    grid.sync();
+    spmv_rows<T, NS>(a.rowptr, a.col, a.km, a.n, a.p, a.q, sc, a.red_pq, bid, nb, buf);
+    grid.sync();
+    sum_blocks(a.red_pq, nb, NS, sums);
+    finish_pq(sc, &ctrl, sums, NS);
+    __syncthreads();
+  }
+  if (bid == 0) {
+    if (threadIdx.x < NS) {
+      if (ctrl.done) sc[threadIdx.x].xpend = 0;  // applied above
+      a.sc[threadIdx.x] = sc[threadIdx.x];
+    }
+    if (threadIdx.x == 0) *a.ctrl = ctrl;
+  }
 }
 
 // ------------------------------------------------------------------ tiled SpMV (16 systems, FP64)
@@ -3026,6 +3247,55 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, cudaEve
   if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
 }
 
+// Whether the smoothed iteration runs as one launch (k_small): systems whose steps do not fill the
+// device.
+template <int NS, bool SEG>
+bool small_system(const afem_ctx* c, const SolverWork* w) {
+  return !SEG && (long)w->n * (NS + 2) <= SMALL_ITEMS && c->num_sms > 5 * NS;
+}
+
+// `steps` iterations (fewer when the solve ends) in one cooperative launch.
+template <class T, class PT, int NS>
+void launch_small(afem_ctx* c, SolverWork* w, int steps, const double* d_omega) {
+  using I = Inner<T, NS>;
+  using P = Inner<PT, NS>;
+  using PV = typename P::V;
+  HybridState* h = c->hyb;
+  CoarseState* co = h->co;
+  const size_t vec = (size_t)4 * NS * co->ntot, smem = std::min(SMALL_BYTES, sizeof(PV) * co->tail_vals);
+  SmallArgs<T, PT> a{};
+  a.n = w->n; a.node = h->node; a.nsys = NS; a.steps = steps; a.vals = (int)(smem / sizeof(PV)); a.top = co->tail;
+  a.rowptr = c->rowptr.p; a.col = c->col.p; a.line = c->line.p; a.nptr = h->nptr.p; a.nlist = h->nlist.p;
+  a.hrow = h->rowptr.p; a.hcol = h->col.p; a.cell = co->cell.p; a.lptr = co->lptr.p; a.lidx = co->lidx.p;
+  a.levels = co->d_levels.p; a.bc = c->bc.p;
+  a.km = I::KM(c, w);
+  if constexpr (sizeof(PT) == 8) { a.kmp = c->km.p; a.gkm = co->km.p; }
+  else { a.kmp = w->kmf.p; a.gkm = co->kmf.p; }
+  a.dkm = w->dkm.p; a.hkm = h->km.p; a.l1 = co->l1.p; a.te = co->te.p; a.frac = co->frac.p; a.axw = co->axw.p;
+  a.lw = co->lw.p; a.cheb = w->cheb.p; a.omega = d_omega; a.grids = co->d_grids.p; a.hdd = P::HDD(w);
+  a.r = I::R(w); a.p = I::P(w); a.q = I::Q(w); a.z = P::Z(w);
+  a.sv = reinterpret_cast<PV*>(w->dd.p);
+  a.t = reinterpret_cast<PV*>(w->nbuf.p); a.w = a.t + 4L * h->node * NS; a.hs = P::HY(w);
+  a.R = reinterpret_cast<PV*>(w->cbuf.p); a.Z = a.R + vec; a.O = a.Z + vec;
+  a.x = w->x.p; a.rho = w->rho.p + MAX_SYS; a.sc = w->sc.p; a.ctrl = w->ctrl.p;
+  a.red_r = red_set(w, RED_R); a.red_edge = red_set(w, RED_EDGE); a.red_node = red_set(w, RED_NODE);
+  a.red_pq = red_set(w, RED_PQ); a.red_grid = red_set(w, RED_GRID);
+  auto k = k_small<T, PT, NS>;
+  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(c->num_sms);
+  cfg.blockDim = dim3(SMALL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  AFEM_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+  count_launch();
+}
+
 // Row-order diagonal and smoother coefficients: the edges' once per assembly (k_power covers every
 // frequency), the nodes' once per solve (k_node_power).
 void smoother_values(afem_ctx* c, SolverWork* w, const double* d_omega) {
@@ -3201,7 +3471,9 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   w->epoch_host += 1;
   AFEM_CUDA(cudaMemcpyAsync(&w->ctrl.p->epoch, &w->epoch_host, sizeof(unsigned), cudaMemcpyHostToDevice, s));
   int iters_done = 0;
-  const int chunk = check_every > 0 ? check_every : 32;
+  // iterations between host checks; the one-launch form needs the host less often
+  const bool one_launch = smoothed(c, w, mode) && !c->prof.on && small_system<NS, SEG>(c, w);
+  const int chunk = check_every > 0 ? check_every : (one_launch ? 128 : 32);
   // profiling: 8 events per iteration of a chunk (fwd | scal | bwd | nodal correction | scal | pupd | spmv,
   // or r update | smoother | coarse cycle | prolongation | pupd | spmv)
   const bool prof = c->prof.on;
@@ -3218,7 +3490,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   };
   cudaGraphExec_t gexec = nullptr;
   long graph_kernels = 0;  // kernel nodes of the captured chunk (launch count per graph launch)
-  bool use_graph = o->use_graph != 0 && !prof;
+  bool use_graph = o->use_graph != 0 && !prof && !one_launch;
   if (use_graph) {
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
@@ -3274,7 +3546,9 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   const long chunk_budget = (long)maxit / chunk + 4;
   for (long nchunk = 0;; ++nchunk) {
     AFEM_REQUIRE(nchunk < chunk_budget, AFEM_ESTATE, "COCG: inner solve made no progress");
-    if (use_graph) {
+    if (one_launch) {
+      if constexpr (!SEG) launch_small<T, PT, NS>(c, w, chunk, d_omega);
+    } else if (use_graph) {
       AFEM_CUDA(cudaGraphLaunch(gexec, s));
       count_launch(graph_kernels);
     } else {
@@ -3335,7 +3609,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
     // FP64 inner solves get a long window (64 chunks, 2048 iterations): on the
     // air-dominated systems the recursive residual can flatten out near 1e-7,
     // and a restart from the true residual resumes the descent
-    const int win = learned ? 4 : (sizeof(T) == 4 ? 16 : 64);
+    const int win = std::max(1, (learned ? 4 : (sizeof(T) == 4 ? 16 : 64)) * (one_launch && check_every <= 0 ? 32 : chunk) / chunk);
     if (!w->no_window) {
       AFEM_CUDA(cudaMemcpyAsync(w->h_sc, w->sc.p, sizeof(SysScal) * nsys, cudaMemcpyDeviceToHost, s));
       AFEM_CUDA(cudaStreamSynchronize(s));

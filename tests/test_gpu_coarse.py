@@ -116,3 +116,32 @@ def test_new_conductivities_and_bounds_rebuild_the_matrices(fw, oracle):
         A = oracle.OracleForward(m2).assemble(m2.freqs[0])
         r = fw.solve(m2.freqs[0], precond="HYBRID", tol=1e-9, maxit=2000)
         assert r.ok and oracle.true_residual(A, fw.solution(0)) <= 1.01e-9, r
+
+
+@pytest.mark.parametrize("ns", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("precision", ["fp64", "pc32"])
+def test_one_launch_iteration_gives_the_same_solution(fw, oracle, ns, precision):
+    """Small systems iterate inside one launch, profiled solves by a launch per step: the same polynomial,
+    cycles and formulas, so both reach the tolerance and their site fields agree to 1e-6.  The caps on
+    iterations and an iteration count that ends inside a launch hold for both."""
+    m = synth.tidal_box(9, 8, 10, seed=12, grf=True, block=False)
+    fw.load_model(m, sources=[(m.F, m.v), (m.F, 0.5j * m.v)])
+    fw.assemble()
+    f = 1.0 / (3600.0 * np.array((synth.BATCH_PERIODS_H * 2)[:ns]))
+    src = np.arange(ns) % 2
+    kw = dict(precond="HYBRID", precision=precision)
+    r = fw.solve(f, src, tol=1e-9, maxit=2000, **kw)
+    assert r.ok and r.resid_true <= 1e-9, r
+    one = fw.sites(m.sites)
+    A = oracle.OracleForward(m).assemble(f[0])
+    assert oracle.true_residual(A, fw.solution(0)) <= 1.01e-9
+    fw.set_profiling(True)  # launches per step
+    r2 = fw.solve(f, src, tol=1e-9, maxit=2000, **kw)
+    fw.set_profiling(False)
+    assert r2.ok and abs(r2.iterations - r.iterations) <= 3, (r, r2)
+    assert np.abs(fw.sites(m.sites) - one).max() <= 1e-6 * np.abs(one).max()
+    for cap in (1, 7):  # EMAXITER with exactly that many iterations
+        rc = fw.solve(f, src, tol=1e-9, maxit=cap, **kw)
+        assert rc.status == -4 and rc.iterations == cap, rc
+    rc = fw.solve(f, src, tol=1e-9, maxit=2000, check_every=5, **kw)
+    assert rc.ok and rc.iterations == r.iterations
