@@ -50,6 +50,7 @@ HostTimer::~HostTimer() {
 
 std::atomic<long> g_launches{0};
 thread_local int g_capturing = 0;
+thread_local AllocScope t_alloc;
 
 }  // namespace afem
 
@@ -124,8 +125,13 @@ namespace {
 template <class F>
 int guarded(afem_ctx* c, F&& f) {
   if (!c) return AFEM_EINVAL;
+  struct Scope {  // (a call may run inside another's on the same thread)
+    afem::AllocScope before = afem::t_alloc;
+    ~Scope() { afem::t_alloc = before; }
+  } scope;
   try {
     cudaSetDevice(c->device);
+    afem::t_alloc = afem::AllocScope{c->pool, c->stream};
     int rc = f();
     return rc;
   } catch (const Error& e) {
@@ -152,6 +158,17 @@ afem_ctx* afem_create(int device) {
   try {
     AFEM_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     AFEM_CUDA(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device));
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&c->pool, &props) == cudaSuccess) {
+      unsigned long long keep = afem::POOL_KEEP;
+      cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    } else {
+      c->pool = nullptr;
+      cudaGetLastError();
+    }
     c->status.alloc(1);
     c->status.zero(c->stream);
     AFEM_CUDA(cudaStreamSynchronize(c->stream));
@@ -173,11 +190,13 @@ void afem_destroy(afem_ctx* c) {
   afem::mt_destroy(c);
   for (auto* s : c->src) delete s;
   c->src.clear();
-    if (c->stream) {
+  if (c->stream) {
     cudaStreamSynchronize(c->stream);
     cudaStreamDestroy(c->stream);
   }
-  delete c;
+  const cudaMemPool_t pool = c->pool;
+  delete c;  // the last buffers
+  if (pool) cudaMemPoolDestroy(pool);
 }
 
 const char* afem_last_error(const afem_ctx* c) { return c ? c->err.c_str() : "null context"; }

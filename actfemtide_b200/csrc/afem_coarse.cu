@@ -478,22 +478,27 @@ void coarse_pattern(afem_ctx* c) {
   for (int sg = 0; sg < nseg; ++sg) {
     const int a0 = c->nseg > 0 ? c->seg_node_ptr[sg] : 0, a1 = c->nseg > 0 ? c->seg_node_ptr[sg + 1] : node;
     const int e1 = c->nseg > 0 ? c->seg_row_ptr[sg + 1] : nline;
-    double ext[3], cells[3], prod = 1.0;
+    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, sum[3] = {0.0, 0.0, 0.0}, cells[3];
+    double prod = 1.0;
+    long cnt[3] = {0, 0, 0};
+    for (int a = a0; a < a1; ++a)
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = std::min(lo[d], xyz[3L * a + d]);
+        hi[d] = std::max(hi[d], xyz[3L * a + d]);
+      }
+    for (int d = 0; d < 3; ++d)  // a flat or unreadable mesh: no correction
+      if (!(hi[d] - lo[d] > 0.0) || !std::isfinite(hi[d] - lo[d])) return;
+    for (int e = e0; e < e1; ++e) {
+      const double* p = xyz.data() + 3L * (ln[2L * e] - 1);
+      const double* q = xyz.data() + 3L * (ln[2L * e + 1] - 1);
+      for (int d = 0; d < 3; ++d) {
+        const double t = std::fabs(q[d] - p[d]);
+        if (t > 1e-9 * (hi[d] - lo[d])) { sum[d] += t; cnt[d] += 1; }
+      }
+    }
     for (int d = 0; d < 3; ++d) {
-      double lo = 1e300, hi = -1e300, sum = 0.0;
-      long cnt = 0;
-      for (int a = a0; a < a1; ++a) {
-        lo = std::min(lo, xyz[3L * a + d]);
-        hi = std::max(hi, xyz[3L * a + d]);
-      }
-      ext[d] = hi - lo;
-      if (!(ext[d] > 0.0) || !std::isfinite(ext[d])) return;  // a flat or unreadable mesh: no correction
-      for (int e = e0; e < e1; ++e) {
-        const double t = std::fabs(xyz[3L * (ln[2L * e + 1] - 1) + d] - xyz[3L * (ln[2L * e] - 1) + d]);
-        if (t > 1e-9 * ext[d]) { sum += t; cnt += 1; }
-      }
-      if (!cnt || !std::isfinite(sum)) return;
-      cells[d] = std::max(1.0, 0.5 * ext[d] * cnt / sum);
+      if (!cnt[d] || !std::isfinite(sum[d])) return;
+      cells[d] = std::max(1.0, 0.5 * (hi[d] - lo[d]) * cnt[d] / sum[d]);
       prod *= cells[d];
     }
     e0 = e1;

@@ -24,6 +24,66 @@ namespace {
 
 constexpr int NODE_EDGE_MAX = 128;  // edges meeting at one node
 
+// The node graph from the edges.  bad[0..2]: the first edge with a bad node id, the first node with too
+// many edges, the first with a repeated one.
+__global__ void k_node_degree(const int32_t* __restrict__ line, int nline, int node, int32_t* __restrict__ deg,
+                              int32_t* __restrict__ bad) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nline) return;
+  const int a = line[2L * e] - 1, b = line[2L * e + 1] - 1;
+  if (a < 0 || a >= node || b < 0 || b >= node || a == b) {
+    atomicMin(bad, e);
+    return;
+  }
+  atomicAdd(deg + a, 1);
+  atomicAdd(deg + b, 1);
+}
+
+__global__ void k_check_degree(const int32_t* __restrict__ deg, int node, int32_t* __restrict__ bad) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a < node && deg[a] > NODE_EDGE_MAX) atomicMin(bad + 1, a);
+}
+
+__global__ void k_node_fill(const int32_t* __restrict__ line, int nline, const int32_t* __restrict__ nptr,
+                            int32_t* __restrict__ cur, int32_t* __restrict__ nlist) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nline) return;
+  const int a = line[2L * e] - 1, b = line[2L * e + 1] - 1;
+  nlist[nptr[a] + atomicAdd(cur + a, 1)] = (e << 1) | 1;
+  nlist[nptr[b] + atomicAdd(cur + b, 1)] = e << 1;
+}
+
+// Sorts a node's edges (the atomics above leave any order) and writes its row, a thread per node: an
+// insertion sort of ~14 entries.
+__global__ void k_node_rows(const int32_t* __restrict__ line, int node, const int32_t* __restrict__ nptr,
+                            int32_t* __restrict__ nlist, int32_t* __restrict__ rowptr, int32_t* __restrict__ col,
+                            int32_t* __restrict__ diagpos, int32_t* __restrict__ bad) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a > node) return;
+  const int b = nptr[a];
+  rowptr[a] = a + b;  // a row holds the node and its edges' far ends
+  if (a == node) return;
+  const int e = nptr[a + 1];
+  for (int i = b + 1; i < e; ++i) {
+    const int v = nlist[i];
+    int j = i;
+    for (; j > b && nlist[j - 1] > v; --j) nlist[j] = nlist[j - 1];
+    nlist[j] = v;
+  }
+  int32_t* row = col + a + b;
+  int len = 0;
+  for (int i = b - 1; i < e; ++i) {
+    const int v = i < b ? a : ((nlist[i] & 1) ? line[2L * (nlist[i] >> 1) + 1] : line[2L * (nlist[i] >> 1)]) - 1;
+    int j = len++;
+    for (; j > 0 && row[j - 1] > v; --j) row[j] = row[j - 1];
+    row[j] = v;
+  }
+  for (int k = 0; k < len; ++k) {
+    if (k && row[k] == row[k - 1]) atomicMin(bad + 2, a);
+    if (row[k] == a) diagpos[a] = a + b + k;
+  }
+}
+
 // Nodal matrices on the node graph: A_G = G^T P (K, M) P G, and with VEC the vector components'
 // Pi_k^T P (K, M) P Pi_k (n3[3 * entry + k]).  Half a warp per row, a lane per entry, so an entry stays
 // in registers over the row's edges; an edge's matrix row is fetched by the lanes at once and handed
@@ -142,62 +202,49 @@ void hybrid_prepare(afem_ctx* c, bool coarse, bool colours) {
   if (h->node != node || h->nline != c->nline || !h->pattern_ready) {
     h->node = node;
     h->nline = c->nline;
-    // The node graph, once per mesh, on the host: incident edges per node in
-    // ascending edge order (edge << 1 | 1 at the tail line(1,e), edge << 1 at
-    // the head), rows = the node and the far ends of its edges, ascending.
+    // The node graph, once per mesh: incident edges per node in ascending edge order
+    // (edge << 1 | 1 at the tail line(1,e), edge << 1 at the head), rows = the node and the far
+    // ends of its edges, ascending.
     const int nline = c->nline;
-    std::vector<int32_t> ln(2L * nline);
-    c->line.download(ln.data(), ln.size(), s);
+    const long nnz = node + 2L * nline;
+    DBuf<int32_t> deg, bad;
+    deg.alloc(node);
+    deg.zero(s);
+    const int32_t none[3] = {INT32_MAX, INT32_MAX, INT32_MAX};
+    int32_t found[3];
+    bad.upload(none, 3, s);
+    k_node_degree<<<nblk(nline, 256), 256, 0, s>>>(c->line.p, nline, node, deg.p, bad.p);
+    count_launch();
+    k_check_degree<<<nblk(node, 256), 256, 0, s>>>(deg.p, node, bad.p);
+    count_launch();
+    bad.download(found, 3, s);
     AFEM_CUDA(cudaStreamSynchronize(s));
-    std::vector<int32_t> np(node + 1, 0);
-    for (int e = 0; e < nline; ++e) {
-      const int a = ln[2L * e] - 1, b = ln[2L * e + 1] - 1;
-      AFEM_REQUIRE(a >= 0 && a < node && b >= 0 && b < node && a != b, AFEM_EINVAL,
-                   "hybrid preconditioner: edge " + std::to_string(e + 1) + " has a bad node id");
-      np[a + 1] += 1;
-      np[b + 1] += 1;
-    }
-    for (int a = 0; a < node; ++a) {
-      AFEM_REQUIRE(np[a + 1] <= NODE_EDGE_MAX, AFEM_EPATTERN,
-                   "hybrid preconditioner: more than 128 edges meet at node " + std::to_string(a + 1));
-      np[a + 1] += np[a];
-    }
-    std::vector<int32_t> nl(2L * nline), cur(np.begin(), np.end() - 1);
-    for (int e = 0; e < nline; ++e) {
-      nl[cur[ln[2L * e] - 1]++] = (e << 1) | 1;
-      nl[cur[ln[2L * e + 1] - 1]++] = e << 1;
-    }
-    std::vector<int32_t> rp(node + 1, 0), dp(node);
-    for (int a = 0; a < node; ++a) rp[a + 1] = rp[a] + 1 + (np[a + 1] - np[a]);
-    const long nnz = rp[node];
-    std::vector<int32_t> cl(nnz);
-    for (int a = 0; a < node; ++a) {
-      int32_t* row = cl.data() + rp[a];
-      int len = 0;
-      row[len++] = a;
-      for (int q = np[a]; q < np[a + 1]; ++q) {
-        const int e = nl[q] >> 1;
-        row[len++] = (nl[q] & 1) ? ln[2L * e + 1] - 1 : ln[2L * e] - 1;
-      }
-      std::sort(row, row + len);
-      for (int k = 0; k < len; ++k) {
-        AFEM_REQUIRE(k == 0 || row[k] > row[k - 1], AFEM_EPATTERN,
-                     "hybrid preconditioner: repeated edge at node " + std::to_string(a + 1));
-        if (row[k] == a) dp[a] = rp[a] + k;
-      }
-    }
+    AFEM_REQUIRE(found[0] == INT32_MAX, AFEM_EINVAL,
+                 "hybrid preconditioner: edge " + std::to_string(found[0] + 1L) + " has a bad node id");
+    AFEM_REQUIRE(found[1] == INT32_MAX, AFEM_EPATTERN,
+                 "hybrid preconditioner: more than 128 edges meet at node " + std::to_string(found[1] + 1L));
+    h->nptr.alloc(node + 1);
+    exclusive_scan(deg.p, h->nptr.p, node, s, nullptr);
+    h->nlist.alloc(2L * nline);
+    h->rowptr.alloc(node + 1);
+    h->col.alloc(nnz);
+    h->diagpos.alloc(node);
+    deg.zero(s);
+    k_node_fill<<<nblk(nline, 256), 256, 0, s>>>(c->line.p, nline, h->nptr.p, deg.p, h->nlist.p);
+    count_launch();
+    k_node_rows<<<nblk(node + 1, 128), 128, 0, s>>>(c->line.p, node, h->nptr.p, h->nlist.p, h->rowptr.p, h->col.p,
+                                                    h->diagpos.p, bad.p);
+    count_launch();
+    bad.download(found, 3, s);
+    AFEM_CUDA(cudaStreamSynchronize(s));
+    AFEM_REQUIRE(found[2] == INT32_MAX, AFEM_EPATTERN,
+                 "hybrid preconditioner: repeated edge at node " + std::to_string(found[2] + 1L));
     h->nnz = nnz;
-    h->nptr.upload(np.data(), np.size(), s);
-    h->nlist.upload(nl.data(), nl.size(), s);
-    h->rowptr.upload(rp.data(), rp.size(), s);
-    h->col.upload(cl.data(), cl.size(), s);
-    h->diagpos.upload(dp.data(), dp.size(), s);
     h->km.alloc(nnz);
     h->live.alloc(node);
     h->pattern_ready = true;
     h->values_gen = -1;
     h->coarse_ready = h->colours_ready = false;
-    AFEM_CUDA(cudaStreamSynchronize(s));  // the host arrays go out of scope
   }
   if (c->nseg > 0 && (int)h->seg_nseg != c->nseg) {
     DBuf<int32_t> ptr;

@@ -35,24 +35,48 @@ struct Error {
   } while (0)
 
 // ---------------------------------------------------------------- device buffer
+// Device memory of an entry point comes from its context's own pool, in the order of the context's
+// stream (the only one its kernels and copies use): a call's temporary buffers then cost microseconds,
+// where cudaMalloc and cudaFree drain the device and now and then took 100 to 650 ms of a 30 ms call.
+// A pool keeps at most POOL_KEEP bytes of freed memory and goes with its context.  Outside an entry
+// point (`pool` null) buffers are plain allocations, and any buffer may be freed there.
+struct AllocScope {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t stream = nullptr;
+};
+extern thread_local AllocScope t_alloc;
+constexpr unsigned long long POOL_KEEP = 1ull << 30;
+
 template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
+  cudaStream_t owner = nullptr;  // the stream of a pooled buffer
   DBuf() = default;
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) {
+      if (owner && owner == t_alloc.stream) cudaFreeAsync(p, owner);
+      else cudaFree(p);
+    }
     p = nullptr;
+    owner = nullptr;
     n = 0;
   }
   void alloc(size_t count) {
     if (count == n && p) return;
     release();
     if (count == 0) return;
-    AFEM_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    if (t_alloc.pool) {
+      void* v = nullptr;
+      AFEM_CUDA(cudaMallocFromPoolAsync(&v, count * sizeof(T), t_alloc.pool, t_alloc.stream));
+      p = static_cast<T*>(v);
+      owner = t_alloc.stream;
+    } else {
+      AFEM_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    }
     n = count;
   }
   void upload(const T* h, size_t count, cudaStream_t s) {
@@ -164,6 +188,7 @@ struct MtState;      // afem_mt.cu
 struct afem_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaMemPool_t pool = nullptr;  // of the context's device buffers (null: plain allocations)
   std::string err;
   int num_sms = 0;
 

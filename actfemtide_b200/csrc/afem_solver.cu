@@ -102,6 +102,7 @@ struct SolverWork {
   DBuf<unsigned> cnt;               // their counters
   DBuf<double2> rho;                // shares of rho: the edges', then 4 rows of the grids'
   int nmc_blocks = 0;               // co-resident grid of the nodal multicolour sweeps
+  int rpw_smooth = 0;               // SpMV rows per warp of the smoothed iteration (smooth_rpw)
   int rpw64 = 0, rpw32 = 0;         // SpMV rows per warp chosen by tune_spmv (0 = not tuned; 8: 4 systems per lane)
   int spmv_grid[2][5] = {};         // one-wave grid of each SpMV variant (FP64 / FP32), 0 = not known yet
   int mc_blocks = 0;                // co-resident grid of the forward multicolour sweep
@@ -3055,6 +3056,22 @@ void launch_sweep_block(afem_ctx* c, SolverWork* w) {
   count_launch();
 }
 
+// The SpMV variant of the smoothed iteration, by a rule and not by timing (a new mesh spent 2 ms on the
+// tuner, a tenth of its solve, and two processes could differ in the last bits): four rows per warp, at
+// 16 systems two of them per lane.  Over 12x12x9 to 64x64x48 cells it is the fastest or within 3 % of it,
+// but for 16 systems at 12,000 rows (18.5 us, no other is faster) to 180,000 (106 against 103).  A
+// variant pinned by the caller is kept.
+template <class T, int NS, bool SEG>
+void smooth_rpw(afem_ctx* c, SolverWork* w) {
+  const int pin = c->spmv_rpw;
+  int rpw = NS == 16 ? 8 : 4;
+  if (pin > 0)
+    rpw = pin == 16 ? (NS == 16 && sizeof(T) == 8 ? 16 : 1)
+                    : (pin == 8 ? (NS == 16 ? 8 : 1) : (NS * pin <= 32 ? pin : 1));
+  if (rpw == 16) ensure_spmv_tiles(c);
+  w->rpw_smooth = rpw;
+}
+
 // One COCG iteration (7 launches; the learned preconditioner adds the network's 8).
 // T: COCG vectors and the SpMV; PT: the multicolour preconditioner (its matrix
 // copies and vectors); PT differs from T only on the multicolour path.
@@ -3236,7 +3253,7 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, cudaEve
                                                           w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw, co->te.p);
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
-  const int rpw = sizeof(T) == 8 ? w->rpw64 : w->rpw32;
+  const int rpw = w->rpw_smooth;
   const bool tiles = rpw == 16;
   const int sgrid = launch_spmv<T, NS, SEG>(c, w, rpw, I::KM(c, w), (const V*)I::P(w), I::Q(w), w->ctrl.p,
                                             (const V*)nullptr, tiles ? RedSet{} : red_set(w, RED_PQ), 0);
@@ -3444,7 +3461,9 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   }
   setup_dd<T, PT, NS, SEG>(c, w, use_hyb ? AFEM_PRECOND_HYBRID : precond, w->sd);
   const int mode = precond;
-  {
+  if (smoothed(c, w, mode)) {
+    smooth_rpw<T, NS, SEG>(c, w);
+  } else {
     HostTimer ht(c, "host_setup_spmv_tuner");
     tune_spmv<T, NS, SEG>(c, w);
   }
@@ -3569,7 +3588,8 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       snprintf(nb, sizeof nb, "cocg_bwd_sweep%s_%s_%s%d", mcs ? "_mc" : "", tag, kind, cnt);
       snprintf(nh, sizeof nh, "cocg_nodal_correction_%s_%s%d", tag, kind, cnt);
       snprintf(np_, sizeof np_, "cocg_p_update_%s_%s%d", tag, kind, cnt);
-      snprintf(ns_, sizeof ns_, "cocg_spmv_%s_%s%d_rpw%d", tag, kind, cnt, sizeof(T) == 8 ? w->rpw64 : w->rpw32);
+      snprintf(ns_, sizeof ns_, "cocg_spmv_%s_%s%d_rpw%d", tag, kind, cnt,
+               smooth ? w->rpw_smooth : (sizeof(T) == 8 ? w->rpw64 : w->rpw32));
       for (int k = 0; k < executed; ++k) {
         float a = 0, b = 0, h = 0, d = 0, e = 0;
         cudaEvent_t* E = &evs[8L * k];
