@@ -11,7 +11,7 @@
 //   h <- h + relu(X W_l + c_l)   (l = 0..5, GEMM 144 x 48 on the tensor cores)
 //   z_i = r_i/s_i^2 + rms * (o_i0 + i o_i1)/s_i,  o = h W_out  (Jacobi term + learned correction)
 // One fused kernel per layer: the block aggregates its 64 rows' neighbours (all rows
-// at once, 2 lanes per row, 16-byte loads) into a shared-memory tile, with the
+// at once, 6 lanes per row, 16-byte loads) into a shared-memory tile, with the
 // message weights of every matrix entry computed once per solve, then every warp
 // multiplies its 16 x 144 tile by W_l with
 // mma.sync.m16n8k16 (BF16 in, FP32 accumulate) and applies bias, ReLU and the
@@ -32,7 +32,10 @@ constexpr int L = 6;
 constexpr int FIN = 8;
 constexpr int XW = 3 * H;        // 144 columns of the layer input
 constexpr int XS = XW + 8;       // padded shared-memory stride (bf16), conflict-free fragments
-constexpr int ROWS = 64;         // rows per block (4 warps x 16)
+constexpr int ROWS = 64;         // rows per tile
+constexpr int HV = H / 8, XV = XW / 8, XSV = XS / 8;  // the same widths in 16-byte words
+constexpr int LAYER_THREADS = ROWS * HV;              // forward: a thread per 16-byte word of the tile's h
+constexpr int BWD_WARPS = XW / 16;                    // backward: a warp per 16 rows of dW
 constexpr int NPARAM = FIN * H + L * (XW * H + H) + H * 2;
 
 // parameter offsets in the flat FP32 vector
@@ -82,16 +85,18 @@ __global__ void k_rowinfo(const double2* __restrict__ km, const int32_t* __restr
 // The message weights of every matrix entry for one omega per system, computed once per solve
 // (every layer of every application reuses them): ew[sy*nnz + k] = (K_ij, omega M_ij)/(s_i s_j)
 // for j != i, 0 on the diagonal (which the aggregation leaves out).
+// 8 lanes per row, so that a row's entries are read and written together (16.0 -> 6.3 us for 23,500
+// rows, where one thread walked a row).
 __global__ void k_edge_w(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                          const double2* __restrict__ km, const float* __restrict__ s,
                          const double* __restrict__ omega, int n, int ns, long nnz, float2* __restrict__ ew) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long i = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 3;
   if (i >= (long)n * ns) return;
   const int row = (int)(i % n), sy = (int)(i / n);
   const float si = s[i];
   const double om = omega[sy];
   float2* out = ew + (long)sy * nnz;
-  for (int k = rowptr[row]; k < rowptr[row + 1]; ++k) {
+  for (int k = rowptr[row] + (threadIdx.x & 7); k < rowptr[row + 1]; k += 8) {
     const int j = col[k];
     if (j == row) {
       out[k] = make_float2(0.f, 0.f);
@@ -131,19 +136,22 @@ __global__ void k_encode(const V* __restrict__ r, int n, int ns, const float* __
   }
 }
 
-// One message-passing layer for rows x systems (blockIdx.y = system).
-// save_x / save_y (training) keep the layer input tile and the pre-activation.
-__device__ __forceinline__ void agg_add(float (&aa)[24], float (&ab)[24], float2 w, const uint4 (&u)[3]) {
-  const unsigned* q = reinterpret_cast<const unsigned*>(u);
+__device__ __forceinline__ void agg_add(float (&aa)[8], float (&ab)[8], float2 w, const uint4& u) {
+  const unsigned q[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
-  for (int k = 0; k < 12; ++k) {
+  for (int k = 0; k < 4; ++k) {
     const float2 hj = unpack_bf16(q[k]);
     aa[2 * k] += w.x * hj.x; aa[2 * k + 1] += w.x * hj.y;
     ab[2 * k] += w.y * hj.x; ab[2 * k + 1] += w.y * hj.y;
   }
 }
 
-__global__ void __launch_bounds__(128)
+// One message-passing layer for rows x systems (blockIdx.y = system).
+// save_x / save_y (training) keep the layer input tile and the pre-activation.  Bound by the latency of
+// the neighbours' loads: 12 warps per 64 rows, a row's 96 bytes read by 6 lanes at 16 bytes each with four
+// neighbours in flight (4 warps with two lanes per row and two neighbours in flight: 23.3 us for 23,500
+// rows; now 13.7 us).  The order of every sum is the entries' order either way.
+__global__ void __launch_bounds__(LAYER_THREADS)
     k_layer(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const float2* __restrict__ ew,
             long nnz, int n, const __nv_bfloat16* __restrict__ h_in, __nv_bfloat16* __restrict__ h_out,
             const __nv_bfloat16* __restrict__ wt,  // W_l transposed, bf16 [H][XW]
@@ -154,65 +162,54 @@ __global__ void __launch_bounds__(128)
   __shared__ __align__(16) __nv_bfloat16 ws[H * XS];
   const int sy = blockIdx.y;
   const long base = (long)sy * n;
-  for (int k = threadIdx.x; k < H * XW; k += blockDim.x) ws[(k / XW) * XS + (k % XW)] = wt[k];
+  uint4* ws4 = reinterpret_cast<uint4*>(ws);
+  for (int k = threadIdx.x; k < H * XV; k += LAYER_THREADS)
+    ws4[(k / XV) * XSV + (k % XV)] = reinterpret_cast<const uint4*>(wt)[k];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r0 = blockIdx.x * ROWS + w * 16;
-  // ---- aggregate: all 64 rows of the block at once, two lanes per row, each lane owning
-  // features 24*half .. 24*half+23 (three 16-byte words of the row's 96 bytes), two
-  // neighbours' loads in flight; each feature sums its neighbours in entry order
+  const int rg = w & 3, ng = w >> 2;  // the warp's 16 rows and its third of the columns
+  // ---- aggregate: lane q of a row owns features 8q .. 8q+7; each feature sums its neighbours in entry order
   {
-    const int rr = threadIdx.x >> 1, half = threadIdx.x & 1;
+    const int rr = threadIdx.x / HV, q = threadIdx.x % HV;
     const int row = blockIdx.x * ROWS + rr;
-    unsigned* xrow = reinterpret_cast<unsigned*>(xs + rr * XS);
+    uint4* xrow = reinterpret_cast<uint4*>(xs) + rr * XSV + q;
     if (row < n) {
-      float aa[24], ab[24];
+      float aa[8], ab[8];
 #pragma unroll
-      for (int k = 0; k < 24; ++k) { aa[k] = 0.f; ab[k] = 0.f; }
-      const uint4* own = reinterpret_cast<const uint4*>(h_in + (base + row) * H) + 3 * half;
-      const uint4 o[3] = {own[0], own[1], own[2]};
+      for (int k = 0; k < 8; ++k) { aa[k] = 0.f; ab[k] = 0.f; }
+      const uint4* h4 = reinterpret_cast<const uint4*>(h_in + base * H) + q;
+      const uint4 own = h4[(long)row * HV];
       const float2* ewr = ew + (long)sy * nnz;
       const int k1 = rowptr[row + 1];
       int k = rowptr[row];
-      for (; k + 1 < k1; k += 2) {
-        const int ja = col[k], jb = col[k + 1];
-        const float2 wa = ewr[k], wb = ewr[k + 1];
-        const uint4* pa = reinterpret_cast<const uint4*>(h_in + (base + ja) * H) + 3 * half;
-        const uint4* pb = reinterpret_cast<const uint4*>(h_in + (base + jb) * H) + 3 * half;
-        const uint4 ua[3] = {pa[0], pa[1], pa[2]}, ub[3] = {pb[0], pb[1], pb[2]};
-        agg_add(aa, ab, wa, ua);
-        agg_add(aa, ab, wb, ub);
-      }
-      if (k < k1) {
-        const int j = col[k];
-        const float2 wj = ewr[k];
-        const uint4* pj = reinterpret_cast<const uint4*>(h_in + (base + j) * H) + 3 * half;
-        const uint4 uj[3] = {pj[0], pj[1], pj[2]};
-        agg_add(aa, ab, wj, uj);
-      }
-      const unsigned* ow = reinterpret_cast<const unsigned*>(o);
+      for (; k + 3 < k1; k += 4) {
+        int j[4];
+        float2 wj[4];
+        uint4 u[4];
 #pragma unroll
-      for (int q = 0; q < 12; ++q) {
-        xrow[12 * half + q] = ow[q];
-        xrow[24 + 12 * half + q] = pack_bf16(aa[2 * q], aa[2 * q + 1]);
-        xrow[48 + 12 * half + q] = pack_bf16(ab[2 * q], ab[2 * q + 1]);
+        for (int m = 0; m < 4; ++m) { j[m] = col[k + m]; wj[m] = ewr[k + m]; }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) u[m] = h4[(long)j[m] * HV];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) agg_add(aa, ab, wj[m], u[m]);
       }
+      for (; k < k1; ++k) agg_add(aa, ab, ewr[k], h4[(long)col[k] * HV]);
+      xrow[0] = own;
+      xrow[HV] = make_uint4(pack_bf16(aa[0], aa[1]), pack_bf16(aa[2], aa[3]), pack_bf16(aa[4], aa[5]),
+                            pack_bf16(aa[6], aa[7]));
+      xrow[2 * HV] = make_uint4(pack_bf16(ab[0], ab[1]), pack_bf16(ab[2], ab[3]), pack_bf16(ab[4], ab[5]),
+                                pack_bf16(ab[6], ab[7]));
     } else {
-#pragma unroll
-      for (int q = 0; q < 12; ++q) {
-        xrow[12 * half + q] = 0u;
-        xrow[24 + 12 * half + q] = 0u;
-        xrow[48 + 12 * half + q] = 0u;
-      }
+      xrow[0] = xrow[HV] = xrow[2 * HV] = make_uint4(0u, 0u, 0u, 0u);
     }
   }
   __syncthreads();
-  // ---- GEMM: rows 16w..16w+15 of the tile times W_l (XW x H)
+  // ---- GEMM: 16 rows of the tile times 16 columns of W_l (XW x H)
   const int g = lane >> 2, t = lane & 3;
-  float acc[6][4];
+  float acc[2][4];
 #pragma unroll
-  for (int nt = 0; nt < 6; ++nt)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[nt][q] = 0.f;
+    for (int q = 0; q < 4; ++q) acc[i][q] = 0.f;
   const unsigned* X = reinterpret_cast<const unsigned*>(xs);
   const unsigned* W = reinterpret_cast<const unsigned*>(ws);
   constexpr int XSW = XS / 2;  // row stride in 32-bit words
@@ -220,28 +217,29 @@ __global__ void __launch_bounds__(128)
   for (int ks = 0; ks < XW / 16; ++ks) {
     const int kw = ks * 8;  // word offset of column 16*ks
     unsigned a[4];
-    a[0] = X[(w * 16 + g) * XSW + kw + t];
-    a[1] = X[(w * 16 + g + 8) * XSW + kw + t];
-    a[2] = X[(w * 16 + g) * XSW + kw + 4 + t];
-    a[3] = X[(w * 16 + g + 8) * XSW + kw + 4 + t];
+    a[0] = X[(rg * 16 + g) * XSW + kw + t];
+    a[1] = X[(rg * 16 + g + 8) * XSW + kw + t];
+    a[2] = X[(rg * 16 + g) * XSW + kw + 4 + t];
+    a[3] = X[(rg * 16 + g + 8) * XSW + kw + 4 + t];
 #pragma unroll
-    for (int nt = 0; nt < 6; ++nt) {
+    for (int i = 0; i < 2; ++i) {
+      const int nt = 2 * ng + i;
       unsigned b[2];
       b[0] = W[(nt * 8 + g) * XSW + kw + t];
       b[1] = W[(nt * 8 + g) * XSW + kw + 4 + t];
-      mma_bf16(acc[nt], a, b);
+      mma_bf16(acc[i], a, b);
     }
   }
   // ---- epilogue: bias, relu, residual
 #pragma unroll
-  for (int nt = 0; nt < 6; ++nt) {
-    const int c = nt * 8 + 2 * t;
+  for (int i = 0; i < 2; ++i) {
+    const int c = (2 * ng + i) * 8 + 2 * t;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
-      const int tr = w * 16 + g + half * 8;
+      const int tr = rg * 16 + g + half * 8;
       const int row = blockIdx.x * ROWS + tr;
       if (row >= n) continue;
-      const float y0 = acc[nt][2 * half] + bias[c], y1 = acc[nt][2 * half + 1] + bias[c + 1];
+      const float y0 = acc[i][2 * half] + bias[c], y1 = acc[i][2 * half + 1] + bias[c + 1];
       const float2 hv = unpack_bf16(X[tr * XSW + c / 2]);
       const long o = (base + row) * H + c;
       reinterpret_cast<unsigned*>(h_out + o)[0] = pack_bf16(hv.x + fmaxf(y0, 0.f), hv.y + fmaxf(y1, 0.f));
@@ -249,13 +247,10 @@ __global__ void __launch_bounds__(128)
     }
   }
   if (save_x) {
-    for (int rr = 0; rr < 16; ++rr) {
-      const int row = r0 + rr;
-      if (row >= n) break;
-      const unsigned* xrow = X + (w * 16 + rr) * XSW;
-      unsigned* dst = reinterpret_cast<unsigned*>(save_x + (base + row) * XW);
-      for (int q = lane; q < XW / 2; q += 32) dst[q] = xrow[q];
-    }
+    const int live = min(ROWS, n - (int)blockIdx.x * ROWS);
+    uint4* dst = reinterpret_cast<uint4*>(save_x + (base + (long)blockIdx.x * ROWS) * XW);
+    for (int k = threadIdx.x; k < live * XV; k += LAYER_THREADS)
+      dst[k] = reinterpret_cast<const uint4*>(xs)[(k / XV) * XSV + (k % XV)];
   }
 }
 
@@ -295,7 +290,19 @@ __global__ void k_decode(const __nv_bfloat16* __restrict__ h, int n, int ns, con
 }
 
 // ------------------------------------------------------------------ training: loss
-// res = A z - r and partial sums of |res|^2, |r|^2 (system sy = blockIdx.y, vectors [row][sys]).
+// Sums over the 8 lanes of a row.
+__device__ __forceinline__ void row_sum(double& a, double& b, double& c, double& d) {
+#pragma unroll
+  for (int m = 4; m > 0; m >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, m);
+    b += __shfl_xor_sync(0xffffffffu, b, m);
+    c += __shfl_xor_sync(0xffffffffu, c, m);
+    d += __shfl_xor_sync(0xffffffffu, d, m);
+  }
+}
+
+// res = A z - r and partial sums of |res|^2, |r|^2 (system sy = blockIdx.y, vectors [row][sys]); 8 lanes
+// per row, as in k_loss_grad (14.3 and 11.7 us with one thread per row at 23,500 rows, now 7.0 and 6.6).
 __global__ void k_loss_res(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                            const double2* __restrict__ km, const double* __restrict__ omega, int n, int ns,
                            const double2* __restrict__ z, const double2* __restrict__ r, double2* __restrict__ res,
@@ -303,14 +310,21 @@ __global__ void k_loss_res(const int32_t* __restrict__ rowptr, const int32_t* __
   const int sy = blockIdx.y;
   const double om = omega[sy];
   double a = 0.0, b = 0.0;
-  for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x) {
+  const int sub = threadIdx.x & 7;
+  const int step = (gridDim.x * blockDim.x) >> 3;
+  // the eight lanes of a row stay together, so the warp's four rows share its bounds
+  for (int first = (int)((blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3); first < n; first += step) {
+    const int row = first + ((threadIdx.x >> 3) & 3);
+    const bool live = row < n;
     double t1x = 0, t1y = 0, t2x = 0, t2y = 0;
-    for (int k = rowptr[row]; k < rowptr[row + 1]; ++k) {
+    for (int k = live ? rowptr[row] + sub : 0, k1 = live ? rowptr[row + 1] : 0; k < k1; k += 8) {
       const double2 e = km[k];
       const double2 zj = z[(long)col[k] * ns + sy];
       t1x += e.x * zj.x; t1y += e.x * zj.y;
       t2x += e.y * zj.x; t2y += e.y * zj.y;
     }
+    row_sum(t1x, t1y, t2x, t2y);
+    if (!live || sub) continue;
     const double2 ri = r[(long)row * ns + sy];
     const double2 q = make_double2(t1x - om * t2y - ri.x, t1y + om * t2x - ri.y);
     res[(long)row * ns + sy] = q;
@@ -332,12 +346,19 @@ __global__ void k_loss_res(const int32_t* __restrict__ rowptr, const int32_t* __
   }
 }
 
-__global__ void k_loss_sum(const double* __restrict__ part, int nb, int ns, double* __restrict__ out) {
-  // out[2*sy] = sum |res|^2, out[2*sy+1] = sum |r|^2
-  const int sy = threadIdx.x;
-  if (sy >= ns) return;
+// out[2*sy] = sum |res|^2, out[2*sy+1] = sum |r|^2; one warp per system (blockIdx.x)
+__global__ void k_loss_sum(const double* __restrict__ part, int nb, double* __restrict__ out) {
+  const int sy = blockIdx.x;
   double a = 0, b = 0;
-  for (int i = 0; i < nb; ++i) { a += part[((long)sy * nb + i) * 2]; b += part[((long)sy * nb + i) * 2 + 1]; }
+  for (int i = threadIdx.x; i < nb; i += 32) {
+    a += part[((long)sy * nb + i) * 2];
+    b += part[((long)sy * nb + i) * 2 + 1];
+  }
+  for (int m = 16; m > 0; m >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, m);
+    b += __shfl_xor_sync(0xffffffffu, b, m);
+  }
+  if (threadIdx.x) return;
   out[2 * sy] = a;
   out[2 * sy + 1] = b;
 }
@@ -350,14 +371,21 @@ __global__ void k_loss_grad(const int32_t* __restrict__ rowptr, const int32_t* _
   const int sy = blockIdx.y;
   const double om = omega[sy];
   const double f = 2.0 / sums[2 * sy + 1];
-  for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x) {
+  const int sub = threadIdx.x & 7;
+  const int step = (gridDim.x * blockDim.x) >> 3;
+  // the eight lanes of a row stay together, so the warp's four rows share its bounds
+  for (int first = (int)((blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 3); first < n; first += step) {
+    const int row = first + ((threadIdx.x >> 3) & 3);
+    const bool live = row < n;
     double t1x = 0, t1y = 0, t2x = 0, t2y = 0;
-    for (int k = rowptr[row]; k < rowptr[row + 1]; ++k) {
+    for (int k = live ? rowptr[row] + sub : 0, k1 = live ? rowptr[row + 1] : 0; k < k1; k += 8) {
       const double2 e = km[k];
       const double2 q = res[(long)col[k] * ns + sy];
       t1x += e.x * q.x; t1y += e.x * q.y;
       t2x += e.y * q.x; t2y += e.y * q.y;
     }
+    row_sum(t1x, t1y, t2x, t2y);
+    if (!live || sub) continue;
     // conj(A) q = K q - i omega M q
     const double gx = f * (t1x + om * t2y), gy = f * (t1y - om * t2x);
     const long i = (long)sy * n + row;
@@ -398,133 +426,192 @@ __global__ void k_decode_bwd(const __nv_bfloat16* __restrict__ h, long rows, con
   for (int k = threadIdx.x; k < H * 2; k += blockDim.x) atomicAdd(&gwout[k], red[k]);
 }
 
+__device__ __forceinline__ void ldsm4(unsigned (&r)[4], const __nv_bfloat16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a)
+               : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(unsigned (&r)[4], const __nv_bfloat16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a)
+               : "memory");
+}
+
 // Per 64-row tile: dY = dh * (Y > 0); dX = dY W^T (tensor cores); dW += X^T dY (tensor cores);
 // dc += sum dY.  dX goes to global (the neighbour part is aggregated by k_agg_bwd).
-__global__ void __launch_bounds__(128)
-    k_layer_bwd(long rows, const float* __restrict__ dh, const __nv_bfloat16* __restrict__ sx,
+// What bounded it were the atomic additions of dW (6912 per tile), of dc (3072 per tile in shared memory)
+// and the element-wise transposing copies.  A block takes several tiles and keeps its part of dW
+// (warp w: rows 16w .. 16w+15) and of dc in registers until the end, W_l's fragments stay in registers
+// (warp w: columns 16w .. 16w+15 of dX), and the transposed operands come from ldmatrix on row-major tiles
+// (strides of 304 and 112 bytes: an odd number of 16-byte words, so without bank conflicts).
+// 23,500 rows: 55 -> 21.2 us.
+__global__ void __launch_bounds__(32 * BWD_WARPS)
+    k_layer_bwd(long rows, int tiles, const float* __restrict__ dh, const __nv_bfloat16* __restrict__ sx,
                 const __nv_bfloat16* __restrict__ sy_, const __nv_bfloat16* __restrict__ wl,  // W_l bf16 [XW][H]
                 float* __restrict__ dx, float* __restrict__ gw, float* __restrict__ gc) {
-  // dynamic shared memory (50.6 KB): dY tile [row][H], dY^T [H][row], X^T [XW][row], W_l [XW][H]
-  constexpr int DS = H + 8, TS = ROWS + 8, WS = H + 8;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __nv_bfloat16* dys = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-  __nv_bfloat16* dyt = dys + ROWS * DS;
-  __nv_bfloat16* xt = dyt + H * TS;
-  __nv_bfloat16* wsm = xt + XW * TS;
+  constexpr int DS = H + 8, DSV = DS / 8, NT = 32 * BWD_WARPS;
+  static_assert(NT % HV == 0, "a thread keeps its column chunk of dY");
+  __shared__ __align__(16) __nv_bfloat16 xt[ROWS * XS];   // X tile [row][XW]
+  __shared__ __align__(16) __nv_bfloat16 dys[ROWS * DS];  // dY tile [row][H]
   __shared__ float csum[H];
-  const long r0 = (long)blockIdx.x * ROWS;
-  for (int k = threadIdx.x; k < XW * H; k += blockDim.x) wsm[(k / H) * WS + (k % H)] = wl[k];
-  if (threadIdx.x < H) csum[threadIdx.x] = 0.f;
-  for (int k = threadIdx.x; k < ROWS * H; k += blockDim.x) {
-    const int rr = k / H, c = k % H;
-    const long row = r0 + rr;
-    float v = 0.f;
-    if (row < rows) {
-      const float y = __bfloat162float(sy_[row * H + c]);
-      v = y > 0.f ? dh[row * H + c] : 0.f;
-    }
-    const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    dys[rr * DS + c] = b;
-    dyt[c * TS + rr] = b;
-  }
-  for (int k = threadIdx.x; k < ROWS * XW; k += blockDim.x) {
-    const int rr = k / XW, c = k % XW;
-    const long row = r0 + rr;
-    xt[c * TS + rr] = (row < rows) ? sx[row * XW + c] : __float2bfloat16_rn(0.f);
-  }
-  __syncthreads();
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  // dc
-  for (int k = threadIdx.x; k < ROWS * H; k += blockDim.x)
-    atomicAdd(&csum[k % H], __bfloat162float(dys[(k / H) * DS + (k % H)]));  // the tile's rows are padded to DS
-  // ---- dX (rows 16w.. x XW) = dY (16 x H) * W^T: B[k=j][n=m] = W[m][j] -> [n][k] = wsm rows
-  {
-    const unsigned* A = reinterpret_cast<const unsigned*>(dys);
-    const unsigned* B = reinterpret_cast<const unsigned*>(wsm);
-    for (int nt = 0; nt < XW / 8; ++nt) {
-      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  if (threadIdx.x < H) csum[threadIdx.x] = 0.f;
+  unsigned wf[2][H / 16][2];  // B[k=j][n=m] = W[m][j], m = 8 (2w + i) + g
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int ks = 0; ks < H / 16; ++ks) {
+      const unsigned* p = reinterpret_cast<const unsigned*>(wl + ((2 * w + i) * 8 + g) * H + ks * 16);
+      wf[i][ks][0] = p[t];
+      wf[i][ks][1] = p[4 + t];
+    }
+  float acc[H / 8][4];
+#pragma unroll
+  for (int nt = 0; nt < H / 8; ++nt)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[nt][q] = 0.f;
+  float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const int ch = threadIdx.x % HV;  // columns 8 ch .. 8 ch + 7 of dY
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const long r0 = (long)tile * ROWS;
+    __syncthreads();  // the tile before is read
+    for (int k = threadIdx.x; k < ROWS * XV; k += NT) {
+      const int rr = k / XV, q = k % XV;
+      const long row = r0 + rr;
+      reinterpret_cast<uint4*>(xt)[rr * XSV + q] =
+          row < rows ? reinterpret_cast<const uint4*>(sx + row * XW)[q] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (int rr = threadIdx.x / HV; rr < ROWS; rr += NT / HV) {
+      const long row = r0 + rr;
+      uint4 out = make_uint4(0u, 0u, 0u, 0u);
+      if (row < rows) {
+        const uint4 y4 = reinterpret_cast<const uint4*>(sy_ + row * H)[ch];
+        const float4 da = reinterpret_cast<const float4*>(dh + row * H)[2 * ch];
+        const float4 db = reinterpret_cast<const float4*>(dh + row * H)[2 * ch + 1];
+        const float d[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+        const unsigned y[4] = {y4.x, y4.y, y4.z, y4.w};
+        unsigned o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 v = unpack_bf16(y[k]);
+          o[k] = pack_bf16(v.x > 0.f ? d[2 * k] : 0.f, v.y > 0.f ? d[2 * k + 1] : 0.f);
+          const float2 b = unpack_bf16(o[k]);
+          cs[2 * k] += b.x;
+          cs[2 * k + 1] += b.y;
+        }
+        out = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      reinterpret_cast<uint4*>(dys)[rr * DSV + ch] = out;
+    }
+    __syncthreads();
+    // ---- dX columns 16w .. 16w+15 = dY (64 x H) W^T
+    for (int rg = 0; rg < ROWS / 16; ++rg) {
+      float d[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[i][q] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < H / 16; ++ks) {
-        const int kw = ks * 8;
-        unsigned a[4], b[2];
-        a[0] = A[(w * 16 + g) * (DS / 2) + kw + t];
-        a[1] = A[(w * 16 + g + 8) * (DS / 2) + kw + t];
-        a[2] = A[(w * 16 + g) * (DS / 2) + kw + 4 + t];
-        a[3] = A[(w * 16 + g + 8) * (DS / 2) + kw + 4 + t];
-        b[0] = B[(nt * 8 + g) * (WS / 2) + kw + t];
-        b[1] = B[(nt * 8 + g) * (WS / 2) + kw + 4 + t];
-        mma_bf16(acc, a, b);
+        unsigned a[4];
+        ldsm4(a, dys + (rg * 16 + (lane & 15)) * DS + ks * 16 + (lane >> 4) * 8);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) mma_bf16(d[i], a, wf[i][ks]);
       }
-      const int c = nt * 8 + 2 * t;
-      for (int half = 0; half < 2; ++half) {
-        const long row = r0 + w * 16 + g + half * 8;
-        if (row < rows) {
-          dx[row * XW + c] = acc[2 * half];
-          dx[row * XW + c + 1] = acc[2 * half + 1];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const long row = r0 + rg * 16 + g + half * 8;
+          if (row < rows)
+            *reinterpret_cast<float2*>(dx + row * XW + (2 * w + i) * 8 + 2 * t) =
+                make_float2(d[i][2 * half], d[i][2 * half + 1]);
         }
+    }
+    // ---- dW rows 16w .. 16w+15 += X^T (16 x 64) dY (64 x H): both operands transposed on the way
+#pragma unroll
+    for (int ks = 0; ks < ROWS / 16; ++ks) {
+      unsigned a[4];
+      ldsm4_t(a, xt + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * XS + w * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+      for (int np = 0; np < H / 16; ++np) {
+        unsigned b[4];
+        ldsm4_t(b, dys + (ks * 16 + (lane & 15)) * DS + np * 16 + (lane >> 4) * 8);
+        const unsigned b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+        mma_bf16(acc[2 * np], a, b0);
+        mma_bf16(acc[2 * np + 1], a, b1);
       }
     }
   }
-  // ---- dW (XW x H) += X^T (XW x 64 rows) * dY (64 x H): A = xt [m][k], B[k][n] = dY[k][n] -> [n][k] = dyt
-  {
-    const unsigned* A = reinterpret_cast<const unsigned*>(xt);
-    const unsigned* B = reinterpret_cast<const unsigned*>(dyt);
-    for (int mt = w; mt < XW / 16; mt += 4) {
-      for (int nt = 0; nt < H / 8; ++nt) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int ks = 0; ks < ROWS / 16; ++ks) {
-          const int kw = ks * 8;
-          unsigned a[4], b[2];
-          a[0] = A[(mt * 16 + g) * (TS / 2) + kw + t];
-          a[1] = A[(mt * 16 + g + 8) * (TS / 2) + kw + t];
-          a[2] = A[(mt * 16 + g) * (TS / 2) + kw + 4 + t];
-          a[3] = A[(mt * 16 + g + 8) * (TS / 2) + kw + 4 + t];
-          b[0] = B[(nt * 8 + g) * (TS / 2) + kw + t];
-          b[1] = B[(nt * 8 + g) * (TS / 2) + kw + 4 + t];
-          mma_bf16(acc, a, b);
-        }
-        const int m = mt * 16 + g, c = nt * 8 + 2 * t;
-        atomicAdd(&gw[m * H + c], acc[0]);
-        atomicAdd(&gw[m * H + c + 1], acc[1]);
-        atomicAdd(&gw[(m + 8) * H + c], acc[2]);
-        atomicAdd(&gw[(m + 8) * H + c + 1], acc[3]);
-      }
-    }
+  for (int k = 0; k < 8; ++k) atomicAdd(&csum[8 * ch + k], cs[k]);
+#pragma unroll
+  for (int nt = 0; nt < H / 8; ++nt) {
+    const int m = w * 16 + g, c = nt * 8 + 2 * t;
+    atomicAdd(reinterpret_cast<float2*>(gw + m * H + c), make_float2(acc[nt][0], acc[nt][1]));
+    atomicAdd(reinterpret_cast<float2*>(gw + (m + 8) * H + c), make_float2(acc[nt][2], acc[nt][3]));
   }
   __syncthreads();
   if (threadIdx.x < H) atomicAdd(&gc[threadIdx.x], csum[threadIdx.x]);
 }
 
-constexpr size_t LAYER_BWD_SMEM = sizeof(__nv_bfloat16) * ((size_t)ROWS * (H + 8) + (size_t)H * (ROWS + 8) +
-                                                           (size_t)XW * (ROWS + 8) + (size_t)XW * (H + 8));
-
-// dh_prev = dh + dX[:, :H] + sum_j a_ij dX_j[H:2H] + sum_j b_ij dX_j[2H:3H]   (a, b symmetric)
-__global__ void k_agg_bwd(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
-                          const double2* __restrict__ km, const float* __restrict__ s,
-                          const double* __restrict__ omega, int n, const float* __restrict__ dx,
-                          float* __restrict__ dh) {
+// dh_prev = dh + dX[:, :H] + sum_j a_ij dX_j[H:2H] + sum_j b_ij dX_j[2H:3H]   (a, b symmetric: the row's own
+// message weights).  A warp per row: lanes 0-11 sum the first part, lanes 12-23 the second, 16 bytes each,
+// so a neighbour's 384 bytes are one access and four are in flight; the row's columns and weights come in
+// one access each.  Bound by those gathers from the L2 (23,500 rows: 41 -> 22.5 us, where a neighbour was
+// three accesses of 4 bytes per lane behind its weight's division).
+__global__ void __launch_bounds__(256)
+    k_agg_bwd(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const float2* __restrict__ ew,
+              long nnz, int n, const float* __restrict__ dx, float* __restrict__ dh) {
+  constexpr int QV = H / 4;  // 16-byte words of a row's H values
   const int sy = blockIdx.y;
   const long base = (long)sy * n;
-  const double om = omega[sy];
+  const float2* ewr = ew + (long)sy * nnz;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
+  const bool second = lane >= QV;
+  const int word = QV + min(lane, 2 * QV - 1);
   for (int row = warp; row < n; row += nw) {
-    const float si = s[base + row];
-    float acc0 = 0.f, acc1 = 0.f;  // features lane, lane + 32 (< H)
-    for (int k = rowptr[row]; k < rowptr[row + 1]; ++k) {
-      const int j = col[k];
-      if (j == row) continue;
-      const double2 a = km[k];
-      const float inv = 1.0f / (si * s[base + j]);
-      const float wa = (float)a.x * inv, wb = (float)(om * a.y) * inv;
-      const float* dj = dx + (base + j) * XW;
-      acc0 += wa * dj[H + lane] + wb * dj[2 * H + lane];
-      if (lane + 32 < H) acc1 += wa * dj[H + lane + 32] + wb * dj[2 * H + lane + 32];
+    const int k1 = rowptr[row + 1];
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int kb = rowptr[row]; kb < k1; kb += 32) {
+      const int cnt = min(32, k1 - kb);
+      const int jl = lane < cnt ? col[kb + lane] : row;
+      const float2 wl = lane < cnt ? ewr[kb + lane] : make_float2(0.f, 0.f);
+      for (int m = 0; m < cnt; m += 4) {
+        float4 v[4];
+        float wv[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // m + q <= 31; beyond cnt the lane holds the row itself, which is left out
+          const int j = __shfl_sync(0xffffffffu, jl, m + q);
+          const float wa = __shfl_sync(0xffffffffu, wl.x, m + q), wb = __shfl_sync(0xffffffffu, wl.y, m + q);
+          wv[q] = second ? wb : wa;
+          v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (j != row && lane < 2 * QV) v[q] = reinterpret_cast<const float4*>(dx + (base + j) * XW)[word];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc.x += wv[q] * v[q].x; acc.y += wv[q] * v[q].y;
+          acc.z += wv[q] * v[q].z; acc.w += wv[q] * v[q].w;
+        }
+      }
     }
-    const float* di = dx + (base + row) * XW;
-    dh[(base + row) * H + lane] += di[lane] + acc0;
-    if (lane + 32 < H) dh[(base + row) * H + lane + 32] += di[lane + 32] + acc1;
+    const float bx = __shfl_down_sync(0xffffffffu, acc.x, QV), by = __shfl_down_sync(0xffffffffu, acc.y, QV);
+    const float bz = __shfl_down_sync(0xffffffffu, acc.z, QV), bw = __shfl_down_sync(0xffffffffu, acc.w, QV);
+    if (lane < QV) {
+      const float4 di = reinterpret_cast<const float4*>(dx + (base + row) * XW)[lane];
+      float4* out = reinterpret_cast<float4*>(dh + (base + row) * H) + lane;
+      float4 o = *out;
+      o.x += di.x + (acc.x + bx);
+      o.y += di.y + (acc.y + by);
+      o.z += di.z + (acc.z + bz);
+      o.w += di.w + (acc.w + bw);
+      *out = o;
+    }
   }
 }
 
@@ -670,7 +757,7 @@ void rowinfo(afem_ctx* c, MpnnState* S, int ns) {
                                                        S->feat.p);
   count_launch();
   S->ew.alloc((size_t)ns * c->nnz);
-  k_edge_w<<<blocks(rows, 128), 128, 0, c->stream>>>(c->rowptr.p, c->col.p, c->km.p, S->s.p, S->omega.p, c->nline, ns,
+  k_edge_w<<<blocks(rows * 8, 256), 256, 0, c->stream>>>(c->rowptr.p, c->col.p, c->km.p, S->s.p, S->omega.p, c->nline, ns,
                                                      c->nnz, S->ew.p);
   count_launch();
 }
@@ -688,9 +775,9 @@ void forward(afem_ctx* c, MpnnState* S, int ns, const V* r, V* z, bool train, co
   for (int l = 0; l < L; ++l) {
     const __nv_bfloat16* hin = train ? S->h[l].p : S->h[l & 1].p;
     __nv_bfloat16* hout = train ? S->h[l + 1].p : S->h[(l + 1) & 1].p;
-    k_layer<<<grid, 128, 0, st>>>(c->rowptr.p, c->col.p, S->ew.p, c->nnz, n, hin, hout,
-                                  S->wt.p + (size_t)l * XW * H, S->small.p + FIN * H + l * H,
-                                  train ? S->sx[l].p : nullptr, train ? S->sy[l].p : nullptr, skip);
+    k_layer<<<grid, LAYER_THREADS, 0, st>>>(c->rowptr.p, c->col.p, S->ew.p, c->nnz, n, hin, hout,
+                                            S->wt.p + (size_t)l * XW * H, S->small.p + FIN * H + l * H,
+                                            train ? S->sx[l].p : nullptr, train ? S->sy[l].p : nullptr, skip);
     count_launch();
   }
   const __nv_bfloat16* hl = train ? S->h[L].p : S->h[L & 1].p;
@@ -707,11 +794,6 @@ double loss_backward(afem_ctx* c, MpnnState* S, int ns, const double2* r) {
   const long rows = (long)n * ns;
   S->z64.alloc(rows);
   S->res.alloc(rows);
-  static bool attr_set = false;
-  if (!attr_set) {
-    AFEM_CUDA(cudaFuncSetAttribute(k_layer_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LAYER_BWD_SMEM));
-    attr_set = true;
-  }
   rowinfo(c, S, ns);
   if (S->base) {
     // z = H(r) + correction: the base preconditioner's output first, the network adds to it
@@ -722,33 +804,39 @@ double loss_backward(afem_ctx* c, MpnnState* S, int ns, const double2* r) {
     precond_apply_device(c, om, r, S->z64.p);
   }
   forward<double2>(c, S, ns, r, S->z64.p, true, nullptr, nullptr, S->base);
-  const int nb = std::min(1024, (int)blocks(n, 256));
+  const int nb = std::min(1024, (int)blocks(8L * n, 256));
   S->part.alloc((size_t)2 * nb * ns);
   S->sums.alloc(2 * ns);
   k_loss_res<<<dim3(nb, ns), 256, 0, st>>>(c->rowptr.p, c->col.p, c->km.p, S->omega.p, n, ns, S->z64.p, r, S->res.p,
                                            S->part.p);
   count_launch();
-  k_loss_sum<<<1, 32, 0, st>>>(S->part.p, nb, ns, S->sums.p);
+  k_loss_sum<<<ns, 32, 0, st>>>(S->part.p, nb, S->sums.p);
   count_launch();
   k_loss_grad<<<dim3(nb, ns), 256, 0, st>>>(c->rowptr.p, c->col.p, c->km.p, S->omega.p, n, ns, S->res.p, S->sums.p,
                                             S->rms.p, S->s.p, S->dout.p);
   count_launch();
   float* G = S->grad.p;
-  k_decode_bwd<<<std::min(1024u, blocks(rows, 256)), 256, 0, st>>>(S->h[L].p, rows, S->dout.p,
+  // warps of about 8 rows (4 or 16: 1 to 2 % more of a training pass): enough of them to hide the loads,
+  // few enough for the sums at their ends
+  const unsigned wide = std::min(c->num_sms * 8u, blocks(rows, 64));
+  k_decode_bwd<<<wide, 256, 0, st>>>(S->h[L].p, rows, S->dout.p,
                                                                   S->small.p + FIN * H + L * H, S->dh.p,
                                                                   G + off_wout());
   count_launch();
+  // as many tiles per block as leave two blocks per SM, the blocks evenly loaded (one per SM: 3 % more of a
+  // training pass on 23,500 rows, four: 8 %)
+  const int tiles = (int)blocks(rows, ROWS);
+  const int per = (int)blocks(tiles, c->num_sms * 2);
   for (int l = L - 1; l >= 0; --l) {
-    k_layer_bwd<<<blocks(rows, ROWS), 128, LAYER_BWD_SMEM, st>>>(rows, S->dh.p, S->sx[l].p, S->sy[l].p,
-                                                                 S->wl.p + (size_t)l * XW * H, S->dx.p, G + off_w(l),
-                                                                 G + off_c(l));
+    k_layer_bwd<<<blocks(tiles, per), 32 * BWD_WARPS, 0, st>>>(rows, tiles, S->dh.p, S->sx[l].p, S->sy[l].p,
+                                                               S->wl.p + (size_t)l * XW * H, S->dx.p, G + off_w(l),
+                                                               G + off_c(l));
     count_launch();
-    k_agg_bwd<<<dim3(std::min(4096u, blocks(n, 8)), ns), 256, 0, st>>>(c->rowptr.p, c->col.p, c->km.p, S->s.p,
-                                                                       S->omega.p, n, S->dx.p, S->dh.p);
+    k_agg_bwd<<<dim3(std::min(4096u, blocks(n, 8)), ns), 256, 0, st>>>(c->rowptr.p, c->col.p, S->ew.p, c->nnz, n,
+                                                                       S->dx.p, S->dh.p);
     count_launch();
   }
-  k_encode_bwd<double2><<<std::min(1024u, blocks(rows, 256)), 256, 0, st>>>(r, n, ns, S->s.p, S->feat.p, S->rms.p,
-                                                                            S->dh.p, G + off_win());
+  k_encode_bwd<double2><<<wide, 256, 0, st>>>(r, n, ns, S->s.p, S->feat.p, S->rms.p, S->dh.p, G + off_win());
   count_launch();
   AFEM_CUDA(cudaGetLastError());
   std::vector<double> h(2 * ns);
