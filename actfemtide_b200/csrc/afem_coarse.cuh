@@ -6,7 +6,7 @@
 
 namespace afem {
 
-constexpr int COARSE_TAIL = 500;      // nodes of the first level the one-block cycle takes
+constexpr int COARSE_TAIL = 600;      // nodes of the first level the one-block cycle takes
 constexpr int COARSE_STOP = 300;      // a grid of at most this many nodes is the coarsest
 constexpr int COARSE_SWEEPS = 4;      // smoothing sweeps on the coarsest grid
 constexpr int TAIL_THREADS = 512;

@@ -1512,7 +1512,9 @@ __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename
 // one row, so the 8 threads of a row read and write its FP64 values (p, x) as one
 // 256-byte run of 32-byte accesses and its FP32 values (z, u) as one 128-byte run
 // of 16-byte accesses; the systems' scalars stay in registers.  The grid-stride is
-// a multiple of 8, so a thread keeps the same 2 systems throughout.
+// a multiple of 8, so a thread keeps the same 2 systems throughout.  Four blocks per SM (64 registers): a
+// grid of eight per SM is then two full waves (0.33 -> 0.27 ms for 16 systems of 830,000 rows, where 72
+// registers left three and a last wave two thirds full).
 template <class T, class PT, int NS>
 __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typename Cx<T>::V* p, const SysScal* sc,
                                          bool done, bool first, double2* x, const int32_t* __restrict__ line,
@@ -1595,7 +1597,7 @@ __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typ
 }
 
 template <class T, class PT, int NS>
-__global__ void k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
+__global__ void __launch_bounds__(256, 4) k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
                            const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, double2* __restrict__ x,
                            int nsys, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
                            const typename Cx<PT>::V* __restrict__ u, const double* __restrict__ te) {
@@ -2136,6 +2138,38 @@ __global__ void __launch_bounds__(256)
                             gridDim.x, buf);
   if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
     finish_rho(sc, ctrl, sums, edge_rho, grid_rho, MAX_SYS, nsys);
+}
+
+// r = b in the COCG's type and the block sums of |b|^2 in k_init_sys's layout (one pass over b, where a
+// residual SpMV on x = 0 reads the matrix as well).
+template <class T, int NS, bool SEG>
+__global__ void __launch_bounds__(256)
+    k_start(long total, const double2* __restrict__ b, typename Cx<T>::V* __restrict__ r,
+            const uint8_t* __restrict__ seg, double* __restrict__ part) {
+  double v[1] = {0.0};
+  double (*red)[MAX_SYS][1] = nullptr;
+  if constexpr (SEG) red = seg_sums<8, 1>();
+  const long stride = (long)gridDim.x * blockDim.x;  // a multiple of NS: a lane keeps its system
+  const long span = (total + stride - 1) / stride * stride;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < span; i += stride) {
+    double e[1] = {0.0};
+    int sid = -1;
+    if (i < total) {
+      const double2 x = b[i];
+      r[i] = Cx<T>::make((T)x.x, (T)x.y);
+      e[0] = x.x * x.x + x.y * x.y;
+      if constexpr (SEG) sid = __ldg(seg + i);
+    }
+    if constexpr (SEG) seg_warp_sum<1>(red, threadIdx.x >> 5, sid, e);
+    else v[0] += e[0];
+  }
+  if constexpr (SEG) {
+    seg_partials<8, 1>(red, part);
+  } else {
+#pragma unroll
+    for (int m = NS; m < 32; m <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], m);
+    block_partials<NS, 1>(v, part);
+  }
 }
 
 // One step of the power iteration on D_K^-1 K and D_M^-1 M at once (x and y of the vectors): 8 lanes
@@ -3346,14 +3380,16 @@ void smoother_values(afem_ctx* c, SolverWork* w, const double* d_omega) {
 }
 
 // FP64 true residual r64 = b - A x; returns per-system ||r||^2 and ||b||^2 on the host.
+// fast: several rows per warp, as the smoothed iteration's SpMV (1.67 -> 0.6 ms for one system of 3.2 M
+// rows); the other iterations keep one, and with it the order of their sums.
 template <int NS, bool SEG>
-void true_residual(afem_ctx* c, SolverWork* w, std::vector<double>& rr, std::vector<double>& bb) {
+void true_residual(afem_ctx* c, SolverWork* w, bool fast, std::vector<double>& rr, std::vector<double>& bb) {
   cudaStream_t s = c->stream;
   const int nsys = w->nsys;
-  k_spmv<double, NS, 1, SEG><<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p, c->km.p,
-                                                        w->n, w->x.p, w->r64.p, w->sc.p, (const Ctrl*)nullptr,
-                                                        w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr,
-                                                        RedSet{}, 0, AFEM_SPMV_CHUNK);
+  auto k = fast ? k_spmv<double, NS, (NS <= 8 ? 4 : 2), SEG> : k_spmv<double, NS, 1, SEG>;
+  k<<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p, c->km.p, w->n, w->x.p, w->r64.p,
+                               w->sc.p, (const Ctrl*)nullptr, w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr,
+                               RedSet{}, 0, AFEM_SPMV_CHUNK);
   count_launch();
   DBuf<double> out;
   out.alloc(2 * nsys);
@@ -3410,12 +3446,14 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   const int nsys = w->nsys;
   const long total = (long)n * NS;
   // r = rhs (as T), x = 0, ||b||^2
-  k_copy_r<typename I::V><<<c->num_sms * 8, 256, 0, s>>>(w->r64.p, I::R(w), total);
-  count_launch();
-  // ||r64||^2 via partials of a dedicated pass
-  {
-    // reuse SpMV-with-b path on x = 0: part[0] = ||b||^2
-    AFEM_CUDA(cudaMemsetAsync(w->x.p, 0, sizeof(double2) * total, s));
+  AFEM_CUDA(cudaMemsetAsync(w->x.p, 0, sizeof(double2) * total, s));
+  if (smoothed(c, w, precond)) {
+    k_start<T, NS, SEG><<<w->nblocks, 256, 0, s>>>(total, w->r64.p, I::R(w), SEG ? c->seg_of_row.p : nullptr, w->part.p);
+    count_launch();
+  } else {
+    k_copy_r<typename I::V><<<c->num_sms * 8, 256, 0, s>>>(w->r64.p, I::R(w), total);
+    count_launch();
+    // the SpMV-with-b path on x = 0: part[0] = ||b||^2
     k_spmv<double, NS, 1, SEG><<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p,
                                                           c->km.p, n, w->x.p, w->q.p, w->sc.p, (const Ctrl*)nullptr,
                                                           w->part.p, w->r64.p, SEG ? c->seg_of_row.p : nullptr,
@@ -3805,7 +3843,7 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
   if (ex && ex->x0) {
     xacc.upload(reinterpret_cast<const double2*>(ex->x0), total, s);
     AFEM_CUDA(cudaMemcpyAsync(w->x.p, xacc.p, sizeof(double2) * total, cudaMemcpyDeviceToDevice, s));
-    true_residual<NS, SEG>(c, w, rr, bb);  // r64 = b - A x0
+    true_residual<NS, SEG>(c, w, false, rr, bb);  // r64 = b - A x0
     double worst_r = 0.0;
     for (int k = 0; k < nsys; ++k)
       if (bb[k] > 0) worst_r = std::max(worst_r, std::sqrt(rr[k] / bb[k]));
@@ -3869,7 +3907,7 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
     k_add_x<<<c->num_sms * 8, 256, 0, s>>>(xacc.p, w->x.p, total);
     count_launch();
     AFEM_CUDA(cudaMemcpyAsync(w->x.p, xacc.p, sizeof(double2) * total, cudaMemcpyDeviceToDevice, s));
-    true_residual<NS, SEG>(c, w, rr, bb);  // r64 = b - A x_acc
+    true_residual<NS, SEG>(c, w, smoothed(c, w, precond_now), rr, bb);  // r64 = b - A x_acc
     worst = 0.0;
     rec = 0.0;
     bool all_ok = true, any_fatal = false;
