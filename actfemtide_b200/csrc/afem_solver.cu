@@ -12,6 +12,9 @@
 //   k_pupd  : p = z + beta p
 //   k_spmv  : q = A p, p^T q
 //   k_scal_pq: alpha = rho / p^T q, rho1 = rho, epoch++
+// The hybrid preconditioner's iteration is six steps (k_r_update, k_smooth, the coarse cycle,
+// k_node_prolong, k_pupd, k_spmv: see enqueue_smoothed), their scalar steps in the kernels' last blocks,
+// and one launch for small systems (k_small).
 // Every kernel returns at once after the batch has finished, so a captured
 // chunk of iterations can run past convergence harmlessly.
 //
@@ -2027,6 +2030,9 @@ __global__ void __launch_bounds__(256, (NS >= 8 ? MC_MIN_BLOCKS : 0))
 // w = (u + T O_0, T O_1, T O_2, T O_3) at every mesh node, in [node][4][system], with the nodes'
 // smoother u = c1 hs - c2 D_G^-1 A_G hs (the polynomial of the edges, on A_G = G^T A G) and their
 // share t_0^T u of rho; the last block forms rho and beta.  coef: the edges' and the nodes' pairs.
+// A node's lanes split the entries of its row of A_G, then gather their own component's corners: with the
+// row on component 0's lanes alone three quarters of a warp waited for it (16 systems of 830,000 rows
+// 206 -> 165 us, one of 3.2 M 106 -> 78).
 template <class T, int NS, bool SEG, bool RO>
 __device__ __forceinline__ void prolong(int node, const uint8_t* nseg, const CoarseGrid* grids, const int32_t* cell,
                                         const double* frac, const typename Cx<T>::V* O, const typename Cx<T>::V* t,
@@ -2048,33 +2054,47 @@ __device__ __forceinline__ void prolong(int node, const uint8_t* nseg, const Coa
   }
   double (*red)[MAX_SYS][2] = nullptr;
   if constexpr (SEG) red = seg_sums<8, 2>();
-  const long span = SEG ? (total + stride - 1) / stride * stride : total;  // SEG: whole warps (shuffles)
+  const long whole = SEG ? stride : 32;  // whole warps (shuffles)
+  const long span = (total + whole - 1) / whole * whole;
   for (long i = i0; i < span; i += stride) {
     const int a = (int)(i / GPR);
     int sid = -1;
     double e[2] = {0.0, 0.0};
-    if (i < total) {
+    const bool live = i < total;
+    // the node's row of A_G, a quarter of it per component's lanes
+    T t1x[SP], t1y[SP], t2x[SP], t2y[SP];
+#pragma unroll
+    for (int j = 0; j < SP; ++j) t1x[j] = t1y[j] = t2x[j] = t2y[j] = 0;
+    {
+      const int k1 = live ? __ldg(rowptr + a + 1) : 0;
+#pragma unroll 2
+      for (int k = (live ? __ldg(rowptr + a) : 0) + c; k < k1; k += 4) {
+        const double2 m = __ldg(km + k);
+        V x[SP];
+        load_spl<V, NS, SP, false, RO>(hs + (long)__ldg(col + k) * NS + s0, x);
+#pragma unroll
+        for (int j = 0; j < SP; ++j) {
+          t1x[j] += (T)m.x * x[j].x; t1y[j] += (T)m.x * x[j].y;
+          t2x[j] += (T)m.y * x[j].x; t2y[j] += (T)m.y * x[j].y;
+        }
+      }
+    }
+#pragma unroll
+    for (int m = GPC; m < GPR; m <<= 1)
+#pragma unroll
+      for (int j = 0; j < SP; ++j) {
+        t1x[j] += shfl_xor(t1x[j], m);
+        t1y[j] += shfl_xor(t1y[j], m);
+        t2x[j] += shfl_xor(t2x[j], m);
+        t2y[j] += shfl_xor(t2y[j], m);
+      }
+    if (live) {
       if constexpr (SEG) sid = __ldg(nseg + a);
       V o[SP];
 #pragma unroll
       for (int j = 0; j < SP; ++j) o[j] = Cx<T>::make(0, 0);
       if (c == 0) {
         if constexpr (SEG) om[0] = sc[sid].omega;
-        T t1x[SP], t1y[SP], t2x[SP], t2y[SP];
-#pragma unroll
-        for (int j = 0; j < SP; ++j) t1x[j] = t1y[j] = t2x[j] = t2y[j] = 0;
-        const int k1 = __ldg(rowptr + a + 1);
-#pragma unroll 4
-        for (int k = __ldg(rowptr + a); k < k1; ++k) {
-          const double2 m = __ldg(km + k);
-          V x[SP];
-          load_spl<V, NS, SP, false, RO>(hs + (long)__ldg(col + k) * NS + s0, x);
-#pragma unroll
-          for (int j = 0; j < SP; ++j) {
-            t1x[j] += (T)m.x * x[j].x; t1y[j] += (T)m.x * x[j].y;
-            t2x[j] += (T)m.y * x[j].x; t2y[j] += (T)m.y * x[j].y;
-          }
-        }
         V ti[SP], si[SP], dd[SP];
         load_spl<V, NS, SP, false, RO>(t + (long)a * 4 * NS + s0, ti);
         load_spl<V, NS, SP, false, RO>(hs + (long)a * NS + s0, si);

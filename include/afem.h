@@ -56,17 +56,19 @@ typedef enum afem_precond {
   AFEM_PRECOND_NONE = 3,
   AFEM_PRECOND_LEARNED = 4,  /* flexible COCG with the learned network; SSOR-COCG restart when it stalls */
   AFEM_PRECOND_SSOR_MC = 5,  /* SSOR of the colour-permuted matrix: every sweep is ~10 parallel passes */
-  AFEM_PRECOND_HYBRID = 6    /* multicolour SSOR plus a gradient-space correction G SSOR_node(G^T r)
-                                (Hiptmair's hybrid smoother, additive) and, in afem_solve, a coarse-grid
-                                correction in the nodal scalar and vector spaces; needs the mesh */
+  AFEM_PRECOND_HYBRID = 6    /* polynomial smoothing of the edges and of the gradient space G (Hiptmair's
+                                hybrid smoother, additive) plus a coarse-grid correction in the nodal scalar
+                                and vector spaces; multicolour SSOR sweeps in place of the polynomials
+                                where sigma_diag is not 1 or the mesh is too small for a coarse grid, and in
+                                the learned base; needs the mesh */
 } afem_precond;
 
 typedef enum afem_precision {
   AFEM_FP64 = 0,          /* every kernel in complex FP64 */
   AFEM_MIXED = 1,         /* inner COCG in complex FP32, FP64 iterative refinement outside */
   AFEM_FP32_PRECOND = 2   /* COCG in complex FP64 (SpMV, residuals, x, p, alpha/beta, the true-residual
-                             check) with the multicolour preconditioner (SSOR_MC, HYBRID: its sweeps,
-                             matrix copies, nodal correction and vectors) in complex FP32 */
+                             check) with the preconditioner (SSOR_MC, HYBRID: its sweeps or smoothing,
+                             matrix copies, nodal and coarse corrections and vectors) in complex FP32 */
 } afem_precision;
 
 typedef struct afem_solve_opts {
