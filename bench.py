@@ -13,12 +13,12 @@ and seeded (no dataset exists for it).
 
 Methods (preconditioner, precision, systems per step): plain = SSOR-COCG
 FP64, one system (the reference's solver on the device, natural row order);
-plain-mc = the multicolour SSOR; hybrid = multicolour SSOR plus the
-gradient-space (nodal) correction; mixed = hybrid with FP32 inner COCG
+plain-mc = the multicolour SSOR; hybrid = polynomial smoothing of the edges
+and of the gradient space plus the auxiliary-space coarse correction; mixed = hybrid with FP32 inner COCG
 under FP64 refinement; *-pc32 = FP64 COCG with the preconditioner in FP32;
 batched / batched-mixed / batched-pc32 = 8 tidal periods x 2 source patterns =
 16 systems per solve (batched-pc32 is the default); learned* = flexible COCG with the learned
-network (flexible COCG, z = H(r) + N(r) over the gradient-corrected SSOR H when
+network (flexible COCG, z = H(r) + N(r) over the hybrid preconditioner H when
 that checkpoint exists); packed = 24 uneven meshes (n x n x 3n/4, n in 8..32)
 in one solve.
 
@@ -58,7 +58,6 @@ TRAFFIC = {
     "cocg_spmv_fp64pc32_ns16_rpw8": {"bytes": 4.085e9, "rows": 4193536, "source": _T96},
     "cocg_fwd_sweep_mc_fp64pc32_ns16": {"bytes": 5.877e9, "rows": 4193536, "source": _T96},
     "cocg_bwd_sweep_mc_fp64pc32_ns16": {"bytes": 3.163e9, "rows": 4193536, "source": _T96},
-    "cocg_p_update_fp64pc32_ns16": {"bytes": 4.931e9, "rows": 4193536, "source": _T96},
     "cocg_nodal_correction_fp64pc32_ns16": {"bytes": 1.991e9, "rows": 4193536, "source": _T96},
 }
 DEFAULT_METHOD = "batched-pc32"
@@ -153,7 +152,8 @@ def kernel_bytes(name: str, n: int, nnz: int, ns: int, ntet: int = 0, nsrc: int 
     """Algorithmic bytes of one launch of the named kernel (values read/written once).
 
     mc: multicolour iteration (x += alpha p moves from the forward sweep to the p
-    update); fold: the hybrid's z += G u is formed inside the p update.  The COCG
+    update); fold: the hybrid's nodal correction (gradient and vector parts) is added inside
+    the p update.  The COCG
     vectors (r, p, q) and the SpMV use the COCG width, the preconditioner's matrix
     copies and vectors (y, z, nodal t, u) the preconditioner width (the name's tag)."""
     rb, pb = widths(name)
@@ -173,13 +173,28 @@ def kernel_bytes(name: str, n: int, nnz: int, ns: int, ntet: int = 0, nsrc: int 
         # rho from the diagonal, packed batches read r instead for their per-mesh rho
         b = pent * off + 8 * n + 16 * n + n * 2 * pvec
         return b + n * vec if "_seg" in name else b
+    nnz_g = node + 2 * n              # node graph: the node and its edge neighbours
+    if name.startswith("cocg_r_update"):
+        # r read and write, q read, s = D^-1 r written, the FP64 (K, M) diagonal pair
+        return n * (3 * vec + pvec + 16)
+    if name.startswith("cocg_smoother"):
+        # edges: all entries and rowptr; s (gathers counted once) and r read, z written, diagonal pair;
+        # nodes: the edge list of each node, Dirichlet flags, edge vectors, t (4 components) and hs written,
+        # the nodal diagonal read
+        edge = pent * nnz + 4 * (n + 1) + n * (2 * pvec + vec + 16)
+        return edge + 8 * n + 4 * (node + 1) + n + 24 * n + 6 * node * pvec
+    if name.startswith("cocg_coarse_cycle"):
+        # of its launches only what touches the mesh: t and the 8 weights of every node (the grids are small)
+        return node * (4 * pvec + 96)
+    if name.startswith("cocg_prolongation"):
+        # node graph with FP64 values; t_0, hs and the nodal diagonal read, 4 components written; cell and weights
+        return 20 * nnz_g + 4 * (node + 1) + node * (7 * pvec + 28)
     if name.startswith("cocg_nodal_correction"):
-        nnz_n = node + 2 * n          # node graph: the node and its edge neighbours
         pvn = pvec                    # nodal vectors have the edge vectors' width
         gt = 4 * (node + 1) + 8 * n + n + n * vec + node * pvn
         # two sweeps, each over its half of the off-diagonal entries, with pointers and ids;
         # forward: t, dd read, y write; backward: y read and write, dd read
-        sweeps = 2 * (pent * (nnz_n - node) // 2 + 4 * (node + 1) + 4 * node + 3 * node * pvn)
+        sweeps = 2 * (pent * (nnz_g - node) // 2 + 4 * (node + 1) + 4 * node + 3 * node * pvn)
         if fold:  # the backward nodal sweep also reads t for t^T u
             return gt + sweeps + node * pvn
         gadd = 8 * n + n + 2 * n * pvec + n * vec + node * pvn
@@ -198,7 +213,7 @@ def kernel_bytes(name: str, n: int, nnz: int, ns: int, ntet: int = 0, nsrc: int 
         if mc:
             b += n * 32 * ns                # x read and write (FP64)
         if fold:
-            b += 8 * n + n + node * pvec    # line, bc, u (each node once)
+            b += 8 * n + n + 24 * n + 4 * node * pvec  # line, bc, edge vectors, u's 4 components (each node once)
         return b
     if name.startswith("assemble_rows"):
         # tetrahedron data (n4, n6line, tag, sigma), node coordinates, adjacency, pattern, values, rhs
@@ -452,7 +467,7 @@ def run_gpu(args):
             dom, dom_ms, dom_n = name, kms, cnt
     pc = kw["precond"]
     mc = pc in ("SSOR_MC", "HYBRID") or "learned" in args.method
-    fold = pc == "HYBRID" and not args.method.startswith("packed")
+    fold = pc == "HYBRID"
     per_launch = kernel_bytes(dom or "", n, nnz, ns, job.ntet, job.nsrc, job.node, job.nodes, mc=mc, fold=fold)
     achieved = per_launch / (dom_ms / max(1, dom_n) / 1e3) / 1e9 if dom_ms > 0 else 0.0
     traffic, traffic_src = None, None
@@ -490,7 +505,7 @@ def run_gpu(args):
                    else {"workload": job.desc.format(n=n, nnz=nnz), "solves_per_step": ns,
                          "parallelism": f"replicas x{ws}"}),
         "method": {"name": args.method, "preconditioner": kw["precond"], "precision": kw["precision"],
-                   "note": "batched gradient-corrected (Hiptmair hybrid) multicolour-SSOR COCG; the learned network "
+                   "note": "batched COCG with polynomial smoothing and auxiliary-space coarse correction; the learned network "
                            "is not in this method (it does not pay on these models)" if "learned" not in args.method
                    else "flexible COCG with the learned correction"},
         "solver": {"iterations_median": int(np.median(iters)), "refinements_median": int(np.median(refs)),
