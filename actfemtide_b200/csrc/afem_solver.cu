@@ -66,7 +66,9 @@ struct SysScal {
   int status;     // afem_status of this system
   int iter;       // iterations done
   int xpend;      // multicolour path: this iteration's x += alpha p waits for the p update
+  int renew;      // smoothed path: r is formed anew from x once (see exact_residual)
 };
+enum Renew { RENEW_WAIT, RENEW_TURN, RENEW_RESTART, RENEW_FIRST, RENEW_DONE };  // in the order of SysScal::renew
 
 struct Ctrl {
   unsigned epoch;  // flag generation, increases by one per sweep pair, never reset
@@ -74,6 +76,9 @@ struct Ctrl {
   int iter;        // iterations of the current inner solve
   int maxit;
   double tol;
+  double renew_tol;     // smoothed path: a system at this residual has its r formed anew (0: none)
+  int renew_mask;       // ... in the iterations whose number has these bits set
+  int renew;            // ... a system's turn is this iteration
   unsigned spin_limit;  // polls of a bounded wait before DEV_TIMEOUT (0: SPIN_LIMIT)
 };
 
@@ -1367,10 +1372,10 @@ __device__ __forceinline__ void sum_partials(const double* part, int nblocks, in
 __device__ __forceinline__ double2 d_cdiv(double2 a, double2 b) { return cdiv(a, b); }
 
 // The three scalar steps of an iteration, run by one block on the sums v[system]:
-// ||r||^2 -> RESID, convergence, iteration cap, pending x update;
+// ||r||^2 -> RESID, convergence, iteration cap, pending x update, residuals to be formed anew;
 __device__ __forceinline__ void finish_r(SysScal* sc, Ctrl* ctrl, const double2* v, int nsys) {
-  __shared__ int any_active;
-  if (threadIdx.x == 0) any_active = 0;
+  __shared__ int any_active, any_renew;
+  if (threadIdx.x == 0) any_active = any_renew = 0;
   __syncthreads();
   if (threadIdx.x < nsys) {
     SysScal& S = sc[threadIdx.x];
@@ -1384,9 +1389,19 @@ __device__ __forceinline__ void finish_r(SysScal* sc, Ctrl* ctrl, const double2*
       else if (ctrl->iter >= ctrl->maxit) { S.active = 0; S.status = AFEM_EMAXITER; }
       else any_active = 1;
     }
+    if (S.renew == RENEW_RESTART) S.renew = RENEW_FIRST;
+    else if (S.renew != RENEW_WAIT) S.renew = RENEW_DONE;
+    if (S.active && S.renew == RENEW_WAIT && S.resid <= ctrl->renew_tol &&
+        (ctrl->iter & ctrl->renew_mask) == ctrl->renew_mask) {
+      S.renew = RENEW_TURN;
+      any_renew = 1;
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !any_active) ctrl->done = 1;
+  if (threadIdx.x == 0) {
+    ctrl->renew = any_renew;
+    if (!any_active) ctrl->done = 1;
+  }
 }
 
 // rho = r^T z from the edges', the nodes' and the grids' shares -> beta;
@@ -1399,6 +1414,7 @@ __device__ __forceinline__ void finish_rho(SysScal* sc, const Ctrl* ctrl, const 
   S.rho = a;
   if (S.active) {
     if (a.x == 0.0 && a.y == 0.0) { S.active = 0; S.status = AFEM_EBREAKDOWN; }
+    else if (S.renew == RENEW_FIRST) S.beta = make_double2(0.0, 0.0);
     else if (ctrl->iter > 0) S.beta = d_cdiv(S.rho, S.rho1);
   }
 }
@@ -1741,6 +1757,7 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
 //   coarse_cycle:  the V-cycles;
 //   k_node_prolong: the nodal correction w at the mesh nodes, with the nodes' smoother; rho -> beta;
 //   k_pupd:        x += alpha p, p = z + (correction of w) + beta p;
+//   k_exact_residual: r = b - A x, once a solve;
 //   k_spmv:        q = A p, p^T q -> alpha.
 // The scalar steps run in the last block of the kernel that produced their sums.
 constexpr double CHEB_SAFETY = 1.25;  // on the power iteration's estimate of the largest eigenvalue (0.79 of it
@@ -1858,6 +1875,165 @@ __global__ void __launch_bounds__(256)
   __shared__ double2 sums[MAX_SYS], buf[8 * NS];
   r_update<T, PT, NS, SEG>(n, r, q, s, dkm, sc, ctrl->iter > 0, seg, R, blockIdx.x, gridDim.x, buf);
   if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_r(sc, ctrl, sums, nsys);
+}
+
+// r = b - A x with products and sums carried in two doubles (two-sum, and the product's error by FMA;
+// Ogita, Rump and Oishi, SIAM J. Sci. Comput. 26, 2005): rounded once, and not term by term.
+// The recursion's r -= alpha q leaves in x what the products q rounded off.  On the gradients A is
+// i omega M alone, 1e-12 of the rest in the air, so that these roundings, harmless to the residual, are
+// an error of 2 to 5e-6 of x, and of up to 1e-10 in sensitivities, at every tolerance: 1.3 to 5 times
+// what the colour sweeps leave, whose updates are smaller.  One such r in the course of a solve, about
+// half way down, lets the second half remove what the first has gathered, and the second half's own
+// updates are small: 1e-9 of x instead of 4e-6, sensitivities 4 to 30 times nearer (14x14x11 cells).
+// The iteration goes on with its p unless r changed by more than RENEW_KEEP of itself: then beta is zero
+// once.  (Adjoint right-hand sides, whose x is large on the gradients, change by 5e-5; the gradients weigh
+// so much in r^T M^-1 r that the old p held some systems up for 25 to 100 iterations.)
+// NORMS: every row, and the sums of |r|^2 and |b|^2 in k_spmv's layout; else the systems whose turn it
+// is, and the sums of what changed.
+constexpr double RENEW_KEEP = 1e-5;
+struct Dd {
+  double h, l;
+};
+__device__ __forceinline__ void dd_add(Dd& s, double v) {
+  const double t = __dadd_rn(s.h, v), u = __dsub_rn(t, s.h);
+  s.l = __dadd_rn(s.l, __dadd_rn(__dsub_rn(s.h, __dsub_rn(t, u)), __dsub_rn(v, u)));
+  s.h = t;
+}
+__device__ __forceinline__ void dd_mul_add(Dd& s, double a, double b) {
+  const double p = __dmul_rn(a, b);
+  s.l = __dadd_rn(s.l, __fma_rn(a, b, -p));
+  dd_add(s, p);
+}
+// b - k + om m
+__device__ __forceinline__ double dd_residual(double b, const Dd& k, double om, const Dd& m) {
+  Dd s{b, 0.0};
+  dd_add(s, -k.h);
+  dd_mul_add(s, om, m.h);
+  return s.h + (s.l - k.l + om * m.l);
+}
+template <int NS, bool SEG, bool NORMS>
+__device__ __forceinline__ void exact_residual(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                                               const double2* __restrict__ km, int n, const double2* x, const double2* b,
+                                               double2* r, const SysScal* sc, const uint8_t* seg,
+                                               double* part, const RedSet& R, int bid, int nb, double2* buf) {
+  using S = SmShape<NS, SEG>;
+  constexpr int SPL = S::SPL;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
+  double om[SPL], acc[SPL][3];
+  bool turn[SPL];
+#pragma unroll
+  for (int i = 0; i < SPL; ++i) {
+    om[i] = sc[s0 + i].omega;
+    turn[i] = NORMS || sc[s0 + i].renew == RENEW_TURN;
+    acc[i][0] = acc[i][1] = acc[i][2] = 0.0;
+  }
+  double (*red)[MAX_SYS][3] = nullptr;
+  if constexpr (SEG) red = seg_sums<32, 3>();
+  for (long r0 = ((long)bid * nw + w) * S::RPW; r0 < n; r0 += (long)nb * nw * S::RPW) {
+    const int row = (int)r0 + sub;
+    const bool live = row < n;
+    int sid = 0;
+    if constexpr (SEG) {
+      sid = live ? (int)__ldg(seg + row) : 0;
+      om[0] = sc[sid].omega;
+      turn[0] = NORMS || (live && sc[sid].renew == RENEW_TURN);
+    }
+    bool any = false;
+#pragma unroll
+    for (int i = 0; i < SPL; ++i) any |= turn[i];
+    const int k1 = live && any ? __ldg(rowptr + row + 1) : 0;
+    Dd t[4][SPL];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) t[c][i] = Dd{0.0, 0.0};
+    for (int k = (k1 ? __ldg(rowptr + row) : 0) + g; k < k1; k += S::G) {
+      const double2 a = __ldg(km + k);
+      double2 v[SPL];
+      load_spl<double2, NS, SPL, true>(x + (long)__ldg(col + k) * NS + s0, v);
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        dd_mul_add(t[0][i], a.x, v[i].x);
+        dd_mul_add(t[1][i], a.x, v[i].y);
+        dd_mul_add(t[2][i], a.y, v[i].x);
+        dd_mul_add(t[3][i], a.y, v[i].y);
+      }
+    }
+#pragma unroll
+    for (int m = S::NG; m < S::LPR; m <<= 1)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int i = 0; i < SPL; ++i) {
+          const double h = shfl_xor(t[c][i].h, m), l = shfl_xor(t[c][i].l, m);
+          dd_add(t[c][i], h);
+          t[c][i].l += l;
+        }
+    if (g == 0 && live && any) {
+      const long base = (long)row * NS + s0;
+      double2 bi[SPL];
+      load_spl<double2, NS, SPL, false>(b + base, bi);
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        if (!turn[i]) continue;
+        const double2 v = make_double2(dd_residual(bi[i].x, t[0][i], om[i], t[3][i]),
+                                       dd_residual(bi[i].y, t[1][i], -om[i], t[2][i]));
+        double e0, e2 = 0.0;
+        if constexpr (NORMS) {
+          e0 = v.x * v.x + v.y * v.y;
+          e2 = bi[i].x * bi[i].x + bi[i].y * bi[i].y;
+        } else {
+          const double2 was = r[base + i];
+          e0 = (v.x - was.x) * (v.x - was.x) + (v.y - was.y) * (v.y - was.y);
+        }
+        r[base + i] = v;
+        if constexpr (SEG) {
+          red[w * 4 + sub][sid][0] += e0;
+          red[w * 4 + sub][sid][2] += e2;
+        } else {
+          acc[i][0] += e0;
+          acc[i][2] += e2;
+        }
+      }
+    }
+  }
+  if constexpr (NORMS) {
+    if constexpr (SEG) seg_partials<32, 3>(red, part);
+    else block_partials_spl<NS, SPL, S::LPR, 3>(acc, s0, g == 0, part);
+  } else {
+    if constexpr (SEG) {
+      seg_pair<32, 3>(red, R, bid);
+    } else {
+      double d[SPL][2];
+#pragma unroll
+      for (int i = 0; i < SPL; ++i) {
+        d[i][0] = acc[i][0];
+        d[i][1] = 0.0;
+      }
+      block_pair<NS, SPL, S::LPR>(d, s0, g == 0, R, bid, buf);
+    }
+  }
+}
+
+// Whether the systems whose turn it was keep their p (d: the sums above).
+__device__ __forceinline__ void finish_renew(SysScal* sc, const double2* d, int nsys) {
+  if (threadIdx.x >= nsys) return;
+  SysScal& S = sc[threadIdx.x];
+  if (S.renew == RENEW_TURN && !(d[threadIdx.x].x <= RENEW_KEEP * RENEW_KEEP * S.rr)) S.renew = RENEW_RESTART;
+}
+
+template <int NS, bool SEG, bool NORMS>
+__global__ void __launch_bounds__(256)
+    k_exact_residual(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
+                     const double2* __restrict__ km, int n, const double2* __restrict__ x,
+                     const double2* __restrict__ b, double2* __restrict__ r, SysScal* sc, const Ctrl* ctrl,
+                     const uint8_t* __restrict__ seg, double* __restrict__ part, RedSet R, int nsys) {
+  if (!NORMS && (ctrl->done || !ctrl->renew)) return;
+  __shared__ double2 sums[MAX_SYS], buf[8 * NS];
+  exact_residual<NS, SEG, NORMS>(rowptr, col, km, n, x, b, r, sc, seg, part, R, blockIdx.x, gridDim.x, buf);
+  if constexpr (!NORMS)
+    if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums)) finish_renew(sc, sums, nsys);
 }
 
 // z = c1 s - c2 D^-1 A s by rows, and the edges' share r^T z of rho.  (RO: nothing of what is read is
@@ -2324,6 +2500,7 @@ struct SmallArgs {
   const int32_t *rowptr, *col, *line, *nptr, *nlist, *hrow, *hcol, *cell, *lptr, *lidx, *levels;
   const uint8_t* bc;
   const V* km;     // the COCG's matrix
+  const double2* b;
   const PV* kmp;   // the smoother's copy
   const double2 *dkm, *hkm, *l1;
   const double *te, *frac, *axw, *lw, *cheb, *omega;
@@ -2335,7 +2512,7 @@ struct SmallArgs {
   double2 *x, *rho;
   SysScal* sc;
   Ctrl* ctrl;
-  RedSet red_r, red_edge, red_node, red_pq, red_grid;
+  RedSet red_r, red_edge, red_node, red_pq, red_grid, red_renew;
 };
 
 // q = A p and p^T q, lane geometry of the smoother's edges
@@ -2449,8 +2626,17 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(const __grid_constant__
                              nb);
     if (ctrl.done) break;
     grid.sync();
+    if constexpr (sizeof(T) == 8)
+      if (ctrl.renew)
+        exact_residual<NS, false, false>(a.rowptr, a.col, a.km, a.n, a.x, a.b, a.r, sc, nullptr, nullptr, a.red_renew,
+                                         bid, nb, buf);
     spmv_rows<T, NS>(a.rowptr, a.col, a.km, a.n, a.p, a.q, sc, a.red_pq, bid, nb, buf);
     grid.sync();
+    if (ctrl.renew) {
+      sum_blocks(a.red_renew, nb, NS, sums);
+      finish_renew(sc, sums, NS);
+      __syncthreads();
+    }
     sum_blocks(a.red_pq, nb, NS, sums);
     finish_pq(sc, &ctrl, sums, NS);
     __syncthreads();
@@ -2830,7 +3016,7 @@ __global__ void k_copy_r<float2>(const double2* __restrict__ in, float2* __restr
 
 // Start of an inner solve: x_inner = 0, ||b||^2 from the partials of the residual SpMV.
 __global__ void k_init_sys(SysScal* sc, Ctrl* ctrl, const double* part, int nblocks, int ns, double tol, int maxit,
-                           const double* omega, unsigned spin_limit) {
+                           const double* omega, unsigned spin_limit, double renew_tol, int renew_mask) {
   const int s = threadIdx.x >> 5;
   if (s < ns) {
     double v[1];
@@ -2843,7 +3029,7 @@ __global__ void k_init_sys(SysScal* sc, Ctrl* ctrl, const double* part, int nblo
       S.resid = 1.0;
       S.rho = S.rho1 = S.alpha = S.beta = S.pq = make_double2(0.0, 0.0);
       S.iter = 0;
-      S.xpend = 0;
+      S.xpend = S.renew = 0;
       // a NaN / Inf in the matrix or the right-hand side shows in ||b - A 0||^2
       const bool finite = isfinite(v[0]);
       S.active = finite && v[0] > 0.0;
@@ -2857,6 +3043,9 @@ __global__ void k_init_sys(SysScal* sc, Ctrl* ctrl, const double* part, int nblo
     ctrl->tol = tol;
     ctrl->maxit = maxit;
     ctrl->spin_limit = spin_limit;
+    ctrl->renew_tol = renew_tol;
+    ctrl->renew_mask = renew_mask;
+    ctrl->renew = 0;
   }
 }
 
@@ -3250,16 +3439,31 @@ bool smoothed(const afem_ctx* c, const SolverWork* w, int precond) {
 }
 
 // The sets of block sums (each kernel its own: a kernel may start while the one before it ends).
-enum { RED_R, RED_EDGE, RED_NODE, RED_PQ, RED_GRID, RED_SETS };
+enum { RED_R, RED_EDGE, RED_NODE, RED_PQ, RED_GRID, RED_RENEW, RED_SETS };
 RedSet red_set(SolverWork* w, int k) {
   const long vals = (long)RED_SYS * (w->prows + RED_GROUPS);
   double2* p = w->red.p + k * vals;
   return RedSet{p, p + (long)RED_SYS * w->prows, w->cnt.p + k * (RED_GROUPS + 1), w->prows};
 }
 
+// Iterations from one chance of a new residual to the next (a launch that mostly returns at once): four,
+// where the chunks of iterations keep that step.
+int renew_every(int chunk) { return chunk % 4 == 0 ? 4 : 1; }
+
+// r = b - A x into r (see k_exact_residual).
+template <int NS, bool SEG, bool NORMS>
+void launch_exact_residual(afem_ctx* c, SolverWork* w, const double2* b, double2* r) {
+  const long lanes = (long)w->n * SmShape<NS, SEG>::LPR;
+  const int g = NORMS ? w->nblocks : (int)std::max(1L, std::min(c->num_sms * 8L, (lanes + 255) / 256));
+  k_exact_residual<NS, SEG, NORMS><<<g, 256, 0, c->stream>>>(
+      c->rowptr.p, c->col.p, c->km.p, w->n, w->x.p, b, r, w->sc.p, NORMS ? (const Ctrl*)nullptr : w->ctrl.p,
+      SEG ? c->seg_of_row.p : nullptr, w->part.p, red_set(w, RED_RENEW), w->nsys);
+  count_launch();
+}
+
 // One smoothed iteration (see k_r_update).
 template <class T, class PT, int NS, bool SEG>
-void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, cudaEvent_t* ev) {
+void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, bool renew, cudaEvent_t* ev) {
   using I = Inner<T, NS>;
   using P = Inner<PT, NS>;
   using V = typename I::V;
@@ -3306,6 +3510,8 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, cudaEve
     k_pupd<T, PT, NS, SEG><<<grid((long)n * NS), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg,
                                                           w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw, co->te.p);
   count_launch();
+  if constexpr (sizeof(T) == 8)
+    if (renew) launch_exact_residual<NS, SEG, false>(c, w, w->r64.p, w->r.p);
   if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
   const int rpw = w->rpw_smooth;
   const bool tiles = rpw == 16;
@@ -3340,6 +3546,7 @@ void launch_small(afem_ctx* c, SolverWork* w, int steps, const double* d_omega) 
   a.hrow = h->rowptr.p; a.hcol = h->col.p; a.cell = co->cell.p; a.lptr = co->lptr.p; a.lidx = co->lidx.p;
   a.levels = co->d_levels.p; a.bc = c->bc.p;
   a.km = I::KM(c, w);
+  a.b = w->r64.p;
   if constexpr (sizeof(PT) == 8) { a.kmp = c->km.p; a.gkm = co->km.p; }
   else { a.kmp = w->kmf.p; a.gkm = co->kmf.p; }
   a.dkm = w->dkm.p; a.hkm = h->km.p; a.l1 = co->l1.p; a.te = co->te.p; a.frac = co->frac.p; a.axw = co->axw.p;
@@ -3350,7 +3557,7 @@ void launch_small(afem_ctx* c, SolverWork* w, int steps, const double* d_omega) 
   a.R = reinterpret_cast<PV*>(w->cbuf.p); a.Z = a.R + vec; a.O = a.Z + vec;
   a.x = w->x.p; a.rho = w->rho.p + MAX_SYS; a.sc = w->sc.p; a.ctrl = w->ctrl.p;
   a.red_r = red_set(w, RED_R); a.red_edge = red_set(w, RED_EDGE); a.red_node = red_set(w, RED_NODE);
-  a.red_pq = red_set(w, RED_PQ); a.red_grid = red_set(w, RED_GRID);
+  a.red_pq = red_set(w, RED_PQ); a.red_grid = red_set(w, RED_GRID); a.red_renew = red_set(w, RED_RENEW);
   auto k = k_small<T, PT, NS>;
   AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
@@ -3400,17 +3607,20 @@ void smoother_values(afem_ctx* c, SolverWork* w, const double* d_omega) {
 }
 
 // FP64 true residual r64 = b - A x; returns per-system ||r||^2 and ||b||^2 on the host.
-// fast: several rows per warp, as the smoothed iteration's SpMV (1.67 -> 0.6 ms for one system of 3.2 M
-// rows); the other iterations keep one, and with it the order of their sums.
+// exact: by k_exact_residual, as the smoothed iteration's own; the other iterations keep the plain sums
+// and their order.
 template <int NS, bool SEG>
-void true_residual(afem_ctx* c, SolverWork* w, bool fast, std::vector<double>& rr, std::vector<double>& bb) {
+void true_residual(afem_ctx* c, SolverWork* w, bool exact, std::vector<double>& rr, std::vector<double>& bb) {
   cudaStream_t s = c->stream;
   const int nsys = w->nsys;
-  auto k = fast ? k_spmv<double, NS, (NS <= 8 ? 4 : 2), SEG> : k_spmv<double, NS, 1, SEG>;
-  k<<<w->nblocks, 256, 0, s>>>((const int32_t*)c->rowptr.p, (const int32_t*)c->col.p, c->km.p, w->n, w->x.p, w->r64.p,
-                               w->sc.p, (const Ctrl*)nullptr, w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr,
-                               RedSet{}, 0, AFEM_SPMV_CHUNK);
-  count_launch();
+  if (exact) {
+    launch_exact_residual<NS, SEG, true>(c, w, w->b.p, w->r64.p);
+  } else {
+    k_spmv<double, NS, 1, SEG><<<w->nblocks, 256, 0, s>>>(
+        (const int32_t*)c->rowptr.p, (const int32_t*)c->col.p, c->km.p, w->n, w->x.p, w->r64.p, w->sc.p,
+        (const Ctrl*)nullptr, w->part.p, w->b.p, SEG ? c->seg_of_row.p : nullptr, RedSet{}, 0, AFEM_SPMV_CHUNK);
+    count_launch();
+  }
   DBuf<double> out;
   out.alloc(2 * nsys);
   k_true_resid<<<1, 32 * MAX_SYS, 0, s>>>(w->part.p, w->nblocks, nsys, out.p);
@@ -3480,8 +3690,13 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
                                                           RedSet{}, 0, AFEM_SPMV_CHUNK);
     count_launch();
   }
+  // iterations between host checks; the one-launch form needs the host less often
+  const bool one_launch = smoothed(c, w, precond) && !c->prof.on && small_system<NS, SEG>(c, w);
+  const int chunk = check_every > 0 ? check_every : (one_launch ? 128 : 32);
+  const bool renew = smoothed(c, w, precond) && sizeof(T) == 8 && tol < 1e-4;
+  const int renew_mask = renew_every(chunk) - 1;
   k_init_sys<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, w->nblocks, nsys, tol, maxit, d_omega,
-                                       c->wait_limit);
+                                       c->wait_limit, renew ? std::sqrt(tol) : 0.0, renew_mask);
   count_launch();
   const bool use_hyb = precond == AFEM_PRECOND_HYBRID || (precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1);
   if (use_hyb) {
@@ -3548,9 +3763,6 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   w->epoch_host += 1;
   AFEM_CUDA(cudaMemcpyAsync(&w->ctrl.p->epoch, &w->epoch_host, sizeof(unsigned), cudaMemcpyHostToDevice, s));
   int iters_done = 0;
-  // iterations between host checks; the one-launch form needs the host less often
-  const bool one_launch = smoothed(c, w, mode) && !c->prof.on && small_system<NS, SEG>(c, w);
-  const int chunk = check_every > 0 ? check_every : (one_launch ? 128 : 32);
   // profiling: 8 events per iteration of a chunk (fwd | scal | bwd | nodal correction | scal | pupd | spmv,
   // or r update | smoother | coarse cycle | prolongation | pupd | spmv)
   const bool prof = c->prof.on;
@@ -3562,7 +3774,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   auto ev_of = [&](int k) -> cudaEvent_t* { return prof ? &evs[8L * k] : nullptr; };
   const bool smooth = smoothed(c, w, mode);
   auto enqueue = [&](int k) {
-    if (smooth) enqueue_smoothed<T, PT, NS, SEG>(c, w, d_omega, ev_of(k));
+    if (smooth) enqueue_smoothed<T, PT, NS, SEG>(c, w, d_omega, (k & renew_mask) == renew_mask, ev_of(k));
     else enqueue_iteration<T, PT, NS, SEG>(c, w, mode, sblocks, ev_of(k));
   };
   cudaGraphExec_t gexec = nullptr;
