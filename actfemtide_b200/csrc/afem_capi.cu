@@ -182,6 +182,8 @@ afem_ctx* afem_create(int device) {
 void afem_destroy(afem_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
+  // a call that failed may have left kernels in flight, and cudaFree of a pool's memory waits for none
+  if (c->stream) cudaStreamSynchronize(c->stream);
   afem::destroy_work(c);
   afem::destroy_ctl(c);
   afem::mpnn_destroy(c);
@@ -190,10 +192,7 @@ void afem_destroy(afem_ctx* c) {
   afem::mt_destroy(c);
   for (auto* s : c->src) delete s;
   c->src.clear();
-  if (c->stream) {
-    cudaStreamSynchronize(c->stream);
-    cudaStreamDestroy(c->stream);
-  }
+  if (c->stream) cudaStreamDestroy(c->stream);
   const cudaMemPool_t pool = c->pool;
   delete c;  // the last buffers
   if (pool) cudaMemPoolDestroy(pool);
