@@ -696,7 +696,7 @@ const void* coarse_cycle(afem_ctx* c, const CoarseArgs& a) {
     }
   const size_t smem = std::min(TAIL_BYTES, sizeof(V) * co->tail_vals);
   auto tail = k_grid_tail<PT, NS, SEG>;
-  AFEM_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_shared(tail, TAIL_BYTES);
   tail<<<dim3(4, SEG ? co->nseg : NS), TAIL_THREADS, smem, s>>>(
       co->d_grids.p, co->d_levels.p, co->tail, (int)(smem / sizeof(V)), km, co->l1.p, co->axw.p, a.omega, R, O, co->lptr.p, co->lidx.p,
       co->lw.p, t, a.done, co->tail == 0 ? a.rho : nullptr);

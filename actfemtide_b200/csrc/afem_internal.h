@@ -34,6 +34,13 @@ struct Error {
     if (!(cond)) throw ::afem::Error{(code), (msg)};  \
   } while (0)
 
+// A kernel's limit of dynamic shared memory belongs to the device and not to a context: set to what any
+// mesh may need (never to one mesh's size, which would lower it under another thread's launch).
+template <class K>
+void allow_shared(K kernel, size_t most) {
+  AFEM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+}
+
 // ---------------------------------------------------------------- device buffer
 // Device memory of an entry point comes from its context's own pool, in the order of the context's
 // stream (the only one its kernels and copies use): a call's temporary buffers then cost microseconds,

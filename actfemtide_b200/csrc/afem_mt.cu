@@ -787,7 +787,11 @@ void run_faces(afem_ctx* c, const std::vector<double>& s2tet, int nf, const doub
     AFEM_CUDA(cudaMemcpyAsync(R.rf0.p, R.rf.p, sizeof(double2) * roff, cudaMemcpyDeviceToDevice, s));
   }
   const size_t shm = 2 * sizeof(double2) * (size_t)(maxbw + 1);
-  AFEM_CUDA(cudaFuncSetAttribute(k_band_ldlt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+  int optin = 0;
+  cudaFuncAttributes fa;
+  AFEM_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  AFEM_CUDA(cudaFuncGetAttributes(&fa, k_band_ldlt));
+  allow_shared(k_band_ldlt, optin - fa.sharedSizeBytes);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c->prof.on) {
     AFEM_CUDA(cudaEventCreate(&e0));

@@ -3206,7 +3206,7 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
       auto k = k_spmv_tile<NS>;
       constexpr size_t smem = sizeof(double2) * SPT_UCAP * NS;
       if (!grid) {
-        AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared(k, smem);
         grid = one_wave_grid(c, k, w->nblocks, smem);
       }
       k<<<grid, 256, smem, s>>>(rp, cl, (const double2*)km, n, c->spt_ptr.p, c->spt_uniq.p, c->spt_lidx.p,
@@ -3292,7 +3292,7 @@ void launch_sweep_block(afem_ctx* c, SolverWork* w) {
   auto k = k_sweep_block<T, NS, BWD>;
   const int nlev = BWD ? c->levels_b : c->levels_f;
   const int smem = (int)(sizeof(V) * w->n * NS + sizeof(int) * (nlev + 1));
-  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  allow_shared(k, SWEEP_BYTES + sizeof(int) * SWEEP_LEVELS);
   k<<<1, SWEEP_THREADS, smem, c->stream>>>(BWD ? c->rows_b.p : c->rows_f.p, c->col.p, I::KM(c, w), w->n,
                                            (const V*)I::R(w), I::Z(w), (const V*)I::DD(w), w->sc.p, w->ctrl.p,
                                            BWD ? c->lev_b.p : c->lev_f.p, nlev);
@@ -3559,7 +3559,7 @@ void launch_small(afem_ctx* c, SolverWork* w, int steps, const double* d_omega) 
   a.red_r = red_set(w, RED_R); a.red_edge = red_set(w, RED_EDGE); a.red_node = red_set(w, RED_NODE);
   a.red_pq = red_set(w, RED_PQ); a.red_grid = red_set(w, RED_GRID); a.red_renew = red_set(w, RED_RENEW);
   auto k = k_small<T, PT, NS>;
-  AFEM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_shared(k, SMALL_BYTES);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(c->num_sms);
   cfg.blockDim = dim3(SMALL_THREADS);

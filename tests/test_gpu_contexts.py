@@ -29,3 +29,41 @@ def test_context_closed_right_after_a_failed_call(gpulib):
             fw.close()
             again = keep.solve(m.freqs[0], precond="HYBRID", tol=1e-9)
             assert again.iterations == ref.iterations and np.array_equal(keep.solution(0), x)
+
+
+@pytest.mark.parametrize("precond", ["HYBRID", "SSOR"])
+def test_two_threads_with_meshes_of_two_sizes(gpulib, precond):
+    """A kernel's limit of shared memory belongs to the device: one context's mesh must not lower another's."""
+    import threading
+
+    from actfemtide_b200.forward import Forward
+    models = [synth.tidal_box(*d, seed=4, block=False, half_km=10.0) for d in ((9, 9, 8), (4, 4, 4))]
+    if precond == "SSOR":
+        models = [synth.tidal_box(*d, seed=4, block=False, half_km=10.0) for d in ((7, 7, 6), (3, 3, 3))]
+    errors, got = [], [[], []]
+
+    def work(k):
+        try:
+            m = models[k]
+            with Forward(0) as fw:
+                fw.load_model(m)
+                fw.set_sigma(np.maximum(m.sigma_per_tet(), 1e-2))
+                fw.assemble()
+                fw.set_profiling(precond == "HYBRID")  # every kernel launched by itself
+                for _ in range(12):
+                    r = fw.solve(m.freqs[0], precond=precond, tol=1e-8, maxit=400 if precond == "SSOR" else 2000,
+                                 use_graph=False)
+                    got[k].append((r.status, r.iterations, fw.solution(0)))
+        except Exception as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for runs in got:
+        assert len(runs) == 12
+        for status, its, x in runs[1:]:
+            assert (status, its) == runs[0][:2] and np.array_equal(x, runs[0][2])
