@@ -103,9 +103,10 @@ struct SolverWork {
   DBuf<unsigned char> cbuf, nbuf;   // smoothed iteration: the grids' vectors; the mesh nodes' right-hand
                                     // sides and corrections, [node][4][system] each
   DBuf<double2> dkm;                // (K, M) diagonal in row order
-  DBuf<double> cheb;                // polynomial coefficients of the smoother: edges, nodes
-  DBuf<double2> pw;                 // power iteration: two vectors (K and M parts as x, y)
-  long cheb_gen = -1;               // assembly generation of dkm and cheb
+  DBuf<double> cheb;                // polynomial coefficients of the smoother: edges, nodes, of each mesh
+  DBuf<unsigned long long> lam;     // eigenvalue bounds: the meshes' edges, then their nodes (bits of doubles)
+  DBuf<double2> pw;                 // the bounds' iteration: two vectors (K and M parts as x, y)
+  long cheb_gen = -1;               // assembly generation of dkm and the edges' bounds
   DBuf<double2> red;                // block sums finished inside a launch: RED_SETS sets (red_set)
   DBuf<unsigned> cnt;               // their counters
   DBuf<double2> rho;                // shares of rho: the edges', then 4 rows of the grids'
@@ -1760,10 +1761,10 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
 //   k_exact_residual: r = b - A x, once a solve;
 //   k_spmv:        q = A p, p^T q -> alpha.
 // The scalar steps run in the last block of the kernel that produced their sums.
-constexpr double CHEB_SAFETY = 1.25;  // on the power iteration's estimate of the largest eigenvalue (0.79 of it
-                                      // after four steps on Kuhn meshes, from below)
+constexpr double CHEB_TOP = 0.92;     // the smoothed interval ends at this part of the bound on the largest eigenvalue
+                                      // (k_power), b; c1 - c2 lambda is positive below 1.125 b, past the bound
 constexpr double CHEB_RATIO = 8.0;    // the smoothed interval is [b / 8, b]
-constexpr int CHEB_POWER = 4;         // steps of the power iteration
+constexpr int CHEB_POWER = 4;         // steps of the bound's iteration
 // The smoothed iteration's recursive residual goes to this fraction of the tolerance before the true
 // residual is judged.  At the same residual its error is spread differently from the sweeps': the
 // phases of an MT model's small impedances were 2 to 12e-10 off where the sweeps left 3 to 4e-10
@@ -2053,7 +2054,7 @@ __device__ __forceinline__ void smooth_edges(const int32_t* __restrict__ rowptr,
   using S = SmShape<NS, SEG>;
   constexpr int SPL = S::SPL;
   const int sub = lane / S::LPR, ql = lane % S::LPR, s0 = (ql % S::NG) * SPL, g = ql / S::NG;
-  const PT c1 = (PT)coef[0], c2 = (PT)coef[1];
+  PT c1 = (PT)coef[0], c2 = (PT)coef[1];
   double om[SPL], acc[SPL][2];
 #pragma unroll
   for (int i = 0; i < SPL; ++i) {
@@ -2072,6 +2073,8 @@ __device__ __forceinline__ void smooth_edges(const int32_t* __restrict__ rowptr,
     if constexpr (SEG) {
       sid = live ? (int)__ldg(seg + row) : 0;
       om[0] = sc[sid].omega;
+      c1 = (PT)coef[4 * sid];
+      c2 = (PT)coef[4 * sid + 1];
     }
     const int k0 = live ? nk0 : 0, k1 = live ? nk1 : 0;
     if (next >= 0 && next + sub < n) { nk0 = __ldg(rowptr + next + sub); nk1 = __ldg(rowptr + next + sub + 1); }
@@ -2219,7 +2222,7 @@ __device__ __forceinline__ void prolong(int node, const uint8_t* nseg, const Coa
   using V = typename Cx<T>::V;
   constexpr int SP = NS >= 2 ? 2 : 1, GPC = NS / SP, GPR = 4 * GPC;
   const long total = (long)node * GPR, stride = (long)nb * blockDim.x;
-  const T c1 = (T)coef[2], c2 = (T)coef[3];
+  T c1 = (T)coef[2], c2 = (T)coef[3];
   const long i0 = bid * (long)blockDim.x + threadIdx.x;
   const int c = (int)(i0 % GPR) / GPC, s0 = (int)(i0 % GPC) * SP;  // the stride is a multiple of GPR
   double om[SP], acc[SP][2];
@@ -2270,7 +2273,11 @@ __device__ __forceinline__ void prolong(int node, const uint8_t* nseg, const Coa
 #pragma unroll
       for (int j = 0; j < SP; ++j) o[j] = Cx<T>::make(0, 0);
       if (c == 0) {
-        if constexpr (SEG) om[0] = sc[sid].omega;
+        if constexpr (SEG) {
+          om[0] = sc[sid].omega;
+          c1 = (T)coef[4 * sid + 2];
+          c2 = (T)coef[4 * sid + 3];
+        }
         V ti[SP], si[SP], dd[SP];
         load_spl<V, NS, SP, false, RO>(t + (long)a * 4 * NS + s0, ti);
         load_spl<V, NS, SP, false, RO>(hs + (long)a * NS + s0, si);
@@ -2368,31 +2375,41 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// One step of the power iteration on D_K^-1 K and D_M^-1 M at once (x and y of the vectors): 8 lanes
-// per row; first: the start vector is a hash of the row in [-1, 1].  The last block of the last step
-// turns the two Rayleigh quotients into the smoother's coefficients: [b / CHEB_RATIO, b] with b
-// CHEB_SAFETY times the larger quotient (|x^H A x| <= b |x^H D x| at every frequency, as K and M are
-// semi-definite).
-__device__ __forceinline__ void cheb_coefficients(double lam, double fallback, double* coef) {
-  if (!(lam > 0.5 && lam < 64.0)) lam = fallback;  // an unusable estimate (non-finite values end the solve by themselves)
-  const double b = CHEB_SAFETY * lam, a = b / CHEB_RATIO;
-  const double th = 0.5 * (b + a), de = 0.5 * (b - a), sg = th / de, rho0 = 1.0 / sg, rn = 1.0 / (2.0 * sg - rho0);
-  coef[0] = (1.0 + rn * rho0) / th + 2.0 * rn / de;
-  coef[1] = 2.0 * rn / (de * th);
-}
-__device__ __forceinline__ double power_start(int row) {
-  unsigned h = (unsigned)row * 2654435761u;
-  h ^= h >> 15;
-  h *= 2246822519u;
-  h ^= h >> 13;
-  return (double)(h & 0xffff) / 32768.0 - 1.0;
-}
+// Upper bounds of the eigenvalues of D^-1 K and D^-1 M: for a positive vector v the largest of
+// (|A| v)_i / (D_i v_i) bounds every eigenvalue of D^-1 A in modulus (Collatz and Wielandt), and v <- D^-1
+// |A| v from v = D^-1/2 tightens it: after four steps it is 1.01 to 1.05 times the largest eigenvalue on
+// Kuhn meshes and 1.0 to 1.3 times on Delaunay meshes, thin elements among them.  (Four steps of a power
+// iteration gave 0.67 to 0.96 times, from below, and in a packed batch one mean of all meshes; the polynomial
+// was negative above 1.41 times the estimate.)  K and M being semi-definite, the larger bound is one of
+// |x^H A x| / |x^H D x| at every frequency, so c1 - c2 lambda is positive on the whole spectrum.  Ten thin
+// elements in 16x16x12 cells: 103 iterations -> 69 (49 without them).
+// One step for K and M at once (x and y of the vectors), 8 lanes per row.  The last step leaves the larger
+// bound of each mesh in lam, as the bits of a positive double.
+__device__ __forceinline__ double bound_start(double d) { return d > 0.0 ? 1.0 / sqrt(d) : 0.0; }
+
+// The largest value of each mesh: rows of one mesh are kept in a register until the mesh changes.
+struct MeshMax {
+  int mesh = -1;
+  double v = 0.0;
+  __device__ __forceinline__ void put(unsigned long long* lam) const {
+    if (mesh >= 0 && v > 0.0) atomicMax(lam + mesh, (unsigned long long)__double_as_longlong(v));
+  }
+  __device__ __forceinline__ void add(int k, double x, unsigned long long* lam) {
+    if (k != mesh) {
+      put(lam);
+      mesh = k;
+      v = 0.0;
+    }
+    if (x > v) v = x;
+  }
+};
+
 __global__ void __launch_bounds__(256)
     k_power(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const double2* __restrict__ km, int n,
-            const double2* __restrict__ dkm, const double2* __restrict__ in, double2* __restrict__ out, int first,
-            RedSet R, double* __restrict__ coef) {
+            const double2* __restrict__ dkm, const uint8_t* __restrict__ seg, const double2* __restrict__ in,
+            double2* __restrict__ out, int first, unsigned long long* __restrict__ lam) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, g = lane & 7;
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  MeshMax most;
   for (long r0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; r0 < n; r0 += (long)gridDim.x * 32) {
     const int row = (int)r0 + sub;
     double kx = 0.0, my = 0.0;
@@ -2400,9 +2417,9 @@ __global__ void __launch_bounds__(256)
       for (int k = __ldg(rowptr + row) + g; k < __ldg(rowptr + row + 1); k += 8) {
         const int j = __ldg(col + k);
         const double2 a = km[k];
-        const double2 v = first ? make_double2(power_start(j), power_start(j)) : in[j];
-        kx += a.x * v.x;
-        my += a.y * v.y;
+        const double2 v = first ? dkm[j] : in[j];
+        kx += fabs(a.x) * (first ? bound_start(v.x) : v.x);
+        my += fabs(a.y) * (first ? bound_start(v.y) : v.y);
       }
     for (int m = 1; m < 8; m <<= 1) {
       kx += shfl_xor(kx, m);
@@ -2410,70 +2427,56 @@ __global__ void __launch_bounds__(256)
     }
     if (row < n && g == 0) {
       const double2 d = dkm[row];
-      const double2 v = first ? make_double2(power_start(row), power_start(row)) : in[row];
-      s[0] += v.x * kx; s[1] += v.x * v.x * d.x;
-      s[2] += v.y * my; s[3] += v.y * v.y * d.y;
-      out[row] = make_double2(d.x != 0.0 ? kx / d.x : 0.0, d.y != 0.0 ? my / d.y : 0.0);
+      const double2 v = first ? make_double2(bound_start(d.x), bound_start(d.y)) : in[row];
+      const double2 o = make_double2(d.x > 0.0 ? kx / d.x : 0.0, d.y > 0.0 ? my / d.y : 0.0);
+      out[row] = o;
+      if (lam) most.add(seg ? (int)__ldg(seg + row) : 0, fmax(v.x > 0.0 ? o.x / v.x : 0.0, v.y > 0.0 ? o.y / v.y : 0.0), lam);
     }
   }
-  if (!coef) return;
-  // two sums as two "systems": K's quotient and M's
-  __shared__ double2 sums[MAX_SYS];
-  double v[2][2] = {{s[0], s[1]}, {s[2], s[3]}};
-  __shared__ double2 buf[16];
-  block_pair<2, 2, 1>(v, 0, true, R, blockIdx.x, buf);
-  if (reduce_blocks(R, blockIdx.x, gridDim.x, 2, sums) && threadIdx.x == 0) {
-    double lam = sums[0].y > 0.0 ? sums[0].x / sums[0].y : 0.0;
-    if (sums[1].y > 0.0) lam = fmax(lam, sums[1].x / sums[1].y);
-    cheb_coefficients(lam, 3.5, coef);
-  }
+  if (lam) most.put(lam);
 }
 
-// Steps of a power iteration on D_G^-1 A_G at each mesh's first frequency (8 lanes per node); the
-// last one leaves the quotient of the last two vectors' norms in coefficients like k_power's.
+// The same for D_G^-1 A_G at each mesh's first frequency (A_G is i omega M_G but for rounding).
 __global__ void __launch_bounds__(256)
     k_node_power(int node, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                  const double2* __restrict__ km, const int32_t* __restrict__ diagpos, const uint8_t* __restrict__ live,
-                 const uint8_t* __restrict__ nseg, const double* __restrict__ omega, const double2* __restrict__ in,
-                 double2* __restrict__ out, int first, RedSet R, double* __restrict__ coef) {
+                 const uint8_t* __restrict__ nseg, const double* __restrict__ omega, const double* __restrict__ in,
+                 double* __restrict__ out, int first, unsigned long long* __restrict__ lam) {
   const int lane = threadIdx.x & 31, sub = lane >> 3, g = lane & 7;
-  double s[1][2] = {{0.0, 0.0}};
+  MeshMax most;
   for (long r0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; r0 < node; r0 += (long)gridDim.x * 32) {
     const int a = (int)r0 + sub;
-    double kx = 0.0, ky = 0.0;
-    if (a < node) {
-      const double om = omega[nseg ? (int)nseg[a] : 0];
+    const int mesh = a < node && nseg ? (int)nseg[a] : 0;
+    const double om = omega[mesh];
+    auto size = [&](double2 m) { return sqrt(m.x * m.x + om * m.y * (om * m.y)); };
+    double s = 0.0;
+    if (a < node)
       for (int k = rowptr[a] + g; k < rowptr[a + 1]; k += 8) {
         const int j = col[k];
-        const double2 m = km[k];
-        const double2 v = first ? make_double2(power_start(j), 0.0) : in[j];
-        kx += m.x * v.x - om * m.y * v.y;
-        ky += m.x * v.y + om * m.y * v.x;
+        s += size(km[k]) * (first ? (live[j] ? bound_start(size(km[diagpos[j]])) : 0.0) : in[j]);
       }
-      for (int m = 1; m < 8; m <<= 1) {
-        kx += __shfl_xor_sync(0xffu << (8 * sub), kx, m);
-        ky += __shfl_xor_sync(0xffu << (8 * sub), ky, m);
-      }
-      if (g == 0) {
-        const double2 d = km[diagpos[a]];
-        const double2 D = make_double2(d.x, om * d.y);
-        const double2 v = first ? make_double2(power_start(a), 0.0) : in[a];
-        double2 o = make_double2(0.0, 0.0);
-        if (live[a] && (D.x != 0.0 || D.y != 0.0)) {
-          o = cdiv(make_double2(kx, ky), D);
-          s[0][0] += o.x * o.x + o.y * o.y;
-          s[0][1] += v.x * v.x + v.y * v.y;
-        }
-        out[a] = o;
-      }
+    for (int m = 1; m < 8; m <<= 1) s += shfl_xor(s, m);
+    if (a < node && g == 0) {
+      const double d = live[a] ? size(km[diagpos[a]]) : 0.0, v = first ? bound_start(d) : in[a];
+      const double o = d > 0.0 ? s / d : 0.0;
+      out[a] = o;
+      if (lam) most.add(mesh, v > 0.0 ? o / v : 0.0, lam);
     }
   }
-  if (!coef) return;
-  __shared__ double2 sums[MAX_SYS];
-  __shared__ double2 buf[8];
-  block_pair<1, 1, 1>(s, 0, true, R, blockIdx.x, buf);
-  if (reduce_blocks(R, blockIdx.x, gridDim.x, 1, sums) && threadIdx.x == 0)
-    cheb_coefficients(sums[0].y > 0.0 ? sqrt(sums[0].x / sums[0].y) : 0.0, 2.0, coef + 2);
+  if (lam) most.put(lam);
+}
+
+// Polynomial coefficients of each mesh from its bounds: the edges' pair, the nodes' pair.
+__global__ void k_cheb(const unsigned long long* __restrict__ edge, const unsigned long long* __restrict__ nodes,
+                       int nmesh, double* __restrict__ coef) {
+  const int i = threadIdx.x;
+  if (i >= 2 * nmesh) return;
+  double lam = __longlong_as_double((long long)((i & 1) ? nodes : edge)[i >> 1]);
+  if (!(lam > 0.5 && lam < 64.0)) lam = (i & 1) ? 2.0 : 3.5;  // (non-finite values end the solve by themselves)
+  const double b = CHEB_TOP * lam, a = b / CHEB_RATIO;
+  const double th = 0.5 * (b + a), de = 0.5 * (b - a), sg = th / de, rho0 = 1.0 / sg, rn = 1.0 / (2.0 * sg - rho0);
+  coef[2 * i] = (1.0 + rn * rho0) / th + 2.0 * rn / de;
+  coef[2 * i + 1] = 2.0 * rn / (de * th);
 }
 
 // ------------------------------------------------------------------ one-launch iteration of small systems
@@ -3581,29 +3584,36 @@ void smoother_values(afem_ctx* c, SolverWork* w, const double* d_omega) {
   HybridState* h = c->hyb;
   const int n = w->n, node = h->node;
   auto grid = [&](long rows) { return (int)std::max(1L, std::min((long)c->num_sms * 8, (rows + 31) / 32)); };
-  const RedSet R = red_set(w, RED_EDGE);
   const long m = std::max(n, node);  // (a mesh may have nodes without edges)
-  w->cheb.alloc(4);
+  const int nmesh = std::max(1, c->nseg);
+  w->cheb.alloc(4 * MAX_SYS);
+  w->lam.alloc(2 * MAX_SYS);
   w->pw.alloc(2 * m);
   if (w->cheb_gen != c->assemble_gen) {
     w->dkm.alloc(n);
     k_gather_entries<double2><<<c->num_sms * 8, 256, 0, s>>>(c->km.p, c->diagpos.p, (long)n, w->dkm.p);
     count_launch();
+    w->lam.zero(s);
     for (int k = 0; k < CHEB_POWER; ++k) {
-      k_power<<<grid(n), 256, 0, s>>>(c->rowptr.p, c->col.p, c->km.p, n, w->dkm.p, w->pw.p + (k & 1 ? m : 0),
-                                      w->pw.p + (k & 1 ? 0 : m), k == 0, R,
-                                      k + 1 == CHEB_POWER ? w->cheb.p : (double*)nullptr);
+      k_power<<<grid(n), 256, 0, s>>>(c->rowptr.p, c->col.p, c->km.p, n, w->dkm.p,
+                                      c->nseg > 0 ? c->seg_of_row.p : nullptr, w->pw.p + (k & 1 ? m : 0),
+                                      w->pw.p + (k & 1 ? 0 : m), k == 0,
+                                      k + 1 == CHEB_POWER ? w->lam.p : (unsigned long long*)nullptr);
       count_launch();
     }
     w->cheb_gen = c->assemble_gen;
   }
+  AFEM_CUDA(cudaMemsetAsync(w->lam.p + MAX_SYS, 0, sizeof(unsigned long long) * MAX_SYS, s));
+  double* v = reinterpret_cast<double*>(w->pw.p);
   for (int k = 0; k < CHEB_POWER; ++k) {
     k_node_power<<<grid(node), 256, 0, s>>>(node, h->rowptr.p, h->col.p, h->km.p, h->diagpos.p, h->live.p,
-                                            c->nseg > 0 ? h->seg.p : nullptr, d_omega, w->pw.p + (k & 1 ? m : 0),
-                                            w->pw.p + (k & 1 ? 0 : m), k == 0, R,
-                                            k + 1 == CHEB_POWER ? w->cheb.p : (double*)nullptr);
+                                            c->nseg > 0 ? h->seg.p : nullptr, d_omega, v + (k & 1 ? m : 0),
+                                            v + (k & 1 ? 0 : m), k == 0,
+                                            k + 1 == CHEB_POWER ? w->lam.p + MAX_SYS : (unsigned long long*)nullptr);
     count_launch();
   }
+  k_cheb<<<1, 2 * MAX_SYS, 0, s>>>(w->lam.p, w->lam.p + MAX_SYS, nmesh, w->cheb.p);
+  count_launch();
 }
 
 // FP64 true residual r64 = b - A x; returns per-system ||r||^2 and ||b||^2 on the host.

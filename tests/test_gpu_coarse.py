@@ -145,3 +145,61 @@ def test_one_launch_iteration_gives_the_same_solution(fw, oracle, ns, precision)
         assert rc.status == -4 and rc.iterations == cap, rc
     rc = fw.solve(f, src, tol=1e-9, maxit=2000, check_every=5, **kw)
     assert rc.ok and rc.iterations == r.iterations
+
+
+def test_packed_iterates_do_not_depend_on_the_companions(fw):
+    """The smoother's interval is each mesh's own: after 12 iterations a mesh's iterate is the same, but for
+    the order of sums (1e-16 a step, grown at most a thousandfold each by the iteration's scalars), whatever
+    it is packed with."""
+    a = synth.tidal_box(7, 8, 6, seed=3, grf=True, block=False)
+    others = [synth.tidal_box(8, 8, 6, seed=2, block=False), synth.tidal_box(20, 3, 9, seed=2, grf=True, block=False)]
+    xs = []
+    for b in others:
+        fw.load_packed(synth.pack([a, b]))
+        fw.assemble()
+        r = fw.solve(np.full(2, a.freqs[0]), precond="HYBRID", tol=1e-12, maxit=12)
+        assert r.iterations == 12
+        xs.append(fw.solution(0))
+    assert np.linalg.norm(xs[0] - xs[1]) < 1e-9 * np.linalg.norm(xs[0])
+
+
+def test_thin_elements_do_not_break_the_smoother(fw):
+    """Ten nodes moved to 1/200 of their way from a face of one of their tetrahedra: the smoother stays positive
+    on the eigenvalues these add, and they may cost half as many iterations again, not twice as many."""
+    m = synth.tidal_box(16, 16, 12, seed=4, grf=True, block=False)
+    rng = np.random.default_rng(3)
+    xyz = m.xyz.copy()
+    lo, hi = xyz.min(axis=0), xyz.max(axis=0)
+    h = (hi - lo) / m.dims
+    sign = np.sign(_volumes(xyz, m.n4))
+    inner = np.where(np.all((xyz > lo + 1.5 * h) & (xyz < hi - 1.5 * h), axis=1))[0]
+    used, moved = set(), 0
+    for a in rng.permutation(inner):
+        around = np.where((m.n4 == a + 1).any(axis=1))[0]
+        nodes = set((m.n4[around] - 1).ravel())
+        if used & nodes:
+            continue
+        face = [b for b in m.n4[around[rng.integers(len(around))]] - 1 if b != a]
+        old = xyz[a].copy()
+        xyz[a] = 0.005 * old + 0.995 * xyz[face].mean(axis=0)
+        if np.all(_volumes(xyz, m.n4[around]) * sign[around] > 0):
+            used |= nodes
+            moved += 1
+            if moved == 10:
+                break
+        else:
+            xyz[a] = old
+    assert moved == 10
+    its = []
+    for q in (m, dataclasses.replace(m, xyz=xyz)):
+        fw.load_model(q)
+        fw.assemble()
+        r = fw.solve(q.freqs[0], precond="HYBRID", tol=1e-9, maxit=2000)
+        assert r.ok, r
+        its.append(r.iterations)
+    assert its[1] <= 1.5 * its[0], its
+
+
+def _volumes(xyz, n4):
+    p = xyz[n4 - 1]
+    return np.linalg.det(p[:, 1:] - p[:, :1]) / 6
