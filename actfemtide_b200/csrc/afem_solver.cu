@@ -3943,9 +3943,10 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   return iters_done;
 }
 
-// The solve workspace for NS systems per row (SEG: a packed batch), FP32 copies when mixed.
+// The solve workspace for NS systems per row (SEG: a packed batch), FP32 copies when mixed.  rows32: of the
+// matrix in row order (the mixed inner solve, the smoothed iteration's FP32 preconditioner).
 template <int NS, bool SEG>
-SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false) {
+SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false, bool rows32 = false) {
   SolverWork* w = c->work;
   cudaStream_t s = c->stream;
   const int n = c->nline;
@@ -3976,7 +3977,7 @@ SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false) {
     w->rf.alloc(total); w->pf.alloc(total); w->qf.alloc(total); w->ddf.alloc(total);
   }
   if ((mixed || pc32) && w->zf.n != (size_t)total) w->zf.alloc(total);
-  if ((mixed || pc32) && (w->kmf_gen != c->assemble_gen || w->kmf.n != (size_t)c->nnz)) {
+  if (rows32 && (w->kmf_gen != c->assemble_gen || w->kmf.n != (size_t)c->nnz)) {
     w->kmf.alloc(c->nnz);
     k_convert<float2, double2><<<c->num_sms * 8, 256, 0, s>>>(c->km.p, w->kmf.p, c->nnz);
     count_launch();
@@ -4041,7 +4042,9 @@ int solve_ns(afem_ctx* c, const double* freq, const int* srcs, const afem_solve_
   SolverWork* w = nullptr;
   {
     HostTimer ht(c, "host_setup_work");
-    w = ensure_work<NS, SEG>(c, nsys, mixed, pc32);
+    const bool smooth = (o->precond == AFEM_PRECOND_HYBRID || o->precond == AFEM_PRECOND_LEARNED) &&
+                        (o->sigma_diag <= 0 || o->sigma_diag == 1.0) && c->hyb && c->hyb->co && c->hyb->co->on;
+    w = ensure_work<NS, SEG>(c, nsys, mixed, pc32, mixed || (pc32 && smooth));
   }
   // ---- right-hand sides and omegas
   {
