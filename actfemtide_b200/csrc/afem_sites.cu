@@ -60,14 +60,15 @@ __device__ __forceinline__ void nodebasis(const V3 e[4], const V3& x3, double a[
 // the lowest id that holds site s.  A thread takes a tetrahedron, reads it once and runs through the
 // sites (staged in shared memory): the barycentric test is made only where the site lies in the
 // tetrahedron's box, widened far beyond what rounding could let the test accept outside it (a launch
-// row per site, each reading the whole mesh, took 8.6 ms for 400 sites in 2.6 M tetrahedra).
+// row per site, each reading the whole mesh, took 8.6 ms for 400 sites in 2.6 M tetrahedra).  Grid rows share
+// the sites out in groups where the tetrahedra alone do not fill the device (launch_find).
 constexpr int FIND_SITES = 512;
 __global__ void __launch_bounds__(256)
     k_find(const double* __restrict__ xyz, const int32_t* __restrict__ n4, long t0, long t1,
-           const double* __restrict__ obs, int nobs, int* __restrict__ best) {
+           const double* __restrict__ obs, int nobs, int group, int* __restrict__ best) {
   __shared__ double ob[3][FIND_SITES];
-  for (int s0 = 0; s0 < nobs; s0 += FIND_SITES) {
-    const int cnt = min(FIND_SITES, nobs - s0);
+  for (int s0 = blockIdx.y * group; s0 < nobs; s0 += gridDim.y * group) {
+    const int cnt = min(group, nobs - s0);
     __syncthreads();
     for (int i = threadIdx.x; i < 3 * cnt; i += blockDim.x) ob[i % 3][i / 3] = obs[3L * s0 + i];
     __syncthreads();
@@ -257,6 +258,16 @@ __global__ void k_eval(const double2* __restrict__ X, int nline, int nsys, const
   out[i] = acc;
 }
 
+// A block per 256 tetrahedra, and rows for groups of 64 to FIND_SITES sites up to eight blocks per SM (384
+// tetrahedra, two blocks: 1,000 sites 0.31 -> 0.18 ms, 400,000 sites 82 -> 28 ms).
+void launch_find(afem_ctx* c, long t0, long t1, const double* obs, int nobs, int* best) {
+  const long most = 8L * c->num_sms, x = std::max(1L, std::min(most, (t1 - t0 + 255) / 256));
+  const long y = std::max(1L, std::min(most / x, ((long)nobs + 63) / 64));
+  const int group = (int)std::max(1L, std::min((long)FIND_SITES, (nobs + y - 1) / y));
+  k_find<<<dim3((unsigned)x, (unsigned)y), 256, 0, c->stream>>>(c->xyz.p, c->n4.p, t0, t1, obs, nobs, group, best);
+  count_launch();
+}
+
 }  // namespace
 
 // SORT_INDEX (src/solver/sort_index.f90:13-56): heapsort of ra (ascending)
@@ -385,9 +396,7 @@ void site_coeffs_range(afem_ctx* c, int nobs, const double* xyz_obs, long t0, lo
                                                          g->nz, g->stack.p, g->ordered.p, obs.p, nobs, best.p);
     count_launch();
   } else {
-    const int grid = (int)std::max(1L, std::min(8L * c->num_sms, (t1 - t0 + 255) / 256));
-    k_find<<<grid, 256, 0, s>>>(c->xyz.p, c->n4.p, t0, t1, obs.p, nobs, best.p);
-    count_launch();
+    launch_find(c, t0, t1, obs.p, nobs, best.p);
   }
   DBuf<int32_t> ditem;
   DBuf<double> dve, dvf;
@@ -548,9 +557,7 @@ void sites_noalloc_device(afem_ctx* c, int nobs, const double* xyz_obs, double* 
   // the search keeps the smallest holder: every site starts with none
   k_fill_int<<<(nobs + 255) / 256, 256, 0, s>>>(best, nobs, 0x7fffffff);
   count_launch();
-  const int grid = std::max(1, std::min(8 * c->num_sms, (c->ntet + 255) / 256));
-  k_find<<<grid, 256, 0, s>>>(c->xyz.p, c->n4.p, 0, c->ntet, obs, nobs, best);
-  count_launch();
+  launch_find(c, 0, c->ntet, obs, nobs, best);
   k_coeffs<<<(nobs + 63) / 64, 64, 0, s>>>(c->xyz.p, c->n4.p, c->n6line.p, obs, nobs, best, item, ve, vf, c->status.p);
   count_launch();
   check_status(c, "sites_noalloc: a site lies outside every tetrahedron");
