@@ -93,6 +93,12 @@ __global__ void k_node_cells(const double* __restrict__ xyz, int node, const uin
   }
 }
 
+__global__ void k_support_max(int n1, const int32_t* __restrict__ cnt, int* __restrict__ most) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int v = __reduce_max_sync(0xffffffffu, c < n1 ? cnt[c] : 0);
+  if ((threadIdx.x & 31) == 0) atomicMax(most, v);
+}
+
 __global__ void k_support_fill(int node, const uint8_t* __restrict__ seg, const CoarseGrid* __restrict__ grids,
                                const int32_t* __restrict__ corner, const double* __restrict__ frac,
                                const int32_t* __restrict__ lptr, int32_t* __restrict__ cur,
@@ -584,7 +590,7 @@ void coarse_pattern(afem_ctx* c) {
   co->d_levels.upload(co->levels.data(), co->levels.size(), s);
   co->planes.upload(planes.data(), planes.size(), s);
   co->axw.upload(axw.data(), axw.size(), s);
-  DBuf<int32_t> dpofs, cnt;
+  DBuf<int32_t> dpofs, cnt, dmost;
   dpofs.upload(pofs.data(), pofs.size(), s);
   co->corner.alloc(node);
   co->frac.alloc(3L * node);
@@ -601,6 +607,13 @@ void coarse_pattern(afem_ctx* c) {
   count_launch();
   k_cseg<<<nblk(co->n1, 256), 256, 0, s>>>(nseg, co->d_grids.p, co->n1, co->cseg.p);
   count_launch();
+  int most = 0;
+  dmost.upload(&most, 1, s);
+  k_support_max<<<nblk(co->n1, 256), 256, 0, s>>>(co->n1, cnt.p, dmost.p);
+  count_launch();
+  dmost.download(&most, 1, s);
+  AFEM_CUDA(cudaStreamSynchronize(s));  // (the host vectors above may go out of scope, too)
+  if (most > COARSE_CROWD) return;
   long total = 0;
   co->lptr.alloc(co->n1 + 1);
   exclusive_scan(cnt.p, co->lptr.p, co->n1, s, &total);

@@ -14,6 +14,12 @@ constexpr size_t TAIL_BYTES = 212 << 10;  // its shared memory (vectors, and the
 constexpr size_t TAIL_VALS = TAIL_BYTES / 16;
 constexpr int TAIL_AXIS = 1024;       // axis weights of its levels
 constexpr int COARSE_MIN_NODES = 64;  // smaller meshes keep the SSOR corrections alone
+// Mesh nodes in the support of one grid node up to which the correction is taken (36 at most on box
+// meshes).  Where a mesh is refined around a few points, its nodes crowd into few cells of a tensor
+// grid: a step waits for one thread's support, and the correction leaves what varies inside the cell.
+// Solves of 8 systems with the correction / by the colour sweeps alone, by the largest support: 734 125 /
+// 187 ms, 1,240 123 / 125, 1,306 80 / 93, 1,968 153 / 126, 2,271 262 / 201, 7,059 3,466 / 834.
+constexpr int COARSE_CROWD = 1500;
 
 template <class T>
 struct CV;

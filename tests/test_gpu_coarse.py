@@ -203,3 +203,52 @@ def test_thin_elements_do_not_break_the_smoother(fw):
 def _volumes(xyz, n4):
     p = xyz[n4 - 1]
     return np.linalg.det(p[:, 1:] - p[:, :1]) / 6
+
+
+def _refined_around(points, count, n=10, half=50.0):
+    """A Delaunay mesh of a jittered n^3 grid with `count` more nodes around each point, 20 m to 4 km from it."""
+    from scipy.spatial import Delaunay
+    rng = np.random.default_rng(0)
+    g = np.stack(np.meshgrid(*[np.linspace(-half, half, n + 1)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    g += np.all(np.abs(g) < half - 1e-6, axis=1)[:, None] * rng.uniform(-0.5, 0.5, g.shape) * half / n
+    xyz = [g]
+    for p in points:
+        d = rng.normal(size=(count, 3))
+        xyz.append(p + d / np.linalg.norm(d, axis=1)[:, None] * np.exp(rng.uniform(np.log(0.02), np.log(4.0), (count, 1))))
+    xyz = np.concatenate(xyz)
+    n4 = Delaunay(xyz, qhull_options="QJ Pp").simplices + 1
+    like = synth.tidal_box(2, 2, 2, block=False)
+    vol, sign = _volumes(xyz, n4), np.sign(_volumes(like.xyz, like.n4)[0])
+    q = xyz[n4 - 1]
+    edge = np.abs(q[:, [0, 0, 0, 1, 1, 2]] - q[:, [1, 2, 3, 2, 3, 3]]).max(axis=(1, 2))
+    keep = np.abs(vol) > 1e-9 * edge ** 3  # (flat ones on the box's faces)
+    n4 = np.where((np.sign(vol) != sign)[:, None], n4[:, [0, 2, 1, 3]], n4)[keep]
+    cen = xyz[n4 - 1].mean(axis=1)
+    tag = np.where(cen[:, 2] > 0, 1, np.where((cen[:, 2] > -5) & (cen[:, 0] < 0), 2, 3)).astype(np.int32)
+    order = np.argsort(tag, kind="stable")
+    n4, tag = n4[order], tag[order]
+    sea = np.zeros(len(xyz), bool)
+    sea[n4[tag == 2] - 1] = True
+    perm = np.argsort(~sea, kind="stable")
+    new = np.empty(len(xyz), np.int64)
+    new[perm] = np.arange(len(xyz))
+    nodes = int(sea.sum())
+    return dataclasses.replace(like, xyz=np.ascontiguousarray(xyz[perm]), n4=(new[n4 - 1] + 1).astype(np.int32), tag=tag,
+                               sigma_land=np.full(int((tag == 3).sum()), 0.01), nodes=nodes,
+                               F=np.tile(np.array(synth.F_MAIN_NT), (nodes, 1)), v=np.full((nodes, 3), 0.05 + 0.01j),
+                               bounds=dict(zmin=-half, zmax=half, xout=half, yout=half))
+
+
+@pytest.mark.parametrize("count,smoothed", [(100, True), (4000, False)])
+def test_nodes_crowded_around_points_keep_the_sweeps(fw, count, smoothed):
+    """Regions of fine elements around four points: with thousands of nodes in a cell of the tensor grid the
+    solve takes the colour sweeps (their kernels in the profile); either way it converges."""
+    m = _refined_around([(-35.0, -18.0, -3.0), (-12.0, 35.0, -12.0), (13.0, -36.0, -25.0), (34.0, 12.0, -38.0)], count)
+    fw.load_model(m)
+    fw.assemble()
+    fw.set_profiling(True)
+    r = fw.solve(m.freqs[0], precond="HYBRID", tol=1e-8, maxit=3000)
+    names = " ".join(fw.profile())
+    fw.set_profiling(False)
+    assert r.ok and r.iterations > 0, r
+    assert ("cocg_smoother" in names) == smoothed and ("cocg_fwd_sweep_mc" in names) != smoothed, names
