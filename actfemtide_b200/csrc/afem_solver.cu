@@ -4246,13 +4246,13 @@ int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, cons
                  afem_solve_stats* st, const SolveExtra* ex) {
   AFEM_REQUIRE(c->assembled, AFEM_ESTATE, "solve: system not assembled");
   const bool hyb = o->precond == AFEM_PRECOND_HYBRID || (o->precond == AFEM_PRECOND_LEARNED && mpnn_base(c) == 1);
+  const bool coarse = o->sigma_diag <= 0 || o->sigma_diag == 1.0;  // (see smoothed)
   if (hyb) {
     HostTimer ht(c, "host_setup_hybrid");
-    hybrid_prepare(c, true, false);
+    hybrid_prepare(c, coarse, false);
   }
   // the smoothed iteration needs no colouring, the multicolour sweeps no natural-order levels
-  const bool smooth = o->precond == AFEM_PRECOND_HYBRID && (o->sigma_diag <= 0 || o->sigma_diag == 1.0) &&
-                      c->hyb->co->on;
+  const bool smooth = o->precond == AFEM_PRECOND_HYBRID && coarse && c->hyb->co->on;
   const bool mc = o->precond == AFEM_PRECOND_SSOR_MC || (hyb && !smooth);
   if (!smooth) {
     HostTimer ht(c, "host_setup_schedule");
@@ -4261,7 +4261,7 @@ int solve_device(afem_ctx* c, int nsys, const double* freq, const int* src, cons
   if (mc) {
     HostTimer ht(c, "host_setup_mc_values");
     ensure_mc_values(c);
-    if (hyb) hybrid_prepare(c, true, true);
+    if (hyb) hybrid_prepare(c, coarse, true);
   }
   if (c->nseg > 0) {
     AFEM_REQUIRE(nsys == c->nseg, AFEM_EINVAL, "solve: a packed batch solves one system per mesh (nsys = nseg)");

@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import scipy.sparse.linalg as sla
 
-from actfemtide_b200 import synth
+from actfemtide_b200 import capi, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -252,3 +252,22 @@ def test_nodes_crowded_around_points_keep_the_sweeps(fw, count, smoothed):
     fw.set_profiling(False)
     assert r.ok and r.iterations > 0, r
     assert ("cocg_smoother" in names) == smoothed and ("cocg_fwd_sweep_mc" in names) != smoothed, names
+
+
+def test_other_diagonal_scales_leave_the_coarse_matrices_out(fw):
+    """SIGMA_DIAG other than 1 takes the colour sweeps: after an assembly their set-up is six launches (diagonal, lower
+    and upper values of the edges; the nodal matrix and its two halves), and no Galerkin matrix among them."""
+    m = synth.tidal_box(6, 6, 5, seed=1, half_km=10.0)
+    fw.load_model(m)
+    fw.set_spmv_rows_per_warp(1)  # no timing runs
+    count = []
+    for k in range(4):
+        if k != 3:  # the third solve after an assembly with buffers and tables at hand, the fourth without one
+            fw.assemble()
+        before = capi.lib().afem_launch_count()
+        fw.solve(m.freqs[0], precond="HYBRID", tol=1e-10, maxit=8, sigma_diag=1.5, use_graph=False)
+        count.append(capi.lib().afem_launch_count() - before)
+    fw.set_spmv_rows_per_warp(0)
+    assert count[2] - count[3] == 6, count
+    fw.assemble()  # and back to the smoothed iteration
+    assert fw.solve(m.freqs[0], precond="HYBRID", tol=1e-9, maxit=2000).ok
