@@ -268,7 +268,7 @@ void hybrid_prepare(afem_ctx* c, bool coarse, bool colours) {
                                      vec ? h->co->n3.p : nullptr, h->live.p);
     count_launch();
     h->values_gen = c->assemble_gen;
-    h->kmf_valid = false;
+    h->splitf_valid = false;
   }
   if (vec) coarse_values(c);
   if (colours && !h->colours_ready) {
@@ -304,7 +304,7 @@ void hybrid_prepare(afem_ctx* c, bool coarse, bool colours) {
       count_launch();
     }
     h->split_gen = c->assemble_gen;
-    h->kmf_valid = false;
+    h->splitf_valid = false;
   }
   AFEM_CUDA(cudaStreamSynchronize(s));
 }

@@ -20,8 +20,6 @@ struct HybridState {
   DBuf<int32_t> rowptr, col;    // nodal pattern (node graph), columns ascending
   DBuf<int32_t> diagpos;
   DBuf<double2> km;             // (K_G, M_G) per nodal entry
-  DBuf<float2> kmf;             // FP32 copy for the mixed-precision inner solve
-  bool kmf_valid = false;
   DBuf<uint8_t> live;           // 1 when the node has a non-Dirichlet edge
   DBuf<uint8_t> color;          // nodal multicolour order
   DBuf<int32_t> perm, cptr;
@@ -31,6 +29,7 @@ struct HybridState {
   DBuf<int32_t> lptr, lcol, lsrc, uptr, ucol, usrc;
   DBuf<double2> lkm, ukm;
   DBuf<float2> lkmf, ukmf;
+  bool splitf_valid = false;    // lkmf, ukmf match lkm, ukm
   DBuf<uint8_t> seg;            // packed batches: mesh of each node
   int seg_nseg = 0;
   CoarseState* co = nullptr;    // coarse correction (owned; afem_coarse.cu)

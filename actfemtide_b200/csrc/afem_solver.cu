@@ -3115,7 +3115,6 @@ struct Inner<double, NS> {
   static V* HT(SolverWork* w) { return w->ht.p; }
   static V* HY(SolverWork* w) { return w->hy.p; }
   static V* HDD(SolverWork* w) { return w->hdd.p; }
-  static const V* HKM(afem_ctx* c) { return c->hyb->km.p; }
   static const V* HLKM(afem_ctx* c) { return c->hyb->lkm.p; }
   static const V* HUKM(afem_ctx* c) { return c->hyb->ukm.p; }
   static const V* LKM(afem_ctx* c, SolverWork*) { return c->mc_lkm.p; }
@@ -3134,7 +3133,6 @@ struct Inner<float, NS> {
   static V* HT(SolverWork* w) { return w->htf.p; }
   static V* HY(SolverWork* w) { return w->hyf.p; }
   static V* HDD(SolverWork* w) { return w->hddf.p; }
-  static const V* HKM(afem_ctx* c) { return c->hyb->kmf.p; }
   static const V* HLKM(afem_ctx* c) { return c->hyb->lkmf.p; }
   static const V* HUKM(afem_ctx* c) { return c->hyb->ukmf.p; }
   static const V* LKM(afem_ctx*, SolverWork* w) { return w->mc_lkmf.p; }
@@ -3716,10 +3714,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
       w->ht.alloc(nt); w->hy.alloc(nt); w->hdd.alloc(nt);
     } else {
       w->htf.alloc(nt); w->hyf.alloc(nt); w->hddf.alloc(nt);
-      if (!smoothed(c, w, precond) && (!h->kmf_valid || h->kmf.n != (size_t)h->nnz)) {
-        h->kmf.alloc(h->nnz);
-        k_convert<float2, double2><<<c->num_sms * 8, 256, 0, s>>>(h->km.p, h->kmf.p, h->nnz);
-        count_launch();
+      if (!smoothed(c, w, precond) && !h->splitf_valid) {
         h->lkmf.alloc(h->lkm.n);
         h->ukmf.alloc(h->ukm.n);
         if (h->lkm.n) {
@@ -3730,7 +3725,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
           k_convert<float2, double2><<<c->num_sms * 8, 256, 0, s>>>(h->ukm.p, h->ukmf.p, (long)h->ukm.n);
           count_launch();
         }
-        h->kmf_valid = true;
+        h->splitf_valid = true;
       }
     }
     if (smoothed(c, w, precond)) {
