@@ -271,3 +271,26 @@ def test_other_diagonal_scales_leave_the_coarse_matrices_out(fw):
     assert count[2] - count[3] == 6, count
     fw.assemble()  # and back to the smoothed iteration
     assert fw.solve(m.freqs[0], precond="HYBRID", tol=1e-9, maxit=2000).ok
+
+
+@pytest.mark.parametrize("ns,precision", [(1, "fp64"), (16, "fp64"), (16, "pc32")])
+@pytest.mark.parametrize("dims", [(16, 14, 14), (16, 16, 14)])
+def test_either_side_of_the_cycles_and_the_launchs_limit(fw, oracle, dims, ns, precision):
+    """Level-1 grids of 9 x 8 x 8 = 576 and 9 x 9 x 8 = 648 nodes (one block takes up to 600), and with 16 systems
+    430,704 and 490,428 rows x (systems + 2) (one launch takes up to 480,000).  Profiled solves take the launches
+    everywhere: the same solution to the tolerance, site fields within 1e-6."""
+    m = synth.tidal_box(*dims, seed=8, grf=True, block=False)
+    A = oracle.OracleForward(m).assemble(m.freqs[0])
+    fw.load_model(m)
+    fw.assemble()
+    out, its = [], []
+    for profiled in (False, True):
+        fw.set_profiling(profiled)
+        r = fw.solve(np.full(ns, m.freqs[0]), precond="HYBRID", precision=precision, tol=1e-9, maxit=2000)
+        fw.set_profiling(False)
+        assert r.ok and r.resid_true <= 1e-9, r
+        assert oracle.true_residual(A, fw.solution(ns - 1)) <= 1.01e-9
+        out.append(fw.sites(m.sites))
+        its.append(r.iterations)
+    assert abs(its[0] - its[1]) <= 3, its
+    assert np.abs(out[0] - out[1]).max() <= 1e-6 * np.abs(out[0]).max()
