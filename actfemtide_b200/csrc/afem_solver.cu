@@ -1361,13 +1361,12 @@ __device__ __forceinline__ void sum_partials(const double* part, int nblocks, in
   const int lane = threadIdx.x & 31;
   for (int v = 0; v < nvals; ++v) {
     double acc = 0.0;
-    for (int b = lane; b < nblocks; b += 32) acc += __ldcg(part + ((long)b * MAX_SYS + s) * 4 + k + v);
+    for (int b = lane; b < nblocks; b += 32) acc += part[((long)b * MAX_SYS + s) * 4 + k + v];
     for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
     sh[threadIdx.x >> 5][v] = acc;
   }
   __syncwarp();
   for (int v = 0; v < nvals; ++v) out[v] = sh[threadIdx.x >> 5][v];
-  __syncwarp();
 }
 
 __device__ __forceinline__ double2 d_cdiv(double2 a, double2 b) { return cdiv(a, b); }
