@@ -113,7 +113,7 @@ struct SolverWork {
   int nmc_blocks = 0;               // co-resident grid of the nodal multicolour sweeps
   int rpw_smooth = 0;               // SpMV rows per warp of the smoothed iteration (smooth_rpw)
   int rpw64 = 0, rpw32 = 0;         // SpMV rows per warp chosen by tune_spmv (0 = not tuned; 8: 4 systems per lane)
-  int spmv_grid[2][5] = {};         // one-wave grid of each SpMV variant (FP64 / FP32), 0 = not known yet
+  int spmv_grid[4][5] = {};         // one-wave grid of each SpMV variant (FP64 / FP32, then FUSE), 0 = not known yet
   int mc_blocks = 0;                // co-resident grid of the forward multicolour sweep
   int mcb_blocks = 0;               // and of the backward one (fewer registers: more blocks)
   double sd = 1.0;                  // SSOR diagonal scale of the current solve (DD = 1 / (sd D))
@@ -1635,14 +1635,20 @@ __global__ void __launch_bounds__(256, 4) k_pupd_spl(int n, const typename Cx<PT
 // RPW rows per warp, SPL systems per lane: lane = sub * (32/RPW) + g * (NS/SPL) +
 // s0/SPL, so rows of ~16 nonzeros do not leave half a warp idle (RPW and SPL are
 // picked by tune_spmv; SPL = 4 at 16 systems gives 8 rows per warp).
-template <class T, int NS, int RPW = 1, bool SEG = false, int SPL = 1>
-__global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
+// FUSE (the smoothed iteration): `chunk` rounds per chunk, and the last block forms alpha from R's sums.
+// Bound by gathers, so by the warps in flight: a variant of its own, since both decided at run time took
+// registers from the other iterations (8 FP64 systems at 4 rows per warp 48 -> 60 registers, 5 -> 4 blocks
+// per SM, 104 -> 143 us for 350,000 rows; 104 again now), and five blocks per SM asked for, as those have:
+// 8 systems 789 -> 427 us, 4 systems 479 -> 407, 1 system 181 -> 185 for 1.8 M rows.
+template <class T, int NS, int RPW = 1, bool SEG = false, int SPL = 1, bool FUSE = false>
+__global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : (FUSE && sizeof(T) == 8 ? 5 : 0)))
     k_spmv(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
            const typename Cx<T>::V* __restrict__ km, int n, const typename Cx<T>::V* __restrict__ p,
            typename Cx<T>::V* __restrict__ q, const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl,
            double* __restrict__ part, const typename Cx<T>::V* __restrict__ bvec, const uint8_t* __restrict__ seg,
-           RedSet R = RedSet{}, int nsys = 0, int ch = AFEM_SPMV_CHUNK) {
+           RedSet R = RedSet{}, int nsys = 0, int chunk = AFEM_SPMV_CHUNK) {
   using V = typename Cx<T>::V;
+  const int ch = FUSE ? chunk : AFEM_SPMV_CHUNK;
   constexpr int NG = NS / SPL;   // lanes of a row that hold different systems
   static_assert(NG * RPW <= 32, "rows per warp times lanes per row must fit a warp");
   static_assert(!SEG || (NS == 1 && SPL == 1), "packed batches hold one system per row");
@@ -1651,9 +1657,9 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
   constexpr int G = LPR / NG;    // entry groups per row
   const int lane = threadIdx.x & 31, sub = lane / LPR, ql = lane % LPR;
   const int s0 = (ql % NG) * SPL, g = ql / NG;
-  // SPL > 1 never runs in resid_mode (the true residual uses one system per lane):
+  // SPL > 1 and FUSE never run in resid_mode (the true residual uses one system per lane):
   // two sums per system (p^T q) keep the 64-register variant free of spills
-  constexpr int NACC = SPL > 1 ? 2 : 3;
+  constexpr int NACC = SPL > 1 || FUSE ? 2 : 3;
   double om1 = sc[s0].omega;  // SPL = 1: this lane's system (SEG: set per row)
   double acc[SPL][NACC];
 #pragma unroll
@@ -1693,7 +1699,7 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
         const T o = (T)(SPL == 1 ? om1 : __ldg(&sc[s0 + i].omega));
         qi[i] = Cx<T>::make(t1x[i] - o * t2y[i], t1y[i] + o * t2x[i]);
       }
-      if (SPL == 1 && bvec) {  // r = b - A x
+      if (SPL == 1 && !FUSE && bvec) {  // r = b - A x
         load_spl<V, NS, SPL, false>(bvec + base, own);
 #pragma unroll
         for (int i = 0; i < SPL; ++i) {
@@ -1717,27 +1723,20 @@ __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : 0))
       store_spl<V, SPL>(q + base, qi);
     }
   });
-  if (!R.part) {
+  if constexpr (!FUSE) {
     if constexpr (SEG) seg_partials<8 * RPW, 3>(red, part);
     else block_partials_spl<NS, SPL, LPR, NACC>(acc, s0, g == 0, part);
-    return;
-  }
-  // smoothed iteration: alpha is formed here
-  __shared__ double2 sums[MAX_SYS];
-  if constexpr (SEG) {
-    seg_pair<8 * RPW, 3>(red, R, blockIdx.x);
   } else {
-    double pq[SPL][2];
-#pragma unroll
-    for (int i = 0; i < SPL; ++i) {
-      pq[i][0] = acc[i][0];
-      pq[i][1] = acc[i][1];
+    __shared__ double2 sums[MAX_SYS];
+    if constexpr (SEG) {
+      seg_pair<8 * RPW, 3>(red, R, blockIdx.x);
+    } else {
+      __shared__ double2 buf[8 * NS];
+      block_pair<NS, SPL, LPR>(acc, s0, g == 0, R, blockIdx.x, buf);
     }
-    __shared__ double2 buf[8 * NS];
-    block_pair<NS, SPL, LPR>(pq, s0, g == 0, R, blockIdx.x, buf);
+    if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
+      finish_pq(const_cast<SysScal*>(sc), const_cast<Ctrl*>(ctrl), sums, nsys);
   }
-  if (reduce_blocks(R, blockIdx.x, gridDim.x, nsys, sums))
-    finish_pq(const_cast<SysScal*>(sc), const_cast<Ctrl*>(ctrl), sums, nsys);
 }
 
 // ------------------------------------------------------------------ smoothed iteration
@@ -3192,7 +3191,8 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
   const int32_t* cl = c->col.p;
   const uint8_t* sg = SEG ? c->seg_of_row.p : nullptr;
   const int vi = rpw == 16 ? 4 : rpw == 8 ? 3 : rpw == 4 ? 2 : rpw == 2 ? 1 : 0;
-  int& grid = w->spmv_grid[sizeof(T) == 8 ? 0 : 1][vi];
+  const bool fuse = R.part != nullptr;
+  int& grid = w->spmv_grid[(sizeof(T) == 8 ? 0 : 1) + (fuse ? 2 : 0)][vi];
   const bool fit = ch == 0;  // chunk and grid by the number of rows
   auto shape = [&](int rows_per_warp) {
     if (!fit) return grid;
@@ -3215,7 +3215,8 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
       return grid;
     }
   }
-  auto run = [&](auto k, int rows_per_warp) {
+  auto run = [&](auto plain, auto fused, int rows_per_warp) {
+    auto k = fuse ? fused : plain;
     if (!grid) grid = one_wave_grid(c, k, w->nblocks);
     const int g = shape(rows_per_warp);
     k<<<g, 256, 0, s>>>(rp, cl, km, n, p, q, w->sc.p, ctrl, w->part.p, bvec, sg, R, w->nsys, ch);
@@ -3223,10 +3224,13 @@ int launch_spmv(afem_ctx* c, SolverWork* w, int rpw, const typename Cx<T>::V* km
     return g;
   };
   if constexpr (NS == 16 && !SEG)  // AFEM_MC_SPL systems per lane, 2 * AFEM_MC_SPL rows per warp (q = A p only)
-    if (rpw == 8 && !bvec) return run(k_spmv<T, NS, 2 * AFEM_MC_SPL, SEG, AFEM_MC_SPL>, 2 * AFEM_MC_SPL);
-  if (rpw == 4 && NS * 4 <= 32) return run(k_spmv<T, NS, (NS * 4 <= 32 ? 4 : 1), SEG>, 4);
-  if (rpw == 2 && NS * 2 <= 32) return run(k_spmv<T, NS, (NS * 2 <= 32 ? 2 : 1), SEG>, 2);
-  return run(k_spmv<T, NS, 1, SEG>, 1);
+    if (rpw == 8 && !bvec)
+      return run(k_spmv<T, NS, 2 * AFEM_MC_SPL, SEG, AFEM_MC_SPL>, k_spmv<T, NS, 2 * AFEM_MC_SPL, SEG, AFEM_MC_SPL, true>,
+                 2 * AFEM_MC_SPL);
+  constexpr int R4 = NS * 4 <= 32 ? 4 : 1, R2 = NS * 2 <= 32 ? 2 : 1;
+  if (rpw == 4 && R4 == 4) return run(k_spmv<T, NS, R4, SEG>, k_spmv<T, NS, R4, SEG, 1, true>, 4);
+  if (rpw == 2 && R2 == 2) return run(k_spmv<T, NS, R2, SEG>, k_spmv<T, NS, R2, SEG, 1, true>, 2);
+  return run(k_spmv<T, NS, 1, SEG>, k_spmv<T, NS, 1, SEG, 1, true>, 1);
 }
 
 // Rows-per-warp autotuner: times each variant on this matrix (q = A p with the
