@@ -1439,15 +1439,16 @@ __device__ __forceinline__ void finish_pq(SysScal* sc, Ctrl* ctrl, const double2
 }
 
 // ------------------------------------------------------------------ p update, SpMV
-// The nodal correction of edge e for system s of NS: u_head - u_tail, or with edge vectors te (coarse
-// correction on, u then [node][4][system]) also te . (v_head + v_tail) / 2 of the vector part v.
-template <class T, class PT, int NS>
+// The nodal correction of edge e for system s of NS: u_head - u_tail, or with VEC (coarse correction on,
+// edge vectors te, u then [node][4][system]) also te . (v_head + v_tail) / 2 of the vector part v.
+// VEC makes variants of the kernels: decided at run time it cost the sweeps' p update 4 to 18 registers.
+template <class T, class PT, int NS, bool VEC>
 __device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restrict__ line,
                                                         const typename Cx<PT>::V* __restrict__ u,
                                                         const double* __restrict__ te, long e, int s) {
   using PV = typename Cx<PT>::V;
   const long ih = __ldg(line + 2 * e + 1) - 1, it = __ldg(line + 2 * e) - 1;
-  if (!te) {
+  if constexpr (!VEC) {
     const PV uh = u[ih * NS + s], ut = u[it * NS + s];
     return Cx<T>::make((T)(uh.x - ut.x), (T)(uh.y - ut.y));
   }
@@ -1469,7 +1470,7 @@ __device__ __forceinline__ typename Cx<T>::V nodal_term(const int32_t* __restric
 // solve).  Hybrid preconditioner with the nodal part folded in (u != nullptr):
 // z_e + the nodal correction (nodal_term) on the non-Dirichlet edges stands for z.
 // (p in the COCG type T; z and u in the preconditioner type PT)
-template <class T, class PT, int NS, bool SEG>
+template <class T, class PT, int NS, bool SEG, bool VEC>
 __device__ __forceinline__ void pupd(int n, const typename Cx<PT>::V* z, typename Cx<T>::V* p, const SysScal* sc,
                                      bool done, bool first, const uint8_t* seg, double2* x,
                                      const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
@@ -1493,10 +1494,10 @@ __device__ __forceinline__ void pupd(int n, const typename Cx<PT>::V* z, typenam
     if (done) continue;
     const PV zp = z[i];
     V zi = Cx<T>::make((T)zp.x, (T)zp.y);
-    if (u) {
+    if (VEC || u) {
       const int e = (int)(i / NS);
       if (!__ldg(bc + e)) {
-        const V d = nodal_term<T, PT, NS>(line, u, te, e, SEG ? 0 : s);
+        const V d = nodal_term<T, PT, NS, VEC>(line, u, te, e, SEG ? 0 : s);
         zi = Cx<T>::make(zi.x + d.x, zi.y + d.y);
       }
     }
@@ -1511,7 +1512,7 @@ __device__ __forceinline__ void pupd(int n, const typename Cx<PT>::V* z, typenam
   }
 }
 
-template <class T, class PT, int NS, bool SEG = false>
+template <class T, class PT, int NS, bool SEG, bool VEC>
 __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
                        const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, const uint8_t* __restrict__ seg,
                        double2* __restrict__ x, int nsys, const int32_t* __restrict__ line,
@@ -1524,7 +1525,7 @@ __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename
     for (int k = 0; k < nsys; ++k) any |= sc[k].xpend != 0;
     if (!any) return;
   }
-  pupd<T, PT, NS, SEG>(n, z, p, sc, done, ctrl->iter == 0, seg, x, line, bc, u, te, blockIdx.x, gridDim.x);
+  pupd<T, PT, NS, SEG, VEC>(n, z, p, sc, done, ctrl->iter == 0, seg, x, line, bc, u, te, blockIdx.x, gridDim.x);
 }
 
 // k_pupd for 16 systems sharing a matrix: a thread takes 2 consecutive systems of
@@ -1534,7 +1535,7 @@ __global__ void k_pupd(int n, const typename Cx<PT>::V* __restrict__ z, typename
 // a multiple of 8, so a thread keeps the same 2 systems throughout.  Four blocks per SM (64 registers): a
 // grid of eight per SM is then two full waves (0.33 -> 0.27 ms for 16 systems of 830,000 rows, where 72
 // registers left three and a last wave two thirds full).
-template <class T, class PT, int NS>
+template <class T, class PT, int NS, bool VEC>
 __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typename Cx<T>::V* p, const SysScal* sc,
                                          bool done, bool first, double2* x, const int32_t* __restrict__ line,
                                          const uint8_t* __restrict__ bc, const typename Cx<PT>::V* u,
@@ -1579,8 +1580,8 @@ __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typ
     V zi[SP];
 #pragma unroll
     for (int j = 0; j < SP; ++j) zi[j] = Cx<T>::make((T)zp[j].x, (T)zp[j].y);
-    if (u && !__ldg(bc + e)) {
-      const int nc = te ? 4 : 1;  // components of a nodal row (see nodal_term)
+    if ((VEC || u) && !__ldg(bc + e)) {
+      constexpr int nc = VEC ? 4 : 1;  // components of a nodal row (see nodal_term)
       const PV* ph = u + (long)(__ldg(line + 2 * e + 1) - 1) * nc * NS + s0;
       const PV* pt = u + (long)(__ldg(line + 2 * e) - 1) * nc * NS + s0;
       PV uh[SP], ut[SP];
@@ -1589,7 +1590,7 @@ __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typ
 #pragma unroll
       for (int j = 0; j < SP; ++j)
         zi[j] = Cx<T>::make(zi[j].x + (T)(uh[j].x - ut[j].x), zi[j].y + (T)(uh[j].y - ut[j].y));
-      if (te) {
+      if constexpr (VEC) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           const T h = (T)(0.5 * __ldg(te + 3L * e + d));
@@ -1615,7 +1616,7 @@ __device__ __forceinline__ void pupd_spl(int n, const typename Cx<PT>::V* z, typ
   }
 }
 
-template <class T, class PT, int NS>
+template <class T, class PT, int NS, bool VEC>
 __global__ void __launch_bounds__(256, 4) k_pupd_spl(int n, const typename Cx<PT>::V* __restrict__ z, typename Cx<T>::V* __restrict__ p,
                            const SysScal* __restrict__ sc, const Ctrl* __restrict__ ctrl, double2* __restrict__ x,
                            int nsys, const int32_t* __restrict__ line, const uint8_t* __restrict__ bc,
@@ -1627,7 +1628,7 @@ __global__ void __launch_bounds__(256, 4) k_pupd_spl(int n, const typename Cx<PT
     for (int k = 0; k < nsys; ++k) any |= sc[k].xpend != 0;
     if (!any) return;
   }
-  pupd_spl<T, PT, NS>(n, z, p, sc, done, ctrl->iter == 0, x, line, bc, u, te, blockIdx.x, gridDim.x);
+  pupd_spl<T, PT, NS, VEC>(n, z, p, sc, done, ctrl->iter == 0, x, line, bc, u, te, blockIdx.x, gridDim.x);
 }
 
 // q = A p (COCG13_single.f90:273-288) and p^T q partial sums.  With
@@ -2621,9 +2622,9 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_small(const __grid_constant__
     }
     // also when this iteration's residual ended the solve: x += alpha p may be pending
     if constexpr (NS >= 2)
-      pupd_spl<T, PT, NS>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, a.x, a.line, a.bc, a.w, a.te, bid, nb);
+      pupd_spl<T, PT, NS, true>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, a.x, a.line, a.bc, a.w, a.te, bid, nb);
     else
-      pupd<T, PT, NS, false>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, nullptr, a.x, a.line, a.bc, a.w, a.te, bid,
+      pupd<T, PT, NS, false, true>(a.n, a.z, a.p, sc, ctrl.done, ctrl.iter == 0, nullptr, a.x, a.line, a.bc, a.w, a.te, bid,
                              nb);
     if (ctrl.done) break;
     grid.sync();
@@ -3418,12 +3419,12 @@ void enqueue_iteration(afem_ctx* c, SolverWork* w, int mode, int sweep_blocks, c
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
   if constexpr (NS == 16 && !SEG)
-    k_pupd_spl<T, PT, NS><<<c->num_sms * 8, 256, 0, s>>>(
+    k_pupd_spl<T, PT, NS, false><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr,
         fold_grad ? c->bc.p : (const uint8_t*)nullptr, fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr, (const double*)nullptr);
   else
-    k_pupd<T, PT, NS, SEG><<<c->num_sms * 8, 256, 0, s>>>(
+    k_pupd<T, PT, NS, SEG, false><<<c->num_sms * 8, 256, 0, s>>>(
         n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg, mc ? w->x.p : (double2*)nullptr, nsys,
         fold_grad ? (const int32_t*)c->line.p : (const int32_t*)nullptr, fold_grad ? c->bc.p : (const uint8_t*)nullptr,
         fold_grad ? (const PV*)P::HY(w) : (const PV*)nullptr, (const double*)nullptr);
@@ -3507,11 +3508,11 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, bool re
   count_launch();
   if (ev) AFEM_CUDA(cudaEventRecord(ev[4], s));
   if constexpr (NS >= 2)
-    k_pupd_spl<T, PT, NS><<<grid((long)n * NS / 2), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p,
+    k_pupd_spl<T, PT, NS, true><<<grid((long)n * NS / 2), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p,
                                                              w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw,
                                                              co->te.p);
   else
-    k_pupd<T, PT, NS, SEG><<<grid((long)n * NS), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg,
+    k_pupd<T, PT, NS, SEG, true><<<grid((long)n * NS), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg,
                                                           w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw, co->te.p);
   count_launch();
   if constexpr (sizeof(T) == 8)
