@@ -538,7 +538,6 @@ void coarse_pattern(afem_ctx* c) {
     CoarseGrid* G = co->grids.data() + (size_t)sg * COARSE_LEVELS;
     int l = 0;
     for (; l + 1 < COARSE_LEVELS && G[l].n > COARSE_STOP && std::max(G[l].nx, std::max(G[l].ny, G[l].nz)) > 3; ++l) {
-      int* np[3] = {&G[l].nx, &G[l].ny, &G[l].nz};
       int* nc[3] = {&G[l + 1].nx, &G[l + 1].ny, &G[l + 1].nz};
       int* wo[3] = {&G[l].wx, &G[l].wy, &G[l].wz};
       for (int d = 0; d < 3; ++d) {
@@ -558,7 +557,6 @@ void coarse_pattern(afem_ctx* c) {
           axw.push_back((p[i] - q[ci]) / (q[ci + 1] - q[ci]));
         }
         *nc[d] = (int)q.size();
-        (void)np;
         p = q;
       }
       G[l + 1].n = G[l + 1].nx * G[l + 1].ny * G[l + 1].nz;

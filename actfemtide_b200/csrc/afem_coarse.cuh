@@ -267,15 +267,6 @@ __device__ __forceinline__ unsigned grid_mask(const CoarseGrid& g, int l) {
   return m;
 }
 
-// The V-cycle from level `top` down, one block of TAIL_THREADS per (component, system) -- in a packed
-// batch per (component, mesh) -- with `vals` values of shared memory at sh, the levels' R, Z and D^-1 and one scratch vector in shared memory.
-// Starts from R of the top level, or (top = 0) from the mesh nodes' t, and writes the top level's O;
-// rho (top = 0): the component's share of rho of its system.
-// A step is one load latency long, so what bounds it is how many dependent loads it makes: the
-// matrices of the lower levels that fit are copied to shared memory while the restriction runs, the
-// inverse diagonals are formed once, the axis weights sit in shared memory, and the larger levels' rows
-// come seven entries at a time on two lanes a node.  49.6 -> 21 us a cycle on 12x12x9 cells (one 245-node grid,
-// whose four sweeps replaced two more levels).
 template <class T>
 __device__ __forceinline__ void copy_async(typename CV<T>::V* dst, const typename CV<T>::V* src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -283,6 +274,16 @@ __device__ __forceinline__ void copy_async(typename CV<T>::V* dst, const typenam
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
 }
 
+// The V-cycle from level `top` down, one block of TAIL_THREADS per (component, system) -- in a packed
+// batch per (component, mesh) -- with `vals` values of shared memory at sh: the levels' R, Z and D^-1 and
+// one scratch vector, then the matrices that fit.
+// Starts from R of the top level, or (top = 0) from the mesh nodes' t, and writes the top level's O;
+// rho (top = 0): the component's share of rho of its system.
+// A step is one load latency long, so what bounds it is how many dependent loads it makes: the
+// matrices of the lower levels that fit are copied to shared memory while the restriction runs, the
+// inverse diagonals are formed once, the axis weights sit in shared memory, and the larger levels' rows
+// come seven entries at a time on two lanes a node.  49.6 -> 21 us a cycle on 12x12x9 cells (one 245-node grid,
+// whose four sweeps replaced two more levels).
 template <class T, int NS, bool SEG>
 __device__ __forceinline__ void grid_tail(int comp, int by, typename CV<T>::V* sh, const CoarseGrid* grids,
                                           const int32_t* levels, int top, int vals, const typename CV<T>::V* km,

@@ -497,9 +497,10 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------ natural-order sweeps of small systems
-// The triangular sweep of k_fwd / k_bwd alone, for a system whose vector fits the shared memory of one
-// block: the rows of a dependency level are swept side by side (a warp per row, the lanes and sums of
-// k_fwd) and a block barrier parts the levels.  The sync-free sweeps pass every level through L2 flags
+// The triangular sweep of k_fwd / k_bwd alone, for systems whose vectors together fit the shared memory
+// of one block (SWEEP_BYTES: 10,240 rows x systems in FP64, 20,480 in FP32): the rows of a dependency
+// level are swept side by side (a warp per row, the lanes and sums of k_fwd) and a block barrier parts the
+// levels.  The sync-free sweeps pass every level through L2 flags
 // and polls, 6 us a level on 878 rows (380 us a sweep of 61 levels); here a level costs a barrier, the
 // arithmetic's latency and part of a load's, 1 us (60 us a sweep): a warp's rows come through a
 // pipeline, the range of the row after next and the entries of the next row on their way while a row is
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(256)
 // bits by either path.
 constexpr int SWEEP_THREADS = 1024;
 constexpr int SWEEP_LEVELS = 12000;
-constexpr int SWEEP_BYTES = SWEEP_ROWS * 8;  // 160 KB: the vector (the levels' offsets come on top)
+constexpr int SWEEP_BYTES = SWEEP_ROWS * 8;  // 160 KB: the vectors (the levels' offsets come on top)
 
 template <class T, int NS, bool BWD>
 __global__ void __launch_bounds__(SWEEP_THREADS)
@@ -1638,9 +1639,9 @@ __global__ void __launch_bounds__(256, 4) k_pupd_spl(int n, const typename Cx<PT
 // picked by tune_spmv; SPL = 4 at 16 systems gives 8 rows per warp).
 // FUSE (the smoothed iteration): `chunk` rounds per chunk, and the last block forms alpha from R's sums.
 // Bound by gathers, so by the warps in flight: a variant of its own, since both decided at run time took
-// registers from the other iterations (8 FP64 systems at 4 rows per warp 48 -> 60 registers, 5 -> 4 blocks
-// per SM, 104 -> 143 us for 350,000 rows; 104 again now), and five blocks per SM asked for, as those have:
-// 8 systems 789 -> 427 us, 4 systems 479 -> 407, 1 system 181 -> 185 for 1.8 M rows.
+// registers or spilled in the other iterations (350,000 rows in FP64, 4 systems 95 -> 108 us a product, 16 at
+// a row per warp 190 -> 217; 95 and 188 now), and five blocks per SM asked for, as those have (1.8 M rows:
+// 4 systems 478 -> 407 us, 8 systems 491 -> 426, 1 system 181 -> 184).
 template <class T, int NS, int RPW = 1, bool SEG = false, int SPL = 1, bool FUSE = false>
 __global__ void __launch_bounds__(256, (SPL > 1 ? MC_MIN_BLOCKS : (FUSE && sizeof(T) == 8 ? 5 : 0)))
     k_spmv(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
@@ -2435,7 +2436,9 @@ __global__ void __launch_bounds__(256)
   if (lam) most.put(lam);
 }
 
-// The same for D_G^-1 A_G at each mesh's first frequency (A_G is i omega M_G but for rounding).
+// The same for D_G^-1 A_G at each mesh's first frequency: A_G is i omega M_G but for rounding away from the
+// Dirichlet edges and has its K where some are dropped, so that the bound depends little on the frequency
+// (2.03 to 2.16 over 1e-5 to 100 Hz on 6x6x5 and 9x8x7 cells, the largest eigenvalue 1.96 to 1.98).
 __global__ void __launch_bounds__(256)
     k_node_power(int node, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                  const double2* __restrict__ km, const int32_t* __restrict__ diagpos, const uint8_t* __restrict__ live,
@@ -2498,7 +2501,7 @@ struct SmallArgs {
   using V = typename Cx<T>::V;
   using PV = typename Cx<PT>::V;
   // static data
-  int n, node, nsys, steps, vals, top;
+  int n, node, steps, vals, top;
   const int32_t *rowptr, *col, *line, *nptr, *nlist, *hrow, *hcol, *cell, *lptr, *lidx, *levels;
   const uint8_t* bc;
   const V* km;     // the COCG's matrix
@@ -3016,7 +3019,7 @@ __global__ void k_copy_r<float2>(const double2* __restrict__ in, float2* __restr
     out[i] = make_float2((float)in[i].x, (float)in[i].y);
 }
 
-// Start of an inner solve: x_inner = 0, ||b||^2 from the partials of the residual SpMV.
+// Start of an inner solve: x_inner = 0, ||b||^2 from the partials of the residual SpMV or of k_start.
 __global__ void k_init_sys(SysScal* sc, Ctrl* ctrl, const double* part, int nblocks, int ns, double tol, int maxit,
                            const double* omega, unsigned spin_limit, double renew_tol, int renew_mask) {
   const int s = threadIdx.x >> 5;
@@ -3032,7 +3035,8 @@ __global__ void k_init_sys(SysScal* sc, Ctrl* ctrl, const double* part, int nblo
       S.rho = S.rho1 = S.alpha = S.beta = S.pq = make_double2(0.0, 0.0);
       S.iter = 0;
       S.xpend = S.renew = 0;
-      // a NaN / Inf in the matrix or the right-hand side shows in ||b - A 0||^2
+      // a NaN / Inf in the right-hand side shows in ||b||^2, one in the matrix in ||b - A 0||^2 too (k_spmv),
+      // after k_start in the first iteration's sums
       const bool finite = isfinite(v[0]);
       S.active = finite && v[0] > 0.0;
       S.status = finite ? AFEM_OK : AFEM_ENONFINITE;
@@ -3283,7 +3287,7 @@ int tune_spmv(afem_ctx* c, SolverWork* w) {
   return pick;
 }
 
-// Whether the natural-order sweeps run in one block (k_sweep_block): the vector fits its shared memory.
+// Whether the natural-order sweeps run in one block (k_sweep_block): the vectors fit its shared memory.
 template <class T, int NS, bool SEG>
 bool block_sweeps(const afem_ctx* c, const SolverWork* w, int mode) {
   return !SEG && mode <= AFEM_PRECOND_SSOR && (long)w->n * NS * (long)sizeof(typename Cx<T>::V) <= SWEEP_BYTES &&
@@ -3546,7 +3550,7 @@ void launch_small(afem_ctx* c, SolverWork* w, int steps, const double* d_omega) 
   CoarseState* co = h->co;
   const size_t vec = (size_t)4 * NS * co->ntot, smem = std::min(SMALL_BYTES, sizeof(PV) * co->tail_vals);
   SmallArgs<T, PT> a{};
-  a.n = w->n; a.node = h->node; a.nsys = NS; a.steps = steps; a.vals = (int)(smem / sizeof(PV)); a.top = co->tail;
+  a.n = w->n; a.node = h->node; a.steps = steps; a.vals = (int)(smem / sizeof(PV)); a.top = co->tail;
   a.rowptr = c->rowptr.p; a.col = c->col.p; a.line = c->line.p; a.nptr = h->nptr.p; a.nlist = h->nlist.p;
   a.hrow = h->rowptr.p; a.hcol = h->col.p; a.cell = co->cell.p; a.lptr = co->lptr.p; a.lidx = co->lidx.p;
   a.levels = co->d_levels.p; a.bc = c->bc.p;

@@ -59,8 +59,8 @@ typedef enum afem_precond {
   AFEM_PRECOND_HYBRID = 6    /* polynomial smoothing of the edges and of the gradient space G (Hiptmair's
                                 hybrid smoother, additive) plus a coarse-grid correction in the nodal scalar
                                 and vector spaces; multicolour SSOR sweeps in place of the polynomials
-                                where sigma_diag is not 1 or the mesh is too small for a coarse grid, and in
-                                the learned base; needs the mesh */
+                                where sigma_diag is not 1, the mesh is too small for a coarse grid or thousands
+                                of its nodes crowd into one cell of it, and in the learned base; needs the mesh */
 } afem_precond;
 
 typedef enum afem_precision {
