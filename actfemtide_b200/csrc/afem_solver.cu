@@ -3967,6 +3967,7 @@ SolverWork* ensure_work(afem_ctx* c, int nsys, bool mixed, bool pc32 = false, bo
     w->rf.release(); w->zf.release(); w->pf.release(); w->qf.release(); w->ddf.release();
     w->flag_f.alloc(n); w->flag_b.alloc(n);
     w->rpw64 = w->rpw32 = 0;
+    for (auto& g : w->spmv_grid) std::fill(std::begin(g), std::end(g), 0);  // (other kernels than before)
     w->flag_f.zero(s); w->flag_b.zero(s);
     w->sc.alloc(MAX_SYS);
     w->ctrl.alloc(1);

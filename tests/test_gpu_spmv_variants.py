@@ -57,3 +57,21 @@ def test_tiled_pin_on_a_small_batch_falls_back(gpulib, batch_model):
         fw.set_spmv_rows_per_warp(16)
         r = fw.solve(f[:4], srcs=src[:4], precond="HYBRID", precision="fp64", tol=1e-8)
         assert r.ok and r.resid_true <= 1e-8, r
+
+
+@pytest.mark.parametrize("precision,ns", [("mixed", 4), ("fp64", 8)])
+def test_a_solve_does_not_depend_on_earlier_batch_sizes(gpulib, precision, ns):
+    """The SpMV's grid is that of its own variant: a batch gives the same bits in a fresh context and after a solve of
+    one system, whose variant may fit another number of blocks; on enough rows for more than one wave of blocks."""
+    from actfemtide_b200.forward import Forward
+    m = synth.tidal_box(28, 26, 22, seed=3, block=False)
+    xs = []
+    for batches in ((ns,), (1, ns)):
+        with Forward(0) as f:
+            f.load_model(m)
+            f.set_spmv_rows_per_warp(4)
+            f.assemble()
+            for n in batches:
+                f.solve(np.full(n, m.freqs[0]), precond="DIAG", precision=precision, tol=1e-12, maxit=20)
+            xs.append(f.solution(ns - 1))
+    assert np.array_equal(xs[0], xs[1])
