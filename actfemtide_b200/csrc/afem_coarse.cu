@@ -1,8 +1,8 @@
-// Coarse correction of the gradient-corrected multicolour SSOR.
+// Coarse correction of the gradient-corrected COCG (AFEM_PRECOND_HYBRID).
 //
-// SSOR on the edges and on the gradients removes the error that varies from
-// edge to edge; what is left is smooth, and its reduction takes as many
-// iterations as the mesh is cells wide.  Following Hiptmair and Xu (SIAM J.
+// Smoothing on the edges and on the gradients (the polynomials of afem_solver.cu's smoothed iteration)
+// removes the error that varies from edge to edge; what is left is smooth, and its reduction would take
+// as many iterations as the mesh is cells wide.  Following Hiptmair and Xu (SIAM J.
 // Numer. Anal. 45, 2007) the smooth part of an edge field is represented by
 // nodal functions: the gradient of a scalar potential and a vector field whose
 // three components are taken one by one,
@@ -18,9 +18,9 @@
 // halved per axis; its smoother is l1-Jacobi, D = sum_j |K_ij| + i omega
 // sum_j |M_ij|, which needs no estimate of the largest eigenvalue on stretched
 // cells.  Everything is complex symmetric, so COCG applies as before.
-// Measured to 1e-10 on a B200: 461 -> 59 iterations and 370 -> 70 ms on a 48x48x32-cell mesh (8
-// systems, FP64), about 850 -> 65 and 1,290 -> 151 ms on 88x88x56 (one system), 110 -> 43 and
-// 30 -> 16 ms on 12x12x9, where an iteration is all launches and grid barriers.
+// Measured to 1e-10 on a B200 in FP64, the colour sweeps alone against sweeps and correction against the
+// smoothed iteration with it: 461, 59, 69 iterations and 361, 70, 49 ms on 48x48x32 cells (8 systems), about
+// 850, 65, 70 and 1,290, 151, 103 ms on 88x88x56 (one system), 110, 43, 50 and 30, 16, 3.3 ms on 12x12x9.
 //
 // The four components and the systems are independent below the restriction,
 // so the lower levels of the V-cycle run as one block per (component, system)

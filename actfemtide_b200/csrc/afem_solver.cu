@@ -3519,9 +3519,10 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, bool re
     k_pupd<T, PT, NS, SEG, true><<<grid((long)n * NS), 256, 0, s>>>(n, (const PV*)P::Z(w), I::P(w), w->sc.p, w->ctrl.p, sg,
                                                           w->x.p, nsys, c->line.p, c->bc.p, (const PV*)nw, co->te.p);
   count_launch();
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
   if constexpr (sizeof(T) == 8)
     if (renew) launch_exact_residual<NS, SEG, false>(c, w, w->r64.p, w->r.p);
-  if (ev) AFEM_CUDA(cudaEventRecord(ev[5], s));
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
   const int rpw = w->rpw_smooth;
   const bool tiles = rpw == 16;
   const int sgrid = launch_spmv<T, NS, SEG>(c, w, rpw, I::KM(c, w), (const V*)I::P(w), I::Q(w), w->ctrl.p,
@@ -3530,7 +3531,7 @@ void enqueue_smoothed(afem_ctx* c, SolverWork* w, const double* d_omega, bool re
     k_scal_pq<<<1, 32 * MAX_SYS, 0, s>>>(w->sc.p, w->ctrl.p, w->part.p, sgrid, nsys);
     count_launch();
   }
-  if (ev) AFEM_CUDA(cudaEventRecord(ev[6], s));
+  if (ev) AFEM_CUDA(cudaEventRecord(ev[7], s));
 }
 
 // Whether the smoothed iteration runs as one launch (k_small): systems whose steps do not fill the
@@ -3777,7 +3778,7 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
   AFEM_CUDA(cudaMemcpyAsync(&w->ctrl.p->epoch, &w->epoch_host, sizeof(unsigned), cudaMemcpyHostToDevice, s));
   int iters_done = 0;
   // profiling: 8 events per iteration of a chunk (fwd | scal | bwd | nodal correction | scal | pupd | spmv,
-  // or r update | smoother | coarse cycle | prolongation | pupd | spmv)
+  // or r update | smoother | coarse cycle | prolongation | pupd | exact residual | spmv)
   const bool prof = c->prof.on;
   std::vector<cudaEvent_t> evs;
   if (prof) {
@@ -3878,15 +3879,16 @@ int inner_cocg(afem_ctx* c, SolverWork* w, const afem_solve_opts* o, int precond
         cudaEvent_t* E = &evs[8L * k];
         if (smooth) {
           static const char* const step[6] = {"cocg_r_update", "cocg_smoother", "cocg_coarse_cycle", "cocg_prolongation",
-                                              "cocg_p_update", "cocg_spmv"};
-          for (int j = 0; j < 6; ++j) {
+                                              "cocg_p_update", "cocg_exact_residual"};
+          for (int j = 0; j < 7; ++j) {
             float ms = 0;
+            if (j == 5 && (sizeof(T) == 4 || (k & renew_mask) != renew_mask)) continue;  // (not launched)
             if (cudaEventElapsedTime(&ms, E[j], E[j + 1]) != cudaSuccess) {
               cudaGetLastError();
               break;
             }
-            if (j < 5) snprintf(nh, sizeof nh, "%s_%s_%s%d", step[j], tag, kind, cnt);
-            c->prof.add(j < 5 ? nh : ns_, ms);
+            if (j < 6) snprintf(nh, sizeof nh, "%s_%s_%s%d", step[j], tag, kind, cnt);
+            c->prof.add(j < 6 ? nh : ns_, ms);
           }
           continue;
         }
